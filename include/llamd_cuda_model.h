@@ -139,7 +139,8 @@ size_t llamd_model_weight_bytes(llamd_model *m); /* device.rs:473 */
  * projections of every layer; "early_loads"
  * (default 1): the down projection reads its expert ids, and attention its positions and the cached rows of earlier
  * positions, before the launch's dependency wait, so their bytes travel while the launch in front still runs.
- * Prefill: "prefill_tile" (tokens per tile, 1..4096, default 512), "prefill_gemm" (1: the exact integer tensor path,
+ * Prefill: "prefill_tile" (tokens per tile, 1..4096; until it is set one
+ * GPU cuts a prompt into equal tiles of up to 2048, several into tiles of 512), "prefill_gemm" (1: the exact integer tensor path,
  * default; 0: dp4a, 8 tokens per weight pass, exact; 2: tcgen05 on f16 pairs, tolerance level), "prefill_attn" (1: the
  * register-tiled attention kernels, default; 0: the per-token decode kernels), "prefill_prefold" (1: keep the expert
  * matrices a second time, folded for the integer GEMM, +2 bytes per weight; same bits).

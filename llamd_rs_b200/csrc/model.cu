@@ -227,6 +227,7 @@ struct Model {
     int prefill_gemm = 1;    // 1: integer tensor path (mma.sync), exact; 0: dp4a, 8 tokens per weight pass, exact;
                              // 2: tcgen05 on f16 pairs, tolerance level (gemm_tc.cu)
     int prefill_tile = 512;  // VulkanModel::prefill_tile default max_seq.min(512), vulkan_model.rs:343
+    bool prefill_tile_set = false;  // the caller chose the tile; else one GPU takes up to kAutoTile tokens
     int32_t *h_meta = nullptr;  // pinned
     int32_t *h_out = nullptr;   // pinned
     size_t weight_bytes = 0;
@@ -1192,6 +1193,7 @@ int llamd_model_set_option(llamd_model *h, const char *name, int value) {
     if (!strcmp(name, "prefill_tile")) {
         if (value < 1 || value > 4096) return -1;
         m->prefill_tile = value;
+        m->prefill_tile_set = true;
         return 0;
     }
     if (!strcmp(name, "batch_group")) {
@@ -1251,6 +1253,14 @@ int llamd_model_forward_batch(llamd_model *h, const int32_t *tokens, const int32
 // (moe_group), and attention needs no mask because every token of the tile has
 // stored its K and V before any query of the tile runs. Per token the
 // arithmetic is the decode pass's, so prefill == sequential decode exactly.
+// The tile of a caller that never chose one, on one GPU. A tile reads every expert's weights once whatever its size, and
+// folds them for the MMAs once, so the GEMMs of a layer took 743 us for 512 tokens and 2029 us for 2048 (48-layer model's
+// shapes, four to one in tokens). Beyond 2048 the folding is a tenth of the work and the buffers (gate, up, down: 230 MB
+// at 2048) grow on.
+constexpr int kAutoTile = 2048;
+// Attention of a tile runs this many tokens at a time: its score buffer is [tokens][heads][max_kv] floats, and 512 tokens
+// already are thousands of CTAs.
+constexpr int kAttnTokens = 512;
 constexpr int kGroupMaxPairs = 40960;  // what one scatter plan takes (ops.cu: moe_group_kernel)
 
 // The folded copies of the expert matrices (option "prefill_prefold"), made once all tensors are there.
@@ -1285,6 +1295,7 @@ static bool prefill_alloc(Model &m, int tile) {
     if (!ensure_prefold(m)) return false;
     Model::Prefill &p = m.pf;
     if (p.tile >= tile) return true;
+    if (tile > m.prefill_tile) tile = (tile + 511) & ~511;  // (a tile beyond the caller's: prompts that grow re-allocate four times at most)
     if (p.ep_cap) {
         m.err = "prefill: the tile buffers have been shared with the other ranks and cannot grow (set prefill_tile before the attach)";
         return false;
@@ -1305,7 +1316,7 @@ static bool prefill_alloc(Model &m, int tile) {
               p.v.alloc(T * kvd * 4) && p.attn.alloc(T * qd * 4) && p.aq.alloc(T * max_act) && p.ad.alloc(T * (max_act / 256) * 4) &&
               p.aq2.alloc(T * nu * ffe) && p.ad2.alloc(T * nu * (ffe / 256) * 4) && p.ids.alloc(T * nu * 4) && p.w.alloc(T * nu * 4) &&
               p.logits.alloc(T * ne * 4) && p.counter.alloc(T * 4) && p.gate.alloc(T * nu * ffe * 4) && p.up.alloc(T * nu * ffe * 4) &&
-              p.down.alloc(T * nu * E * 4) && p.scores.alloc(T * hp.n_head * (size_t)((m.max_kv + 3) & ~3) * 4) && p.meta.alloc(T * 8) &&
+              p.down.alloc(T * nu * E * 4) && p.scores.alloc((T < kAttnTokens ? T : kAttnTokens) * hp.n_head * (size_t)((m.max_kv + 3) & ~3) * 4) && p.meta.alloc(T * 8) &&
               p.gstart.alloc(ne * 4) && p.gcount.alloc(ne * 4) && p.ptoken.alloc(T * nu * 4 * (size_t)m.ep_world) &&
               p.pslot.alloc(T * nu * 4 * (size_t)m.ep_world) &&
               p.work.alloc((T * nu / 8 + ne + 1) * 12) && p.n_work.alloc(4) && p.aq_rm.alloc(T * max_act * 4) && p.aq2_rm.alloc(T * nu * ffe * 4) &&
@@ -1342,6 +1353,24 @@ static bool prefill_alloc_all_logits(Model &m, bool own_logits) {
                     cudaMallocHost((void **)&p.h_out_tokens, T * 4) == cudaSuccess;
     if (!ok) m.err = std::string("verification buffers: ") + llamd_cuda_last_error_string();
     return ok;
+}
+
+// The tile of a caller that never chose one: as few tiles as kAutoTile allows and the same number of tokens in each, rather
+// than full ones and a small rest that costs nearly as much per layer. A tile beyond prefill_tile has to fit the free memory
+// with room to spare.
+static int auto_tile(const Model &m, int n_tokens) {
+    const llamd_hparams &hp = m.hp;
+    int cap = kAutoTile < kGroupMaxPairs / hp.n_expert_used ? kAutoTile : kGroupMaxPairs / hp.n_expert_used;
+    if (cap < m.prefill_tile) return m.prefill_tile;
+    if (n_tokens > m.prefill_tile && n_tokens > m.pf.tile) {
+        const size_t E = hp.n_embd, qd = (size_t)hp.n_head * hp.head_dim, kvd = (size_t)hp.n_head_kv * hp.head_dim, nu = hp.n_expert_used,
+                     ffe = hp.n_ff_expert, act = E > qd ? E : qd;
+        const size_t per_token = 4 * (3 * E + 2 * qd + 2 * kvd + 2 * hp.n_expert + 4 * nu) + 6 * act + nu * (4 * E + 14 * ffe);
+        if ((size_t)cap * per_token + ((size_t)1 << 30) > llamd_cuda_free_mem()) cap = m.prefill_tile > m.pf.tile ? m.prefill_tile : m.pf.tile;
+        if (cap > kAutoTile) cap = kAutoTile;
+    }
+    const int n = (n_tokens + cap - 1) / cap;
+    return (n_tokens + n - 1) / n;
 }
 
 // The largest tile expert-parallel prefill can take: the scatter plan covers the pairs of ALL ranks' tiles.
@@ -1417,12 +1446,16 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
                                               HKV, hd, meta, m.rope_tab.as<float>(), hp.rms_eps, T);
         }
         if (!multi_seq) {  // (a batch of sequences attended above)
-            if (m.prefill_attn)
-                llamd_fwd_attention_prefill(p.q.as<float>(), kc_view, vc_view, p.attn.as<float>(), p.scores.as<float>(), H, HKV, hd, meta,
-                                            (m.max_kv + 3) & ~3, T, n_kv_max);  // score rows padded to 16 bytes
-            else
-                llamd_fwd_attention_tile(p.q.as<float>(), kc_view, vc_view, p.attn.as<float>(), p.scores.as<float>(), H, HKV, hd, meta,
-                                         m.max_kv, T);
+            for (int t0 = 0; t0 < T; t0 += kAttnTokens) {
+                const int n = T - t0 < kAttnTokens ? T - t0 : kAttnTokens;
+                const float *q = p.q.as<float>() + (size_t)t0 * qd;
+                float *out = p.attn.as<float>() + (size_t)t0 * qd;
+                if (m.prefill_attn)
+                    llamd_fwd_attention_prefill(q, kc_view, vc_view, out, p.scores.as<float>(), H, HKV, hd, meta + 2 * t0,
+                                                (m.max_kv + 3) & ~3, n, n_kv_max - T + t0 + n);  // score rows padded to 16 bytes
+                else
+                    llamd_fwd_attention_tile(q, kc_view, vc_view, out, p.scores.as<float>(), H, HKV, hd, meta + 2 * t0, m.max_kv, n);
+            }
         }
         llamd_fwd_quantize(p.attn.as<float>(), p.aq.as<int8_t>(), p.ad.as<float>(), T * (qd / 256));
         if (tc) {
@@ -1555,6 +1588,7 @@ int llamd_model_prefill(llamd_model *h, const int32_t *tokens, int n_tokens, int
     // (expert parallelism over peer memory: tiles of at most the shared capacity; every rank must bring the same number
     // of tiles, of any length, or the others' bounded waits run out)
     int tile = m->prefill_tile < 1 ? 1 : m->prefill_tile;
+    if (!m->prefill_tile_set && m->ep_world == 1) tile = auto_tile(*m, n_tokens);
     if (m->ep_world > 1 && tile > m->pf.ep_cap) tile = m->pf.ep_cap;
     if (tile > n_tokens) tile = n_tokens;
     if (!prefill_alloc(*m, tile)) return -1;

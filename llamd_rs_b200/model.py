@@ -256,6 +256,8 @@ class CudaModel:
 
     @property
     def prefill_tile(self) -> int:
+        """Tokens per prefill tile. Until it is set, the library cuts a prompt into equal tiles of up to 2048 tokens on one
+        GPU; the results do not depend on it."""
         return getattr(self, "_prefill_tile", 512)
 
     @prefill_tile.setter
