@@ -141,7 +141,7 @@ struct Model {
     Buf tok_embd, output_norm, output, rope_tab;
     // scratch (crates/llamd-runtime/src/device.rs:407-434)
     Buf x, xb, xb2, q, k, v, attn, aq, ad, aq2, ad2, router_logits, router_probs, expert_ids, expert_w;
-    Buf head_fold, head_rm;  // the output matrix folded for the integer GEMM (option "head_gemm"), and a batch's activations in its operand order
+    Buf head_fold, head_rm;  // the output matrix folded for the integer GEMM (option "head_gemm"); a batch's activations in the GEMM's operand order
     bool head_fold_ready = false, head_fold_failed = false;
     Buf slot_order;          // [max_seq * n_expert_used] a batch's (sequence, slot) pairs sorted by expert (decode pass, 8 sequences and more)
     Buf e_gate, e_up, e_down, logits, amax_v, amax_i, out_token, meta;
@@ -695,6 +695,47 @@ bool check_ready(Model &m) {
     return true;
 }
 
+// The folded copies that a pass over n sequences, or a small tile of n tokens, multiplies with (options "dense_gemm" and
+// "head_gemm"), made once and not inside a capture; without the memory for them the matvec serves every pass. False: an error.
+bool ensure_folded(Model &m, int n, bool head = true) {
+    const llamd_hparams &hp = m.hp;
+    const int eb = hp.n_embd / 256, qd = hp.n_head * hp.head_dim, kvd = hp.n_head_kv * hp.head_dim;
+    if (m.dense_gemm && n >= m.dense_gemm && !m.dense_fold_ready && !m.dense_fold_failed) {
+        const size_t need = (size_t)hp.n_layer * (expert_fold_bytes(eb, qd, 1) + 2 * expert_fold_bytes(eb, kvd, 1) + expert_fold_bytes(qd / 256, hp.n_embd, 1));
+        bool ok = qd % 256 == 0 && need + ((size_t)1 << 30) <= llamd_cuda_free_mem();
+        for (size_t i = 0; ok && i < m.layers.size(); i++) {
+            Layer &l = m.layers[i];
+            ok = l.q_fold.alloc(expert_fold_bytes(eb, qd, 1)) && l.k_fold.alloc(expert_fold_bytes(eb, kvd, 1)) &&
+                 l.v_fold.alloc(expert_fold_bytes(eb, kvd, 1)) && l.o_fold.alloc(expert_fold_bytes(qd / 256, hp.n_embd, 1));
+            if (!ok) break;
+            expert_prefold(l.attn_q.p, l.q_fold.p, eb, qd, 1);
+            expert_prefold(l.attn_k.p, l.k_fold.p, eb, kvd, 1);
+            expert_prefold(l.attn_v.p, l.v_fold.p, eb, kvd, 1);
+            expert_prefold(l.attn_out.p, l.o_fold.p, qd / 256, hp.n_embd, 1);
+        }
+        m.dense_fold_ready = ok && llamd_fwd_sync() == 0;
+        if (!m.dense_fold_ready) {
+            for (auto &l : m.layers)
+                for (Buf *b : {&l.q_fold, &l.k_fold, &l.v_fold, &l.o_fold}) b->release();
+            m.dense_fold_failed = true;
+            if (error_code() != 0) return false;
+        }
+    }
+    if (head && m.head_gemm && n >= m.head_gemm && !m.head_fold_ready && !m.head_fold_failed) {
+        const size_t need = expert_fold_bytes(eb, hp.n_vocab, 1);
+        if (need + ((size_t)1 << 30) <= llamd_cuda_free_mem() && m.head_fold.alloc(need)) {
+            expert_prefold(m.output.p ? m.output.p : m.tok_embd.p, m.head_fold.p, eb, hp.n_vocab, 1);
+            m.head_fold_ready = llamd_fwd_sync() == 0;
+        }
+        if (!m.head_fold_ready) {
+            m.head_fold.release();
+            m.head_fold_failed = true;
+            if (error_code() != 0) return false;
+        }
+    }
+    return true;
+}
+
 int run(Model &m, const int32_t *tokens, const int32_t *positions, int nseq, int32_t *out_tokens) {
     const llamd_hparams &hp = m.hp;
     if (nseq < 1 || nseq > m.max_seq) {
@@ -715,49 +756,7 @@ int run(Model &m, const int32_t *tokens, const int32_t *positions, int nseq, int
     }
     if (!check_ready(m)) return -1;
     if (m.resident) mega_prepare(m);  // (uploads a pointer table: not inside a capture)
-    if (m.dense_gemm && nseq >= m.dense_gemm && !m.dense_fold_ready && !m.dense_fold_failed) {
-        // the attention projections folded once for batched passes (not inside a capture); the matvec without the memory
-        const int eb = hp.n_embd / 256, qd = hp.n_head * hp.head_dim, kvd = hp.n_head_kv * hp.head_dim;
-        const size_t need = (size_t)hp.n_layer * (expert_fold_bytes(eb, qd, 1) + 2 * expert_fold_bytes(eb, kvd, 1) + expert_fold_bytes(qd / 256, hp.n_embd, 1));
-        bool ok = qd % 256 == 0 && need + ((size_t)1 << 30) <= llamd_cuda_free_mem();
-        for (size_t i = 0; ok && i < m.layers.size(); i++) {
-            Layer &l = m.layers[i];
-            ok = l.q_fold.alloc(expert_fold_bytes(eb, qd, 1)) && l.k_fold.alloc(expert_fold_bytes(eb, kvd, 1)) &&
-                 l.v_fold.alloc(expert_fold_bytes(eb, kvd, 1)) && l.o_fold.alloc(expert_fold_bytes(qd / 256, hp.n_embd, 1));
-            if (!ok) break;
-            expert_prefold(l.attn_q.p, l.q_fold.p, eb, qd, 1);
-            expert_prefold(l.attn_k.p, l.k_fold.p, eb, kvd, 1);
-            expert_prefold(l.attn_v.p, l.v_fold.p, eb, kvd, 1);
-            expert_prefold(l.attn_out.p, l.o_fold.p, qd / 256, hp.n_embd, 1);
-        }
-        const size_t rm_bytes = (size_t)m.max_seq * (size_t)(qd / 256 > eb ? qd / 256 : eb) * 256;
-        if (ok && m.head_rm.bytes < rm_bytes) {
-            m.head_rm.release();
-            ok = m.head_rm.alloc(rm_bytes);
-        }
-        m.dense_fold_ready = ok && llamd_fwd_sync() == 0;
-        if (!m.dense_fold_ready) {
-            for (auto &l : m.layers)
-                for (Buf *b : {&l.q_fold, &l.k_fold, &l.v_fold, &l.o_fold}) b->release();
-            m.dense_fold_failed = true;
-            if (error_code() != 0) return -1;
-        }
-    }
-    if (m.head_gemm && nseq >= m.head_gemm && !m.head_fold_ready && !m.head_fold_failed) {
-        // the output matrix folded once for the batched output projection (not inside a capture); without the memory for
-        // it the matvec serves batches as it serves one sequence
-        const int eb = hp.n_embd / 256;
-        const size_t need = expert_fold_bytes(eb, hp.n_vocab, 1);
-        if (need + ((size_t)1 << 30) <= llamd_cuda_free_mem() && m.head_fold.alloc(need) && (m.head_rm.p || m.head_rm.alloc((size_t)m.max_seq * eb * 256))) {
-            expert_prefold(m.output.p ? m.output.p : m.tok_embd.p, m.head_fold.p, eb, hp.n_vocab, 1);
-            m.head_fold_ready = llamd_fwd_sync() == 0;
-        }
-        if (!m.head_fold_ready) {
-            m.head_fold.release();
-            m.head_fold_failed = true;
-            if (error_code() != 0) return -1;
-        }
-    }
+    if (!ensure_folded(m, nseq)) return -1;
     // the only per-token host->device traffic: 8 bytes per sequence
     if (cudaMemcpyAsync(m.meta.p, m.h_meta, (size_t)nseq * 8, cudaMemcpyHostToDevice, stream()) != cudaSuccess) {
         set_error(cudaGetLastError(), "meta H2D");
@@ -847,7 +846,7 @@ llamd_model *llamd_model_create(const llamd_hparams *hp, int max_kv, int max_seq
     f(m->x, E); f(m->xb, E); f(m->xb2, E); f(m->q, qd); f(m->k, kvd); f(m->v, kvd); f(m->attn, qd);
     ok = ok && m->aq.alloc(max_act * S);
     f(m->ad, max_act / 256);
-    ok = ok && m->aq2.alloc(nu * ffe * S);
+    ok = ok && m->aq2.alloc(nu * ffe * S) && m->head_rm.alloc(max_act * S);
     f(m->ad2, nu * ffe / 256);
     f(m->router_logits, hp->n_expert); f(m->router_probs, hp->n_expert);
     ok = ok && m->expert_ids.alloc(nu * 4 * S) && m->slot_order.alloc(nu * 4 * S);
@@ -1381,6 +1380,15 @@ static int ep_tile_cap(const Model &m) {
     return cap < 1 ? 1 : cap;
 }
 
+// A small tile of one sequence (a draft, a short turn, a prompt's rest) runs its matrices as a decode pass over as many
+// sequences does: the experts as grouped matvecs with the slots in expert order, the dense matrices on the folded copies.
+// The tile GEMMs fold every weight for 16-token MMA tiles that a handful of tokens leaves nearly empty. The line is where
+// a batch of sequences changes over, which was measured there (matvec_batch_max).
+constexpr int kRouterRowsMax = 12;  // a small tile's router: a chain per warp up to here (16 us for 9 tokens, 36 for 32), tiles of chains beyond (37)
+static bool small_tile(const Model &m, int T, bool multi_seq) {
+    return !multi_seq && m.ep_world == 1 && m.prefill_gemm == 1 && !m.prefold_ready && T <= m.matvec_batch_max && T * m.hp.n_expert_used <= 8192;
+}
+
 // multi_seq: the T tokens belong to T different sequences, token i with its own cache (sequence i) and position:
 // K/V go to the per-sequence caches and attention runs the per-sequence decode kernels. all_logits: the head runs for
 // every token of the tile (logits into `logits_out`, greedy picks into pf.out_tokens), not only for the last one.
@@ -1393,6 +1401,23 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
     const int32_t *meta = p.meta.as<int32_t>();
     float *x = p.x.as<float>();
     const int max_items = T * nu / 8 + ne;
+    const bool small = small_tile(m, T, multi_seq);
+    const bool folded = small && m.dense_gemm && T >= m.dense_gemm && m.dense_fold_ready;
+    // up to three dense matrices of a small tile against the activations in p.aq / p.ad
+    auto small_dense = [&](const Buf &f0, const Buf &f1, const Buf &f2, const Buf &w0, const Buf &w1, const Buf &w2, const Buf &o0, const Buf &o1,
+                           const Buf &o2, int blocks, int rows0, int rows12) {
+        if (folded) {
+            llamd_fwd_q8k_residue_major(p.aq.as<int8_t>(), p.aq_rm.p, (size_t)T * blocks);
+            gemm_tokens_folded3(f0.p, f1.p, f2.p, p.aq_rm.p, p.ad.as<float>(), o0.as<float>(), o1.as<float>(), o2.as<float>(), blocks, rows0, rows12,
+                                rows12, T);
+        } else if (w1.p) {
+            matvec_x3_batch(MatvecPlans{}, w0.p, w1.p, w2.p, p.aq.as<int8_t>(), p.ad.as<float>(), o0.as<float>(), o1.as<float>(), o2.as<float>(),
+                            blocks, rows0, rows12, rows12, T);
+        } else {
+            matvec_batch(MatvecPlans{}, w0.p, p.aq.as<int8_t>(), p.ad.as<float>(), o0.as<float>(), blocks, rows0, T);
+        }
+    };
+    const Buf none;
     llamd_fwd_embed_meta(m.tok_embd.p, meta, x, eb, T);
     for (int il = 0; il < hp.n_layer; il++) {
         Layer &l = m.layers[il];
@@ -1403,7 +1428,9 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
                                              p.aq.as<int8_t>(), p.ad.as<float>(), E, hp.rms_eps, T);
         const bool ep = m.ep_world > 1;  // sharded experts run on the integer GEMM; so then do the dense matmuls
         const bool gemm = m.prefill_gemm != 0 || ep, tc = m.prefill_gemm == 2 && !ep;
-        if (tc) {
+        if (small) {
+            small_dense(l.q_fold, l.k_fold, l.v_fold, l.attn_q, l.attn_k, l.attn_v, p.q, p.k, p.v, eb, qd, kvd);
+        } else if (tc) {
             llamd_fwd_act_f16_rm(p.aq.as<int8_t>(), p.ad.as<float>(), p.aq_rm.p, (size_t)T * eb);
             llamd_fwd_gemm_tokens_tc(l.attn_q.p, l.attn_k.p, l.attn_v.p, p.aq_rm.p, p.q.as<float>(), p.k.as<float>(), p.v.as<float>(), eb, qd,
                                      kvd, kvd, T);
@@ -1458,7 +1485,9 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
             }
         }
         llamd_fwd_quantize(p.attn.as<float>(), p.aq.as<int8_t>(), p.ad.as<float>(), T * (qd / 256));
-        if (tc) {
+        if (small) {
+            small_dense(l.o_fold, none, none, l.attn_out, none, none, p.xb2, none, none, qd / 256, E, 0);
+        } else if (tc) {
             llamd_fwd_act_f16_rm(p.aq.as<int8_t>(), p.ad.as<float>(), p.aq_rm.p, (size_t)T * (qd / 256));
             llamd_fwd_gemm_tokens_tc(l.attn_out.p, nullptr, nullptr, p.aq_rm.p, p.xb2.as<float>(), nullptr, nullptr, qd / 256, E, 0, 0, T);
         } else if (gemm) {
@@ -1471,7 +1500,7 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
         }
         llamd_fwd_add_rms_norm_quant(x, p.xb2.as<float>(), x, l.ffn_norm.as<float>(), p.xb.as<float>(), p.aq.as<int8_t>(), p.ad.as<float>(),
                                      E, hp.rms_eps, T);
-        if (m.prefill_attn && T > 1) {
+        if (m.prefill_attn && T > (small ? kRouterRowsMax : 1)) {
             llamd_fwd_matmul_f32_tokens(l.ffn_gate_inp.as<float>(), p.xb.as<float>(), p.logits.as<float>(), E, ne, T);
             llamd_fwd_router(p.logits.as<float>(), ne, nu, p.ids.as<int32_t>(), p.w.as<float>(), nullptr, T);
         } else {
@@ -1505,6 +1534,19 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
                                 ffe / 256, E, n_local, p.down_tab.as<float *>(), cap * nu);
             ep_signal_rows(m.ep_arrive_tab.as<unsigned int *>());
             ep_wait_rows(m.ep_arrive.as<unsigned int>(), (unsigned)W, m.ep_status.as<int>(), m.ep_poll_limit);
+            continue;
+        }
+        if (small) {
+            MatvecPlans plan = {};
+            if (m.sort_slots && T >= m.sort_slots) {
+                slot_order_launch(p.ids.as<int32_t>(), T * nu, p.pslot.as<int32_t>());
+                plan.slot_order = p.pslot.as<int32_t>();
+            }
+            matvec_grouped_x2_batch(plan, l.gate_exps.p, l.up_exps.p, p.ids.as<int32_t>(), p.aq.as<int8_t>(), p.ad.as<float>(), p.gate.as<float>(),
+                                    p.up.as<float>(), eb, ffe, nu, T);
+            llamd_fwd_silu_mul_quant(p.gate.as<float>(), p.up.as<float>(), nullptr, p.aq2.as<int8_t>(), p.ad2.as<float>(), T * nu * ffe);
+            matvec_grouped_pa_batch(plan, l.down_exps.p, p.ids.as<int32_t>(), p.aq2.as<int8_t>(), p.ad2.as<float>(), p.down.as<float>(), ffe / 256, E,
+                                    nu, T);
             continue;
         }
         // the expert scatter plan: (token, slot) pairs sorted by expert
@@ -1543,9 +1585,16 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
         // the head for every token of the tile: combine + output norm + Q8_K per row, lm_head as a GEMM, greedy pick per row
         llamd_fwd_combine_rms_norm_quant(x, p.down.as<float>(), p.w.as<float>(), nu, x, m.output_norm.as<float>(), nullptr,
                                          p.aq.as<int8_t>(), p.ad.as<float>(), E, hp.rms_eps, T);
-        llamd_fwd_q8k_residue_major(p.aq.as<int8_t>(), p.aq_rm.p, (size_t)T * eb);
-        llamd_fwd_gemm_tokens(m.output.p ? m.output.p : m.tok_embd.p, nullptr, nullptr, p.aq_rm.p, p.ad.as<float>(), logits_out, nullptr,
-                              nullptr, eb, hp.n_vocab, 0, 0, T);
+        if (small && !(m.head_gemm && T >= m.head_gemm && m.head_fold_ready)) {
+            matvec_batch(MatvecPlans{}, m.output.p ? m.output.p : m.tok_embd.p, p.aq.as<int8_t>(), p.ad.as<float>(), logits_out, eb, hp.n_vocab, T);
+        } else {
+            llamd_fwd_q8k_residue_major(p.aq.as<int8_t>(), p.aq_rm.p, (size_t)T * eb);
+            if (small)
+                gemm_tokens_folded(m.head_fold.p, p.aq_rm.p, p.ad.as<float>(), logits_out, eb, hp.n_vocab, T);
+            else
+                llamd_fwd_gemm_tokens(m.output.p ? m.output.p : m.tok_embd.p, nullptr, nullptr, p.aq_rm.p, p.ad.as<float>(), logits_out, nullptr,
+                                      nullptr, eb, hp.n_vocab, 0, 0, T);
+        }
         llamd_fwd_argmax(logits_out, hp.n_vocab, p.amax_v.as<float>(), p.amax_i.as<int32_t>(), p.out_tokens.as<int32_t>(), kArgmaxBlocks, T);
         return;
     }
@@ -1603,6 +1652,7 @@ int llamd_model_prefill(llamd_model *h, const int32_t *tokens, int n_tokens, int
             set_error(cudaGetLastError(), "prefill meta H2D");
             return -1;
         }
+        if (small_tile(*m, T, false) && !ensure_folded(*m, T, false)) return -1;
         queue_prefill_tile(*m, T, base_pos + t0 + T, t0 + T >= n_tokens);
     }
     if (cudaMemcpyAsync(m->h_out, m->out_token.p, 4, cudaMemcpyDeviceToHost, stream()) != cudaSuccess) return -1;
@@ -1664,6 +1714,7 @@ int llamd_model_verify(llamd_model *h, const int32_t *tokens, int n_tokens, int 
             set_error(cudaGetLastError(), "verify meta H2D");
             return -1;
         }
+        if (small_tile(*m, T, false) && !ensure_folded(*m, T)) return -1;
         queue_prefill_tile(*m, T, base_pos + t0 + T, true, false, true, m->pf.logits_all.as<float>());
         if (cudaMemcpyAsync(m->pf.h_out_tokens, m->pf.out_tokens.p, (size_t)T * 4, cudaMemcpyDeviceToHost, stream()) != cudaSuccess) return -1;
         if (llamd_fwd_sync() != 0) return -1;

@@ -294,6 +294,25 @@ def test_batch_attention_per_kv_head(kv_f16):
         gm.free()
 
 
+@pytest.mark.parametrize("n", [1, 8, 9, 12, 13, 56, 57])
+def test_small_tiles_equal_gemm_tiles(tiny, n):
+    """A tile's matrices run on the decode pass's launches up to matvec_batch_max tokens and on the tile GEMMs beyond: the
+    same logits and cache rows on both sides of the line, and the same picks from a verification."""
+    from llamd_rs_b200 import synth
+
+    hp, w, gm, om = tiny
+    prompt = synth.token_ids(n, hp["n_vocab"], 11, "prefill").tolist()
+    runs = []
+    for line in (8, 256):
+        gm.set_option("matvec_batch_max", line)
+        tok = gm.prefill(prompt, 0)
+        runs.append((tok, gm.logits()[0].view(np.uint32).copy(), gm.read_kv(hp["n_layer"] - 1, n), list(gm.verify(prompt, 0))))
+    gm.set_option("matvec_batch_max", 56)
+    a, b = runs
+    assert a[0] == b[0] and np.array_equal(a[1], b[1]) and a[3] == b[3] and a[3][-1] == a[0]
+    assert np.array_equal(a[2][0].view(np.uint32), b[2][0].view(np.uint32)) and np.array_equal(a[2][1].view(np.uint32), b[2][1].view(np.uint32))
+
+
 def test_prefill_equals_sequential_decode(tiny):
     """crates/llamd-testing/tests/vulkan_prefill.rs:48-136: prefill gives the token (and here the logits and the
     K/V cache, bit for bit) of sequential decode, for (tile, length) pairs that straddle tile and chunk boundaries."""
