@@ -305,110 +305,17 @@ __global__ void __launch_bounds__(128) matvec_q8_0_kernel(const uint8_t *__restr
     for (int s = 0; s < NSEQ; s++) out[(size_t)s * rows + row] = acc[s];
 }
 
-// The same result with the row's work spread over a CTA. Above, one thread unpacks, converts, multiplies and adds
-// every element of its row alone and is bound by its own instruction latency (~20 cycles per element). Here a CTA owns
-// 32 rows: seven producer warps turn 8 blocks (256 columns) of the 32 rows into f32 weights d*q in shared memory,
-// [column][row] so that a lane per row reads without bank conflicts, while one chain warp per sequence (lane = row)
-// walks acc = acc + w*x over the previous 256 columns: only the add is on the dependent chain (~4 cycles per element).
-// Raw blocks are loaded two chunks ahead into registers, converted one chunk ahead, double-buffered in shared memory.
-constexpr int kQ80ChunkBlocks = 8;
-constexpr int kQ80Producers = 224;  // 7 warps
-template <int NSEQ>
-__global__ void __launch_bounds__(kQ80Producers + 32 * NSEQ) matvec_q8_0_rows_kernel(const uint8_t *__restrict__ tiled, const float *__restrict__ x,
-                                                                                     float *__restrict__ out, int blocks, int rows) {
-    extern __shared__ __align__(16) float smem_f[];
-    float *s_w = smem_f;                                      // [2][kQ80ChunkBlocks * 32 columns][32 rows]
-    float *sx = smem_f + 2 * kQ80ChunkBlocks * 32 * 32;       // [NSEQ][k]
-    pdl_trigger();
-    pdl_wait();
-    const int k = blocks * 32, tid = threadIdx.x;
-    const bool producer = tid < kQ80Producers;
-    const int n_chunks = (blocks + kQ80ChunkBlocks - 1) / kQ80ChunkBlocks;
-    const uint8_t *tile0 = tiled + (size_t)blockIdx.x * blocks * kQ80TileBytes;  // this CTA's 32 rows, block 0
-    constexpr int kItems = kQ80ChunkBlocks * 64;                                 // (block, half, row): 16 weights each
-    constexpr int kPer = (kItems + kQ80Producers - 1) / kQ80Producers;           // 3
-    uint4 raw[kPer];
-    uint16_t rawd[kPer];
-    auto load_chunk = [&](int ch) {
-#pragma unroll
-        for (int u = 0; u < kPer; u++) {
-            const int item = tid + u * kQ80Producers;
-            const int bl = item >> 6, h = (item >> 5) & 1, r = item & 31;
-            raw[u] = make_uint4(0, 0, 0, 0);
-            rawd[u] = 0;
-            if (item < kItems && ch * kQ80ChunkBlocks + bl < blocks) {
-                const uint8_t *t = tile0 + (size_t)(ch * kQ80ChunkBlocks + bl) * kQ80TileBytes;
-                raw[u] = __ldg(reinterpret_cast<const uint4 *>(t + 512 * h) + r);
-                rawd[u] = __ldg(reinterpret_cast<const uint16_t *>(t + 1024) + r);
-            }
-        }
-    };
-    auto store_chunk = [&](int buf) {
-        float *dst = s_w + buf * (kQ80ChunkBlocks * 32 * 32);
-#pragma unroll
-        for (int u = 0; u < kPer; u++) {
-            const int item = tid + u * kQ80Producers;
-            if (item < kItems) {
-                const int bl = item >> 6, h = (item >> 5) & 1, r = item & 31;
-                const float d = f16_bits_to_f32(rawd[u]);
-                const uint32_t ws[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
-#pragma unroll
-                for (int j = 0; j < 16; j++)
-                    dst[(bl * 32 + h * 16 + j) * 32 + r] = __fmul_rn(d, (float)(int8_t)(ws[j >> 2] >> (8 * (j & 3))));
-            }
-        }
-    };
-    if (producer) load_chunk(0);
-    for (int i = tid; i < NSEQ * k; i += blockDim.x) sx[i] = x[i];
-    if (producer) {
-        store_chunk(0);
-        if (n_chunks > 1) load_chunk(1);
-    }
-    __syncthreads();
-    const int seq = (tid - kQ80Producers) >> 5, lane = tid & 31;  // chain warps
-    float acc = -0.0f;
-    for (int ch = 0; ch < n_chunks; ch++) {
-        if (producer) {
-            if (ch + 1 < n_chunks) store_chunk((ch + 1) & 1);
-            if (ch + 2 < n_chunks) load_chunk(ch + 2);
-        } else {
-            const float *w = s_w + (ch & 1) * (kQ80ChunkBlocks * 32 * 32) + lane;
-            const float *xs = sx + (size_t)seq * k + ch * kQ80ChunkBlocks * 32;
-            const int ncol = min(kQ80ChunkBlocks, blocks - ch * kQ80ChunkBlocks) * 32;
-            // 16 columns at a time, the next 16 loaded while these are added: the loads and the multiplies stay off
-            // the chain, which is then the 16 dependent adds (ncol is a multiple of 32)
-            float wv[16], xv[16];
-            auto fetch = [&](int c0) {
-#pragma unroll
-                for (int j = 0; j < 16; j++) wv[j] = w[(c0 + j) * 32];
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const float4 v = *reinterpret_cast<const float4 *>(xs + c0 + 4 * j);
-                    xv[4 * j] = v.x, xv[4 * j + 1] = v.y, xv[4 * j + 2] = v.z, xv[4 * j + 3] = v.w;
-                }
-            };
-            fetch(0);
-            for (int c0 = 0; c0 < ncol; c0 += 16) {
-                float pr[16];
-#pragma unroll
-                for (int j = 0; j < 16; j++) pr[j] = __fmul_rn(wv[j], xv[j]);
-                if (c0 + 16 < ncol) fetch(c0 + 16);
-#pragma unroll
-                for (int j = 0; j < 16; j++) acc = __fadd_rn(acc, pr[j]);
-            }
-        }
-        __syncthreads();
-    }
-    const int row = blockIdx.x * 32 + lane;
-    if (!producer && row < rows) out[(size_t)seq * rows + row] = acc;
-}
-
-// The same arithmetic again, fed by bulk copies. The form above keeps ONE chunk of raw blocks in flight per CTA (8.7 KB
-// per SM against an HBM round trip of ~2 us: 0.5 TB/s over the whole GPU, which is what it measured). Here one thread
-// asks for the CTA's WHOLE slice of the matrix -- 32 rows x all blocks, one contiguous run of the tiled layout -- as one
-// bulk copy per 256-column chunk (cp.async.bulk, each completing on its own mbarrier) before anything else happens, so
-// the memory latency is paid once and the producers then convert from shared memory. With one sequence the producers
-// store the products (d*q)*x, so the chain warp's loop is a shared load and the dependent add alone.
+// The same result with the row's work spread over a CTA, fed by bulk copies. Above, one thread unpacks, converts, multiplies
+// and adds every element of its row alone and is bound by its own instruction latency (~20 cycles per element). Here a CTA
+// owns 32 rows: seven producer warps turn 8 blocks (256 columns) of the 32 rows into f32 weights d*q in shared memory while
+// one chain warp per sequence (lane = row) walks acc = acc + w*x over the previous 256 columns: only the add is on the
+// dependent chain (~4 cycles per element). The raw blocks come as one bulk copy per chunk (cp.async.bulk, 32 rows x 256
+// columns are one contiguous run of the tiled layout), n_raw chunks ahead, the first ones before anything else happens; the
+// producers convert from shared memory. With one sequence the producers
+// store the products (d*q)*x, so the chain warp's loop is a shared load and the dependent add alone; with more, each has
+// a chain warp that multiplies ahead of its adds. Bound by those chains (2048 dependent adds are 4.3 us at 1.9 GHz).
+// 4096 x 2048, 1 / 2 / 4 / 8 sequences: 13.8 / 26.2 / 27.5 / 37.9 us with the activations staged a load at a time and the
+// multiplies standing between the adds, 11.6 / 16.0 / 17.5 / 23.3 now.
 // Every mbarrier wait is bounded; a wait that runs out sets *status and the CTA leaves its outputs unwritten.
 __device__ __forceinline__ uint32_t q80_smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ bool q80_mbar_wait(uint64_t *bar, uint32_t parity) {
@@ -426,12 +333,20 @@ __device__ __forceinline__ bool q80_mbar_wait(uint64_t *bar, uint32_t parity) {
     }
     return false;
 }
-constexpr int kQ80MaxChunks = 32;  // k <= 8192
+constexpr int kQ80ChunkBlocks = 8;
+constexpr int kQ80Producers = 224;   // 7 warps
+constexpr int kQ80MaxRaw = 32;       // raw chunks in flight
+constexpr int kQ80RingBytes = 2 * kQ80ChunkBlocks * 32 * 32 * 4, kQ80RawBytes = kQ80ChunkBlocks * kQ80TileBytes;
+__device__ __forceinline__ unsigned long long q80_mul2(unsigned long long w, unsigned long long x) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(w), "l"(x));
+    return r;
+}
 template <int NSEQ>
 __global__ void __launch_bounds__(kQ80Producers + 32 * NSEQ) matvec_q8_0_bulk_kernel(const uint8_t *__restrict__ tiled, const float *__restrict__ x,
-                                                                                     float *__restrict__ out, int blocks, int rows, int *status) {
+                                                                                     float *__restrict__ out, int blocks, int rows, int n_raw, int *status) {
     extern __shared__ __align__(16) float smem_f[];
-    __shared__ __align__(8) uint64_t s_bar[kQ80MaxChunks];
+    __shared__ __align__(8) uint64_t s_bar[kQ80MaxRaw];
     __shared__ int s_fail;
     constexpr bool kProd = NSEQ == 1;                         // the ring holds products w*x instead of weights
     // ring: [2][64 column quads][32 rows][4]: a lane (= row) reads four consecutive columns with one 16-byte load, and the
@@ -440,42 +355,59 @@ __global__ void __launch_bounds__(kQ80Producers + 32 * NSEQ) matvec_q8_0_bulk_ke
     float *s_w = smem_f;
     float *sx = smem_f + 2 * kQ80ChunkBlocks * 32 * 32;       // [NSEQ][k]
     const int k = blocks * 32, tid = threadIdx.x;
-    uint8_t *s_raw = reinterpret_cast<uint8_t *>(sx + (size_t)NSEQ * k);  // [blocks][1088]: the tiles as they lie in memory
+    uint8_t *s_raw = reinterpret_cast<uint8_t *>(sx + (size_t)NSEQ * k);  // [n_raw][8 blocks][1088]: the tiles as they lie in memory
     const bool producer = tid < kQ80Producers;
     const int n_chunks = (blocks + kQ80ChunkBlocks - 1) / kQ80ChunkBlocks;
     const uint8_t *tile0 = tiled + (size_t)blockIdx.x * blocks * kQ80TileBytes;  // this CTA's 32 rows, block 0
+    auto request = [&](int ch) {  // one thread
+        const uint32_t bytes = (uint32_t)min(kQ80ChunkBlocks, blocks - ch * kQ80ChunkBlocks) * kQ80TileBytes;  // (1088 = 68 x 16)
+        const int slot = ch % n_raw;
+        const uint32_t bar = q80_smem_u32(&s_bar[slot]);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         q80_smem_u32(s_raw + (size_t)slot * kQ80RawBytes)),
+                     "l"(tile0 + (size_t)ch * kQ80RawBytes), "r"(bytes), "r"(bar)
+                     : "memory");
+    };
     if (tid == 0) {
         s_fail = 0;
-        for (int ch = 0; ch < n_chunks; ch++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(q80_smem_u32(&s_bar[ch])) : "memory");
+        for (int i = 0; i < n_raw; i++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(q80_smem_u32(&s_bar[i])) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         // the weights do not depend on the previous kernel: their copies start before the dependency wait
-        for (int ch = 0; ch < n_chunks; ch++) {
-            const int nb = min(kQ80ChunkBlocks, blocks - ch * kQ80ChunkBlocks);
-            const uint32_t bytes = (uint32_t)nb * kQ80TileBytes;  // (1088 = 68 x 16)
-            const uint32_t bar = q80_smem_u32(&s_bar[ch]);
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                             q80_smem_u32(s_raw + (size_t)ch * kQ80ChunkBlocks * kQ80TileBytes)),
-                         "l"(tile0 + (size_t)ch * kQ80ChunkBlocks * kQ80TileBytes), "r"(bytes), "r"(bar)
-                         : "memory");
-        }
+        for (int ch = 0; ch < n_raw && ch < n_chunks; ch++) request(ch);
     }
     pdl_trigger();
     pdl_wait();
-    for (int i = tid; i < NSEQ * k; i += blockDim.x) sx[i] = x[i];
+    {   // (all of a thread's loads in flight at once: one after the other this loop took 7000 cycles for 2048 columns, a
+        // quarter of the launch, and 15000 for eight sequences)
+        const int n4 = NSEQ * k / 4;
+        for (int i0 = 0; i0 < n4; i0 += 8 * (int)blockDim.x) {
+            float4 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int i = i0 + u * (int)blockDim.x + tid;
+                if (i < n4) v[u] = reinterpret_cast<const float4 *>(x)[i];
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int i = i0 + u * (int)blockDim.x + tid;
+                if (i < n4) reinterpret_cast<float4 *>(sx)[i] = v[u];
+            }
+        }
+    }
     __syncthreads();  // (the barriers are initialised, the activations staged)
     constexpr int kItems = kQ80ChunkBlocks * 64;                        // (block, half, row): 16 weights each
     constexpr int kPer = (kItems + kQ80Producers - 1) / kQ80Producers;  // 3
     auto convert_chunk = [&](int ch) -> bool {
-        if (!q80_mbar_wait(&s_bar[ch], 0)) return false;
+        if (!q80_mbar_wait(&s_bar[ch % n_raw], (uint32_t)(ch / n_raw) & 1)) return false;
         float4 *dst = reinterpret_cast<float4 *>(s_w + (ch & 1) * (kQ80ChunkBlocks * 32 * 32));
 #pragma unroll
         for (int u = 0; u < kPer; u++) {
             const int item = tid + u * kQ80Producers;
             const int bl = item >> 6, h = (item >> 5) & 1, r = item & 31;
             if (item < kItems && ch * kQ80ChunkBlocks + bl < blocks) {
-                const uint8_t *t = s_raw + (size_t)(ch * kQ80ChunkBlocks + bl) * kQ80TileBytes;
+                const uint8_t *t = s_raw + (size_t)(ch % n_raw) * kQ80RawBytes + (size_t)bl * kQ80TileBytes;
                 const uint4 raw = *(reinterpret_cast<const uint4 *>(t + 512 * h) + r);
                 const float d = f16_bits_to_f32(*(reinterpret_cast<const uint16_t *>(t + 1024) + r));
                 const uint32_t ws[4] = {raw.x ^ 0x80808080u, raw.y ^ 0x80808080u, raw.z ^ 0x80808080u, raw.w ^ 0x80808080u};
@@ -497,6 +429,7 @@ __global__ void __launch_bounds__(kQ80Producers + 32 * NSEQ) matvec_q8_0_bulk_ke
         }
         return true;
     };
+    int requested = min(n_raw, n_chunks) - 1;  // thread 0: the last chunk asked for
     if (producer && !convert_chunk(0)) s_fail = 1;
     __syncthreads();
     const int seq = (tid - kQ80Producers) >> 5, lane = tid & 31;  // chain warps
@@ -504,6 +437,8 @@ __global__ void __launch_bounds__(kQ80Producers + 32 * NSEQ) matvec_q8_0_bulk_ke
 #define Q80_ADD4(v) acc = __fadd_rn(acc, v.x), acc = __fadd_rn(acc, v.y), acc = __fadd_rn(acc, v.z), acc = __fadd_rn(acc, v.w)
     for (int ch = 0; ch < n_chunks; ch++) {
         if (producer) {
+            // (chunk ch was converted behind the barrier: its slot is free)
+            if (tid == 0 && !s_fail && ch + n_raw < n_chunks) request(requested = ch + n_raw);
             if (ch + 1 < n_chunks && !s_fail && !convert_chunk(ch + 1)) s_fail = 1;
         } else {
             const float4 *w = reinterpret_cast<const float4 *>(s_w + (ch & 1) * (kQ80ChunkBlocks * 32 * 32)) + lane;
@@ -520,20 +455,31 @@ __global__ void __launch_bounds__(kQ80Producers + 32 * NSEQ) matvec_q8_0_bulk_ke
                     b0 = w[qb], b1 = w[qb + 32], b2 = w[qb + 64], b3 = w[qb + 96];
                 }
             } else {
-                const float4 *xs = reinterpret_cast<const float4 *>(sx + (size_t)seq * k + ch * kQ80ChunkBlocks * 32);
-                float4 wv[4], xv[4];
+                // the products of 16 columns (packed: w and x of neighbouring columns are register pairs as they lie) and the
+                // loads of the 16 after them do not depend on the adds that they are scheduled among
+                const ulonglong2 *w2 = reinterpret_cast<const ulonglong2 *>(w), *xs = reinterpret_cast<const ulonglong2 *>(sx + (size_t)seq * k + ch * kQ80ChunkBlocks * 32);
+                ulonglong2 wv[4], xv[4], pr[4];
                 auto fetch = [&](int q0) {
 #pragma unroll
-                    for (int j = 0; j < 4; j++) wv[j] = w[(q0 + j) * 32], xv[j] = xs[q0 + j];
+                    for (int j = 0; j < 4; j++) wv[j] = w2[(q0 + j) * 32], xv[j] = xs[q0 + j];
+                };
+                auto products = [&](ulonglong2 (&o)[4]) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) o[j].x = q80_mul2(wv[j].x, xv[j].x), o[j].y = q80_mul2(wv[j].y, xv[j].y);
                 };
                 fetch(0);
+                products(pr);
+                fetch(4);  // (nq is a multiple of 8)
                 for (int q0 = 0; q0 < nq; q0 += 4) {
-                    float4 pr[4];
+                    ulonglong2 nx[4];
+                    products(nx);
+                    fetch(min(q0 + 8, nq - 4));
 #pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        pr[j] = make_float4(__fmul_rn(wv[j].x, xv[j].x), __fmul_rn(wv[j].y, xv[j].y), __fmul_rn(wv[j].z, xv[j].z), __fmul_rn(wv[j].w, xv[j].w));
-                    if (q0 + 4 < nq) fetch(q0 + 4);
-                    Q80_ADD4(pr[0]), Q80_ADD4(pr[1]), Q80_ADD4(pr[2]), Q80_ADD4(pr[3]);
+                    for (int j = 0; j < 4; j++) {
+                        acc = __fadd_rn(acc, __uint_as_float((uint32_t)pr[j].x)), acc = __fadd_rn(acc, __uint_as_float((uint32_t)(pr[j].x >> 32)));
+                        acc = __fadd_rn(acc, __uint_as_float((uint32_t)pr[j].y)), acc = __fadd_rn(acc, __uint_as_float((uint32_t)(pr[j].y >> 32)));
+                        pr[j] = nx[j];
+                    }
                 }
             }
         }
@@ -544,8 +490,8 @@ __global__ void __launch_bounds__(kQ80Producers + 32 * NSEQ) matvec_q8_0_bulk_ke
         // a copy did not arrive within the limit: wait (bounded again) for the ones still in flight before this CTA's shared
         // memory is given up, record it, write nothing
         if (tid == 0) {
-            for (int ch = 0; ch < n_chunks; ch++) q80_mbar_wait(&s_bar[ch], 0);
-            atomicExch(status, 1 + (int)blockIdx.x);
+            for (int ch = max(0, requested - n_raw + 1); ch <= requested; ch++) q80_mbar_wait(&s_bar[ch % n_raw], (uint32_t)(ch / n_raw) & 1);
+            *(volatile int *)status = 1 + (int)blockIdx.x;
         }
         return;
     }
@@ -1785,14 +1731,17 @@ void llamd::norm_router_flags(const float *w, const float *x, const float *resid
 }
 extern "C" {
 
-static int g_q80_rows_max_ctas = 148 * 4;
+// Measured, this form / thread per row: 20000 x 4096 (625 CTAs) 57 / 86 us for one sequence, 137 / 120 for four (one CTA
+// per SM beside their activations); 20000 x 1056 21 / 26 and 33 / 35.
+constexpr int kQ80MaxCtasOne = 148 * 8, kQ80MaxCtas = 148 * 4;
 static int *g_q80_status = nullptr;
-static int *q80_status_word() {
+static int *q80_status_word() {  // mapped host memory: reading it after a synchronise costs no copy
     if (!g_q80_status) {
-        if (cudaMalloc(&g_q80_status, sizeof(int)) != cudaSuccess || cudaMemsetAsync(g_q80_status, 0, sizeof(int), stream()) != cudaSuccess) {
+        if (cudaHostAlloc((void **)&g_q80_status, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
             cudaGetLastError();
-            g_q80_status = nullptr;
+            return g_q80_status = nullptr;
         }
+        *g_q80_status = 0;
     }
     return g_q80_status;
 }
@@ -1800,10 +1749,8 @@ static int *q80_status_word() {
 // 32 rows were not written). Synchronises the stream.
 int llamd_fwd_matvec_q8_0_status(void) {
     if (!g_q80_status) return 0;
-    int h = 0;
-    if (cudaMemcpyAsync(&h, g_q80_status, sizeof(int), cudaMemcpyDeviceToHost, stream()) != cudaSuccess) return -1;
     if (cudaStreamSynchronize(stream()) != cudaSuccess) return -1;
-    return h;
+    return *(volatile int *)g_q80_status;
 }
 void llamd_fwd_matvec_q8_0(const void *w, const float *x, float *out, int blocks32, int rows, int nseq) {
     const size_t smem = (size_t)nseq * blocks32 * 32 * sizeof(float);
@@ -1812,19 +1759,22 @@ void llamd_fwd_matvec_q8_0(const void *w, const float *x, float *out, int blocks
         return;
     }
     const uint8_t *t = (const uint8_t *)w;
-    // the CTA-per-32-rows form needs 64 KiB of staged weights beside the activations; the thread-per-row form takes the rest
-    const size_t smem_rows = smem + 2 * kQ80ChunkBlocks * 32 * 32 * sizeof(float);
-    // measured: it wins while its CTAs fit one wave (attn_q 40 -> 10s of us); beyond that the thread-per-row form's
-    // deeper occupancy does (lm_head)
-    const bool by_rows = smem_rows <= 220 * 1024 && (rows + 31) / 32 <= g_q80_rows_max_ctas;
-    // ... and with the CTA's whole slice of the matrix brought in by bulk copies, where that fits beside the rest
-    const size_t smem_bulk = smem_rows + (size_t)blocks32 * kQ80TileBytes;
-    const bool by_bulk = by_rows && smem_bulk <= 226 * 1024 && (blocks32 + kQ80ChunkBlocks - 1) / kQ80ChunkBlocks <= kQ80MaxChunks &&
-                         ((uintptr_t)w & 15) == 0 && q80_status_word() != nullptr;
-    const dim3 grid(by_rows ? (rows + 31) / 32 : (rows + 127) / 128);
+    // The CTA-per-32-rows form: 64 KiB of converted weights and at least two raw chunks beside the activations. Its CTAs are
+    // bound by their chains, so where they do not all fit at one per SM the raw ring gives way to a second CTA per SM. It
+    // wins while they are a few waves; beyond that the thread-per-row form's deeper occupancy does (lm_head).
+    const int ctas = (rows + 31) / 32, chunks = (blocks32 + kQ80ChunkBlocks - 1) / kQ80ChunkBlocks;
+    auto raw_fit = [&](size_t budget) { return budget < smem + kQ80RingBytes ? 0 : (int)((budget - smem - kQ80RingBytes) / kQ80RawBytes); };
+    int n_raw = ctas > 148 ? raw_fit(111 * 1024) : 0;
+    if (n_raw < 2) n_raw = raw_fit(225 * 1024);
+    if (n_raw > kQ80MaxRaw) n_raw = kQ80MaxRaw;
+    if (n_raw > chunks) n_raw = chunks;
+    const bool by_bulk = ctas <= (nseq == 1 ? kQ80MaxCtasOne : kQ80MaxCtas) && n_raw >= (chunks < 2 ? 1 : 2) && ((uintptr_t)w & 15) == 0 && ((uintptr_t)x & 15) == 0 &&
+                         q80_status_word() != nullptr;
+    const size_t smem_bulk = smem + kQ80RingBytes + (size_t)n_raw * kQ80RawBytes;
+    const dim3 grid(by_bulk ? ctas : (rows + 127) / 128);
 #define Q80_CASE(N)                                                                                                   \
     case N: {                                                                                                          \
-        static size_t configured = 0, configured_rows = 0;                                                             \
+        static size_t configured = 0;                                                                                  \
         if (by_bulk) {                                                                                                 \
             static size_t configured_bulk = 0;                                                                         \
             if (smem_bulk > configured_bulk) {                                                                         \
@@ -1834,15 +1784,7 @@ void llamd_fwd_matvec_q8_0(const void *w, const float *x, float *out, int blocks
                 }                                                                                                      \
                 configured_bulk = smem_bulk;                                                                           \
             }                                                                                                          \
-            launch_kc(PDL_OTHER, "matvec_q8_0_bulk", matvec_q8_0_bulk_kernel<N>, grid, dim3(kQ80Producers + 32 * N), smem_bulk, t, x, out, blocks32, rows, q80_status_word()); \
-            break;                                                                                                     \
-        }                                                                                                              \
-        if (by_rows) {                                                                                                 \
-            if (smem_rows > configured_rows) {                                                                         \
-                cudaFuncSetAttribute(matvec_q8_0_rows_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows); \
-                configured_rows = smem_rows;                                                                           \
-            }                                                                                                          \
-            launch_k("matvec_q8_0_rows", matvec_q8_0_rows_kernel<N>, grid, dim3(kQ80Producers + 32 * N), smem_rows, t, x, out, blocks32, rows); \
+            launch_kc(PDL_OTHER, "matvec_q8_0_bulk", matvec_q8_0_bulk_kernel<N>, grid, dim3(kQ80Producers + 32 * N), smem_bulk, t, x, out, blocks32, rows, n_raw, q80_status_word()); \
             break;                                                                                                     \
         }                                                                                                              \
         if (smem > 48 * 1024 && smem > configured) {                                                                   \
