@@ -41,6 +41,8 @@ unsafe extern "C" {
     pub fn llamd_cuda_last_error_string() -> *const c_char;
     pub fn llamd_cuda_upload(host: *const c_void, bytes: usize) -> *mut c_void;
     pub fn llamd_cuda_release(dev: *mut c_void);
+    pub fn llamd_cuda_host_alloc(bytes: usize) -> *mut c_void;
+    pub fn llamd_cuda_host_free(p: *mut c_void);
     pub fn llamd_fwd_alloc(bytes: usize) -> *mut c_void;
     pub fn llamd_fwd_free(p: *mut c_void);
     pub fn llamd_fwd_upload(dst: *mut c_void, src: *const c_void, bytes: usize) -> c_int;

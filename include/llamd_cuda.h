@@ -51,6 +51,10 @@ const char *llamd_cuda_last_error_string(void);
  *      crates/llamd-rocm/src/forward.rs:270-277 --------------------------- */
 void *llamd_cuda_upload(const void *host, size_t bytes); /* NULL on failure */
 void llamd_cuda_release(void *dev);
+/* Pinned host memory for a caller's own buffers: results copied into it (llamd_cuda_matvec_q6k_f32, llamd_model_logits,
+ * ...) skip the driver's pageable staging. NULL when there is none to be had; any host memory will do instead. */
+void *llamd_cuda_host_alloc(size_t bytes);
+void llamd_cuda_host_free(void *p);
 void *llamd_fwd_alloc(size_t bytes);
 void llamd_fwd_free(void *p);
 int llamd_fwd_upload(void *dst, const void *src, size_t bytes);

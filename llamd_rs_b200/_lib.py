@@ -24,6 +24,8 @@ SIGNATURES = {
     "llamd_cuda_last_error_string": (C.c_char_p, []),
     "llamd_cuda_upload": (vp, [vp, sz]),
     "llamd_cuda_release": (None, [vp]),
+    "llamd_cuda_host_alloc": (vp, [sz]),
+    "llamd_cuda_host_free": (None, [vp]),
     "llamd_fwd_alloc": (vp, [sz]),
     "llamd_fwd_free": (None, [vp]),
     "llamd_fwd_upload": (i32, [vp, vp, sz]),

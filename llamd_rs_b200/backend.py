@@ -10,6 +10,7 @@ This module is for tests, the bench and Python users; the compiled host side
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from dataclasses import dataclass
 
 import numpy as np
@@ -45,6 +46,67 @@ class Other(LlamdError):
 
 def _ptr(a: np.ndarray):
     return a.ctypes.data_as(C.c_void_p)
+
+
+class _Block:
+    """A pinned block of the pool below, lent to one array; back in the pool when the last view of the array is gone."""
+    __slots__ = ("pool", "ptr", "size", "__array_interface__")
+
+    def __init__(self, pool, ptr, size):
+        self.pool, self.ptr, self.size = pool, ptr, size
+
+    def __del__(self):
+        try:
+            self.pool.give_back(self.ptr, self.size)
+        except Exception:  # the interpreter is shutting down: the process's memory goes with it
+            pass
+
+
+class _ResultPool:
+    """Pinned memory for large result arrays: the device copies straight into the array that the caller gets, where an
+    ordinary new array costs a page fault per 4 KB and a copy through the driver's staging (0.2 ms for the four rows of
+    logits of a 151936-token vocabulary). At most LIMIT bytes are pinned, KEEP of them while nobody holds them; beyond that,
+    and below MIN, a result is an ordinary array."""
+    MIN, KEEP, LIMIT = 1 << 15, 64 << 20, 256 << 20
+
+    def __init__(self):
+        self.lock = threading.RLock()  # (re-entrant: a garbage collection inside may give a block back)
+        self.free = {}                 # size -> pointers
+        self.idle = self.total = 0
+
+    def empty(self, shape) -> np.ndarray:
+        n = 4 * int(np.prod(shape))
+        if n < self.MIN:
+            return np.empty(shape, dtype=np.float32)
+        size = 1 << (n - 1).bit_length()
+        ptr = None
+        with self.lock:
+            have = self.free.get(size)
+            if have:
+                ptr = have.pop()
+                self.idle -= size
+            elif self.total + size <= self.LIMIT:
+                self.total += size
+                ptr = lib().llamd_cuda_host_alloc(size)
+                if not ptr:
+                    self.total -= size
+        if not ptr:
+            return np.empty(shape, dtype=np.float32)
+        b = _Block(self, ptr, size)
+        b.__array_interface__ = {"data": (ptr, False), "typestr": "<f4", "shape": tuple(shape), "version": 3}
+        return np.asarray(b)
+
+    def give_back(self, ptr, size):
+        with self.lock:
+            if self.idle + size <= self.KEEP:
+                self.free.setdefault(size, []).append(ptr)
+                self.idle += size
+                return
+            self.total -= size
+        lib().llamd_cuda_host_free(ptr)
+
+
+results = _ResultPool()
 
 
 def _last_error() -> str:
@@ -248,11 +310,11 @@ class DeviceWeights:
         x = np.ascontiguousarray(x, dtype=np.float32).ravel()
         if nseq < 1 or nseq > MAX_SEQ or x.size != nseq * self._blocks * QK_K:
             raise ShapeError(f"expected {nseq}x{self._blocks * QK_K} activations, got {x.size}")
-        out = np.zeros(nseq * self._rows, dtype=np.float32)
-        rc = lib().llamd_cuda_matvec_q6k_f32(self.ptr, _ptr(x), _ptr(out), self._blocks, self._rows, nseq)
+        out = results.empty((nseq, self._rows))
+        rc = lib().llamd_cuda_matvec_q6k_f32(self.ptr, x.ctypes.data, out.ctypes.data, self._blocks, self._rows, nseq)
         if rc != 0:
             raise Other("CUDA matvec failed: " + _last_error())
-        return out.reshape(nseq, self._rows)
+        return out
 
     def _check_grouped(self, expert_ids, rows_per_expert: int):
         ids = np.ascontiguousarray(expert_ids, dtype=np.int32).ravel()
@@ -351,11 +413,11 @@ class Q80Weights:
         x = np.ascontiguousarray(x, dtype=np.float32).ravel()
         if nseq < 1 or nseq > MAX_SEQ or x.size != nseq * self._blocks * 32:
             raise ShapeError(f"expected {nseq}x{self._blocks * 32} activations, got {x.size}")
-        out = np.zeros(nseq * self._rows, dtype=np.float32)
-        rc = lib().llamd_cuda_matvec_q8_0_f32(self.ptr, _ptr(x), _ptr(out), self._blocks, self._rows, nseq)
+        out = results.empty((nseq, self._rows))
+        rc = lib().llamd_cuda_matvec_q8_0_f32(self.ptr, x.ctypes.data, out.ctypes.data, self._blocks, self._rows, nseq)
         if rc != 0:
             raise Other("CUDA Q8_0 matvec failed: " + _last_error())
-        return out.reshape(nseq, self._rows)
+        return out
 
     def dequantize(self) -> np.ndarray:
         tmp = DevBuf(self._rows * self._blocks * 32 * 4)

@@ -279,6 +279,7 @@ void combine_rms_norm_quant_wait(const WaitPlan &wait, const float *x, const flo
 // Grow-only device scratch for the host-facing entry points, the counterpart
 // of g_aq/g_ad/g_out in crates/llamd-rocm/kernels/llamd.hip:1027-1051.
 void *scratch(int slot, size_t bytes);
+void *host_stage(int slot, size_t bytes);  // runtime.cu
 
 constexpr int kTileUnits = 32;
 constexpr int kTileBytes = 6720;       // 32 blocks x 210 B

@@ -203,6 +203,29 @@ void *scratch(int slot, size_t bytes) {
     return g_scratch[slot];
 }
 
+// Pinned, device-visible host memory of this library's own, kept and grown per slot (0: a call's inputs, 1: its results).
+// A host-facing call copies through it instead of handing the driver pageable memory: the driver's own staging of a
+// pageable copy, or the result copy's wait for it, cost several microseconds of a call that takes a dozen.
+void *host_stage(int slot, size_t bytes) {
+    static void *buf[2] = {nullptr, nullptr};
+    static size_t have[2] = {0, 0};
+    if (bytes <= have[slot] && buf[slot]) return buf[slot];
+    if (buf[slot]) {
+        cudaStreamSynchronize(stream());
+        cudaFreeHost(buf[slot]);
+        buf[slot] = nullptr;
+        have[slot] = 0;
+    }
+    const size_t want = bytes < 65536 ? 65536 : bytes;
+    cudaError_t e = cudaHostAlloc(&buf[slot], want, cudaHostAllocMapped);
+    if (e != cudaSuccess) {
+        set_error(e, "host staging");
+        return buf[slot] = nullptr;
+    }
+    have[slot] = want;
+    return buf[slot];
+}
+
 }  // namespace llamd
 
 using namespace llamd;
@@ -278,6 +301,18 @@ void *llamd_cuda_upload(const void *host, size_t bytes) {
 }
 void llamd_cuda_release(void *dev) {
     if (dev) cudaFree(dev);
+}
+
+void *llamd_cuda_host_alloc(size_t bytes) {
+    void *p = nullptr;
+    if (!stream() || cudaHostAlloc(&p, bytes ? bytes : 1, cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();  // (the caller has ordinary memory to fall back to)
+        return nullptr;
+    }
+    return p;
+}
+void llamd_cuda_host_free(void *p) {
+    if (p) cudaFreeHost(p);
 }
 
 void *llamd_fwd_alloc(size_t bytes) {

@@ -429,8 +429,8 @@ class CudaModel:
         return dict(zip(self.PHASES, ms.tolist()))
 
     def logits(self, nseq: int = 1) -> np.ndarray:
-        out = np.zeros((nseq, self.hp["n_vocab"]), dtype=np.float32)
-        if self._L.llamd_model_logits(self._h, out.ctypes.data_as(C.c_void_p), nseq) != 0:
+        out = backend.results.empty((nseq, self.hp["n_vocab"]))
+        if self._L.llamd_model_logits(self._h, out.ctypes.data, nseq) != 0:
             raise backend.Other("logits: " + self._err())
         return out
 
