@@ -344,7 +344,14 @@ static __device__ __noinline__ float chain_sum(const float *s, int n, float acc)
             i++;
         }
     }
-    for (int k = i * 16; k < n; k++) acc = __fadd_rn(acc, s[k]);
+    if (i * 16 < n) {  // the last terms all loaded at once; -0.0 in the missing places changes nothing, whatever acc is
+        float r[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) r[k] = i * 16 + k < n ? s[i * 16 + k] : -0.0f;
+#pragma unroll
+        for (int k = 0; k < 16; k++) acc = __fadd_rn(acc, r[k]);
+        for (int k = i * 16 + 16; k < n; k++) acc = __fadd_rn(acc, s[k]);  // (fewer than 32 terms in all)
+    }
     return acc;
 }
 #undef LLAMD_CHAIN_ADD16

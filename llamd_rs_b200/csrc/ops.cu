@@ -12,6 +12,7 @@
 
 #include "q6k_layout.cuh"
 #include "quant.cuh"
+#include "pos_sum.cuh"
 #include "route.cuh"
 
 namespace llamd {
@@ -153,6 +154,7 @@ __global__ void __launch_bounds__(128) norm_router_kernel(const float *__restric
     __shared__ float s_red[40 + kMaxUsed];
     __shared__ int s_redi[40 + kMaxUsed];
     __shared__ float s_scale;
+    __shared__ PosScratch s_pos;
     __shared__ bool s_last;
     pdl_trigger();
     const int seq = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -199,7 +201,8 @@ __global__ void __launch_bounds__(128) norm_router_kernel(const float *__restric
         for (int i = tid; i < k; i += 128) part = __fadd_rn(part, ssq[i]);
         scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(block_tree_sum(part, s_tree), (float)k), eps)));
     } else {
-        if (tid == 0) s_scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(chain_sum(ssq, k, 0.0f), (float)k), eps)));
+        const float sum = pos_chain_sum<128>(ssq, k, s_pos);
+        if (tid == 0) s_scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)k), eps)));
         __syncthreads();
         scale = s_scale;
     }
@@ -1008,6 +1011,7 @@ __global__ void __launch_bounds__(256) attn_out_kernel(const float *__restrict__
     extern __shared__ __align__(16) float sm[];
     __shared__ float s_red[16];
     __shared__ float s_tree[32];
+    __shared__ PosScratch s_pos;
     __shared__ float s_part[256];
     pdl_trigger();
     const bool clusters = !tail.counter && tail.qs;  // launched as clusters that quantize the result (below); uniform
@@ -1072,7 +1076,8 @@ __global__ void __launch_bounds__(256) attn_out_kernel(const float *__restrict__
         for (int t = tid; t < n_kv; t += blockDim.x) part = __fadd_rn(part, sl[t]);
         inv = __fdiv_rn(1.0f, block_tree_sum(part, s_tree));
     } else {
-        if (tid == 0) s_red[8] = __fdiv_rn(1.0f, chain_sum(sl, n_kv, 0.0f));
+        const float sum = pos_chain_sum<256>(sl, n_kv, s_pos);
+        if (tid == 0) s_red[8] = __fdiv_rn(1.0f, sum);
         __syncthreads();
         inv = s_red[8];
     }
@@ -1883,7 +1888,7 @@ static void attention_split_launch(const float *q, const void *kc, const void *v
     // (the library runs on one device per process: llamd_cuda_set_device is refused once the stream exists, so a
     // per-process record of the configured size is a per-device one)
     static size_t conf_a[2] = {0, 0}, conf_b[2] = {0, 0};
-    if (smem_a > 48 * 1024 && smem_a > conf_a[kv16]) {
+    if (smem_a > 40 * 1024 && smem_a > conf_a[kv16]) {
         const cudaError_t e = kv16 ? cudaFuncSetAttribute(attn_scores_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a)
                                    : cudaFuncSetAttribute(attn_scores_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a);
         if (e != cudaSuccess) {
@@ -1892,7 +1897,7 @@ static void attention_split_launch(const float *q, const void *kc, const void *v
         }
         conf_a[kv16] = smem_a;
     }
-    if (smem_b > 48 * 1024 && smem_b > conf_b[kv16]) {
+    if (smem_b > 40 * 1024 && smem_b > conf_b[kv16]) {
         const cudaError_t e = kv16 ? cudaFuncSetAttribute(attn_out_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b)
                                    : cudaFuncSetAttribute(attn_out_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b);
         if (e != cudaSuccess) {
@@ -1999,7 +2004,7 @@ static void attention_rope_launch(const float *q, const float *wq, const float *
         return;
     }
     static size_t conf_a[2] = {0, 0}, conf_b[2] = {0, 0};
-    if (smem_a > 48 * 1024 && smem_a > conf_a[kv16]) {
+    if (smem_a > 40 * 1024 && smem_a > conf_a[kv16]) {
         const cudaError_t e = kv16 ? cudaFuncSetAttribute(attn_rope_scores_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a)
                                    : cudaFuncSetAttribute(attn_rope_scores_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a);
         if (e != cudaSuccess) {
@@ -2008,7 +2013,7 @@ static void attention_rope_launch(const float *q, const float *wq, const float *
         }
         conf_a[kv16] = smem_a;
     }
-    if (smem_b > 48 * 1024 && smem_b > conf_b[kv16]) {
+    if (smem_b > 40 * 1024 && smem_b > conf_b[kv16]) {
         const cudaError_t e = kv16 ? cudaFuncSetAttribute(attn_out_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b)
                                    : cudaFuncSetAttribute(attn_out_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b);
         if (e != cudaSuccess) {

@@ -3,6 +3,7 @@
 // Everything here reproduces the reference's scalar f32 arithmetic in its
 // order (no FMA contraction, no reassociation), because each value ends up in
 // an int8 quant or a routing decision where the last bit is observable.
+#include "pos_sum.cuh"
 #include "quant.cuh"
 
 namespace llamd {
@@ -20,8 +21,8 @@ __global__ void __launch_bounds__(256) q8k_quantize_kernel(const float *__restri
 }
 
 // ---- rms_norm: crates/llamd-cpu/src/lib.rs:55-75, then `* w` --------------
-// The sum of squares is a left-to-right f32 chain in the reference; thread 0
-// walks it from shared memory while the other threads wait. One CTA per row.
+// The sum of squares is a left-to-right f32 chain in the reference: rms_norm_kernel
+// takes it with the whole CTA (pos_sum.cuh), the per-head norm below with one thread.
 // ssq holds the squares x[i]*x[i] (computed by all threads); n % 4 == 0.
 __device__ __forceinline__ float rms_scale_sequential(const float *__restrict__ ssq, int n, float eps) {
     const float sum = chain_sum(ssq, n, 0.0f);
@@ -44,6 +45,7 @@ __global__ void __launch_bounds__(256) rms_norm_kernel(const float *__restrict__
     float *ssq = sx + n;
     __shared__ float s_scale;
     __shared__ float s_tree[32];
+    __shared__ PosScratch s_pos;
     pdl_trigger();
     const int seq = blockIdx.x, tid = threadIdx.x;
     // Thread t owns the float4 groups t, t+256, ...: every global load of the
@@ -146,7 +148,8 @@ __global__ void __launch_bounds__(256) rms_norm_kernel(const float *__restrict__
         const float sum = block_tree_sum(part, s_tree);
         scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)n), eps)));
     } else {
-        if (tid == 0) s_scale = rms_scale_sequential(ssq, n, eps);
+        const float sum = pos_chain_sum<256>(ssq, n, s_pos);
+        if (tid == 0) s_scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)n), eps)));
         __syncthreads();
         scale = s_scale;
     }
@@ -269,8 +272,11 @@ template <typename... Args>
 static void launch_rms_norm(const char *what, int nseq, int n, Args... args) {
     if (n <= 2048)
         launch_kc(PDL_NORM, what, rms_norm_kernel<2>, dim3(nseq), dim3(256), 2 * n * sizeof(float), args...);
-    else
+    else {
+        static bool configured = false;  // (a row of 6144 is 48 KB of dynamic shared memory, to which the static part comes)
+        if (!configured) configured = cudaFuncSetAttribute(rms_norm_kernel<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024) == cudaSuccess;
         launch_kc(PDL_NORM, what, rms_norm_kernel<6>, dim3(nseq), dim3(256), 2 * n * sizeof(float), args...);
+    }
 }
 
 // `wait`: with expert parallelism the rows of `down` are stored by other GPUs; the launch first waits for their arrivals.

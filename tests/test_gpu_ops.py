@@ -42,6 +42,27 @@ def max_dev(a, b):
     return float(np.max(np.abs(a - b) / np.maximum(np.maximum(np.abs(a), np.abs(b)), 1.0)))
 
 
+@pytest.mark.parametrize("n", [768, 772, 1024, 2048, 4096, 4100, 6144])
+@pytest.mark.parametrize("kind", ["normal", "ties", "mixed", "tiny", "huge"])
+def test_sum_of_squares_in_runs_is_the_chain(ops, orc, n, kind):
+    """The CTA-wide ordered sum against the oracle's chain: from the longest sum that is walked as it is to several passes of
+    the scratch, with terms that tie, vanish against the sum, stay subnormal, or overflow."""
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((16, n))
+    if kind == "ties":
+        x = np.exp2(-rng.integers(0, 14, (16, n))) * rng.integers(1, 4, (16, n))
+    elif kind == "mixed":
+        x = x * np.exp2(rng.integers(-20, 20, (16, n))) * (rng.random((16, n)) < 0.7)
+    elif kind == "tiny":
+        x = x * 2.0 ** -70
+    elif kind == "huge":
+        x = x * 2.0 ** 62
+    x = x.astype(np.float32)
+    with np.errstate(all="ignore"):
+        want = orc.rms_norm(x, 1e-6)
+    assert bit_equal(ops.rms_norm_mul(x, np.ones(n, np.float32), 1e-6), want)
+
+
 def test_rms_norm_is_bit_exact(ops, orc, synth):
     x = synth.normal_f32(3 * 2048, 1, "rms").reshape(3, 2048)
     w = synth.normal_f32(2048, 1, "rms.w")
