@@ -100,6 +100,10 @@ int ep_bounded_sync();  // ep.cu: the stream synchronise of a pass that has NCCL
 
 namespace {
 
+// A pass of up to this many tokens or sequences makes its router logits and decisions in one launch, a chain per warp; beyond
+// it the tokens' chains share the operands (f32_gemm.cu) and the routing follows. us, one launch / two: 8 tokens 19.7 / 20.7,
+// 16: 23.3 / 20.7, 32: 32.7 / 20.7.
+constexpr int kRouterRowsMax = 10;
 constexpr int kArgmaxBlocks = 512;  // crates/llamd-runtime/src/device.rs ARGMAX_BLOCKS
 
 struct Buf {
@@ -540,8 +544,13 @@ void queue_token(Model &m, int nseq) {
             add_rms_norm_quant_flags(x, m.xb2.as<float>(), x, l.ffn_norm.as<float>(), m.xb.as<float>(), m.aq.as<int8_t>(), m.ad.as<float>(), E,
                                      hp.rms_eps, nseq, pf);
             mark(LLAMD_PH_FFN_NORM);
-            llamd_fwd_router_matvec(l.ffn_gate_inp.as<float>(), m.xb.as<float>(), E, hp.n_expert, nu, m.router_logits.as<float>(),
-                                    m.expert_ids.as<int32_t>(), m.expert_w.as<float>(), nullptr, m.router_counter.as<unsigned int>(), nseq);
+            if (nseq > kRouterRowsMax) {
+                llamd_fwd_matmul_f32_tokens(l.ffn_gate_inp.as<float>(), m.xb.as<float>(), m.router_logits.as<float>(), E, hp.n_expert, nseq);
+                llamd_fwd_router(m.router_logits.as<float>(), hp.n_expert, nu, m.expert_ids.as<int32_t>(), m.expert_w.as<float>(), nullptr, nseq);
+            } else {
+                llamd_fwd_router_matvec(l.ffn_gate_inp.as<float>(), m.xb.as<float>(), E, hp.n_expert, nu, m.router_logits.as<float>(),
+                                        m.expert_ids.as<int32_t>(), m.expert_w.as<float>(), nullptr, m.router_counter.as<unsigned int>(), nseq);
+            }
         }
         mark(LLAMD_PH_ROUTER);
         if (m.ep_world > 1) {
@@ -1384,7 +1393,6 @@ static int ep_tile_cap(const Model &m) {
 // sequences does: the experts as grouped matvecs with the slots in expert order, the dense matrices on the folded copies.
 // The tile GEMMs fold every weight for 16-token MMA tiles that a handful of tokens leaves nearly empty. The line is where
 // a batch of sequences changes over, which was measured there (matvec_batch_max).
-constexpr int kRouterRowsMax = 12;  // a small tile's router: a chain per warp up to here (16 us for 9 tokens, 36 for 32), tiles of chains beyond (37)
 static bool small_tile(const Model &m, int T, bool multi_seq) {
     return !multi_seq && m.ep_world == 1 && m.prefill_gemm == 1 && !m.prefold_ready && T <= m.matvec_batch_max && T * m.hp.n_expert_used <= 8192;
 }
@@ -1500,7 +1508,7 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
         }
         llamd_fwd_add_rms_norm_quant(x, p.xb2.as<float>(), x, l.ffn_norm.as<float>(), p.xb.as<float>(), p.aq.as<int8_t>(), p.ad.as<float>(),
                                      E, hp.rms_eps, T);
-        if (m.prefill_attn && T > (small ? kRouterRowsMax : 1)) {
+        if (m.prefill_attn && T > kRouterRowsMax) {
             llamd_fwd_matmul_f32_tokens(l.ffn_gate_inp.as<float>(), p.xb.as<float>(), p.logits.as<float>(), E, ne, T);
             llamd_fwd_router(p.logits.as<float>(), ne, nu, p.ids.as<int32_t>(), p.w.as<float>(), nullptr, T);
         } else {

@@ -207,7 +207,7 @@ def test_router_matvec_logits_are_bit_exact(ops, orc, synth):
     assert bit_equal(ops.matvec_f32(w, x), np.stack([orc.matvec_dequant(orc.F32, w, x[s], k, ne) for s in range(3)]))
 
 
-@pytest.mark.parametrize("rows,k,ntok", [(128, 2048, 37), (8, 256, 1), (50, 100, 19), (33, 68, 16)])
+@pytest.mark.parametrize("rows,k,ntok", [(128, 2048, 37), (8, 256, 1), (50, 100, 19), (33, 68, 16), (33, 772, 129), (128, 640, 593)])
 def test_matmul_f32_tokens(ops, orc, synth, rows, k, ntok):
     """The tile form of the f32 matvec: every output is the same -0.0-seeded left-to-right sum."""
     w = synth.normal_f32(rows * k, 5, "mm.w", rows, k, std=0.02).reshape(rows, k)
