@@ -1001,6 +1001,8 @@ __global__ void __launch_bounds__(256) attn_rope_scores_kernel(const float *__re
 }
 
 constexpr int kPvTile = 256;  // positions per V tile
+constexpr int kPvRows = 224, kPvStride = 228;  // positions per tile of products (7 warps), and a column's stride: 16-byte aligned, neighbours in different bank groups
+static_assert(32 * kPvStride <= 32 * kPvTile, "a tile of products fits where a tile of 32 columns does");
 
 // With a TailPlan the CTA that finishes a sequence last also writes the Q8_K form of that sequence's whole
 // attention output (what llamd_fwd_quantize would do one launch later).
@@ -1056,7 +1058,19 @@ __global__ void __launch_bounds__(256) attn_out_kernel(const float *__restrict__
             asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char *>(vb + (size_t)t * kv_dim)));
         pdl_wait();
     }
-    fetch(0);  // V tile 0 travels while the softmax runs
+    // The weighted values in their usual form: seven warps make the products, thread = position, transposed in shared
+    // memory, and warp 0 adds them, lane = column, at the latency of an add. (One warp that loaded, multiplied and added took
+    // 20 cycles per position: 58 us of a launch at position 4001, @@D@@ now, 11.8 -> @@E@@ at 512.)
+    const bool wide = !(fast & 4) && cols == 32;
+    float4 row_v[8];
+    auto fetch_row = [&](int ti) {
+        const int t = ti * kPvRows + tid - 32;
+        const bool on = tid >= 32 && t < n_kv;
+#pragma unroll
+        for (int q = 0; q < 8; q++) row_v[q] = on ? KvIo<KVT>::ld4(vb + (size_t)t * kv_dim + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    if (wide) fetch_row(0);  // V tile 0 travels while the softmax runs
+    else fetch(0);
     float lmax = -INFINITY;
     for (int t = tid; t < n_kv; t += blockDim.x) {
         const float l = sc[t];
@@ -1082,7 +1096,35 @@ __global__ void __launch_bounds__(256) attn_out_kernel(const float *__restrict__
         inv = s_red[8];
     }
     float acc = 0.0f;
-    for (int ti = 0; ti < n_tiles; ti++) {
+    if (wide) {
+        auto store_row = [&](int ti) {
+            const int t = ti * kPvRows + tid - 32;
+            if (tid < 32 || t >= n_kv) return;
+            const float w = __fmul_rn(sl[t], inv);
+            float *dst = tile + (ti & 1) * 32 * kPvStride + tid - 32;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                dst[(4 * q + 0) * kPvStride] = __fmul_rn(w, row_v[q].x);
+                dst[(4 * q + 1) * kPvStride] = __fmul_rn(w, row_v[q].y);
+                dst[(4 * q + 2) * kPvStride] = __fmul_rn(w, row_v[q].z);
+                dst[(4 * q + 3) * kPvStride] = __fmul_rn(w, row_v[q].w);
+            }
+        };
+        const int n = (n_kv + kPvRows - 1) / kPvRows;
+        store_row(0);
+        fetch_row(1);
+        __syncthreads();
+        for (int ti = 0; ti < n; ti++) {
+            if (tid >= 32) {
+                if (ti + 1 < n) store_row(ti + 1);
+                fetch_row(ti + 2);
+            } else {
+                acc = chain_sum(tile + ((ti & 1) * 32 + tid) * kPvStride, min(kPvRows, n_kv - ti * kPvRows), acc);
+            }
+            __syncthreads();
+        }
+    }
+    for (int ti = 0; ti < n_tiles && !wide; ti++) {
         float *cur = tile + (ti & 1) * kPvTile * cols;
         stash(cur);
         __syncthreads();
@@ -1197,12 +1239,15 @@ __global__ void __launch_bounds__(256) attn_out_kernel(const float *__restrict__
     }
 }
 
-// ---- the same two launches for a batch of sequences -----------------------------------------------------------------
-// With several sequences per pass the grids above are many small CTAs in which a quarter (scores) or an eighth (values) of
-// the threads walk chains while the rest wait, several waves of them. Here a CTA serves ALL the query heads that share
-// a kv head: the cached tile is read once for them instead of once each, every thread has a chain to walk, and the grid is
-// one wave. The same operations on the same values in the same order per (head, position) and per (head, column), hence
-// the same bits as the per-head kernels.
+// ---- the same two launches with the query heads of a kv head together -------------------------------------------------
+// In the grids above a quarter (scores) of the threads walk chains while the rest wait, and every cached row is read once
+// per query head. Here a CTA serves ALL the query heads that share a kv head: the cached tile is read once for them, and
+// every thread walks the chains of two heads for one position, whose key it reads once for both. The position split is
+// the launch's (gridDim.y: enough CTAs for about two per SM where the context has the tiles for them); a CTA whose first
+// tile lies beyond the sequence leaves at once. The same operations on the same values in the same order per (head,
+// position) and per (head, column), hence the same bits as the per-head kernels. Scores, us: one sequence at position 4001
+// 29.0 per head / @@A@@ here, at 512 9.9 / @@B@@; 128 sequences of 30 to 264 positions @@C@@ (82.4 with eight CTAs each and one chain
+// per thread).
 constexpr int kGqaMax = 8;  // query heads per kv head these kernels hold
 
 template <class KVT>
@@ -1213,7 +1258,7 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
                                                                    const int32_t *__restrict__ meta, int max_kv, int kv_stride,
                                                                    const float *__restrict__ rope_tab, float eps, int flags) {
     extern __shared__ __align__(16) float sm[];
-    const int stride = hd + 1, half = hd / 2, ratio = n_head / n_head_kv;
+    const int stride = hd + 4, half = hd / 2, ratio = n_head / n_head_kv;
     float *sq = sm;                               // [ratio][hd] the roped queries
     float *tile = sq + ratio * hd;                // [2][kAttTile][stride]
     float *s_raw = tile + 2 * kAttTile * stride;  // [ratio + 1][hd] raw queries, raw key
@@ -1222,11 +1267,12 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
     pdl_trigger();
     const bool early = (flags & kPassEarlyLoads) != 0;  // (see attn_rope_scores_kernel)
     if (!early) pdl_wait();
-    const int kvh = blockIdx.x, c = blockIdx.y, seq = blockIdx.z, tid = threadIdx.x;
+    const int kvh = blockIdx.x, c = blockIdx.y, split = gridDim.y, seq = blockIdx.z, tid = threadIdx.x;
     const int pos = meta[2 * seq + 1], n_kv = pos + 1;
+    if (c * kAttTile >= n_kv) return;
     const int kv_dim = n_head_kv * hd, h0 = kvh * ratio;
     const int ti_pos = pos / kAttTile;
-    const bool need_k = (ti_pos % kSplitT) == c;  // this CTA scores the new key, and stores the K and V rows of the position
+    const bool need_k = (ti_pos % split) == c;  // this CTA scores the new key, and stores the K and V rows of the position
     KVT *krow = kc + ((size_t)seq * kv_stride + pos) * kv_dim + (size_t)kvh * hd;
     KVT *vrow = vc + ((size_t)seq * kv_stride + pos) * kv_dim + (size_t)kvh * hd;
     const KVT *kb = kc + (size_t)seq * kv_stride * kv_dim + (size_t)kvh * hd;
@@ -1250,8 +1296,7 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
             const int idx = tid + j * 256;
             const int r = idx / hd4, cc = idx - r * hd4;
             if (idx < per_tile4 && ti * kAttTile + r != pos) {  // (the token's own row is written below, by other threads)
-                float *p = dst + r * stride + 4 * cc;
-                p[0] = reg[j].x; p[1] = reg[j].y; p[2] = reg[j].z; p[3] = reg[j].w;
+                *reinterpret_cast<float4 *>(dst + r * stride + 4 * cc) = reg[j];
             }
         }
     };
@@ -1259,7 +1304,7 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
     if (early) {
         const int lpr = hd * (int)sizeof(KVT) / 128;
         if (lpr > 0)
-            for (int ti = c + kSplitT; ti < n_tiles; ti += kSplitT)
+            for (int ti = c + split; ti < n_tiles; ti += split)
                 for (int i = tid; i < kAttTile * lpr; i += blockDim.x) {
                     const int r = i / lpr, l = i - r * lpr, t = ti * kAttTile + r;
                     if (t < pos) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char *>(kb + (size_t)t * kv_dim) + l * 128));
@@ -1269,18 +1314,17 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
     // ---- QK-norm (crates/llamd-runtime/src/layer.rs:62-79) and RoPE (crates/llamd-cpu/src/lib.rs:158-209) of the kv head's
     // query heads (adjacent in q_raw) and, where needed, of the new key
     const int n_vec = ratio + (need_k ? 1 : 0);
-    for (int i = tid; i < ratio * hd; i += blockDim.x) s_raw[i] = q_raw[((size_t)seq * n_head + h0) * hd + i];
-    if (need_k)
-        for (int i = tid; i < hd; i += blockDim.x) s_raw[ratio * hd + i] = k_raw[((size_t)seq * n_head_kv + kvh) * hd + i];
+    for (int i = tid; i < n_vec * hd; i += blockDim.x) {
+        const float x = i < ratio * hd ? q_raw[((size_t)seq * n_head + h0) * hd + i] : k_raw[((size_t)seq * n_head_kv + kvh) * hd + i - ratio * hd];
+        s_raw[i] = x;
+        tile[i] = __fmul_rn(x, x);  // (no cached tile is in place yet)
+    }
     __syncthreads();
     {
         // vector v's sum of squares is walked in order by lane v / 8 of warp v % 8: the chains run side by side
         const int warp = tid >> 5, lane = tid & 31, v = lane * 8 + warp;
         if (lane < 2 && v < n_vec && (v < ratio ? wq != nullptr : wk != nullptr)) {
-            const float *sx = s_raw + v * hd;
-            float sum = 0.0f;
-#pragma unroll 8
-            for (int t = 0; t < hd; t++) sum = __fadd_rn(sum, __fmul_rn(sx[t], sx[t]));
+            const float sum = chain_sum(tile + v * hd, hd, 0.0f);
             s_scale[v] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)hd), eps)));
         }
     }
@@ -1318,36 +1362,33 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
     __syncthreads();
     // ---- scores: (query head, position) pairs of the tile over the threads ----
     int buf = 0;
-    for (int ti = c; ti < n_tiles; ti += kSplitT, buf ^= 1) {
+    for (int ti = c; ti < n_tiles; ti += split, buf ^= 1) {
         float *cur = tile + buf * kAttTile * stride;
         stash(cur, ti);
         if (ti == ti_pos)
             for (int i = tid; i < hd; i += blockDim.x) cur[(pos - ti * kAttTile) * stride + i] = sk[i];
         __syncthreads();
-        if (ti + kSplitT < n_tiles) fetch(ti + kSplitT);
-        for (int idx = tid; idx < ratio * kAttTile; idx += blockDim.x) {
-            const int j = idx / kAttTile, r = idx - j * kAttTile;
+        if (ti + split < n_tiles) fetch(ti + split);
+        for (int idx = tid; idx < (ratio / 2) * kAttTile; idx += blockDim.x) {  // (ratio is kGqaMax)
+            const int j = 2 * (idx / kAttTile), r = idx % kAttTile;
             const int t = ti * kAttTile + r;
             if (t >= n_kv) continue;
-            const float *kr = cur + r * stride, *q = sq + j * hd;
-            float dot = 0.0f;
-            if ((hd & 15) == 0) {
-                float pa[16], pb[16];
-#pragma unroll
-                for (int i = 0; i < 16; i++) pa[i] = __fmul_rn(q[i], kr[i]);
-                for (int d0 = 0; d0 < hd; d0 += 16) {
-                    const int dn = (d0 + 16 < hd) ? d0 + 16 : d0;
-#pragma unroll
-                    for (int i = 0; i < 16; i++) pb[i] = __fmul_rn(q[dn + i], kr[dn + i]);
-#pragma unroll
-                    for (int i = 0; i < 16; i++) dot = __fadd_rn(dot, pa[i]);
-#pragma unroll
-                    for (int i = 0; i < 16; i++) pa[i] = pb[i];
-                }
-            } else {
-                for (int d = 0; d < hd; d++) dot = __fadd_rn(dot, __fmul_rn(q[d], kr[d]));
+            const float4 *kr = reinterpret_cast<const float4 *>(cur + r * stride), *qa = reinterpret_cast<const float4 *>(sq + j * hd), *qb = qa + hd4;
+            float da = 0.0f, db = 0.0f;
+            float4 k0 = kr[0], a0 = qa[0], b0 = qb[0];
+#pragma unroll 4
+            for (int d = 0; d < hd4; d++) {
+                const int dn = min(d + 1, hd4 - 1);
+                const float4 k1 = kr[dn], a1 = qa[dn], b1 = qb[dn];
+                da = __fadd_rn(da, __fmul_rn(a0.x, k0.x)), db = __fadd_rn(db, __fmul_rn(b0.x, k0.x));
+                da = __fadd_rn(da, __fmul_rn(a0.y, k0.y)), db = __fadd_rn(db, __fmul_rn(b0.y, k0.y));
+                da = __fadd_rn(da, __fmul_rn(a0.z, k0.z)), db = __fadd_rn(db, __fmul_rn(b0.z, k0.z));
+                da = __fadd_rn(da, __fmul_rn(a0.w, k0.w)), db = __fadd_rn(db, __fmul_rn(b0.w, k0.w));
+                k0 = k1, a0 = a1, b0 = b1;
             }
-            scores[((size_t)seq * n_head + h0 + j) * max_kv + t] = __fmul_rn(dot, scale);
+            float *out = scores + ((size_t)seq * n_head + h0 + j) * max_kv + t;
+            out[0] = __fmul_rn(da, scale);
+            out[max_kv] = __fmul_rn(db, scale);
         }
     }
 }
@@ -2022,15 +2063,15 @@ static void attention_rope_launch(const float *q, const float *wq, const float *
         }
         conf_b[kv16] = smem_b;
     }
-    // A batch of sequences: one CTA per (kv head, ...) for all the query heads that share it (the decode pass asks for it)
+    // One CTA per (kv head, ...) for all the query heads that share it (the decode pass asks for it)
     const int ratio = n_head / n_head_kv, cap = (max_kv + 3) & ~3;
-    const size_t smem_ga = (size_t)(ratio * hd + 2 * kAttTile * (hd + 1) + (ratio + 1) * hd + hd) * sizeof(float);
+    const size_t smem_ga = (size_t)(ratio * hd + 2 * kAttTile * (hd + 4) + (ratio + 1) * hd + hd) * sizeof(float);
     const size_t smem_gb = (size_t)((size_t)ratio * cap + 2 * kPvTile * (hd / kSplit)) * sizeof(float);
-    // (measured, 48 layers at position ~520: 8 sequences 814.7 -> 1044.8 tok/s, 4 sequences 641.8 -> 717.2, 2 sequences 456.2 -> 439.7,
-    // so from four sequences on)
-    if ((flags & kPassAttnGqa) && !(flags & 4) && nseq >= 4 && ratio == kGqaMax && hd / kSplit == 32 && smem_ga <= 200 * 1024 &&
-        smem_gb <= 200 * 1024) {
-        static size_t conf_ga[2] = {0, 0}, conf_gb[2] = {0, 0};
+    // (values, measured, 48 layers at position ~520: 8 sequences 814.7 -> 1044.8 tok/s, 4 sequences 641.8 -> 717.2, 2 sequences
+    // 456.2 -> 439.7, so from four sequences on; the scores from one on)
+    const bool gqa = (flags & kPassAttnGqa) && !(flags & 4) && ratio == kGqaMax && hd / kSplit == 32 && smem_ga <= 200 * 1024;
+    if (gqa) {
+        static size_t conf_ga[2] = {0, 0};
         if (smem_ga > conf_ga[kv16]) {
             const cudaError_t e = kv16 ? cudaFuncSetAttribute(attn_rope_scores_gqa_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_ga)
                                        : cudaFuncSetAttribute(attn_rope_scores_gqa_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_ga);
@@ -2040,6 +2081,26 @@ static void attention_rope_launch(const float *q, const float *wq, const float *
             }
             conf_ga[kv16] = smem_ga;
         }
+        const int tiles = (max_kv + kAttTile - 1) / kAttTile;
+        int split = 2 * 148 / (n_head_kv * nseq);
+        split = split < kSplitT ? kSplitT : split;
+        split = split > tiles ? tiles : split;
+        const dim3 grid(n_head_kv, split, nseq);
+        if (kv16)
+            launch_kc(PDL_ATTN, "attn_rope_scores_gqa", attn_rope_scores_gqa_kernel<__half>, grid, dim3(256), smem_ga, q, wq, k, wk, v, (__half *)kc,
+                      (__half *)vc, scores, n_head, n_head_kv, hd, meta, max_kv, max_kv, rope_tab, eps, flags);
+        else
+            launch_kc(PDL_ATTN, "attn_rope_scores_gqa", attn_rope_scores_gqa_kernel<float>, grid, dim3(256), smem_ga, q, wq, k, wk, v, (float *)kc,
+                      (float *)vc, scores, n_head, n_head_kv, hd, meta, max_kv, max_kv, rope_tab, eps, flags);
+    } else if (kv16) {
+        launch_kc(PDL_ATTN, "attn_rope_scores", attn_rope_scores_kernel<__half>, dim3(n_head, kSplitT, nseq), dim3(256), smem_a, q, wq, k, wk, v,
+                  (__half *)kc, (__half *)vc, scores, n_head, n_head_kv, hd, meta, max_kv, max_kv, rope_tab, eps, flags);
+    } else {
+        launch_kc(PDL_ATTN, "attn_rope_scores", attn_rope_scores_kernel<float>, dim3(n_head, kSplitT, nseq), dim3(256), smem_a, q, wq, k, wk, v,
+                  (float *)kc, (float *)vc, scores, n_head, n_head_kv, hd, meta, max_kv, max_kv, rope_tab, eps, flags);
+    }
+    if (gqa && nseq >= 4 && smem_gb <= 200 * 1024) {
+        static size_t conf_gb[2] = {0, 0};
         if (smem_gb > conf_gb[kv16]) {
             const cudaError_t e = kv16 ? cudaFuncSetAttribute(attn_out_gqa_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_gb)
                                        : cudaFuncSetAttribute(attn_out_gqa_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_gb);
@@ -2049,38 +2110,26 @@ static void attention_rope_launch(const float *q, const float *wq, const float *
             }
             conf_gb[kv16] = smem_gb;
         }
-        if (kv16) {
-            launch_kc(PDL_ATTN, "attn_rope_scores_gqa", attn_rope_scores_gqa_kernel<__half>, dim3(n_head_kv, kSplitT, nseq), dim3(256), smem_ga, q, wq, k,
-                      wk, v, (__half *)kc, (__half *)vc, scores, n_head, n_head_kv, hd, meta, max_kv, max_kv, rope_tab, eps, flags);
+        if (kv16)
             launch_kc(PDL_ATTN, "attn_out_gqa", attn_out_gqa_kernel<__half>, dim3(n_head_kv, kSplit, nseq), dim3(256), smem_gb, (const float *)scores,
                       (const __half *)vc, out, n_head, n_head_kv, hd, meta, max_kv, max_kv, flags);
-        } else {
-            launch_kc(PDL_ATTN, "attn_rope_scores_gqa", attn_rope_scores_gqa_kernel<float>, dim3(n_head_kv, kSplitT, nseq), dim3(256), smem_ga, q, wq, k,
-                      wk, v, (float *)kc, (float *)vc, scores, n_head, n_head_kv, hd, meta, max_kv, max_kv, rope_tab, eps, flags);
+        else
             launch_kc(PDL_ATTN, "attn_out_gqa", attn_out_gqa_kernel<float>, dim3(n_head_kv, kSplit, nseq), dim3(256), smem_gb, (const float *)scores,
                       (const float *)vc, out, n_head, n_head_kv, hd, meta, max_kv, max_kv, flags);
-        }
         if (qs && qd) llamd_fwd_quantize(out, qs, qd, nseq * (n_head * hd / 256));
         return;
     }
     const bool clusters = qs && qd && attn_out_cluster_ok(n_head, hd);
-    if (kv16) {
-        launch_kc(PDL_ATTN, "attn_rope_scores", attn_rope_scores_kernel<__half>, dim3(n_head, kSplitT, nseq), dim3(256), smem_a, q, wq, k, wk, v,
-                  (__half *)kc, (__half *)vc, scores, n_head, n_head_kv, hd, meta, max_kv, max_kv, rope_tab, eps, flags);
-        if (clusters)
-            attn_out_cluster_launch<__half>(smem_b, scores, (const __half *)vc, out, n_head, n_head_kv, hd, meta, max_kv, nseq, qs, qd, flags);
-        else
-            launch_kc(PDL_ATTN, "attn_out", attn_out_kernel<__half>, dim3(n_head, kSplit, nseq), dim3(256), smem_b, (const float *)scores,
-                      (const __half *)vc, out, n_head, n_head_kv, hd, meta, 0, max_kv, max_kv, TailPlan{}, flags);
-    } else {
-        launch_kc(PDL_ATTN, "attn_rope_scores", attn_rope_scores_kernel<float>, dim3(n_head, kSplitT, nseq), dim3(256), smem_a, q, wq, k, wk, v,
-                  (float *)kc, (float *)vc, scores, n_head, n_head_kv, hd, meta, max_kv, max_kv, rope_tab, eps, flags);
-        if (clusters)
-            attn_out_cluster_launch<float>(smem_b, scores, (const float *)vc, out, n_head, n_head_kv, hd, meta, max_kv, nseq, qs, qd, flags);
-        else
-            launch_kc(PDL_ATTN, "attn_out", attn_out_kernel<float>, dim3(n_head, kSplit, nseq), dim3(256), smem_b, (const float *)scores,
-                      (const float *)vc, out, n_head, n_head_kv, hd, meta, 0, max_kv, max_kv, TailPlan{}, flags);
-    }
+    if (clusters && kv16)
+        attn_out_cluster_launch<__half>(smem_b, scores, (const __half *)vc, out, n_head, n_head_kv, hd, meta, max_kv, nseq, qs, qd, flags);
+    else if (clusters)
+        attn_out_cluster_launch<float>(smem_b, scores, (const float *)vc, out, n_head, n_head_kv, hd, meta, max_kv, nseq, qs, qd, flags);
+    else if (kv16)
+        launch_kc(PDL_ATTN, "attn_out", attn_out_kernel<__half>, dim3(n_head, kSplit, nseq), dim3(256), smem_b, (const float *)scores, (const __half *)vc, out,
+                  n_head, n_head_kv, hd, meta, 0, max_kv, max_kv, TailPlan{}, flags);
+    else
+        launch_kc(PDL_ATTN, "attn_out", attn_out_kernel<float>, dim3(n_head, kSplit, nseq), dim3(256), smem_b, (const float *)scores, (const float *)vc, out,
+                  n_head, n_head_kv, hd, meta, 0, max_kv, max_kv, TailPlan{}, flags);
     if (qs && qd && !clusters) llamd_fwd_quantize(out, qs, qd, nseq * (n_head * hd / 256));
 }
 } // extern "C"
