@@ -511,16 +511,23 @@ template <class T>
 struct KvIo;
 template <>
 struct KvIo<float> {
+    // four elements as they lie in the cache: loaded ahead and widened where they are used (a widening right behind the
+    // load would wait for it)
+    typedef float4 Raw;
+    static __device__ __forceinline__ Raw raw4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
+    static __device__ __forceinline__ float4 wide4(const Raw &r) { return r; }
     static __device__ __forceinline__ float4 ld4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
     static __device__ __forceinline__ void st(float *p, float v) { *p = v; }
 };
 template <>
 struct KvIo<__half> {
-    static __device__ __forceinline__ float4 ld4(const __half *p) {
-        const uint2 u = __ldg(reinterpret_cast<const uint2 *>(p));
-        const __half2 a = *reinterpret_cast<const __half2 *>(&u.x), b = *reinterpret_cast<const __half2 *>(&u.y);
+    typedef uint2 Raw;
+    static __device__ __forceinline__ Raw raw4(const __half *p) { return __ldg(reinterpret_cast<const uint2 *>(p)); }
+    static __device__ __forceinline__ float4 wide4(const Raw &r) {
+        const __half2 a = *reinterpret_cast<const __half2 *>(&r.x), b = *reinterpret_cast<const __half2 *>(&r.y);
         return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
     }
+    static __device__ __forceinline__ float4 ld4(const __half *p) { return wide4(raw4(p)); }
     static __device__ __forceinline__ void st(__half *p, float v) { *p = __float2half_rn(v); }
 };
 
@@ -772,14 +779,15 @@ __global__ void __launch_bounds__(256) attn_scores_kernel(const float *__restric
     const int hd4 = hd / 4, per_tile4 = kAttTile * hd4;
     const int n_tiles = (n_kv + kAttTile - 1) / kAttTile;
     constexpr int kMaxLd = 8;
-    float4 reg[kMaxLd];
+    typename KvIo<KVT>::Raw reg[kMaxLd];
     auto fetch = [&](int ti) {
 #pragma unroll
         for (int j = 0; j < kMaxLd; j++) {
             const int idx = tid + j * 256;
             const int r = idx / hd4, cc = idx - r * hd4;
             const int t = ti * kAttTile + r;
-            reg[j] = (idx < per_tile4 && t < n_kv) ? KvIo<KVT>::ld4(kb + (size_t)t * kv_dim + 4 * cc) : make_float4(0.f, 0.f, 0.f, 0.f);
+            reg[j] = typename KvIo<KVT>::Raw{};
+            if (idx < per_tile4 && t < n_kv) reg[j] = KvIo<KVT>::raw4(kb + (size_t)t * kv_dim + 4 * cc);
         }
     };
     auto stash = [&](float *dst) {
@@ -789,7 +797,8 @@ __global__ void __launch_bounds__(256) attn_scores_kernel(const float *__restric
             if (idx < per_tile4) {
                 const int r = idx / hd4, cc = idx - r * hd4;
                 float *p = dst + r * stride + 4 * cc;
-                p[0] = reg[j].x; p[1] = reg[j].y; p[2] = reg[j].z; p[3] = reg[j].w;
+                const float4 x = KvIo<KVT>::wide4(reg[j]);
+                p[0] = x.x; p[1] = x.y; p[2] = x.z; p[3] = x.w;
             }
         }
     };
@@ -866,7 +875,7 @@ __global__ void __launch_bounds__(256) attn_rope_scores_kernel(const float *__re
     const int hd4 = hd / 4, per_tile4 = kAttTile * hd4;
     const int n_tiles = (n_kv + kAttTile - 1) / kAttTile;
     constexpr int kMaxLd = 8;
-    float4 reg[kMaxLd];
+    typename KvIo<KVT>::Raw reg[kMaxLd];
     auto fetch = [&](int ti) {
 #pragma unroll
         for (int j = 0; j < kMaxLd; j++) {
@@ -874,7 +883,8 @@ __global__ void __launch_bounds__(256) attn_rope_scores_kernel(const float *__re
             const int r = idx / hd4, cc = idx - r * hd4;
             const int t = ti * kAttTile + r;
             // (the token's own row is not in the cache yet: it comes from shared memory below)
-            reg[j] = (idx < per_tile4 && t < pos) ? KvIo<KVT>::ld4(kb + (size_t)t * kv_dim + 4 * cc) : make_float4(0.f, 0.f, 0.f, 0.f);
+            reg[j] = typename KvIo<KVT>::Raw{};
+            if (idx < per_tile4 && t < pos) reg[j] = KvIo<KVT>::raw4(kb + (size_t)t * kv_dim + 4 * cc);
         }
     };
     auto stash = [&](float *dst, int ti) {
@@ -884,7 +894,8 @@ __global__ void __launch_bounds__(256) attn_rope_scores_kernel(const float *__re
             const int r = idx / hd4, cc = idx - r * hd4;
             if (idx < per_tile4 && ti * kAttTile + r != pos) {  // (the token's own row is written below, by other threads)
                 float *p = dst + r * stride + 4 * cc;
-                p[0] = reg[j].x; p[1] = reg[j].y; p[2] = reg[j].z; p[3] = reg[j].w;
+                const float4 x = KvIo<KVT>::wide4(reg[j]);
+                p[0] = x.x; p[1] = x.y; p[2] = x.z; p[3] = x.w;
             }
         }
     };
@@ -1001,8 +1012,24 @@ __global__ void __launch_bounds__(256) attn_rope_scores_kernel(const float *__re
 }
 
 constexpr int kPvTile = 256;  // positions per V tile
-constexpr int kPvRows = 224, kPvStride = 228;  // positions per tile of products (7 warps), and a column's stride: 16-byte aligned, neighbours in different bank groups
-static_assert(32 * kPvStride <= 32 * kPvTile, "a tile of products fits where a tile of 32 columns does");
+constexpr int kPvRows = 224;  // positions per tile of products: 8 per thread of seven warps, a multiple of 32
+static_assert(kPvRows <= kPvTile && kPvRows % 32 == 0, "a tile of products fits where a tile of 32 columns does");
+// chain_sum over n32 runs of 32 floats whose 16-byte pieces are permuted by XOR with `key` (bits 4 to 6 of the byte offset)
+static __device__ __noinline__ float chain_sum_keyed(const float *s, int n32, uint32_t key, float acc) {
+    const uint32_t p = (uint32_t)__cvta_generic_to_shared(s);
+    auto at = [&](int run, uint32_t piece) { return chain_lds(p + 128u * (uint32_t)run + ((16u * piece) ^ key)); };
+#define ADD4(q) acc = __fadd_rn(acc, q.x), acc = __fadd_rn(acc, q.y), acc = __fadd_rn(acc, q.z), acc = __fadd_rn(acc, q.w)
+    float4 a0 = at(0, 0), a1 = at(0, 1), a2 = at(0, 2), a3 = at(0, 3), b0 = at(0, 4), b1 = at(0, 5), b2 = at(0, 6), b3 = at(0, 7);
+    for (int i = 0; i < n32; i++) {
+        const int next = min(i + 1, n32 - 1);  // (past the end: a harmless re-load)
+        ADD4(a0), ADD4(a1), ADD4(a2), ADD4(a3);
+        a0 = at(next, 0), a1 = at(next, 1), a2 = at(next, 2), a3 = at(next, 3);
+        ADD4(b0), ADD4(b1), ADD4(b2), ADD4(b3);
+        b0 = at(next, 4), b1 = at(next, 5), b2 = at(next, 6), b3 = at(next, 7);
+    }
+#undef ADD4
+    return acc;
+}
 
 // With a TailPlan the CTA that finishes a sequence last also writes the Q8_K form of that sequence's whole
 // attention output (what llamd_fwd_quantize would do one launch later).
@@ -1034,21 +1061,22 @@ __global__ void __launch_bounds__(256) attn_out_kernel(const float *__restrict__
     const int per_tile4 = kPvTile * cols4;
     const int n_tiles = (n_kv + kPvTile - 1) / kPvTile;
     constexpr int kMaxLd = 8;  // 256 rows x 32 cols / 4 / 256
-    float4 reg[kMaxLd];
+    typename KvIo<KVT>::Raw reg[kMaxLd];
     auto fetch = [&](int ti) {
 #pragma unroll
         for (int j = 0; j < kMaxLd; j++) {
             const int idx = tid + j * 256;
             const int r = idx / cols4, cc = idx - r * cols4;
             const int t = ti * kPvTile + r;
-            reg[j] = (idx < per_tile4 && t < n_kv) ? KvIo<KVT>::ld4(vb + (size_t)t * kv_dim + 4 * cc) : make_float4(0.f, 0.f, 0.f, 0.f);
+            reg[j] = typename KvIo<KVT>::Raw{};
+            if (idx < per_tile4 && t < n_kv) reg[j] = KvIo<KVT>::raw4(vb + (size_t)t * kv_dim + 4 * cc);
         }
     };
     auto stash = [&](float *dst) {
 #pragma unroll
         for (int j = 0; j < kMaxLd; j++) {
             const int idx = tid + j * 256;
-            if (idx < per_tile4) reinterpret_cast<float4 *>(dst)[idx] = reg[j];
+            if (idx < per_tile4) reinterpret_cast<float4 *>(dst)[idx] = KvIo<KVT>::wide4(reg[j]);
         }
     };
     if (early) {
@@ -1058,31 +1086,42 @@ __global__ void __launch_bounds__(256) attn_out_kernel(const float *__restrict__
             asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char *>(vb + (size_t)t * kv_dim)));
         pdl_wait();
     }
-    // The weighted values in their usual form: seven warps make the products, thread = position, transposed in shared
-    // memory, and warp 0 adds them, lane = column, at the latency of an add. (One warp that loaded, multiplied and added took
-    // 20 cycles per position: 58 us of a launch at position 4001, @@D@@ now, 11.8 -> @@E@@ at 512.)
+    // The weighted values in their usual form: seven warps make the products, transposed in shared memory, and warp 0 adds
+    // them, lane = column, at the latency of an add. (One warp that loaded, multiplied and added took 20 cycles per position:
+    // 58 us of a launch at position 4001, 36.7 now; the rest is the softmax, of which every column slice
+    // makes its own.) Eight lanes read a row's 32 columns; position t of column col
+    // lies at t ^ 4 * key(col) of its column, where key makes both the lanes that store (four positions, columns 4 apart)
+    // and those that read (eight neighbouring columns) meet eight different bank groups.
     const bool wide = !(fast & 4) && cols == 32;
-    float4 row_v[8];
+    const int pv_cc = tid & 7, pv_r = (tid - 32) >> 3;
     auto fetch_row = [&](int ti) {
-        const int t = ti * kPvRows + tid - 32;
-        const bool on = tid >= 32 && t < n_kv;
 #pragma unroll
-        for (int q = 0; q < 8; q++) row_v[q] = on ? KvIo<KVT>::ld4(vb + (size_t)t * kv_dim + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int u = 0; u < 8; u++) {
+            const int t = ti * kPvRows + pv_r + 28 * u;
+            reg[u] = typename KvIo<KVT>::Raw{};
+            if (tid >= 32 && t < n_kv) reg[u] = KvIo<KVT>::raw4(vb + (size_t)t * kv_dim + 4 * pv_cc);
+        }
     };
     if (wide) fetch_row(0);  // V tile 0 travels while the softmax runs
     else fetch(0);
     float lmax = -INFINITY;
-    for (int t = tid; t < n_kv; t += blockDim.x) {
-        const float l = sc[t];
-        sl[t] = l;
-        lmax = fmaxf(lmax, l);
+    for (int t0 = 0; t0 < n_kv; t0 += 8 * 256) {  // (eight loads in flight: one after the other they were a round trip to L2 each)
+        float l[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) l[u] = t0 + u * 256 + tid < n_kv ? sc[t0 + u * 256 + tid] : -INFINITY;
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            if (t0 + u * 256 + tid < n_kv) sl[t0 + u * 256 + tid] = l[u];
+            lmax = fmaxf(lmax, l[u]);
+        }
     }
     for (int off = 16; off > 0; off >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, off));
     if ((tid & 31) == 0) s_red[tid >> 5] = lmax;
     __syncthreads();
     lmax = s_red[0];
     for (int w = 1; w < 8; w++) lmax = fmaxf(lmax, s_red[w]);
-    for (int t = tid; t < n_kv; t += blockDim.x) sl[t] = ref_expf(__fsub_rn(sl[t], lmax));
+#pragma unroll 4
+    for (int t = tid; t < n_kv; t += 256) sl[t] = ref_expf(__fsub_rn(sl[t], lmax));
     __syncthreads();
     float inv;
     if (fast & 4) {  // the `fast` arithmetic: the softmax sum as a reduction tree
@@ -1098,18 +1137,21 @@ __global__ void __launch_bounds__(256) attn_out_kernel(const float *__restrict__
     float acc = 0.0f;
     if (wide) {
         auto store_row = [&](int ti) {
-            const int t = ti * kPvRows + tid - 32;
-            if (tid < 32 || t >= n_kv) return;
-            const float w = __fmul_rn(sl[t], inv);
-            float *dst = tile + (ti & 1) * 32 * kPvStride + tid - 32;
+            if (tid < 32) return;
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
-                dst[(4 * q + 0) * kPvStride] = __fmul_rn(w, row_v[q].x);
-                dst[(4 * q + 1) * kPvStride] = __fmul_rn(w, row_v[q].y);
-                dst[(4 * q + 2) * kPvStride] = __fmul_rn(w, row_v[q].z);
-                dst[(4 * q + 3) * kPvStride] = __fmul_rn(w, row_v[q].w);
+            for (int u = 0; u < 8; u++) {
+                const int r = pv_r + 28 * u, t = ti * kPvRows + r;
+                const bool on = t < n_kv;  // (-0.0 behind the last position: adding it changes nothing)
+                const float w = on ? __fmul_rn(sl[t], inv) : 0.0f;
+                const float4 x = KvIo<KVT>::wide4(reg[u]);
+                float *dst = tile + ((ti & 1) * 32 + 4 * pv_cc) * kPvRows;
+                dst[0 * kPvRows + (r ^ (4 * (pv_cc ^ 0)))] = on ? __fmul_rn(w, x.x) : -0.0f;
+                dst[1 * kPvRows + (r ^ (4 * (pv_cc ^ 2)))] = on ? __fmul_rn(w, x.y) : -0.0f;
+                dst[2 * kPvRows + (r ^ (4 * (pv_cc ^ 4)))] = on ? __fmul_rn(w, x.z) : -0.0f;
+                dst[3 * kPvRows + (r ^ (4 * (pv_cc ^ 6)))] = on ? __fmul_rn(w, x.w) : -0.0f;
             }
         };
+        const uint32_t key = 16u * (uint32_t)(((tid >> 2) ^ (2 * (tid & 3))) & 7);
         const int n = (n_kv + kPvRows - 1) / kPvRows;
         store_row(0);
         fetch_row(1);
@@ -1119,7 +1161,7 @@ __global__ void __launch_bounds__(256) attn_out_kernel(const float *__restrict__
                 if (ti + 1 < n) store_row(ti + 1);
                 fetch_row(ti + 2);
             } else {
-                acc = chain_sum(tile + ((ti & 1) * 32 + tid) * kPvStride, min(kPvRows, n_kv - ti * kPvRows), acc);
+                acc = chain_sum_keyed(tile + ((ti & 1) * 32 + tid) * kPvRows, (min(kPvRows, n_kv - ti * kPvRows) + 31) >> 5, key, acc);
             }
             __syncthreads();
         }
@@ -1246,7 +1288,7 @@ __global__ void __launch_bounds__(256) attn_out_kernel(const float *__restrict__
 // the launch's (gridDim.y: enough CTAs for about two per SM where the context has the tiles for them); a CTA whose first
 // tile lies beyond the sequence leaves at once. The same operations on the same values in the same order per (head,
 // position) and per (head, column), hence the same bits as the per-head kernels. Scores, us: one sequence at position 4001
-// 29.0 per head / @@A@@ here, at 512 9.9 / @@B@@; 128 sequences of 30 to 264 positions @@C@@ (82.4 with eight CTAs each and one chain
+// 29.0 per head / 11.8 here, at 512 9.9 / 10.3; 128 sequences of 30 to 264 positions 34.2 (82.4 with eight CTAs each and one chain
 // per thread).
 constexpr int kGqaMax = 8;  // query heads per kv head these kernels hold
 
@@ -1280,14 +1322,15 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
     const int hd4 = hd / 4, per_tile4 = kAttTile * hd4;
     const int n_tiles = (n_kv + kAttTile - 1) / kAttTile;
     constexpr int kMaxLd = 8;
-    float4 reg[kMaxLd];
+    typename KvIo<KVT>::Raw reg[kMaxLd];
     auto fetch = [&](int ti) {
 #pragma unroll
         for (int j = 0; j < kMaxLd; j++) {
             const int idx = tid + j * 256;
             const int r = idx / hd4, cc = idx - r * hd4;
             const int t = ti * kAttTile + r;
-            reg[j] = (idx < per_tile4 && t < pos) ? KvIo<KVT>::ld4(kb + (size_t)t * kv_dim + 4 * cc) : make_float4(0.f, 0.f, 0.f, 0.f);
+            reg[j] = typename KvIo<KVT>::Raw{};
+            if (idx < per_tile4 && t < pos) reg[j] = KvIo<KVT>::raw4(kb + (size_t)t * kv_dim + 4 * cc);
         }
     };
     auto stash = [&](float *dst, int ti) {
@@ -1296,7 +1339,7 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
             const int idx = tid + j * 256;
             const int r = idx / hd4, cc = idx - r * hd4;
             if (idx < per_tile4 && ti * kAttTile + r != pos) {  // (the token's own row is written below, by other threads)
-                *reinterpret_cast<float4 *>(dst + r * stride + 4 * cc) = reg[j];
+                *reinterpret_cast<float4 *>(dst + r * stride + 4 * cc) = KvIo<KVT>::wide4(reg[j]);
             }
         }
     };
@@ -1414,21 +1457,22 @@ __global__ void __launch_bounds__(256) attn_out_gqa_kernel(const float *__restri
     const int per_tile4 = kPvTile * cols4;
     const int n_tiles = (n_kv + kPvTile - 1) / kPvTile;
     constexpr int kMaxLd = 8;
-    float4 reg[kMaxLd];
+    typename KvIo<KVT>::Raw reg[kMaxLd];
     auto fetch = [&](int ti) {
 #pragma unroll
         for (int j = 0; j < kMaxLd; j++) {
             const int idx = tid + j * 256;
             const int r = idx / cols4, cc = idx - r * cols4;
             const int t = ti * kPvTile + r;
-            reg[j] = (idx < per_tile4 && t < n_kv) ? KvIo<KVT>::ld4(vb + (size_t)t * kv_dim + 4 * cc) : make_float4(0.f, 0.f, 0.f, 0.f);
+            reg[j] = typename KvIo<KVT>::Raw{};
+            if (idx < per_tile4 && t < n_kv) reg[j] = KvIo<KVT>::raw4(vb + (size_t)t * kv_dim + 4 * cc);
         }
     };
     auto stash = [&](float *dst) {
 #pragma unroll
         for (int j = 0; j < kMaxLd; j++) {
             const int idx = tid + j * 256;
-            if (idx < per_tile4) reinterpret_cast<float4 *>(dst)[idx] = reg[j];
+            if (idx < per_tile4) reinterpret_cast<float4 *>(dst)[idx] = KvIo<KVT>::wide4(reg[j]);
         }
     };
     if (early) {
@@ -1442,10 +1486,15 @@ __global__ void __launch_bounds__(256) attn_out_gqa_kernel(const float *__restri
         const float *sc = scores + ((size_t)seq * n_head + h0 + j) * max_kv;
         float *slj = sl + (size_t)j * cap;
         float lmax = -INFINITY;
-        for (int t = lane; t < n_kv; t += 32) {
-            const float l = sc[t];
-            slj[t] = l;
-            lmax = fmaxf(lmax, l);
+        for (int t0 = 0; t0 < n_kv; t0 += 8 * 32) {
+            float l[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) l[u] = t0 + u * 32 + lane < n_kv ? sc[t0 + u * 32 + lane] : -INFINITY;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                if (t0 + u * 32 + lane < n_kv) slj[t0 + u * 32 + lane] = l[u];
+                lmax = fmaxf(lmax, l[u]);
+            }
         }
         for (int off = 16; off > 0; off >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, off));
         for (int t = lane; t < n_kv; t += 32) slj[t] = ref_expf(__fsub_rn(slj[t], lmax));
