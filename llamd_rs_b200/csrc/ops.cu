@@ -1120,7 +1120,7 @@ __global__ void __launch_bounds__(256) attn_out_kernel(const float *__restrict__
     __syncthreads();
     lmax = s_red[0];
     for (int w = 1; w < 8; w++) lmax = fmaxf(lmax, s_red[w]);
-#pragma unroll 4
+#pragma unroll 1
     for (int t = tid; t < n_kv; t += 256) sl[t] = ref_expf(__fsub_rn(sl[t], lmax));
     __syncthreads();
     float inv;
