@@ -32,6 +32,8 @@ namespace llamd {
 constexpr int kGemmRows = 16;
 constexpr int kTokStride = 68;  // words per staged token row: 16-byte aligned, conflict-free fragment reads
 constexpr int kChunkTiles = 8;  // token tiles per dense work item
+constexpr int kGroupTiles = 4;  // token tiles that the four warps of the folded kernel take together
+constexpr int kTeamWords = 4 * kGroupTiles * 8 * 16;  // their staged activations: 4 warps x 32 tokens x one residue pair's 16 words
 
 struct GemmParams {
     const uint8_t *w[3];  // tiled Q6_K; up to three matrices that share the activations
@@ -55,7 +57,33 @@ struct GemmParams {
     // each exactly what fold_row_tile leaves in shared memory (A fragments, then the 16 x nb block scales)
     const uint8_t *folded[3];
     long long fold_tile_bytes;
+    unsigned long long one;  // 1.0f twice (see gemm_add2)
 };
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 gemm_pack(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 gemm_unpack(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 gemm_mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 gemm_fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// s + t, rounded once, as an fma with 1.0 in a value the compiler cannot see: a packed multiply feeding a packed add is
+// contracted into one fma, which rounds once where the reference rounds twice.
+__device__ __forceinline__ f32x2 gemm_add2(f32x2 s, f32x2 t, f32x2 one) { return gemm_fma2(t, one, s); }
 
 // Ask L2 for the tiles that hold the 16 x nb blocks starting at block `unit0` (a hint: nothing waits on it).
 __device__ __forceinline__ void prefetch_row_tile(const uint8_t *w, size_t unit0, int live_rows, int nb) {
@@ -65,10 +93,11 @@ __device__ __forceinline__ void prefetch_row_tile(const uint8_t *w, size_t unit0
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
+template <int C = 0>  // what the sums land on
 __device__ __forceinline__ void mma_s8(int (&c)[4], const uint4 &a, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                  : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
-                 : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1), "r"(0));
+                 : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1), "r"(C));
 }
 
 // Natural-order Q8_K quants -> residue-major words (t32_element order), one thread per word.
@@ -382,6 +411,165 @@ __global__ void __launch_bounds__(128, HOIST ? 3 : 5) q6k_gemm_grouped_kernel(co
     mma_token_tiles<1>(p, j, row0, rows, first, count, 0, (count + 7) >> 3, s_frag, s_d, s_b, warp, 4, lane);
 }
 
+// ---- few tokens against one matrix kept folded (the dense matrices and the head of a batch): four warps, a residue pair each
+// mma_token_tiles gives a warp whole token tiles, so 8 tokens keep one warp of a CTA at work, and every warp reads every
+// fragment (1 KB of shared memory a residue). Here the four warps of a CTA take up to 32 tokens together: each reads only
+// its own residues' fragments, once for all of them. The tail is packed, two tokens per instruction: the MMAs accumulate onto
+// 1.5 * 2^23, so that hi and lo come out as floats with that offset, and 64*hi + lo is exact because |aux| < 2^24. The image's
+// copy starts before the dependency wait. Bound by the image (2 bytes per weight); us, a warp per tile / this: QKV of 8
+// sequences 10.3 / 5.7, output projection 14.3 / 6.7, head 142 / 127; 32 sequences 13.5 / 10.7, 14.8 / 9.4, 196 / 180. For many tokens the
+// kernels above are quicker (2048: 906 us against 1024, gate and up), which spend less on staging and exchanging.
+// Warp rp owns residues 2rp and 2rp + 1. Per block it copies its 16 words of every token into its own part of
+// s_b (coalesced 16-byte loads; the next block's wait in registers meanwhile), 16-byte pieces swizzled by the token so that
+// the MMA's fragment reads meet 32 banks. At the end the eight residues' sums meet in s_b and are added in order.
+template <int NT>
+__device__ __forceinline__ void mma_group(const GemmParams &p, int j, int row0, int rows, int first, int count, int n0, const uint4 *s_frag,
+                                          const float *s_d, uint32_t *s_b, float *s_ad, int tid) {
+    const int nb = p.nb, rp = tid >> 5, lane = tid & 31;
+    const int g4 = lane >> 2, q4 = lane & 3;
+    auto pair_of = [&](int tok) { return first + min(n0 + tok, count - 1); };
+    for (int i = tid; i < NT * 8 * nb; i += 128) {  // the group's activation scales, [block][token]
+        const int tok = i / nb, b = i - tok * nb, pr = pair_of(tok);
+        s_ad[b * (8 * kGroupTiles) + tok] = __ldg(p.ad + (long long)(p.act_map ? p.act_map[pr] : pr) * nb + b);
+    }
+    const uint4 *src[NT];
+    uint4 st[NT];
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+        const int pr = pair_of(t * 8 + g4);
+        const long long it = p.act_map ? p.act_map[pr] : pr;
+        src[t] = reinterpret_cast<const uint4 *>(p.aq_rm + (size_t)it * nb * 64) + rp * 4 + q4;
+        st[t] = __ldg(src[t]);
+    }
+    uint32_t *mine = s_b + rp * (kTeamWords / 4);
+    const int key = (g4 >> 1) & 3;
+    uint32_t *put = mine + g4 * 16 + 4 * (q4 ^ key);
+    f32x2 sum[NT][2][2];
+#pragma unroll
+    for (int t = 0; t < NT; t++) sum[t][0][0] = sum[t][0][1] = sum[t][1][0] = sum[t][1][1] = 0ull;
+    const f32x2 one = p.one, off = 0xCB400000CB400000ull, c64 = 0x4280000042800000ull;  // -1.5 * 2^23 and 64.0, twice
+    __syncthreads();
+    for (int b = 0; b < nb; b++) {
+#pragma unroll
+        for (int t = 0; t < NT; t++) *reinterpret_cast<uint4 *>(put + t * 128) = st[t];
+        __syncwarp();
+        if (b + 1 < nb) {
+#pragma unroll
+            for (int t = 0; t < NT; t++) st[t] = __ldg(src[t] + (size_t)(b + 1) * 16);
+        }
+        const float d0 = s_d[g4 * nb + b], d1 = s_d[(g4 + 8) * nb + b];
+        f32x2 dsc[NT][2];
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+            const f32x2 a = *reinterpret_cast<const f32x2 *>(s_ad + b * (8 * kGroupTiles) + t * 8 + 2 * q4);
+            dsc[t][0] = gemm_mul2(gemm_pack(d0, d0), a);
+            dsc[t][1] = gemm_mul2(gemm_pack(d1, d1), a);
+        }
+        const uint4 *fr = s_frag + ((size_t)(b * 8 + 2 * rp) * 2) * 32 + (lane ^ (lane >> 3) ^ (b & 7));
+#pragma unroll
+        for (int rr = 0; rr < 2; rr++) {
+            const uint4 ah = fr[(rr * 2 + 0) * 32], al = fr[(rr * 2 + 1) * 32];
+            const uint32_t *bt = mine + g4 * 16 + q4;
+            const int o0 = 4 * ((2 * rr) ^ key), o1 = 4 * ((2 * rr + 1) ^ key);
+#pragma unroll
+            for (int t = 0; t < NT; t++) {
+                const uint32_t b0w = bt[t * 128 + o0], b1w = bt[t * 128 + o1];
+                int ch[4], cl[4];
+                mma_s8<0x4B400000>(ch, ah, b0w, b1w);
+                mma_s8<0x4B400000>(cl, al, b0w, b1w);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {  // rows g4 and g4 + 8, tokens 2 q4 and 2 q4 + 1
+                    const f32x2 hi = gemm_add2(gemm_pack(__int_as_float(ch[2 * h]), __int_as_float(ch[2 * h + 1])), off, one);
+                    const f32x2 lo = gemm_add2(gemm_pack(__int_as_float(cl[2 * h]), __int_as_float(cl[2 * h + 1])), off, one);
+                    sum[t][rr][h] = gemm_add2(sum[t][rr][h], gemm_mul2(dsc[t][h], gemm_fma2(hi, c64, lo)), one);
+                }
+            }
+        }
+        __syncwarp();
+    }
+    // y = ((((((s0+s1)+s2)+s3)+s4)+s5)+s6)+s7, two tiles at a time: [7 terms][16 token places][16 rows]
+    float *s_x = reinterpret_cast<float *>(s_b);
+#pragma unroll
+    for (int t0 = 0; t0 < NT; t0 += 2) {
+        __syncthreads();
+#pragma unroll
+        for (int t = t0; t < t0 + 2 && t < NT; t++) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                float *x = s_x + ((t - t0) * 8 + q4) * 16 + g4 + 8 * h;  // (token 2 q4 + e has place q4 + 4 e)
+                if (rp == 0) {
+                    const float2 v = gemm_unpack(gemm_add2(sum[t][0][h], sum[t][1][h], one));
+                    x[0] = v.x, x[4 * 16] = v.y;
+                } else {
+                    const float2 v = gemm_unpack(sum[t][0][h]), u = gemm_unpack(sum[t][1][h]);
+                    x += (2 * rp - 1) * 256;
+                    x[0] = v.x, x[4 * 16] = v.y, x[256] = u.x, x[256 + 4 * 16] = u.y;
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int t = t0; t < t0 + 2 && t < NT; t++) {
+            const int row = tid & 15, place = tid >> 4;
+            const float *x = s_x + ((t - t0) * 8 + place) * 16 + row;
+            float y = x[0];
+#pragma unroll
+            for (int r = 1; r < 7; r++) y = __fadd_rn(y, x[r * 256]);
+            const int n = n0 + t * 8 + 2 * (place & 3) + (place >> 2);
+            if (n < count && row0 + row < rows) {
+                long long o = p.out_map ? p.out_map[first + n] : first + n;
+                float *out = p.out[j];
+                if (p.out_tab) {  // the rows of a pair go to the GPU the pair's token lives on (plain peer stores)
+                    out = p.out_tab[o / p.out_div];
+                    o %= p.out_div;
+                }
+                out[o * rows + row0 + row] = y;
+            }
+        }
+    }
+}
+
+template <int NT>
+__device__ __forceinline__ void folded_tiles(const GemmParams &p, int j, int row0, int t, const uint4 *s_frag, const float *s_d, uint32_t *s_b, float *s_ad, int tid) {
+    mma_group<NT>(p, j, row0, p.rows[j], 0, p.n_tokens, t * 8, s_frag, s_d, s_b, s_ad, tid);
+}
+static_assert(7 * 256 * 4 <= kTeamWords * 4, "the residues' sums of two tiles fit where the activations were");
+
+__host__ __device__ inline size_t folded_smem_bytes(int nb) {
+    return (size_t)nb * 8 * 2 * 32 * 16 + (size_t)kGemmRows * nb * 4 + (size_t)kTeamWords * 4 + (size_t)nb * 8 * kGroupTiles * 4;
+}
+// grid (row tiles of all jobs), one group of n_tokens
+__global__ void __launch_bounds__(128, 3) q6k_gemm_folded_kernel(const GemmParams p) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int nb = p.nb, tid = threadIdx.x;
+    uint4 *s_frag = reinterpret_cast<uint4 *>(smem);
+    float *s_d = reinterpret_cast<float *>(smem + (size_t)nb * 8 * 2 * 32 * 16);
+    uint32_t *s_b = reinterpret_cast<uint32_t *>(s_d + kGemmRows * nb);
+    float *s_ad = reinterpret_cast<float *>(s_b + kTeamWords);
+    const int j = job_of_tile(p, blockIdx.x), rt = (int)blockIdx.x - p.tile_begin[j];
+    const uint8_t *src = p.folded[j] + (size_t)rt * (size_t)p.fold_tile_bytes;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem);
+    const int n16 = (int)(p.fold_tile_bytes >> 4);
+    for (int i = tid; i < n16; i += 128)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (uint32_t)i), "l"(src + 16 * (size_t)i) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    pdl_trigger();
+    pdl_wait();
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    // (the first barrier of a group stands between everyone's pieces of the image and their first use)
+    const int tiles = (p.n_tokens + 7) >> 3, groups = (tiles + kGroupTiles - 1) / kGroupTiles;
+    for (int g = 0, t = 0; g < groups; g++) {  // as few equal groups as kGroupTiles allows
+        const int nt = (tiles - t + groups - g - 1) / (groups - g);
+        switch (nt) {
+        case 1: folded_tiles<1>(p, j, rt * kGemmRows, t, s_frag, s_d, s_b, s_ad, tid); break;
+        case 2: folded_tiles<2>(p, j, rt * kGemmRows, t, s_frag, s_d, s_b, s_ad, tid); break;
+        case 3: folded_tiles<3>(p, j, rt * kGemmRows, t, s_frag, s_d, s_b, s_ad, tid); break;
+        default: folded_tiles<4>(p, j, rt * kGemmRows, t, s_frag, s_d, s_b, s_ad, tid); break;
+        }
+        t += nt;
+    }
+}
+
 // Folds every (expert, row tile) of one matrix once and keeps the image: grid (row tiles, experts).
 __global__ void __launch_bounds__(128) q6k_prefold_kernel(const uint8_t *__restrict__ w, uint8_t *__restrict__ dst, int rows, int nb,
                                                           long long expert_units, long long tile_bytes) {
@@ -439,7 +627,7 @@ __global__ void __launch_bounds__(256, 2) q6k_gemm_dense_kernel(const GemmParams
 using namespace llamd;
 
 static void gemm_launch(GemmParams &p, int n_groups) {
-    const int threads = n_groups > 1 || p.gstart || p.folded[0] ? 128 : 256;  // (a folded matrix: the kernel that copies tiles)
+    const int threads = n_groups > 1 || p.gstart ? 128 : 256;
     const size_t smem = gemm_smem_bytes(p.nb, threads);
     if (p.nb < 1 || smem > 220 * 1024) {
         set_error_msg("q6k gemm: blocks per row must be 1..24");
@@ -580,7 +768,7 @@ void llamd::expert_gemm_scatter(const void *wa, const void *wb, const int32_t *g
 }
 
 // Up to three matrices kept folded (expert_prefold with one "expert" each) against ntok activations: out_i[ntok][rows_i].
-// The grouped kernel with a single group: a CTA copies its row tile's image and multiplies; 2 bytes per weight whatever
+// A CTA copies its row tile's image and multiplies (q6k_gemm_folded_kernel); 2 bytes per weight whatever
 // ntok is, where the matvec repeats its integer work per sequence. Same results as llamd_fwd_gemm_tokens.
 void llamd::gemm_tokens_folded3(const void *f0, const void *f1, const void *f2, const void *aq_rm, const float *ad, float *o0, float *o1,
                                 float *o2, int blocks, int rows0, int rows1, int rows2, int ntok) {
@@ -595,7 +783,23 @@ void llamd::gemm_tokens_folded3(const void *f0, const void *f1, const void *f2, 
     p.aq_rm = (const uint32_t *)aq_rm;
     p.ad = ad;
     p.n_tokens = ntok;
-    gemm_launch(p, 1);
+    p.one = 0x3F8000003F800000ull;
+    const size_t smem = folded_smem_bytes(blocks);
+    if (blocks < 1 || smem > 220 * 1024) {
+        set_error_msg("q6k gemm: blocks per row must be 1..24");
+        return;
+    }
+    static size_t configured = 0;
+    if (smem > 48 * 1024 && smem > configured) {
+        cudaFuncSetAttribute(q6k_gemm_folded_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        configured = smem;
+    }
+    int tiles = 0;
+    for (int i = 0; i < p.njobs; i++) {
+        p.tile_begin[i] = tiles;
+        tiles += (p.rows[i] + kGemmRows - 1) / kGemmRows;
+    }
+    launch_kc(PDL_MATVEC, "q6k_gemm_folded", q6k_gemm_folded_kernel, dim3(tiles), dim3(128), smem, p);
 }
 void llamd::gemm_tokens_folded(const void *folded, const void *aq_rm, const float *ad, float *out, int blocks, int rows, int ntok) {
     gemm_tokens_folded3(folded, nullptr, nullptr, aq_rm, ad, out, nullptr, nullptr, blocks, rows, 0, 0, ntok);

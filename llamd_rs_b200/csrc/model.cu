@@ -1389,6 +1389,11 @@ static int ep_tile_cap(const Model &m) {
     return cap < 1 ? 1 : cap;
 }
 
+// Up to kFoldedMax tokens the dense matrices run on the folded copies whatever the experts do, us folded / folding on the
+// way: QKV of 64 tokens 18.0 / 31, 128: 33 / 40, 160: 40 / 47, 250: 62 / 60.
+constexpr int kFoldedMax = 192;
+static bool folded_tile(const Model &m, int T) { return m.ep_world == 1 && m.prefill_gemm == 1 && T <= kFoldedMax; }
+
 // A small tile of one sequence (a draft, a short turn, a prompt's rest) runs its matrices as a decode pass over as many
 // sequences does: the experts as grouped matvecs with the slots in expert order, the dense matrices on the folded copies.
 // The tile GEMMs fold every weight for 16-token MMA tiles that a handful of tokens leaves nearly empty. The line is where
@@ -1410,8 +1415,8 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
     float *x = p.x.as<float>();
     const int max_items = T * nu / 8 + ne;
     const bool small = small_tile(m, T, multi_seq);
-    const bool folded = small && m.dense_gemm && T >= m.dense_gemm && m.dense_fold_ready;
-    // up to three dense matrices of a small tile against the activations in p.aq / p.ad
+    const bool folded = folded_tile(m, T) && m.dense_gemm && T >= m.dense_gemm && m.dense_fold_ready;
+    // up to three dense matrices of a small or folded tile against the activations in p.aq / p.ad
     auto small_dense = [&](const Buf &f0, const Buf &f1, const Buf &f2, const Buf &w0, const Buf &w1, const Buf &w2, const Buf &o0, const Buf &o1,
                            const Buf &o2, int blocks, int rows0, int rows12) {
         if (folded) {
@@ -1436,7 +1441,7 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
                                              p.aq.as<int8_t>(), p.ad.as<float>(), E, hp.rms_eps, T);
         const bool ep = m.ep_world > 1;  // sharded experts run on the integer GEMM; so then do the dense matmuls
         const bool gemm = m.prefill_gemm != 0 || ep, tc = m.prefill_gemm == 2 && !ep;
-        if (small) {
+        if (small || folded) {
             small_dense(l.q_fold, l.k_fold, l.v_fold, l.attn_q, l.attn_k, l.attn_v, p.q, p.k, p.v, eb, qd, kvd);
         } else if (tc) {
             llamd_fwd_act_f16_rm(p.aq.as<int8_t>(), p.ad.as<float>(), p.aq_rm.p, (size_t)T * eb);
@@ -1493,7 +1498,7 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
             }
         }
         llamd_fwd_quantize(p.attn.as<float>(), p.aq.as<int8_t>(), p.ad.as<float>(), T * (qd / 256));
-        if (small) {
+        if (small || folded) {
             small_dense(l.o_fold, none, none, l.attn_out, none, none, p.xb2, none, none, qd / 256, E, 0);
         } else if (tc) {
             llamd_fwd_act_f16_rm(p.aq.as<int8_t>(), p.ad.as<float>(), p.aq_rm.p, (size_t)T * (qd / 256));
@@ -1593,11 +1598,12 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
         // the head for every token of the tile: combine + output norm + Q8_K per row, lm_head as a GEMM, greedy pick per row
         llamd_fwd_combine_rms_norm_quant(x, p.down.as<float>(), p.w.as<float>(), nu, x, m.output_norm.as<float>(), nullptr,
                                          p.aq.as<int8_t>(), p.ad.as<float>(), E, hp.rms_eps, T);
-        if (small && !(m.head_gemm && T >= m.head_gemm && m.head_fold_ready)) {
+        const bool head_folded = folded_tile(m, T) && m.head_gemm && T >= m.head_gemm && m.head_fold_ready;
+        if (small && !head_folded) {
             matvec_batch(MatvecPlans{}, m.output.p ? m.output.p : m.tok_embd.p, p.aq.as<int8_t>(), p.ad.as<float>(), logits_out, eb, hp.n_vocab, T);
         } else {
             llamd_fwd_q8k_residue_major(p.aq.as<int8_t>(), p.aq_rm.p, (size_t)T * eb);
-            if (small)
+            if (head_folded)
                 gemm_tokens_folded(m.head_fold.p, p.aq_rm.p, p.ad.as<float>(), logits_out, eb, hp.n_vocab, T);
             else
                 llamd_fwd_gemm_tokens(m.output.p ? m.output.p : m.tok_embd.p, nullptr, nullptr, p.aq_rm.p, p.ad.as<float>(), logits_out, nullptr,
@@ -1660,7 +1666,7 @@ int llamd_model_prefill(llamd_model *h, const int32_t *tokens, int n_tokens, int
             set_error(cudaGetLastError(), "prefill meta H2D");
             return -1;
         }
-        if (small_tile(*m, T, false) && !ensure_folded(*m, T, false)) return -1;
+        if (folded_tile(*m, T) && !ensure_folded(*m, T, false)) return -1;
         queue_prefill_tile(*m, T, base_pos + t0 + T, t0 + T >= n_tokens);
     }
     if (cudaMemcpyAsync(m->h_out, m->out_token.p, 4, cudaMemcpyDeviceToHost, stream()) != cudaSuccess) return -1;
@@ -1722,7 +1728,7 @@ int llamd_model_verify(llamd_model *h, const int32_t *tokens, int n_tokens, int 
             set_error(cudaGetLastError(), "verify meta H2D");
             return -1;
         }
-        if (small_tile(*m, T, false) && !ensure_folded(*m, T)) return -1;
+        if (folded_tile(*m, T) && !ensure_folded(*m, T)) return -1;
         queue_prefill_tile(*m, T, base_pos + t0 + T, true, false, true, m->pf.logits_all.as<float>());
         if (cudaMemcpyAsync(m->pf.h_out_tokens, m->pf.out_tokens.p, (size_t)T * 4, cudaMemcpyDeviceToHost, stream()) != cudaSuccess) return -1;
         if (llamd_fwd_sync() != 0) return -1;
@@ -1759,6 +1765,7 @@ static int run_wide_batch(Model &m, const int32_t *tokens, const int32_t *positi
         return -1;
     }
     if (!prefill_alloc(m, nseq) || !prefill_alloc_all_logits(m, false)) return -1;
+    if (folded_tile(m, nseq) && !ensure_folded(m, nseq)) return -1;
     if (llamd_fwd_sync() != 0) return -1;
     int n_kv_max = 0;
     for (int s = 0; s < nseq; s++) {
