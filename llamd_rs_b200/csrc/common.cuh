@@ -213,13 +213,15 @@ struct MatvecPlans {
     // L2 instead of reading them from HBM again. Produced by slot_order_launch; must be complete when the ids are.
     const int32_t *slot_order;
 };
-// order[] = the slots 0..n_slots-1 sorted by (ids[slot], slot). One small launch.
-void slot_order_launch(const int32_t *ids, int n_slots, int32_t *order);
+// order[] = the slots 0..n_slots-1 sorted by ids[slot]. One small launch.
+void slot_order_launch(const int32_t *ids, int n_slots, int n_expert, int32_t *order);
 
 // The decode pass's attention (QK-norm, RoPE and the K/V store inside the scores launch) leaving its result quantized as well.
 void attention_rope_quant(const float *q, const float *wq, const float *k, const float *wk, const float *v, void *kc, void *vc, float *out,
                           float *scores, int n_head, int n_head_kv, int hd, const int32_t *meta, const float *rope_tab, float eps, int max_kv,
                           int nseq, bool kv16, int8_t *qs, float *d, int flags);
+bool attention_small_tile(const float *q, const void *kc, const void *vc, float *out, float *scores, int n_head, int n_head_kv, int hd,
+                          const int32_t *meta, int n_kv_max, int ntok, bool kv16);
 void attention_meta_flags(const float *q, const void *kc, const void *vc, float *out, float *scores, int n_head, int n_head_kv, int hd,
                           const int32_t *meta, int max_kv, int nseq, bool kv16, int flags);
 void norm_router_flags(const float *w, const float *x, const float *residual, float *x_out, const float *w_norm, float *xn_out, int8_t *qs,

@@ -598,7 +598,7 @@ void queue_token(Model &m, int nseq) {
         // launch; measured worth it from 8 sequences on)
         const int32_t *order = nullptr;
         if (m.sort_slots && nseq >= m.sort_slots) {
-            slot_order_launch(m.expert_ids.as<int32_t>(), nseq * nu, m.slot_order.as<int32_t>());
+            slot_order_launch(m.expert_ids.as<int32_t>(), nseq * nu, hp.n_expert, m.slot_order.as<int32_t>());
             order = m.slot_order.as<int32_t>();
         }
         gu.slot_order = order;
@@ -1399,7 +1399,7 @@ static bool folded_tile(const Model &m, int T) { return m.ep_world == 1 && m.pre
 // The tile GEMMs fold every weight for 16-token MMA tiles that a handful of tokens leaves nearly empty. The line is where
 // a batch of sequences changes over, which was measured there (matvec_batch_max).
 static bool small_tile(const Model &m, int T, bool multi_seq) {
-    return !multi_seq && m.ep_world == 1 && m.prefill_gemm == 1 && !m.prefold_ready && T <= m.matvec_batch_max && T * m.hp.n_expert_used <= 8192;
+    return !multi_seq && m.ep_world == 1 && m.prefill_gemm == 1 && !m.prefold_ready && T <= m.matvec_batch_max;
 }
 
 // multi_seq: the T tokens belong to T different sequences, token i with its own cache (sequence i) and position:
@@ -1478,14 +1478,17 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
             // f32 view that the tiled kernels read as they read an f32 cache
             llamd_fwd_qk_norm_rope_store_tile_kv16(p.q.as<float>(), wqn, p.k.as<float>(), wkn, p.v.as<float>(), l.kc.p, l.vc.p, H, HKV, hd, meta,
                                                    m.rope_tab.as<float>(), hp.rms_eps, T);
-            llamd_fwd_kv16_expand(l.kc.p, l.vc.p, m.kc32.as<float>(), m.vc32.as<float>(), n_kv_max, kvd);
             kc_view = m.kc32.as<float>();
             vc_view = m.vc32.as<float>();
         } else {
             llamd_fwd_qk_norm_rope_store_tile(p.q.as<float>(), wqn, p.k.as<float>(), wkn, p.v.as<float>(), l.kc.as<float>(), l.vc.as<float>(), H,
                                               HKV, hd, meta, m.rope_tab.as<float>(), hp.rms_eps, T);
         }
-        if (!multi_seq) {  // (a batch of sequences attended above)
+        const bool attended = multi_seq || (small && m.prefill_attn && m.attn_gqa &&
+                                            attention_small_tile(p.q.as<float>(), l.kc.p, l.vc.p, p.attn.as<float>(), p.scores.as<float>(), H, HKV, hd, meta,
+                                                                 n_kv_max, T, m.kv16 != 0));
+        if (!attended) {  // (a batch of sequences attended above)
+            if (m.kv16) llamd_fwd_kv16_expand(l.kc.p, l.vc.p, m.kc32.as<float>(), m.vc32.as<float>(), n_kv_max, kvd);
             for (int t0 = 0; t0 < T; t0 += kAttnTokens) {
                 const int n = T - t0 < kAttnTokens ? T - t0 : kAttnTokens;
                 const float *q = p.q.as<float>() + (size_t)t0 * qd;
@@ -1552,7 +1555,7 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
         if (small) {
             MatvecPlans plan = {};
             if (m.sort_slots && T >= m.sort_slots) {
-                slot_order_launch(p.ids.as<int32_t>(), T * nu, p.pslot.as<int32_t>());
+                slot_order_launch(p.ids.as<int32_t>(), T * nu, ne, p.pslot.as<int32_t>());
                 plan.slot_order = p.pslot.as<int32_t>();
             }
             matvec_grouped_x2_batch(plan, l.gate_exps.p, l.up_exps.p, p.ids.as<int32_t>(), p.aq.as<int8_t>(), p.ad.as<float>(), p.gate.as<float>(),

@@ -1361,7 +1361,9 @@ __global__ void __launch_bounds__(256) attn_out_kernel(const float *__restrict__
 // per thread).
 constexpr int kGqaMax = 8;  // query heads per kv head these kernels hold
 
-template <class KVT>
+// ROPE: with the query's and the new key's norm and rotation and the K/V store, for the new token of a sequence. Otherwise for
+// the tokens of a small tile of one sequence: the queries are ready and every key is in the cache (kv_stride 0).
+template <class KVT, bool ROPE>
 __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *__restrict__ q_raw, const float *__restrict__ wq,
                                                                    const float *__restrict__ k_raw, const float *__restrict__ wk,
                                                                    const float *__restrict__ v_raw, KVT *__restrict__ kc, KVT *__restrict__ vc,
@@ -1376,14 +1378,14 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
     float *sk = s_raw + (ratio + 1) * hd;         // [hd] the roped new key, as the cache holds it
     __shared__ float s_scale[kGqaMax + 1];
     pdl_trigger();
-    const bool early = (flags & kPassEarlyLoads) != 0;  // (see attn_rope_scores_kernel)
+    const bool early = ROPE && (flags & kPassEarlyLoads) != 0;  // (see attn_rope_scores_kernel)
     if (!early) pdl_wait();
     const int kvh = blockIdx.x, c = blockIdx.y, split = gridDim.y, seq = blockIdx.z, tid = threadIdx.x;
     const int pos = meta[2 * seq + 1], n_kv = pos + 1;
     if (c * kAttTile >= n_kv) return;
     const int kv_dim = n_head_kv * hd, h0 = kvh * ratio;
     const int ti_pos = pos / kAttTile;
-    const bool need_k = (ti_pos % split) == c;  // this CTA scores the new key, and stores the K and V rows of the position
+    const bool need_k = ROPE && (ti_pos % split) == c;  // this CTA scores the new key, and stores the K and V rows of the position
     KVT *krow = kc + ((size_t)seq * kv_stride + pos) * kv_dim + (size_t)kvh * hd;
     KVT *vrow = vc + ((size_t)seq * kv_stride + pos) * kv_dim + (size_t)kvh * hd;
     const KVT *kb = kc + (size_t)seq * kv_stride * kv_dim + (size_t)kvh * hd;
@@ -1399,7 +1401,7 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
             const int r = idx / hd4, cc = idx - r * hd4;
             const int t = ti * kAttTile + r;
             reg[j] = typename KvIo<KVT>::Raw{};
-            if (idx < per_tile4 && t < pos) reg[j] = KvIo<KVT>::raw4(kb + (size_t)t * kv_dim + 4 * cc);
+            if (idx < per_tile4 && (ROPE ? t < pos : t < n_kv)) reg[j] = KvIo<KVT>::raw4(kb + (size_t)t * kv_dim + 4 * cc);
         }
     };
     auto stash = [&](float *dst, int ti) {
@@ -1407,7 +1409,7 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
         for (int j = 0; j < kMaxLd; j++) {
             const int idx = tid + j * 256;
             const int r = idx / hd4, cc = idx - r * hd4;
-            if (idx < per_tile4 && ti * kAttTile + r != pos) {  // (the token's own row is written below, by other threads)
+            if (idx < per_tile4 && (!ROPE || ti * kAttTile + r != pos)) {  // (the token's own row is written below, by other threads)
                 *reinterpret_cast<float4 *>(dst + r * stride + 4 * cc) = KvIo<KVT>::wide4(reg[j]);
             }
         }
@@ -1423,6 +1425,7 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
                 }
         pdl_wait();
     }
+    if (ROPE) {
     // ---- QK-norm (crates/llamd-runtime/src/layer.rs:62-79) and RoPE (crates/llamd-cpu/src/lib.rs:158-209) of the kv head's
     // query heads (adjacent in q_raw) and, where needed, of the new key
     const int n_vec = ratio + (need_k ? 1 : 0);
@@ -1471,13 +1474,16 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
             KvIo<KVT>::st(vrow + i + half, vs[i + half]);
         }
     }
+    } else {
+        for (int i = tid; i < ratio * hd; i += blockDim.x) sq[i] = q_raw[((size_t)seq * n_head + h0) * hd + i];
+    }
     __syncthreads();
     // ---- scores: (query head, position) pairs of the tile over the threads ----
     int buf = 0;
     for (int ti = c; ti < n_tiles; ti += split, buf ^= 1) {
         float *cur = tile + buf * kAttTile * stride;
         stash(cur, ti);
-        if (ti == ti_pos)
+        if (ROPE && ti == ti_pos)
             for (int i = tid; i < hd; i += blockDim.x) cur[(pos - ti * kAttTile) * stride + i] = sk[i];
         __syncthreads();
         if (ti + split < n_tiles) fetch(ti + split);
@@ -1628,23 +1634,38 @@ static bool attn_out_cluster_ok(int n_head, int hd) {
     return hd == 128 && hd / kSplit == 32 && (256 / hd) * kSplit <= 8 && n_head % (256 / hd) == 0;
 }
 
-// order[] = the slots sorted by (expert id, slot): every slot counts the slots that come before it (a few hundred slots:
-// one CTA, no scratch memory).
-__global__ void __launch_bounds__(256) slot_order_kernel(const int32_t *__restrict__ ids, int n_slots, int32_t *__restrict__ order) {
-    extern __shared__ int32_t s_ids[];
+// order[] = the slots sorted by expert id: histogram, scan over the experts, scatter, one CTA. (Which of an expert's slots comes
+// first is of no consequence: each has its own output.) Ranking every slot against every other took 5.1 us for 256 slots and 8.3 for
+// 296; this 4.4 up to 1024.
+__global__ void __launch_bounds__(512) slot_order_kernel(const int32_t *__restrict__ ids, int n_slots, int n_expert, int32_t *__restrict__ order) {
+    __shared__ int s_at[1024];
     pdl_trigger();
+    const int tid = threadIdx.x;
+    for (int e = tid; e < n_expert; e += blockDim.x) s_at[e] = 0;
     pdl_wait();
-    for (int i = threadIdx.x; i < n_slots; i += blockDim.x) s_ids[i] = ids[i];
     __syncthreads();
-    for (int i = threadIdx.x; i < n_slots; i += blockDim.x) {
-        const int mine = s_ids[i];
-        int rank = 0;
-        for (int j = 0; j < n_slots; j++) {
-            const int o = s_ids[j];
-            rank += (o < mine || (o == mine && j < i)) ? 1 : 0;
+    auto expert = [&](int i) {
+        const int e = ids[i];
+        return e < 0 || e >= n_expert ? 0 : e;
+    };
+    for (int i = tid; i < n_slots; i += blockDim.x) atomicAdd(&s_at[expert(i)], 1);
+    __syncthreads();
+    if (tid < 32) {
+        int start = 0;
+        for (int e0 = 0; e0 < n_expert; e0 += 32) {
+            const int e = e0 + tid, c = e < n_expert ? s_at[e] : 0;
+            int incl = c;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, off);
+                if (tid >= off) incl += v;
+            }
+            if (e < n_expert) s_at[e] = start + incl - c;
+            start += __shfl_sync(0xffffffffu, incl, 31);
         }
-        order[rank] = i;
     }
+    __syncthreads();
+    for (int i = tid; i < n_slots; i += blockDim.x) order[atomicAdd(&s_at[expert(i)], 1)] = i;
 }
 
 // ---- argmax, lowest index on a tie (llamd_forward.hip:353-389) -------------
@@ -2203,8 +2224,8 @@ static void attention_rope_launch(const float *q, const float *wq, const float *
     if (gqa) {
         static size_t conf_ga[2] = {0, 0};
         if (smem_ga > conf_ga[kv16]) {
-            const cudaError_t e = kv16 ? cudaFuncSetAttribute(attn_rope_scores_gqa_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_ga)
-                                       : cudaFuncSetAttribute(attn_rope_scores_gqa_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_ga);
+            const cudaError_t e = kv16 ? cudaFuncSetAttribute(attn_rope_scores_gqa_kernel<__half, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_ga)
+                                       : cudaFuncSetAttribute(attn_rope_scores_gqa_kernel<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_ga);
             if (e != cudaSuccess) {
                 set_error(e, "attention (rope + scores, per kv head) smem attribute");
                 return;
@@ -2217,10 +2238,10 @@ static void attention_rope_launch(const float *q, const float *wq, const float *
         split = split > tiles ? tiles : split;
         const dim3 grid(n_head_kv, split, nseq);
         if (kv16)
-            launch_kc(PDL_ATTN, "attn_rope_scores_gqa", attn_rope_scores_gqa_kernel<__half>, grid, dim3(256), smem_ga, q, wq, k, wk, v, (__half *)kc,
+            launch_kc(PDL_ATTN, "attn_rope_scores_gqa", attn_rope_scores_gqa_kernel<__half, true>, grid, dim3(256), smem_ga, q, wq, k, wk, v, (__half *)kc,
                       (__half *)vc, scores, n_head, n_head_kv, hd, meta, max_kv, max_kv, rope_tab, eps, flags);
         else
-            launch_kc(PDL_ATTN, "attn_rope_scores_gqa", attn_rope_scores_gqa_kernel<float>, grid, dim3(256), smem_ga, q, wq, k, wk, v, (float *)kc,
+            launch_kc(PDL_ATTN, "attn_rope_scores_gqa", attn_rope_scores_gqa_kernel<float, true>, grid, dim3(256), smem_ga, q, wq, k, wk, v, (float *)kc,
                       (float *)vc, scores, n_head, n_head_kv, hd, meta, max_kv, max_kv, rope_tab, eps, flags);
     } else if (kv16) {
         launch_kc(PDL_ATTN, "attn_rope_scores", attn_rope_scores_kernel<__half>, dim3(n_head, kSplitT, nseq), dim3(256), smem_a, q, wq, k, wk, v,
@@ -2232,13 +2253,13 @@ static void attention_rope_launch(const float *q, const float *wq, const float *
     if (gqa && nseq >= 4 && smem_gb <= 200 * 1024) {
         static size_t conf_gb[2] = {0, 0};
         if (smem_gb > conf_gb[kv16]) {
-            const cudaError_t e = kv16 ? cudaFuncSetAttribute(attn_out_gqa_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_gb)
-                                       : cudaFuncSetAttribute(attn_out_gqa_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_gb);
+            const cudaError_t e = kv16 ? cudaFuncSetAttribute(attn_out_gqa_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024  /* (the small tile's launch sets the same) */)
+                                       : cudaFuncSetAttribute(attn_out_gqa_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024  /* (the small tile's launch sets the same) */);
             if (e != cudaSuccess) {
                 set_error(e, "attention (output, per kv head) smem attribute");
                 return;
             }
-            conf_gb[kv16] = smem_gb;
+            conf_gb[kv16] = 200 * 1024;
         }
         if (kv16)
             launch_kc(PDL_ATTN, "attn_out_gqa", attn_out_gqa_kernel<__half>, dim3(n_head_kv, kSplit, nseq), dim3(256), smem_gb, (const float *)scores,
@@ -2276,6 +2297,49 @@ void attention_meta_flags(const float *q, const void *kc, const void *vc, float 
                           const int32_t *meta, int max_kv, int nseq, bool kv16, int flags) {
     attention_launch(q, (const float *)kc, (const float *)vc, out, scores, n_head, n_head_kv, hd, meta, 0, max_kv, nseq, max_kv, TailPlan{}, kv16,
                      flags);
+}
+// Attention of a small tile of one sequence whose keys and values are in the cache: the batch kernels, every token a "sequence"
+// of the same cache. n_kv_max bounds pos + 1 over the tokens. False: a shape they do not cover.
+bool attention_small_tile(const float *q, const void *kc, const void *vc, float *out, float *scores, int n_head, int n_head_kv, int hd,
+                          const int32_t *meta, int n_kv_max, int ntok, bool kv16) {
+    if (n_head_kv <= 0 || n_head != kGqaMax * n_head_kv || hd != 32 * kSplit) return false;
+    const int row = (n_kv_max + 3) & ~3;  // a row of scores
+    const size_t smem_a = (size_t)(kGqaMax * hd + 2 * kAttTile * (hd + 4) + (kGqaMax + 1) * hd + hd) * sizeof(float);
+    const size_t smem_b = (size_t)((size_t)kGqaMax * row + 2 * kPvTile * (hd / kSplit)) * sizeof(float);
+    if (smem_b > 200 * 1024) return false;
+    static size_t conf_a[2] = {0, 0}, conf_b[2] = {0, 0};
+    if (smem_a > conf_a[kv16] || smem_b > conf_b[kv16]) {
+        const cudaError_t e =
+            kv16 ? cudaFuncSetAttribute(attn_rope_scores_gqa_kernel<__half, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a)
+                 : cudaFuncSetAttribute(attn_rope_scores_gqa_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a);
+        const cudaError_t f = kv16 ? cudaFuncSetAttribute(attn_out_gqa_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)
+                                   : cudaFuncSetAttribute(attn_out_gqa_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        if (e != cudaSuccess || f != cudaSuccess) {
+            set_error(e != cudaSuccess ? e : f, "attention (small tile) smem attribute");
+            return true;
+        }
+        conf_a[kv16] = smem_a;
+        conf_b[kv16] = 200 * 1024;
+    }
+    const int tiles = (n_kv_max + kAttTile - 1) / kAttTile;
+    int split = 2 * 148 / (n_head_kv * ntok);
+    split = split < kSplitT ? kSplitT : split;
+    split = split > tiles ? tiles : split;
+    const dim3 grid_a(n_head_kv, split, ntok), grid_b(n_head_kv, kSplit, ntok);
+    if (kv16) {
+        launch_kc(PDL_ATTN, "attn_scores_small_tile", attn_rope_scores_gqa_kernel<__half, false>, grid_a, dim3(256), smem_a, q, (const float *)nullptr,
+                  (const float *)nullptr, (const float *)nullptr, (const float *)nullptr, (__half *)kc, (__half *)vc, scores, n_head, n_head_kv, hd, meta, row, 0,
+                  (const float *)nullptr, 0.0f, 0);
+        launch_kc(PDL_ATTN, "attn_out_small_tile", attn_out_gqa_kernel<__half>, grid_b, dim3(256), smem_b, (const float *)scores, (const __half *)vc, out, n_head,
+                  n_head_kv, hd, meta, row, 0, 0);
+    } else {
+        launch_kc(PDL_ATTN, "attn_scores_small_tile", attn_rope_scores_gqa_kernel<float, false>, grid_a, dim3(256), smem_a, q, (const float *)nullptr,
+                  (const float *)nullptr, (const float *)nullptr, (const float *)nullptr, (float *)kc, (float *)vc, scores, n_head, n_head_kv, hd, meta, row, 0,
+                  (const float *)nullptr, 0.0f, 0);
+        launch_kc(PDL_ATTN, "attn_out_small_tile", attn_out_gqa_kernel<float>, grid_b, dim3(256), smem_b, (const float *)scores, (const float *)vc, out, n_head,
+                  n_head_kv, hd, meta, row, 0, 0);
+    }
+    return true;
 }
 }  // namespace llamd
 extern "C" {
@@ -2396,10 +2460,10 @@ void llamd_fwd_moe_group(const int32_t *ids, int n_expert, int n_used, int nseq,
 
 }  // extern "C"
 
-void llamd::slot_order_launch(const int32_t *ids, int n_slots, int32_t *order) {
-    if (n_slots < 1 || n_slots > 8192) {
-        set_error_msg("slot_order: 1..8192 slots");
+void llamd::slot_order_launch(const int32_t *ids, int n_slots, int n_expert, int32_t *order) {
+    if (n_slots < 1 || n_expert < 1 || n_expert > 1024) {
+        set_error_msg("slot_order: at least one slot, 1..1024 experts");
         return;
     }
-    launch_kc(PDL_SMALL, "slot_order", slot_order_kernel, dim3(1), dim3(256), (size_t)n_slots * sizeof(int32_t), ids, n_slots, order);
+    launch_kc(PDL_SMALL, "slot_order", slot_order_kernel, dim3(1), dim3(512), 0, ids, n_slots, n_expert, order);
 }

@@ -313,6 +313,30 @@ def test_small_tiles_equal_gemm_tiles(tiny, n):
     assert np.array_equal(a[2][0].view(np.uint32), b[2][0].view(np.uint32)) and np.array_equal(a[2][1].view(np.uint32), b[2][1].view(np.uint32))
 
 
+@pytest.mark.parametrize("kv16", [0, 1])
+def test_small_tile_attention_equals_the_tile_kernels(kv16):
+    """Eight heads of 128 per kv head: a small tile's attention runs on the kernels that take a kv head's query heads together.
+    Against the tile kernels (option attn_gqa off) across the 64-position score tiles and the 224- and 256-position value tiles."""
+    from llamd_rs_b200 import synth
+    from llamd_rs_b200.model import CudaModel
+
+    hp = dict(synth.TINY, n_layer=1, n_head=8, n_head_kv=1, head_dim=128)
+    gm = CudaModel.load_batched(hp, synth.make_model(hp, seed=9), max_kv=400, max_seq=1)
+    try:
+        if kv16:
+            gm.set_option("kv_f16", 1)
+        toks = synth.token_ids(400, hp["n_vocab"], 3, "small tile").tolist()
+        gm.prefill(toks[:340], 0)
+        for base, n in [(0, 1), (0, 9), (60, 9), (200, 56), (220, 8), (250, 40), (340, 37)]:
+            runs = []
+            for gqa in (1, 0):
+                gm.set_option("attn_gqa", gqa)
+                runs.append((list(gm.verify(toks[base:base + n], base)), gm.prefill(toks[base:base + n], base), gm.logits()[0].view(np.uint32).copy()))
+            assert runs[0][:2] == runs[1][:2] and np.array_equal(runs[0][2], runs[1][2]), f"{n} tokens from {base}"
+    finally:
+        gm.free()
+
+
 def test_prefill_equals_sequential_decode(tiny):
     """crates/llamd-testing/tests/vulkan_prefill.rs:48-136: prefill gives the token (and here the logits and the
     K/V cache, bit for bit) of sequential decode, for (tile, length) pairs that straddle tile and chunk boundaries."""
