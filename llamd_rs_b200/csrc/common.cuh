@@ -227,9 +227,12 @@ void attention_meta_flags(const float *q, const void *kc, const void *vc, float 
 void norm_router_flags(const float *w, const float *x, const float *residual, float *x_out, const float *w_norm, float *xn_out, int8_t *qs,
                        float *d, int k, float eps, int n_expert, int n_used, float *logits, int32_t *ids, float *weights, float *probs,
                        unsigned int *counter, int nseq, int flags);
-void rms_norm_quant_flags(const float *x, const float *w, float *out, int8_t *qs, float *d, int n, float eps, int nseq, int flags);
+// rm (here and below): the residue-major form of the quants as well, or null
+void quantize_rm(const float *x, int8_t *qs, float *d, int nblocks, int8_t *rm);
+void silu_mul_quant_rm(const float *gate, const float *up, float *out, int8_t *qs, float *d, int n, int8_t *rm);
+void rms_norm_quant_flags(const float *x, const float *w, float *out, int8_t *qs, float *d, int n, float eps, int nseq, int flags, int8_t *rm = nullptr);
 void add_rms_norm_quant_flags(const float *x, const float *residual, float *sum_out, const float *w, float *out, int8_t *qs, float *d, int n,
-                              float eps, int nseq, int flags);
+                              float eps, int nseq, int flags, int8_t *rm = nullptr);
 // Internal launch functions behind the extern "C" entry points of the same names; the model passes its plans here.
 void launch_matvec(int njobs, const void *const *w, float *const *out, const int *rows, int blocks, const int8_t *aq,
                    const float *ad, int nseq, const int32_t *ids, int n_slots, int n_expert, int act_div, int act_mode = 0,
@@ -276,7 +279,7 @@ void ep_wait_requests(unsigned int *counter, const unsigned int *epoch, int *sta
 void ep_wait_rows(unsigned int *counter, unsigned int target, int *status, unsigned int limit);
 void ep_signal_rows(unsigned int *const *arrive_tab);
 void combine_rms_norm_quant_wait(const WaitPlan &wait, const float *x, const float *down, const float *weights, int n_used, float *sum_out,
-                                 const float *w, float *out, int8_t *qs, float *d, int n, float eps, int nseq, int flags);
+                                 const float *w, float *out, int8_t *qs, float *d, int n, float eps, int nseq, int flags, int8_t *rm = nullptr);
 
 // Grow-only device scratch for the host-facing entry points, the counterpart
 // of g_aq/g_ad/g_out in crates/llamd-rocm/kernels/llamd.hip:1027-1051.

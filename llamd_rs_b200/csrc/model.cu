@@ -403,6 +403,8 @@ void queue_token(Model &m, int nseq) {
     const int pf = (m.arith_fast && m.fuse_norm_router && !m.fuse_tails ? m.arith_fast : 0) | (m.early_loads ? kPassEarlyLoads : 0) |
                    (m.attn_gqa ? kPassAttnGqa : 0);
     const bool dense_gemm = m.dense_gemm && nseq >= m.dense_gemm && m.dense_fold_ready && !m.fuse_norm_qkv;
+    int8_t *rm = dense_gemm ? m.head_rm.as<int8_t>() : nullptr;  // the GEMMs' operand, made with the quants
+    bool rm_made = false;
     size_t n_marks = 0;
     auto mark = [&](int phase) {
         if (!m.profiling) return;
@@ -469,17 +471,16 @@ void queue_token(Model &m, int nseq) {
             mark(LLAMD_PH_ATTN_NORM);
         } else {
             if (il == 0) {
-                rms_norm_quant_flags(x, l.attn_norm.as<float>(), nullptr, m.aq.as<int8_t>(), m.ad.as<float>(), E, hp.rms_eps, nseq, pf);
+                rms_norm_quant_flags(x, l.attn_norm.as<float>(), nullptr, m.aq.as<int8_t>(), m.ad.as<float>(), E, hp.rms_eps, nseq, pf, rm);
             } else {
                 combine_rms_norm_quant_wait(plan_ep_wait(), x_res, m.e_down.as<float>(), m.expert_w.as<float>(), nu, x, l.attn_norm.as<float>(),
-                                            nullptr, m.aq.as<int8_t>(), m.ad.as<float>(), E, hp.rms_eps, nseq, pf);
+                                            nullptr, m.aq.as<int8_t>(), m.ad.as<float>(), E, hp.rms_eps, nseq, pf, rm);
                 x_res = x;
                 trace_x(il - 1);
             }
             mark(LLAMD_PH_ATTN_NORM);
             if (dense_gemm) {
                 // a batch: the folded matrices once for all the sequences, on the integer tensor path (the same bits)
-                llamd_fwd_q8k_residue_major(m.aq.as<int8_t>(), m.head_rm.p, (size_t)nseq * eb);
                 gemm_tokens_folded3(l.q_fold.p, l.k_fold.p, l.v_fold.p, m.head_rm.p, m.ad.as<float>(), m.q.as<float>(), m.k.as<float>(),
                                     m.v.as<float>(), eb, qd, kvd, kvd, nseq);
             } else {
@@ -501,7 +502,8 @@ void queue_token(Model &m, int nseq) {
                                  quant_in_launch ? m.aq.as<int8_t>() : nullptr, quant_in_launch ? m.ad.as<float>() : nullptr, pf);
             mark(LLAMD_PH_ROPE);
             mark(LLAMD_PH_ATTENTION);
-            if (!quant_in_launch) llamd_fwd_quantize(m.attn.as<float>(), m.aq.as<int8_t>(), m.ad.as<float>(), nseq * (qd / 256));
+            if (!quant_in_launch) quantize_rm(m.attn.as<float>(), m.aq.as<int8_t>(), m.ad.as<float>(), nseq * (qd / 256), rm);
+            rm_made = !quant_in_launch;
         } else {
             if (m.kv16)
                 llamd_fwd_qk_norm_rope_store_kv16(m.q.as<float>(), wqn, m.k.as<float>(), wkn, m.v.as<float>(), l.kc.p, l.vc.p, H, HKV, hd, meta,
@@ -521,12 +523,13 @@ void queue_token(Model &m, int nseq) {
                                      m.kv16, pf);
                 mark(LLAMD_PH_ATTENTION);
                 // (llamd_fwd_matvec_f32act fuses these two; measured 2 % slower per token: every CTA repeats the quantization)
-                llamd_fwd_quantize(m.attn.as<float>(), m.aq.as<int8_t>(), m.ad.as<float>(), nseq * (qd / 256));
+                quantize_rm(m.attn.as<float>(), m.aq.as<int8_t>(), m.ad.as<float>(), nseq * (qd / 256), rm);
+                rm_made = true;
             }
         }
         mark(LLAMD_PH_QUANT);
         if (dense_gemm) {
-            llamd_fwd_q8k_residue_major(m.aq.as<int8_t>(), m.head_rm.p, (size_t)nseq * (qd / 256));
+            if (!rm_made) llamd_fwd_q8k_residue_major(m.aq.as<int8_t>(), m.head_rm.p, (size_t)nseq * (qd / 256));
             gemm_tokens_folded(l.o_fold.p, m.head_rm.p, m.ad.as<float>(), m.xb2.as<float>(), qd / 256, E, nseq);
         } else {
             matvec_batch(plan_static(m, &l.ffn_gate_inp), l.attn_out.p, m.aq.as<int8_t>(), m.ad.as<float>(), m.xb2.as<float>(), qd / 256, E,
@@ -634,13 +637,14 @@ void queue_token(Model &m, int nseq) {
                             cudaMemcpyDeviceToDevice, stream());
     }
     // the last layer's combine, fused with the output norm
+    const bool head_gemm = m.head_gemm && nseq >= m.head_gemm && m.head_fold_ready;
     combine_rms_norm_quant_wait(plan_ep_wait(), x_res, m.e_down.as<float>(), m.expert_w.as<float>(), nu, x, m.output_norm.as<float>(), nullptr,
-                                m.aq.as<int8_t>(), m.ad.as<float>(), E, hp.rms_eps, nseq, pf);
+                                m.aq.as<int8_t>(), m.ad.as<float>(), E, hp.rms_eps, nseq, pf,
+                                head_gemm ? m.head_rm.as<int8_t>() : nullptr);
     trace_x(hp.n_layer - 1);
     mark(LLAMD_PH_ATTN_NORM);
-    if (m.head_gemm && nseq >= m.head_gemm && m.head_fold_ready) {
+    if (head_gemm) {
         // a batch: the folded matrix once for all the sequences, on the integer tensor path (the same bits)
-        llamd_fwd_q8k_residue_major(m.aq.as<int8_t>(), m.head_rm.p, (size_t)nseq * eb);
         gemm_tokens_folded(m.head_fold.p, m.head_rm.p, m.ad.as<float>(), m.logits.as<float>(), eb, hp.n_vocab, nseq);
     } else {
         // (the prefetch plan names where the next token starts)
@@ -1420,7 +1424,6 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
     auto small_dense = [&](const Buf &f0, const Buf &f1, const Buf &f2, const Buf &w0, const Buf &w1, const Buf &w2, const Buf &o0, const Buf &o1,
                            const Buf &o2, int blocks, int rows0, int rows12) {
         if (folded) {
-            llamd_fwd_q8k_residue_major(p.aq.as<int8_t>(), p.aq_rm.p, (size_t)T * blocks);
             gemm_tokens_folded3(f0.p, f1.p, f2.p, p.aq_rm.p, p.ad.as<float>(), o0.as<float>(), o1.as<float>(), o2.as<float>(), blocks, rows0, rows12,
                                 rows12, T);
         } else if (w1.p) {
@@ -1431,14 +1434,17 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
         }
     };
     const Buf none;
+    // the GEMMs' operand is made with the quants
+    const bool exact_gemm = (m.prefill_gemm != 0 && m.prefill_gemm != 2) || m.ep_world > 1;
+    int8_t *rm = folded || (exact_gemm && !small) ? p.aq_rm.as<int8_t>() : nullptr;
     llamd_fwd_embed_meta(m.tok_embd.p, meta, x, eb, T);
     for (int il = 0; il < hp.n_layer; il++) {
         Layer &l = m.layers[il];
         if (il == 0)
-            llamd_fwd_rms_norm_quant(x, l.attn_norm.as<float>(), nullptr, p.aq.as<int8_t>(), p.ad.as<float>(), E, hp.rms_eps, T);
+            rms_norm_quant_flags(x, l.attn_norm.as<float>(), nullptr, p.aq.as<int8_t>(), p.ad.as<float>(), E, hp.rms_eps, T, 0, rm);
         else
-            llamd_fwd_combine_rms_norm_quant(x, p.down.as<float>(), p.w.as<float>(), nu, x, l.attn_norm.as<float>(), nullptr,
-                                             p.aq.as<int8_t>(), p.ad.as<float>(), E, hp.rms_eps, T);
+            combine_rms_norm_quant_wait(WaitPlan{}, x, p.down.as<float>(), p.w.as<float>(), nu, x, l.attn_norm.as<float>(), nullptr,
+                                             p.aq.as<int8_t>(), p.ad.as<float>(), E, hp.rms_eps, T, 0, rm);
         const bool ep = m.ep_world > 1;  // sharded experts run on the integer GEMM; so then do the dense matmuls
         const bool gemm = m.prefill_gemm != 0 || ep, tc = m.prefill_gemm == 2 && !ep;
         if (small || folded) {
@@ -1448,7 +1454,6 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
             llamd_fwd_gemm_tokens_tc(l.attn_q.p, l.attn_k.p, l.attn_v.p, p.aq_rm.p, p.q.as<float>(), p.k.as<float>(), p.v.as<float>(), eb, qd,
                                      kvd, kvd, T);
         } else if (gemm) {
-            llamd_fwd_q8k_residue_major(p.aq.as<int8_t>(), p.aq_rm.p, (size_t)T * eb);
             llamd_fwd_gemm_tokens(l.attn_q.p, l.attn_k.p, l.attn_v.p, p.aq_rm.p, p.ad.as<float>(), p.q.as<float>(), p.k.as<float>(),
                                   p.v.as<float>(), eb, qd, kvd, kvd, T);
         } else {
@@ -1500,22 +1505,21 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
                     llamd_fwd_attention_tile(q, kc_view, vc_view, out, p.scores.as<float>(), H, HKV, hd, meta + 2 * t0, m.max_kv, n);
             }
         }
-        llamd_fwd_quantize(p.attn.as<float>(), p.aq.as<int8_t>(), p.ad.as<float>(), T * (qd / 256));
+        quantize_rm(p.attn.as<float>(), p.aq.as<int8_t>(), p.ad.as<float>(), T * (qd / 256), rm);
         if (small || folded) {
             small_dense(l.o_fold, none, none, l.attn_out, none, none, p.xb2, none, none, qd / 256, E, 0);
         } else if (tc) {
             llamd_fwd_act_f16_rm(p.aq.as<int8_t>(), p.ad.as<float>(), p.aq_rm.p, (size_t)T * (qd / 256));
             llamd_fwd_gemm_tokens_tc(l.attn_out.p, nullptr, nullptr, p.aq_rm.p, p.xb2.as<float>(), nullptr, nullptr, qd / 256, E, 0, 0, T);
         } else if (gemm) {
-            llamd_fwd_q8k_residue_major(p.aq.as<int8_t>(), p.aq_rm.p, (size_t)T * (qd / 256));
             llamd_fwd_gemm_tokens(l.attn_out.p, nullptr, nullptr, p.aq_rm.p, p.ad.as<float>(), p.xb2.as<float>(), nullptr, nullptr, qd / 256,
                                   E, 0, 0, T);
         } else {
             llamd_fwd_matvec_tokens(l.attn_out.p, nullptr, nullptr, p.aq.as<int8_t>(), p.ad.as<float>(), p.xb2.as<float>(), nullptr, nullptr,
                                     qd / 256, E, 0, 0, T);
         }
-        llamd_fwd_add_rms_norm_quant(x, p.xb2.as<float>(), x, l.ffn_norm.as<float>(), p.xb.as<float>(), p.aq.as<int8_t>(), p.ad.as<float>(),
-                                     E, hp.rms_eps, T);
+        add_rms_norm_quant_flags(x, p.xb2.as<float>(), x, l.ffn_norm.as<float>(), p.xb.as<float>(), p.aq.as<int8_t>(), p.ad.as<float>(),
+                                     E, hp.rms_eps, T, 0, small || ep ? nullptr : rm);
         if (m.prefill_attn && T > kRouterRowsMax) {
             llamd_fwd_matmul_f32_tokens(l.ffn_gate_inp.as<float>(), p.xb.as<float>(), p.logits.as<float>(), E, ne, T);
             llamd_fwd_router(p.logits.as<float>(), ne, nu, p.ids.as<int32_t>(), p.w.as<float>(), nullptr, T);
@@ -1577,13 +1581,11 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
             llamd_fwd_expert_gemm_tc(l.down_exps.p, nullptr, p.gstart.as<int32_t>(), p.gcount.as<int32_t>(), p.pslot.as<int32_t>(),
                                      p.pslot.as<int32_t>(), p.aq2_rm.p, p.down.as<float>(), nullptr, ffe / 256, E, ne, T);
         } else if (gemm) {
-            llamd_fwd_q8k_residue_major(p.aq.as<int8_t>(), p.aq_rm.p, (size_t)T * eb);
             const bool pre = m.prefold_ready;
             expert_gemm_scatter(l.gate_exps.p, l.up_exps.p, p.gstart.as<int32_t>(), p.gcount.as<int32_t>(), p.ptoken.as<int32_t>(),
                                 p.pslot.as<int32_t>(), p.aq_rm.p, p.ad.as<float>(), p.gate.as<float>(), p.up.as<float>(), eb, ffe, ne, nullptr, 1,
                                 pre ? l.gate_fold.p : nullptr, pre ? l.up_fold.p : nullptr);
-            llamd_fwd_silu_mul_quant(p.gate.as<float>(), p.up.as<float>(), nullptr, p.aq2.as<int8_t>(), p.ad2.as<float>(), T * nu * ffe);
-            llamd_fwd_q8k_residue_major(p.aq2.as<int8_t>(), p.aq2_rm.p, (size_t)T * nu * (ffe / 256));
+            silu_mul_quant_rm(p.gate.as<float>(), p.up.as<float>(), nullptr, p.aq2.as<int8_t>(), p.ad2.as<float>(), T * nu * ffe, p.aq2_rm.as<int8_t>());
             expert_gemm_scatter(l.down_exps.p, nullptr, p.gstart.as<int32_t>(), p.gcount.as<int32_t>(), p.pslot.as<int32_t>(),
                                 p.pslot.as<int32_t>(), p.aq2_rm.p, p.ad2.as<float>(), p.down.as<float>(), nullptr, ffe / 256, E, ne, nullptr, 1,
                                 pre ? l.down_fold.p : nullptr, nullptr);
@@ -1599,13 +1601,12 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
     }
     if (all_logits) {
         // the head for every token of the tile: combine + output norm + Q8_K per row, lm_head as a GEMM, greedy pick per row
-        llamd_fwd_combine_rms_norm_quant(x, p.down.as<float>(), p.w.as<float>(), nu, x, m.output_norm.as<float>(), nullptr,
-                                         p.aq.as<int8_t>(), p.ad.as<float>(), E, hp.rms_eps, T);
+        combine_rms_norm_quant_wait(WaitPlan{}, x, p.down.as<float>(), p.w.as<float>(), nu, x, m.output_norm.as<float>(), nullptr,
+                                         p.aq.as<int8_t>(), p.ad.as<float>(), E, hp.rms_eps, T, 0, p.aq_rm.as<int8_t>());
         const bool head_folded = folded_tile(m, T) && m.head_gemm && T >= m.head_gemm && m.head_fold_ready;
         if (small && !head_folded) {
             matvec_batch(MatvecPlans{}, m.output.p ? m.output.p : m.tok_embd.p, p.aq.as<int8_t>(), p.ad.as<float>(), logits_out, eb, hp.n_vocab, T);
         } else {
-            llamd_fwd_q8k_residue_major(p.aq.as<int8_t>(), p.aq_rm.p, (size_t)T * eb);
             if (head_folded)
                 gemm_tokens_folded(m.head_fold.p, p.aq_rm.p, p.ad.as<float>(), logits_out, eb, hp.n_vocab, T);
             else

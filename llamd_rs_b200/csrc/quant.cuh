@@ -66,9 +66,11 @@ static ExpBinderRegistration s_exp_binder_registration;
 
 // ---- Q8_K: crates/llamd-quant/src/dot.rs:88-128 ---------------------------
 // One warp per 256-element block; lane l owns elements 8l..8l+7.
-// Produces qs[256] (natural order), d and optionally bsums[16].
+// Produces qs[256] (natural order), d and optionally bsums[16], and optionally the quants residue-major as well, the GEMMs'
+// operand order: word j of residue r holds elements 32j + 8k + r, so lane l's byte r belongs at 32r + l, and a warp stores
+// eight runs of 32 bytes. (A launch of its own for that order cost 3 to 4 us four times a layer.)
 __device__ __forceinline__ void q8k_quantize_block(const float v[8], int lane, int8_t *__restrict__ qs, float *__restrict__ d_out,
-                                                   int16_t *__restrict__ bsums) {
+                                                   int16_t *__restrict__ bsums, int8_t *__restrict__ rm = nullptr) {
     // the SIGNED value at the largest magnitude, first such element
     float amax = 0.0f, mx = 0.0f;
     int idx = 0;
@@ -110,6 +112,10 @@ __device__ __forceinline__ void q8k_quantize_block(const float v[8], int lane, i
         w1 |= ((uint32_t)q[4 + i] & 0xFFu) << (8 * i);
     }
     *reinterpret_cast<uint2 *>(qs + lane * 8) = make_uint2(w0, w1);
+    if (rm) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) rm[32 * i + lane] = (int8_t)q[i];
+    }
     if (lane == 0) *d_out = dd;
     if (bsums) {
         int s = 0;

@@ -9,7 +9,7 @@
 namespace llamd {
 
 __global__ void __launch_bounds__(256) q8k_quantize_kernel(const float *__restrict__ x, int8_t *__restrict__ qs, float *__restrict__ d,
-                                                           int16_t *__restrict__ bsums, int nblocks) {
+                                                           int16_t *__restrict__ bsums, int8_t *__restrict__ rm, int nblocks) {
     pdl_trigger();
     pdl_wait();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -17,7 +17,8 @@ __global__ void __launch_bounds__(256) q8k_quantize_kernel(const float *__restri
     const float4 *p = reinterpret_cast<const float4 *>(x + (size_t)warp * 256 + lane * 8);
     const float4 a = p[0], b = p[1];
     const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    q8k_quantize_block(v, lane, qs + (size_t)warp * 256, d + warp, bsums ? bsums + (size_t)warp * 16 : nullptr);
+    q8k_quantize_block(v, lane, qs + (size_t)warp * 256, d + warp, bsums ? bsums + (size_t)warp * 16 : nullptr,
+                       rm ? rm + (size_t)warp * 256 : nullptr);
 }
 
 // ---- rms_norm: crates/llamd-cpu/src/lib.rs:55-75, then `* w` --------------
@@ -40,7 +41,8 @@ template <int kMaxV>  // float4 groups per thread: rows of up to 1024 * kMaxV el
 __global__ void __launch_bounds__(256) rms_norm_kernel(const float *__restrict__ x, const float *__restrict__ residual,
                                                        const float *__restrict__ down, const float *__restrict__ cw, int n_used,
                                                        float *__restrict__ sum_out, const float *__restrict__ w, float *__restrict__ out,
-                                                       int8_t *__restrict__ qs, float *__restrict__ d, int n, float eps, const WaitPlan wait, int fast) {
+                                                       int8_t *__restrict__ qs, float *__restrict__ d, int8_t *__restrict__ rm, int n, float eps, const WaitPlan wait,
+                                                       int fast) {
     extern __shared__ __align__(16) float sx[];  // [n] values, then [n] squares
     float *ssq = sx + n;
     __shared__ float s_scale;
@@ -170,7 +172,8 @@ __global__ void __launch_bounds__(256) rms_norm_kernel(const float *__restrict__
         float v[8];
         const float4 a = reinterpret_cast<const float4 *>(sx + b * 256 + lane * 8)[0], c = reinterpret_cast<const float4 *>(sx + b * 256 + lane * 8)[1];
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
-        q8k_quantize_block(v, lane, qs + (size_t)seq * n + (size_t)b * 256, d + (size_t)seq * (n / 256) + b, nullptr);
+        q8k_quantize_block(v, lane, qs + (size_t)seq * n + (size_t)b * 256, d + (size_t)seq * (n / 256) + b, nullptr,
+                           rm ? rm + (size_t)seq * n + (size_t)b * 256 : nullptr);
     }
 }
 
@@ -207,7 +210,7 @@ __global__ void silu_mul_kernel(const float *__restrict__ gate, const float *__r
 // One warp per 256-element block: act = silu(gate)*up, then Q8_K of act.
 __global__ void __launch_bounds__(256) silu_mul_quant_kernel(const float *__restrict__ gate, const float *__restrict__ up,
                                                              float *__restrict__ out, int8_t *__restrict__ qs, float *__restrict__ d,
-                                                             int nblocks) {
+                                                             int8_t *__restrict__ rm, int nblocks) {
     pdl_trigger();
     pdl_wait();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -221,7 +224,7 @@ __global__ void __launch_bounds__(256) silu_mul_quant_kernel(const float *__rest
         *reinterpret_cast<float4 *>(out + base) = make_float4(v[0], v[1], v[2], v[3]);
         *reinterpret_cast<float4 *>(out + base + 4) = make_float4(v[4], v[5], v[6], v[7]);
     }
-    q8k_quantize_block(v, lane, qs + (size_t)warp * 256, d + warp, nullptr);
+    q8k_quantize_block(v, lane, qs + (size_t)warp * 256, d + warp, nullptr, rm ? rm + (size_t)warp * 256 : nullptr);
 }
 
 // The same for a handful of blocks (a decode token: 8 experts x 3 blocks): a CTA per block, one element per thread, so
@@ -229,7 +232,7 @@ __global__ void __launch_bounds__(256) silu_mul_quant_kernel(const float *__rest
 // from shared memory. Same operations per element, same bits.
 __global__ void __launch_bounds__(256) silu_mul_quant_small_kernel(const float *__restrict__ gate, const float *__restrict__ up,
                                                                    float *__restrict__ out, int8_t *__restrict__ qs, float *__restrict__ d,
-                                                                   int nblocks) {
+                                                                   int8_t *__restrict__ rm, int nblocks) {
     __shared__ __align__(16) float s_v[256];
     pdl_trigger();
     pdl_wait();
@@ -242,7 +245,7 @@ __global__ void __launch_bounds__(256) silu_mul_quant_small_kernel(const float *
     if (tid < 32) {
         const float4 a = reinterpret_cast<const float4 *>(s_v + tid * 8)[0], b = reinterpret_cast<const float4 *>(s_v + tid * 8)[1];
         const float w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        q8k_quantize_block(w, tid, qs + (size_t)blk * 256, d + blk, nullptr);
+        q8k_quantize_block(w, tid, qs + (size_t)blk * 256, d + blk, nullptr, rm ? rm + (size_t)blk * 256 : nullptr);
     }
 }
 
@@ -281,38 +284,44 @@ static void launch_rms_norm(const char *what, int nseq, int n, Args... args) {
 
 // `wait`: with expert parallelism the rows of `down` are stored by other GPUs; the launch first waits for their arrivals.
 void llamd::combine_rms_norm_quant_wait(const WaitPlan &wait, const float *x, const float *down, const float *weights, int n_used,
-                                        float *sum_out, const float *w, float *out, int8_t *qs, float *d, int n, float eps, int nseq, int flags) {
+                                        float *sum_out, const float *w, float *out, int8_t *qs, float *d, int n, float eps, int nseq, int flags, int8_t *rm) {
     if (n % 256 || (size_t)n * 8 > 48 * 1024) {
         set_error_msg("combine_rms_norm_quant: n must be a multiple of 256 and at most 6144");
         return;
     }
-    launch_rms_norm("combine_rms_norm_quant", nseq, n, x, (const float *)nullptr, down, weights, n_used, sum_out, w, out, qs, d, n, eps, wait,
+    launch_rms_norm("combine_rms_norm_quant", nseq, n, x, (const float *)nullptr, down, weights, n_used, sum_out, w, out, qs, d, rm, n, eps, wait,
                     flags);
 }
 // llamd_fwd_rms_norm_quant / llamd_fwd_add_rms_norm_quant with a decode pass's flags (kPass... in common.cuh).
-void llamd::rms_norm_quant_flags(const float *x, const float *w, float *out, int8_t *qs, float *d, int n, float eps, int nseq, int flags) {
+void llamd::rms_norm_quant_flags(const float *x, const float *w, float *out, int8_t *qs, float *d, int n, float eps, int nseq, int flags, int8_t *rm) {
     if (n % 256 || (size_t)n * 8 > 48 * 1024) {
         set_error_msg("rms_norm_quant: n must be a multiple of 256 and at most 6144");
         return;
     }
     launch_rms_norm("rms_norm_quant", nseq, n, x, (const float *)nullptr, (const float *)nullptr, (const float *)nullptr, 0, (float *)nullptr, w, out,
-                    qs, d, n, eps, WaitPlan{}, flags);
+                    qs, d, rm, n, eps, WaitPlan{}, flags);
 }
 void llamd::add_rms_norm_quant_flags(const float *x, const float *residual, float *sum_out, const float *w, float *out, int8_t *qs, float *d,
-                                     int n, float eps, int nseq, int flags) {
+                                     int n, float eps, int nseq, int flags, int8_t *rm) {
     if (n % 256 || (size_t)n * 8 > 48 * 1024) {
         set_error_msg("add_rms_norm_quant: n must be a multiple of 256 and at most 6144");
         return;
     }
-    launch_rms_norm("add_rms_norm_quant", nseq, n, x, residual, (const float *)nullptr, (const float *)nullptr, 0, sum_out, w, out, qs, d, n, eps,
+    launch_rms_norm("add_rms_norm_quant", nseq, n, x, residual, (const float *)nullptr, (const float *)nullptr, 0, sum_out, w, out, qs, d, rm, n, eps,
                     WaitPlan{}, flags);
+}
+
+// llamd_fwd_quantize with the residue-major form beside the natural one.
+void llamd::quantize_rm(const float *x, int8_t *qs, float *d, int nblocks, int8_t *rm) {
+    if (nblocks <= 0) return;
+    launch_kc(PDL_SMALL, "q8k_quantize", q8k_quantize_kernel, dim3((nblocks + 7) / 8), dim3(256), 0, x, qs, d, (int16_t *)nullptr, rm, nblocks);
 }
 
 extern "C" {
 
 void llamd_fwd_quantize_bsums(const float *x, int8_t *qs, float *d, int16_t *bsums, int nblocks) {
     if (nblocks <= 0) return;
-    launch_kc(PDL_SMALL, "q8k_quantize", q8k_quantize_kernel, dim3((nblocks + 7) / 8), dim3(256), 0, x, qs, d, bsums, nblocks);
+    launch_kc(PDL_SMALL, "q8k_quantize", q8k_quantize_kernel, dim3((nblocks + 7) / 8), dim3(256), 0, x, qs, d, bsums, (int8_t *)nullptr, nblocks);
 }
 void llamd_fwd_quantize(const float *x, int8_t *qs, float *d, int nblocks) {
     llamd_fwd_quantize_bsums(x, qs, d, nullptr, nblocks);
@@ -324,7 +333,7 @@ void llamd_fwd_rms_norm_mul(const float *x, const float *w, float *out, int n, f
         return;
     }
     launch_rms_norm("rms_norm_mul", nseq, n, x, (const float *)nullptr, (const float *)nullptr, (const float *)nullptr, 0, (float *)nullptr, w, out,
-                    (int8_t *)nullptr, (float *)nullptr, n, eps, WaitPlan{}, 0);
+                    (int8_t *)nullptr, (float *)nullptr, (int8_t *)nullptr, n, eps, WaitPlan{}, 0);
 }
 void llamd_fwd_rms_norm_quant(const float *x, const float *w, float *out, int8_t *qs, float *d, int n, float eps, int nseq) {
     rms_norm_quant_flags(x, w, out, qs, d, n, eps, nseq, 0);
@@ -358,17 +367,22 @@ void llamd_fwd_silu_mul(const float *gate, const float *up, float *out, int n) {
     silu_mul_kernel<<<(n + 255) / 256, 256, 0, stream()>>>(gate, up, out, n);
     LLAMD_CHECK_LAUNCH("silu_mul");
 }
-void llamd_fwd_silu_mul_quant(const float *gate, const float *up, float *out, int8_t *qs, float *d, int n) {
+}
+void llamd::silu_mul_quant_rm(const float *gate, const float *up, float *out, int8_t *qs, float *d, int n, int8_t *rm) {
     if (n % 256) {
         set_error_msg("silu_mul_quant: n must be a multiple of 256");
         return;
     }
     const int nblocks = n / 256;
     if (nblocks <= 592) {  // (four CTAs per SM: beyond that the warp-per-block form's throughput wins)
-        launch_kc(PDL_SMALL, "silu_mul_quant_small", silu_mul_quant_small_kernel, dim3(nblocks), dim3(256), 0, gate, up, out, qs, d, nblocks);
+        launch_kc(PDL_SMALL, "silu_mul_quant_small", silu_mul_quant_small_kernel, dim3(nblocks), dim3(256), 0, gate, up, out, qs, d, rm, nblocks);
         return;
     }
-    launch_kc(PDL_SMALL, "silu_mul_quant", silu_mul_quant_kernel, dim3((nblocks + 7) / 8), dim3(256), 0, gate, up, out, qs, d, nblocks);
+    launch_kc(PDL_SMALL, "silu_mul_quant", silu_mul_quant_kernel, dim3((nblocks + 7) / 8), dim3(256), 0, gate, up, out, qs, d, rm, nblocks);
+}
+extern "C" {
+void llamd_fwd_silu_mul_quant(const float *gate, const float *up, float *out, int8_t *qs, float *d, int n) {
+    silu_mul_quant_rm(gate, up, out, qs, d, n, nullptr);
 }
 void llamd_fwd_moe_combine(const float *down, const float *weights, float *out, int n_used, int n_embd) {
     moe_combine_kernel<<<dim3((n_embd + 255) / 256, 1), 256, 0, stream()>>>(down, weights, nullptr, out, n_used, n_embd);
