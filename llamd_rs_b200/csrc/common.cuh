@@ -213,6 +213,8 @@ struct MatvecPlans {
     // L2 instead of reading them from HBM again. Produced by slot_order_launch; must be complete when the ids are.
     const int32_t *slot_order;
 };
+// A tile's scatter plan, pairs in any order within an expert. One small launch.
+void moe_plan_launch(const int32_t *ids, int npair, int n_expert, int n_used, int32_t *gstart, int32_t *gcount, int32_t *ptoken, int32_t *pslot);
 // order[] = the slots 0..n_slots-1 sorted by ids[slot]. One small launch.
 void slot_order_launch(const int32_t *ids, int n_slots, int n_expert, int32_t *order);
 

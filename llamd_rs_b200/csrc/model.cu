@@ -1569,9 +1569,13 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
                                     nu, T);
             continue;
         }
-        // the expert scatter plan: (token, slot) pairs sorted by expert
-        llamd_fwd_moe_group_work(p.ids.as<int32_t>(), ne, nu, T, p.gstart.as<int32_t>(), p.gcount.as<int32_t>(), p.ptoken.as<int32_t>(),
-                                 p.pslot.as<int32_t>(), p.work.as<int32_t>(), p.n_work.as<int32_t>());
+        // the expert scatter plan: (token, slot) pairs sorted by expert (the dp4a path's work list comes from the stable one)
+        if (gemm)
+            moe_plan_launch(p.ids.as<int32_t>(), T * nu, ne, nu, p.gstart.as<int32_t>(), p.gcount.as<int32_t>(), p.ptoken.as<int32_t>(),
+                            p.pslot.as<int32_t>());
+        else
+            llamd_fwd_moe_group_work(p.ids.as<int32_t>(), ne, nu, T, p.gstart.as<int32_t>(), p.gcount.as<int32_t>(), p.ptoken.as<int32_t>(),
+                                     p.pslot.as<int32_t>(), p.work.as<int32_t>(), p.n_work.as<int32_t>());
         if (tc) {
             llamd_fwd_act_f16_rm(p.aq.as<int8_t>(), p.ad.as<float>(), p.aq_rm.p, (size_t)T * eb);
             llamd_fwd_expert_gemm_tc(l.gate_exps.p, l.up_exps.p, p.gstart.as<int32_t>(), p.gcount.as<int32_t>(), p.ptoken.as<int32_t>(),

@@ -1668,6 +1668,62 @@ __global__ void __launch_bounds__(512) slot_order_kernel(const int32_t *__restri
     for (int i = tid; i < n_slots; i += blockDim.x) order[atomicAdd(&s_at[expert(i)], 1)] = i;
 }
 
+// The scatter plan of a tile whose pairs may stand in any order within an expert (each pair has its own output row): gstart,
+// gcount, and the pairs by expert. The kernel below keeps the reference's stable order, which it pays for with ranks in
+// registers and a walk over all warps' counts: 11.5 us for 128 tokens of 8 experts, 17.7 for 512; this 7.6 for 512.
+__global__ void __launch_bounds__(1024) moe_plan_kernel(const int32_t *__restrict__ ids, int npair, int n_expert, int n_used, int32_t *__restrict__ gstart,
+                                                        int32_t *__restrict__ gcount, int32_t *__restrict__ ptoken, int32_t *__restrict__ pslot) {
+    __shared__ int s_at[1024];
+    pdl_trigger();
+    const int tid = threadIdx.x;
+    s_at[tid] = 0;
+    pdl_wait();
+    __syncthreads();
+    auto expert = [&](int e) { return e < 0 || e >= n_expert ? 0 : e; };
+    for (int i0 = 0; i0 < npair; i0 += 4 * 1024) {
+        int e[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) e[u] = i0 + u * 1024 + tid < npair ? ids[i0 + u * 1024 + tid] : -2;
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (i0 + u * 1024 + tid < npair) atomicAdd(&s_at[expert(e[u])], 1);
+    }
+    __syncthreads();
+    if (tid < 32) {
+        int start = 0;
+        for (int e0 = 0; e0 < n_expert; e0 += 32) {
+            const int e = e0 + tid, c = e < n_expert ? s_at[e] : 0;
+            int incl = c;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, off);
+                if (tid >= off) incl += v;
+            }
+            if (e < n_expert) {
+                s_at[e] = start + incl - c;
+                gstart[e] = start + incl - c;
+                gcount[e] = c;
+            }
+            start += __shfl_sync(0xffffffffu, incl, 31);
+        }
+    }
+    __syncthreads();
+    for (int i0 = 0; i0 < npair; i0 += 4 * 1024) {
+        int e[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) e[u] = i0 + u * 1024 + tid < npair ? ids[i0 + u * 1024 + tid] : -2;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int i = i0 + u * 1024 + tid;
+            if (i < npair) {
+                const int at = atomicAdd(&s_at[expert(e[u])], 1);
+                ptoken[at] = i / n_used;
+                pslot[at] = i;
+            }
+        }
+    }
+}
+
 // ---- argmax, lowest index on a tie (llamd_forward.hip:353-389) -------------
 __device__ __forceinline__ void argmax_combine(float &v, int &i, float ov, int oi) {
     if (ov > v || (ov == v && oi < i)) {
@@ -2460,6 +2516,13 @@ void llamd_fwd_moe_group(const int32_t *ids, int n_expert, int n_used, int nseq,
 
 }  // extern "C"
 
+void llamd::moe_plan_launch(const int32_t *ids, int npair, int n_expert, int n_used, int32_t *gstart, int32_t *gcount, int32_t *ptoken, int32_t *pslot) {
+    if (n_expert < 1 || n_expert > 1024 || npair < 1 || n_used < 1) {
+        set_error_msg("moe_plan: 1..1024 experts, at least one pair");
+        return;
+    }
+    launch_k("moe_plan", moe_plan_kernel, dim3(1), dim3(1024), 0, ids, npair, n_expert, n_used, gstart, gcount, ptoken, pslot);
+}
 void llamd::slot_order_launch(const int32_t *ids, int n_slots, int n_expert, int32_t *order) {
     if (n_slots < 1 || n_expert < 1 || n_expert > 1024) {
         set_error_msg("slot_order: at least one slot, 1..1024 experts");
