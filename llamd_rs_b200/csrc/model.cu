@@ -1312,6 +1312,7 @@ static bool prefill_alloc(Model &m, int tile) {
         m.err = "prefill: the tile buffers have been shared with the other ranks and cannot grow (set prefill_tile before the attach)";
         return false;
     }
+    p.tile = 0;  // until every new buffer is there: a growth that fails leaves no tile behind, and the next call allocates again
     for (Buf *b : {&p.x, &p.xb, &p.xb2, &p.q, &p.k, &p.v, &p.attn, &p.aq, &p.ad, &p.aq2, &p.ad2, &p.ids, &p.w, &p.logits, &p.counter,
                    &p.gate, &p.up, &p.down, &p.scores, &p.meta, &p.gstart, &p.gcount, &p.ptoken, &p.pslot, &p.work, &p.n_work, &p.aq_rm,
                    &p.aq2_rm})
@@ -1355,7 +1356,7 @@ static bool prefill_alloc(Model &m, int tile) {
 static bool prefill_alloc_all_logits(Model &m, bool own_logits) {
     Model::Prefill &p = m.pf;
     const size_t T = p.tile;
-    if (p.out_tokens.p && p.out_tokens.bytes >= T * 4 && (!own_logits || (p.logits_all.p && p.logits_all.bytes >= T * (size_t)m.hp.n_vocab * 4))) return true;
+    if (p.h_out_tokens && p.out_tokens.p && p.out_tokens.bytes >= T * 4 && (!own_logits || (p.logits_all.p && p.logits_all.bytes >= T * (size_t)m.hp.n_vocab * 4))) return true;
     for (Buf *b : {&p.amax_v, &p.amax_i, &p.out_tokens}) b->release();
     if (own_logits) p.logits_all.release();
     if (p.h_out_tokens) cudaFreeHost(p.h_out_tokens);

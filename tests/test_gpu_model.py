@@ -384,3 +384,55 @@ def test_prefill_equals_sequential_decode(tiny):
     with pytest.raises(backend.Malformed):
         gm.prefill([], 0)
     gm.prefill_tile = 512
+
+
+class _FullDevice:
+    """All but `leave` bytes of the device's free memory taken, in as few allocations as it allows."""
+
+    def __init__(self, leave):
+        from llamd_rs_b200 import backend
+        from llamd_rs_b200._lib import lib
+
+        self.L, self.held = lib(), []
+        for size in (8 << 30, 1 << 30, 128 << 20, 16 << 20, 2 << 20):
+            while backend.free_memory() >= leave + size:
+                p = self.L.llamd_fwd_alloc(size)
+                if not p:
+                    self.L.llamd_fwd_last_error()  # (refused: smaller pieces)
+                    break
+                self.held.append(p)
+
+    def release(self):
+        for p in self.held:
+            self.L.llamd_fwd_free(p)
+        self.held = []
+
+
+def test_prefill_after_a_failed_growth():
+    """Tile buffers that could not grow for a long prompt: the call is refused, and the next prompt, whose tile is no larger
+    than the old one, allocates again instead of running on what was released."""
+    from llamd_rs_b200 import backend, synth
+    from llamd_rs_b200._lib import lib
+    from llamd_rs_b200.model import CudaModel
+
+    hp = dict(synth.TINY, n_layer=1, n_ff_expert=2048)
+    gm = CudaModel.load_batched(hp, synth.make_model(hp, seed=9), max_kv=4096, max_seq=1)
+    try:
+        toks = synth.token_ids(4096, hp["n_vocab"], 3, "growth").tolist()
+        gm.prefill_tile = 16
+        want = gm.prefill(toks[:20], 0), gm.logits()[0].view(np.uint32).copy()
+        gm.verify(toks[:9], 0)
+        gm.prefill_tile = 4096
+        full = _FullDevice(96 << 20)  # (the buffers of 4096 tokens take 300 MB)
+        try:
+            with pytest.raises(backend.Other):
+                gm.prefill(toks, 0)
+        finally:
+            full.release()
+        lib().llamd_fwd_last_error()
+        gm.prefill_tile = 16
+        got = gm.prefill(toks[:20], 0), gm.logits()[0].view(np.uint32).copy()
+        assert got[0] == want[0] and np.array_equal(got[1], want[1])
+        assert gm.verify(toks[:20], 0)[-1] == want[0]
+    finally:
+        gm.free()
