@@ -1273,6 +1273,7 @@ constexpr int kAutoTile = 2048;
 // Attention of a tile runs this many tokens at a time: its score buffer is [tokens][heads][max_kv] floats, and 512 tokens
 // already are thousands of CTAs.
 constexpr int kAttnTokens = 512;
+constexpr int kVerifyRows = 64;   // tokens of a verification tile: every one's logits are kept, 0.6 MB each at 151936
 constexpr int kGroupMaxPairs = 40960;  // what one scatter plan takes (ops.cu: moe_group_kernel)
 
 // The folded copies of the expert matrices (option "prefill_prefold"), made once all tensors are there.
@@ -1353,9 +1354,11 @@ static bool prefill_alloc(Model &m, int tile) {
     return true;
 }
 
-static bool prefill_alloc_all_logits(Model &m, bool own_logits) {
+// The buffers of a pass that keeps every row's pick: `rows` of them, and with own_logits their logits. They grow with what is
+// asked for, not with the tile: an automatic tile of 2048 tokens would make the logits of 64 verified ones 1.2 GB.
+static bool prefill_alloc_all_logits(Model &m, int rows, bool own_logits) {
     Model::Prefill &p = m.pf;
-    const size_t T = p.tile;
+    const size_t T = rows;
     if (p.h_out_tokens && p.out_tokens.p && p.out_tokens.bytes >= T * 4 && (!own_logits || (p.logits_all.p && p.logits_all.bytes >= T * (size_t)m.hp.n_vocab * 4))) return true;
     for (Buf *b : {&p.amax_v, &p.amax_i, &p.out_tokens}) b->release();
     if (own_logits) p.logits_all.release();
@@ -1723,9 +1726,9 @@ int llamd_model_verify(llamd_model *h, const int32_t *tokens, int n_tokens, int 
         }
     if (!check_ready(*m)) return -1;
     int tile = m->prefill_tile < 1 ? 1 : m->prefill_tile;
-    if (tile > 64) tile = 64;  // every token's logits are kept: 0.6 MB each
+    if (tile > kVerifyRows) tile = kVerifyRows;
     if (tile > n_tokens) tile = n_tokens;
-    if (!prefill_alloc(*m, tile) || !prefill_alloc_all_logits(*m, true)) return -1;
+    if (!prefill_alloc(*m, tile) || !prefill_alloc_all_logits(*m, m->pf.tile < kVerifyRows ? m->pf.tile : kVerifyRows, true)) return -1;
     for (int t0 = 0; t0 < n_tokens; t0 += tile) {
         const int T = n_tokens - t0 < tile ? n_tokens - t0 : tile;
         if (llamd_fwd_sync() != 0) return -1;  // the pinned staging is reused per tile
@@ -1773,7 +1776,7 @@ static int run_wide_batch(Model &m, const int32_t *tokens, const int32_t *positi
         m.err = "forward_batch: too many (sequence, expert) pairs for one scatter plan";
         return -1;
     }
-    if (!prefill_alloc(m, nseq) || !prefill_alloc_all_logits(m, false)) return -1;
+    if (!prefill_alloc(m, nseq) || !prefill_alloc_all_logits(m, m.pf.tile < LLAMD_MAX_BATCH ? m.pf.tile : LLAMD_MAX_BATCH, false)) return -1;
     if (folded_tile(m, nseq) && !ensure_folded(m, nseq)) return -1;
     if (llamd_fwd_sync() != 0) return -1;
     int n_kv_max = 0;

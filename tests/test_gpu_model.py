@@ -436,3 +436,24 @@ def test_prefill_after_a_failed_growth():
         assert gm.verify(toks[:20], 0)[-1] == want[0]
     finally:
         gm.free()
+
+
+def test_verify_buffers_do_not_follow_the_prompt_tile():
+    """A verification keeps the logits of at most 64 tokens, however large the tile of the prompt before it was."""
+    from llamd_rs_b200 import backend, synth
+    from llamd_rs_b200.model import CudaModel
+
+    hp = dict(synth.TINY, n_layer=1, n_vocab=32768)
+    gm = CudaModel.load_batched(hp, synth.make_model(hp, seed=9), max_kv=2048, max_seq=1)
+    try:
+        toks = synth.token_ids(2048, hp["n_vocab"], 3, "verify memory").tolist()
+        gm.set_option("head_gemm", 0)  # (no folded copy of the head in the figures below)
+        gm.set_option("dense_gemm", 0)
+        gm.prefill(toks[:80], 0)
+        want = list(gm.verify(toks[:80], 0))
+        gm.prefill(toks, 0)  # one tile of 2048
+        free = backend.free_memory()
+        assert list(gm.verify(toks[:80], 0)) == want
+        assert free - backend.free_memory() <= 64 * 4 * hp["n_vocab"] + (8 << 20)
+    finally:
+        gm.free()
