@@ -708,6 +708,20 @@ bool check_ready(Model &m) {
     return true;
 }
 
+// Attention of a tile runs this many tokens at a time: its score buffer is [tokens][heads][max_kv] floats, and 512 tokens
+// already are thousands of CTAs.
+constexpr int kAttnTokens = 512;
+
+// What the buffers of a tile of T tokens take on one GPU (prefill_alloc), with what the allocator rounds up.
+size_t prefill_bytes(const Model &m, size_t T) {
+    const llamd_hparams &hp = m.hp;
+    const size_t E = hp.n_embd, qd = (size_t)hp.n_head * hp.head_dim, kvd = (size_t)hp.n_head_kv * hp.head_dim, nu = hp.n_expert_used,
+                 ffe = hp.n_ff_expert, act = E > qd ? E : qd;
+    const size_t per_token = 4 * (3 * E + 2 * qd + 2 * kvd + 2 * hp.n_expert + 8 * nu + 4) + 6 * act + nu * (4 * E + 14 * ffe);
+    const size_t scores = (T < kAttnTokens ? T : kAttnTokens) * hp.n_head * (size_t)((m.max_kv + 3) & ~3) * 4;
+    return T * per_token + scores + 30 * ((size_t)2 << 20);  // (30 buffers, 2 MB pages)
+}
+
 // The folded copies that a pass over n sequences, or a small tile of n tokens, multiplies with (options "dense_gemm" and
 // "head_gemm"), made once and not inside a capture; without the memory for them the matvec serves every pass. False: an error.
 bool ensure_folded(Model &m, int n, bool head = true) {
@@ -1270,9 +1284,6 @@ int llamd_model_forward_batch(llamd_model *h, const int32_t *tokens, const int32
 // shapes, four to one in tokens). Beyond 2048 the folding is a tenth of the work and the buffers (gate, up, down: 230 MB
 // at 2048) grow on.
 constexpr int kAutoTile = 2048;
-// Attention of a tile runs this many tokens at a time: its score buffer is [tokens][heads][max_kv] floats, and 512 tokens
-// already are thousands of CTAs.
-constexpr int kAttnTokens = 512;
 constexpr int kVerifyRows = 64;   // tokens of a verification tile: every one's logits are kept, 0.6 MB each at 151936
 constexpr int kGroupMaxPairs = 40960;  // what one scatter plan takes (ops.cu: moe_group_kernel)
 
@@ -1308,7 +1319,6 @@ static bool prefill_alloc(Model &m, int tile) {
     if (!ensure_prefold(m)) return false;
     Model::Prefill &p = m.pf;
     if (p.tile >= tile) return true;
-    if (tile > m.prefill_tile) tile = (tile + 511) & ~511;  // (a tile beyond the caller's: prompts that grow re-allocate four times at most)
     if (p.ep_cap) {
         m.err = "prefill: the tile buffers have been shared with the other ranks and cannot grow (set prefill_tile before the attach)";
         return false;
@@ -1375,14 +1385,10 @@ static bool prefill_alloc_all_logits(Model &m, int rows, bool own_logits) {
 // than full ones and a small rest that costs nearly as much per layer. A tile beyond prefill_tile has to fit the free memory
 // with room to spare.
 static int auto_tile(const Model &m, int n_tokens) {
-    const llamd_hparams &hp = m.hp;
-    int cap = kAutoTile < kGroupMaxPairs / hp.n_expert_used ? kAutoTile : kGroupMaxPairs / hp.n_expert_used;
+    int cap = kAutoTile < kGroupMaxPairs / m.hp.n_expert_used ? kAutoTile : kGroupMaxPairs / m.hp.n_expert_used;
     if (cap < m.prefill_tile) return m.prefill_tile;
     if (n_tokens > m.prefill_tile && n_tokens > m.pf.tile) {
-        const size_t E = hp.n_embd, qd = (size_t)hp.n_head * hp.head_dim, kvd = (size_t)hp.n_head_kv * hp.head_dim, nu = hp.n_expert_used,
-                     ffe = hp.n_ff_expert, act = E > qd ? E : qd;
-        const size_t per_token = 4 * (3 * E + 2 * qd + 2 * kvd + 2 * hp.n_expert + 4 * nu) + 6 * act + nu * (4 * E + 14 * ffe);
-        if ((size_t)cap * per_token + ((size_t)1 << 30) > llamd_cuda_free_mem()) cap = m.prefill_tile > m.pf.tile ? m.prefill_tile : m.pf.tile;
+        if (prefill_bytes(m, cap) + ((size_t)1 << 30) > llamd_cuda_free_mem()) cap = m.prefill_tile > m.pf.tile ? m.prefill_tile : m.pf.tile;
         if (cap > kAutoTile) cap = kAutoTile;
     }
     const int n = (n_tokens + cap - 1) / cap;
@@ -1666,6 +1672,17 @@ int llamd_model_prefill(llamd_model *h, const int32_t *tokens, int n_tokens, int
     if (!m->prefill_tile_set && m->ep_world == 1) tile = auto_tile(*m, n_tokens);
     if (m->ep_world > 1 && tile > m->pf.ep_cap) tile = m->pf.ep_cap;
     if (tile > n_tokens) tile = n_tokens;
+    if (tile > m->prefill_tile) {
+        // an automatic tile: buffers for whole 512s of tokens (prompts that grow re-allocate four times at most), and the
+        // ordinary tile if they cannot be had after all
+        const bool clean = error_code() == 0;
+        if (!prefill_alloc(*m, (tile + 511) & ~511)) {
+            if (!clean) return -1;
+            llamd_fwd_last_error();
+            m->err.clear();
+            tile = m->prefill_tile;
+        }
+    }
     if (!prefill_alloc(*m, tile)) return -1;
     for (int t0 = 0; t0 < n_tokens; t0 += tile) {
         const int T = n_tokens - t0 < tile ? n_tokens - t0 : tile;

@@ -457,3 +457,26 @@ def test_verify_buffers_do_not_follow_the_prompt_tile():
         assert free - backend.free_memory() <= 64 * 4 * hp["n_vocab"] + (8 << 20)
     finally:
         gm.free()
+
+
+def test_automatic_tile_counts_the_score_buffer():
+    """A long context's score buffer is most of what a tile takes. With memory for a tile of 512 tokens but not of 2048, a
+    prompt that never chose a tile runs, and gives what it gives with memory to spare."""
+    from llamd_rs_b200 import synth
+    from llamd_rs_b200.model import CudaModel
+
+    hp = dict(synth.TINY, n_layer=1, n_embd=512, n_head=16, n_head_kv=1, n_expert_used=8, n_ff_expert=1024)
+    w = synth.make_model(hp, seed=9)
+    toks = synth.token_ids(2000, hp["n_vocab"], 3, "score buffer").tolist()
+    runs = []
+    for tight in (False, True):
+        gm = CudaModel.load_batched(hp, w, max_kv=40000, max_seq=1)
+        # (scores 1.31 GB, the rest of a tile of 512 tokens 0.08 GB, of 2048 0.31 GB)
+        full = _FullDevice(1540 << 20) if tight else None
+        try:
+            runs.append((gm.prefill(toks, 0), gm.logits()[0].view(np.uint32).copy()))
+        finally:
+            if full:
+                full.release()
+            gm.free()
+    assert runs[0][0] == runs[1][0] and np.array_equal(runs[0][1], runs[1][1])
