@@ -133,7 +133,7 @@ struct Layer {
     Buf attn_norm, attn_q, attn_k, attn_v, attn_q_norm, attn_k_norm, attn_out, ffn_norm, ffn_gate_inp;
     Buf gate_exps, up_exps, down_exps;
     Buf gate_fold, up_fold, down_fold;  // option "prefill_prefold": the expert matrices folded once for the prefill GEMM
-    Buf q_fold, k_fold, v_fold, o_fold;  // option "dense_gemm": the attention projections folded for batched decode
+    uint8_t *q_fold = nullptr, *k_fold = nullptr, *v_fold = nullptr, *o_fold = nullptr;  // option "dense_gemm": the attention projections folded, in Model::dense_fold
     bool has_q_norm = false, has_k_norm = false;
     Buf kc, vc;
 };
@@ -205,7 +205,9 @@ struct Model {
                                 // 32: 1810 / 1247, 40: 1797 / 1446, 48: 1882 / 1649, 64: 1968 / 2048, 80: 1972 / 2330
     int dense_gemm = 8;      // option "dense_gemm" = n: from n sequences per pass the attention projections run on the integer GEMM over folded
                              // copies of their matrices (as "head_gemm"; +2 bytes per weight of the four matrices of every layer); 0: never
+    Buf dense_fold;          // the folded projections of all layers
     bool dense_fold_ready = false, dense_fold_failed = false;
+    bool prompt_no_dense = false, prompt_no_head = false;  // a prompt found too little memory free to make these copies (a batch may still)
     int head_gemm = 4;       // option "head_gemm" = n: from n sequences per pass the output projection runs on the integer GEMM over a folded
                              // copy of the matrix (2 bytes per weight once per pass, where the matvec repeats its integer work per sequence;
                              // +0.6 GB for a 151936 x 2048 matrix, made at the first such pass); 0: never
@@ -481,7 +483,7 @@ void queue_token(Model &m, int nseq) {
             mark(LLAMD_PH_ATTN_NORM);
             if (dense_gemm) {
                 // a batch: the folded matrices once for all the sequences, on the integer tensor path (the same bits)
-                gemm_tokens_folded3(l.q_fold.p, l.k_fold.p, l.v_fold.p, m.head_rm.p, m.ad.as<float>(), m.q.as<float>(), m.k.as<float>(),
+                gemm_tokens_folded3(l.q_fold, l.k_fold, l.v_fold, m.head_rm.p, m.ad.as<float>(), m.q.as<float>(), m.k.as<float>(),
                                     m.v.as<float>(), eb, qd, kvd, kvd, nseq);
             } else {
                 matvec_x3_batch(plan_static(m, &l.attn_out), l.attn_q.p, l.attn_k.p, l.attn_v.p, m.aq.as<int8_t>(), m.ad.as<float>(),
@@ -530,7 +532,7 @@ void queue_token(Model &m, int nseq) {
         mark(LLAMD_PH_QUANT);
         if (dense_gemm) {
             if (!rm_made) llamd_fwd_q8k_residue_major(m.aq.as<int8_t>(), m.head_rm.p, (size_t)nseq * (qd / 256));
-            gemm_tokens_folded(l.o_fold.p, m.head_rm.p, m.ad.as<float>(), m.xb2.as<float>(), qd / 256, E, nseq);
+            gemm_tokens_folded(l.o_fold, m.head_rm.p, m.ad.as<float>(), m.xb2.as<float>(), qd / 256, E, nseq);
         } else {
             matvec_batch(plan_static(m, &l.ffn_gate_inp), l.attn_out.p, m.aq.as<int8_t>(), m.ad.as<float>(), m.xb2.as<float>(), qd / 256, E,
                          nseq);
@@ -723,41 +725,66 @@ size_t prefill_bytes(const Model &m, size_t T) {
 }
 
 // The folded copies that a pass over n sequences, or a small tile of n tokens, multiplies with (options "dense_gemm" and
-// "head_gemm"), made once and not inside a capture; without the memory for them the matvec serves every pass. False: an error.
-bool ensure_folded(Model &m, int n, bool head = true) {
+// "head_gemm"), made once and not inside a capture; without the memory for them the matvec serves every pass. They stay, so
+// a prompt or a draft (`prompt` tokens per tile that it may take) makes them only where a full tile's buffers fit beside them.
+// False: an error. The projections of a 48-layer model (1.9 GB, one allocation) cost the first prompt of 8 tokens or more 5 ms;
+// with four allocations per layer it was 66.
+bool ensure_folded(Model &m, int n, int prompt = 0, bool head = true) {
     const llamd_hparams &hp = m.hp;
     const int eb = hp.n_embd / 256, qd = hp.n_head * hp.head_dim, kvd = hp.n_head_kv * hp.head_dim;
-    if (m.dense_gemm && n >= m.dense_gemm && !m.dense_fold_ready && !m.dense_fold_failed) {
-        const size_t need = (size_t)hp.n_layer * (expert_fold_bytes(eb, qd, 1) + 2 * expert_fold_bytes(eb, kvd, 1) + expert_fold_bytes(qd / 256, hp.n_embd, 1));
-        bool ok = qd % 256 == 0 && need + ((size_t)1 << 30) <= llamd_cuda_free_mem();
-        for (size_t i = 0; ok && i < m.layers.size(); i++) {
-            Layer &l = m.layers[i];
-            ok = l.q_fold.alloc(expert_fold_bytes(eb, qd, 1)) && l.k_fold.alloc(expert_fold_bytes(eb, kvd, 1)) &&
-                 l.v_fold.alloc(expert_fold_bytes(eb, kvd, 1)) && l.o_fold.alloc(expert_fold_bytes(qd / 256, hp.n_embd, 1));
-            if (!ok) break;
-            expert_prefold(l.attn_q.p, l.q_fold.p, eb, qd, 1);
-            expert_prefold(l.attn_k.p, l.k_fold.p, eb, kvd, 1);
-            expert_prefold(l.attn_v.p, l.v_fold.p, eb, kvd, 1);
-            expert_prefold(l.attn_out.p, l.o_fold.p, qd / 256, hp.n_embd, 1);
-        }
-        m.dense_fold_ready = ok && llamd_fwd_sync() == 0;
-        if (!m.dense_fold_ready) {
-            for (auto &l : m.layers)
-                for (Buf *b : {&l.q_fold, &l.k_fold, &l.v_fold, &l.o_fold}) b->release();
+    const bool clean = error_code() == 0;
+    auto room = [&](size_t need) {
+        const size_t tile = prompt > m.pf.tile ? prefill_bytes(m, prompt) : 0;
+        return need + tile + ((size_t)1 << 30) <= llamd_cuda_free_mem();
+    };
+    auto failed = [&](Buf &b) {  // (an allocation that was refused is no error of the pass)
+        b.release();
+        if (clean) llamd_fwd_last_error();
+    };
+    if (m.dense_gemm && n >= m.dense_gemm && !m.dense_fold_ready && !m.dense_fold_failed && !(prompt && m.prompt_no_dense)) {
+        auto padded = [](size_t b) { return (b + 255) & ~(size_t)255; };
+        const size_t q = padded(expert_fold_bytes(eb, qd, 1)), kv = padded(expert_fold_bytes(eb, kvd, 1)),
+                     o = padded(expert_fold_bytes(qd / 256, hp.n_embd, 1)), layer = q + 2 * kv + o;
+        if (!room(hp.n_layer * layer)) {
+            (prompt ? m.prompt_no_dense : m.dense_fold_failed) = true;
+        } else if (!m.dense_fold.alloc(hp.n_layer * layer)) {
+            failed(m.dense_fold);
             m.dense_fold_failed = true;
-            if (error_code() != 0) return false;
+        } else {
+            for (size_t i = 0; i < m.layers.size(); i++) {
+                Layer &l = m.layers[i];
+                l.q_fold = m.dense_fold.as<uint8_t>() + i * layer;
+                l.k_fold = l.q_fold + q;
+                l.v_fold = l.k_fold + kv;
+                l.o_fold = l.v_fold + kv;
+                expert_prefold(l.attn_q.p, l.q_fold, eb, qd, 1);
+                expert_prefold(l.attn_k.p, l.k_fold, eb, kvd, 1);
+                expert_prefold(l.attn_v.p, l.v_fold, eb, kvd, 1);
+                expert_prefold(l.attn_out.p, l.o_fold, qd / 256, hp.n_embd, 1);
+            }
+            m.dense_fold_ready = llamd_fwd_sync() == 0;
+            if (!m.dense_fold_ready) {
+                m.dense_fold.release();
+                m.dense_fold_failed = true;
+                return false;
+            }
         }
     }
-    if (head && m.head_gemm && n >= m.head_gemm && !m.head_fold_ready && !m.head_fold_failed) {
+    if (head && m.head_gemm && n >= m.head_gemm && !m.head_fold_ready && !m.head_fold_failed && !(prompt && m.prompt_no_head)) {
         const size_t need = expert_fold_bytes(eb, hp.n_vocab, 1);
-        if (need + ((size_t)1 << 30) <= llamd_cuda_free_mem() && m.head_fold.alloc(need)) {
+        if (!room(need)) {
+            (prompt ? m.prompt_no_head : m.head_fold_failed) = true;
+        } else if (!m.head_fold.alloc(need)) {
+            failed(m.head_fold);
+            m.head_fold_failed = true;
+        } else {
             expert_prefold(m.output.p ? m.output.p : m.tok_embd.p, m.head_fold.p, eb, hp.n_vocab, 1);
             m.head_fold_ready = llamd_fwd_sync() == 0;
-        }
-        if (!m.head_fold_ready) {
-            m.head_fold.release();
-            m.head_fold_failed = true;
-            if (error_code() != 0) return false;
+            if (!m.head_fold_ready) {
+                m.head_fold.release();
+                m.head_fold_failed = true;
+                return false;
+            }
         }
     }
     return true;
@@ -922,11 +949,10 @@ void llamd_model_free(llamd_model *h) {
     }
     for (auto &l : m->layers)
         for (Buf *b : {&l.attn_norm, &l.attn_q, &l.attn_k, &l.attn_v, &l.attn_q_norm, &l.attn_k_norm, &l.attn_out, &l.ffn_norm,
-                       &l.ffn_gate_inp, &l.gate_exps, &l.up_exps, &l.down_exps, &l.gate_fold, &l.up_fold, &l.down_fold, &l.q_fold, &l.k_fold,
-                       &l.v_fold, &l.o_fold, &l.kc, &l.vc})
+                       &l.ffn_gate_inp, &l.gate_exps, &l.up_exps, &l.down_exps, &l.gate_fold, &l.up_fold, &l.down_fold, &l.kc, &l.vc})
             b->release();
     for (Buf *b : {&m->tok_embd, &m->output_norm, &m->output, &m->rope_tab, &m->x, &m->xb, &m->xb2, &m->q, &m->k, &m->v, &m->attn,
-                   &m->aq, &m->ad, &m->aq2, &m->ad2, &m->router_logits, &m->router_probs, &m->expert_ids, &m->slot_order, &m->head_fold, &m->head_rm, &m->expert_w, &m->e_gate,
+                   &m->aq, &m->ad, &m->aq2, &m->ad2, &m->router_logits, &m->router_probs, &m->expert_ids, &m->slot_order, &m->head_fold, &m->dense_fold, &m->head_rm, &m->expert_w, &m->e_gate,
                    &m->e_up, &m->e_down, &m->logits, &m->amax_v, &m->amax_i, &m->out_token, &m->meta, &m->trace_x, &m->trace_ids,
                    &m->tok_log, &m->tok_count, &m->router_counter, &m->tail_counter, &m->scores, &m->ids_all, &m->ad_all, &m->aq_all, &m->gate_all,
                    &m->up_all, &m->aq2_all, &m->ad2_all, &m->down_all, &m->recv_all, &m->ep_arrive, &m->ep_status, &m->ep_out_tab,
@@ -983,8 +1009,7 @@ int llamd_model_set_tensor(llamd_model *h, int layer, int which, size_t first_bl
         if ((which == LLAMD_T_ATTN_Q || which == LLAMD_T_ATTN_K || which == LLAMD_T_ATTN_V || which == LLAMD_T_ATTN_OUT) &&
             (m->dense_fold_ready || m->dense_fold_failed)) {  // the folded copies are of the old bytes
             if (g_graph_owner == m->id) llamd_fwd_graph_destroy();
-            for (auto &ll : m->layers)
-                for (Buf *b : {&ll.q_fold, &ll.k_fold, &ll.v_fold, &ll.o_fold}) b->release();
+            m->dense_fold.release();
             m->dense_fold_ready = m->dense_fold_failed = false;
         }
         switch (which) {
@@ -1381,11 +1406,19 @@ static bool prefill_alloc_all_logits(Model &m, int rows, bool own_logits) {
     return ok;
 }
 
+static int auto_tile_cap(const Model &m) {
+    return kAutoTile < kGroupMaxPairs / m.hp.n_expert_used ? kAutoTile : kGroupMaxPairs / m.hp.n_expert_used;
+}
+// The tokens of the largest tile that a prompt may still ask for.
+static int full_tile(const Model &m) {
+    const int cap = m.prefill_tile_set || auto_tile_cap(m) < m.prefill_tile ? m.prefill_tile : auto_tile_cap(m);
+    return cap < m.max_kv ? cap : m.max_kv;
+}
 // The tile of a caller that never chose one: as few tiles as kAutoTile allows and the same number of tokens in each, rather
 // than full ones and a small rest that costs nearly as much per layer. A tile beyond prefill_tile has to fit the free memory
 // with room to spare.
 static int auto_tile(const Model &m, int n_tokens) {
-    int cap = kAutoTile < kGroupMaxPairs / m.hp.n_expert_used ? kAutoTile : kGroupMaxPairs / m.hp.n_expert_used;
+    int cap = auto_tile_cap(m);
     if (cap < m.prefill_tile) return m.prefill_tile;
     if (n_tokens > m.prefill_tile && n_tokens > m.pf.tile) {
         if (prefill_bytes(m, cap) + ((size_t)1 << 30) > llamd_cuda_free_mem()) cap = m.prefill_tile > m.pf.tile ? m.prefill_tile : m.pf.tile;
@@ -1431,10 +1464,10 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
     const bool small = small_tile(m, T, multi_seq);
     const bool folded = folded_tile(m, T) && m.dense_gemm && T >= m.dense_gemm && m.dense_fold_ready;
     // up to three dense matrices of a small or folded tile against the activations in p.aq / p.ad
-    auto small_dense = [&](const Buf &f0, const Buf &f1, const Buf &f2, const Buf &w0, const Buf &w1, const Buf &w2, const Buf &o0, const Buf &o1,
+    auto small_dense = [&](const void *f0, const void *f1, const void *f2, const Buf &w0, const Buf &w1, const Buf &w2, const Buf &o0, const Buf &o1,
                            const Buf &o2, int blocks, int rows0, int rows12) {
         if (folded) {
-            gemm_tokens_folded3(f0.p, f1.p, f2.p, p.aq_rm.p, p.ad.as<float>(), o0.as<float>(), o1.as<float>(), o2.as<float>(), blocks, rows0, rows12,
+            gemm_tokens_folded3(f0, f1, f2, p.aq_rm.p, p.ad.as<float>(), o0.as<float>(), o1.as<float>(), o2.as<float>(), blocks, rows0, rows12,
                                 rows12, T);
         } else if (w1.p) {
             matvec_x3_batch(MatvecPlans{}, w0.p, w1.p, w2.p, p.aq.as<int8_t>(), p.ad.as<float>(), o0.as<float>(), o1.as<float>(), o2.as<float>(),
@@ -1517,7 +1550,7 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
         }
         quantize_rm(p.attn.as<float>(), p.aq.as<int8_t>(), p.ad.as<float>(), T * (qd / 256), rm);
         if (small || folded) {
-            small_dense(l.o_fold, none, none, l.attn_out, none, none, p.xb2, none, none, qd / 256, E, 0);
+            small_dense(l.o_fold, nullptr, nullptr, l.attn_out, none, none, p.xb2, none, none, qd / 256, E, 0);
         } else if (tc) {
             llamd_fwd_act_f16_rm(p.aq.as<int8_t>(), p.ad.as<float>(), p.aq_rm.p, (size_t)T * (qd / 256));
             llamd_fwd_gemm_tokens_tc(l.attn_out.p, nullptr, nullptr, p.aq_rm.p, p.xb2.as<float>(), nullptr, nullptr, qd / 256, E, 0, 0, T);
@@ -1695,7 +1728,7 @@ int llamd_model_prefill(llamd_model *h, const int32_t *tokens, int n_tokens, int
             set_error(cudaGetLastError(), "prefill meta H2D");
             return -1;
         }
-        if (folded_tile(*m, T) && !ensure_folded(*m, T, false)) return -1;
+        if (folded_tile(*m, T) && !ensure_folded(*m, T, full_tile(*m), false)) return -1;
         queue_prefill_tile(*m, T, base_pos + t0 + T, t0 + T >= n_tokens);
     }
     if (cudaMemcpyAsync(m->h_out, m->out_token.p, 4, cudaMemcpyDeviceToHost, stream()) != cudaSuccess) return -1;
@@ -1757,7 +1790,7 @@ int llamd_model_verify(llamd_model *h, const int32_t *tokens, int n_tokens, int 
             set_error(cudaGetLastError(), "verify meta H2D");
             return -1;
         }
-        if (folded_tile(*m, T) && !ensure_folded(*m, T)) return -1;
+        if (folded_tile(*m, T) && !ensure_folded(*m, T, full_tile(*m))) return -1;
         queue_prefill_tile(*m, T, base_pos + t0 + T, true, false, true, m->pf.logits_all.as<float>());
         if (cudaMemcpyAsync(m->pf.h_out_tokens, m->pf.out_tokens.p, (size_t)T * 4, cudaMemcpyDeviceToHost, stream()) != cudaSuccess) return -1;
         if (llamd_fwd_sync() != 0) return -1;
@@ -1794,7 +1827,7 @@ static int run_wide_batch(Model &m, const int32_t *tokens, const int32_t *positi
         return -1;
     }
     if (!prefill_alloc(m, nseq) || !prefill_alloc_all_logits(m, m.pf.tile < LLAMD_MAX_BATCH ? m.pf.tile : LLAMD_MAX_BATCH, false)) return -1;
-    if (folded_tile(m, nseq) && !ensure_folded(m, nseq)) return -1;
+    if (folded_tile(m, nseq) && !ensure_folded(m, nseq, full_tile(m))) return -1;
     if (llamd_fwd_sync() != 0) return -1;
     int n_kv_max = 0;
     for (int s = 0; s < nseq; s++) {

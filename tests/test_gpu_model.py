@@ -480,3 +480,31 @@ def test_automatic_tile_counts_the_score_buffer():
                 full.release()
             gm.free()
     assert runs[0][0] == runs[1][0] and np.array_equal(runs[0][1], runs[1][1])
+
+
+@pytest.mark.parametrize("tight", [False, True])
+def test_folded_copies_leave_room_for_a_tile(tight):
+    """A prompt makes the folded copies of the attention projections only where a full tile's buffers still fit beside them,
+    and gives the same bits with and without them."""
+    from llamd_rs_b200 import backend, synth
+    from llamd_rs_b200.model import CudaModel
+
+    hp = dict(synth.TINY, n_layer=8, n_embd=512, n_head=16, n_head_kv=1)
+    gm = CudaModel.load_batched(hp, synth.make_model(hp, seed=9), max_kv=40000, max_seq=1)
+    try:
+        toks = synth.token_ids(20, hp["n_vocab"], 3, "fold room").tolist()
+        gm.set_option("dense_gemm", 0)
+        want = gm.prefill(toks, 0), gm.logits()[0].view(np.uint32).copy()
+        gm.set_option("dense_gemm", 8)
+        full = _FullDevice(2 << 30) if tight else None  # (1 GB besides; a full tile's scores are 1.3 GB)
+        try:
+            free = backend.free_memory()
+            got = gm.prefill(toks, 0), gm.logits()[0].view(np.uint32).copy()
+            took = free - backend.free_memory()
+        finally:
+            if full:
+                full.release()
+        assert got[0] == want[0] and np.array_equal(got[1], want[1])
+        assert took == 0 if tight else took > 0
+    finally:
+        gm.free()
