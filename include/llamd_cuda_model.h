@@ -131,7 +131,7 @@ size_t llamd_model_weight_bytes(llamd_model *m); /* device.rs:473 */
  * neighbouring launches as one ("fuse_attn_quant": the attention-output launch writes the Q8_K form of its result itself,
  * as thread-block clusters of the eight CTAs of a 256-element block; heads of 128, the separate quantize launch
  * otherwise); "attn_gqa" (default 1): attention's scores run with one CTA per kv head and piece of the context for all
- * the query heads that share it, the values too from four sequences on and in tiles of up to "matvec_batch_max" tokens
+ * the query heads that share it (one sequence from position 512 on, two from 256), the values too from four sequences on and in tiles of up to "matvec_batch_max" tokens
  * (eight heads of 128 per kv head; the per-head and tile kernels otherwise); "sort_slots" = n
  * (default 8): from n sequences per pass the expert launches take their (sequence, expert) slots in expert order, so that
  * sequences that chose the same expert read it side by side; "head_gemm" = n (default 4): from n sequences per pass the

@@ -53,7 +53,8 @@ extern int g_pdl;
 // attention kernels read the positions and the cached rows of earlier positions before their dependency wait; true only
 // inside a pass whose first launch waits for everything in front of it.
 constexpr int kPassEarlyLoads = 8;
-// kPassAttnGqa: a batch of sequences runs attention as one CTA per kv head for all the query heads that share it.
+// kPassAttnGqa: attention's scores (from four sequences on the values too) run as one CTA per kv head and piece of the context
+// for all the query heads that share it.
 constexpr int kPassAttnGqa = 16;
 extern int g_batch_group;  // matvec_q6k.cu: sequences per CTA for small ungrouped matrices at batch > 1
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -287,6 +288,9 @@ void combine_rms_norm_quant_wait(const WaitPlan &wait, const float *x, const flo
 // of g_aq/g_ad/g_out in crates/llamd-rocm/kernels/llamd.hip:1027-1051.
 void *scratch(int slot, size_t bytes);
 void *host_stage(int slot, size_t bytes);  // runtime.cu
+// A second captured graph beside the current one (runtime.cu).
+void graph_swap();
+int begin_capture_beside();
 
 constexpr int kTileUnits = 32;
 constexpr int kTileBytes = 6720;       // 32 blocks x 210 B

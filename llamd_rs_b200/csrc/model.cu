@@ -215,7 +215,8 @@ struct Model {
                                    // Measured, tok/s aggregate, fused / separate: 1 sequence 281.3 / 275.7 (when it was built), 2: 460.5 / 485.0,
                                    // 4: 727.1 / 736.8, 8: 1112.5 / 1149.2, 24: 1644.5 / 1718.7, 48: 1876.2 / 1941.4
     int sort_slots = 8;      // option "sort_slots" = n: from n sequences per pass the expert launches take their slots in expert order (0: never)
-    int attn_gqa = 1;        // option "attn_gqa": batches of sequences run attention with one CTA per kv head for all its query heads (the same bits)
+    int attn_gqa = 1;        // option "attn_gqa": attention's scores (from four sequences on the values too) run with one CTA per kv head and piece
+                             // of the context for all its query heads (the same bits), but for near contexts (near_pass)
     int fuse_attn_quant = 0; // option "fuse_attn_quant": the attention-output launch leaves its result quantized (clusters of the CTAs of a
                              // 256-element block exchange their maxima through distributed shared memory); needs fuse_rope_attn. The same
                              // bits, one launch fewer, and measured 7 % SLOWER (270.4 against 291.2 tok/s): a launch of 16 clusters of
@@ -238,7 +239,8 @@ struct Model {
     int32_t *h_out = nullptr;   // pinned
     size_t weight_bytes = 0;
     int use_graph = 1, trace = 0;
-    int graph_nseq = 0;         // nseq the captured graph was recorded for
+    int graph_nseq = 0;         // nseq the captured graphs were recorded for
+    bool graph_near = false;    // ... and whether the current one is the near contexts' (near_pass)
     unsigned long long id = 0;
     std::string err;
 };
@@ -384,10 +386,18 @@ void queue_token_resident(Model &m) {
              m.tok_log.as<int32_t>(), m.tok_count.as<int32_t>(), 1, m.max_kv * m.max_seq);
 }
 
-// Queue one pass for `nseq` sequences. Does not synchronise.
+// Attention's scores of a pass by the per-head launch instead of the one per kv head: while its eight CTAs per head have a
+// 64-position tile each, for one sequence, and while two sequences have half as many. n_kv: positions of the longest sequence.
+// us a layer, per head less per kv head: one sequence at position 16 to 128 -2.3, 256 -1.5, 448 -0.8, 512 +0.7, 1024 +3.0; two at
+// 16 -2.2, 64 to 200 -0.6, 256 +2.1, 512 +3.0; three at 16 +1.8 (binary16 caches: -1.5, -0.8, -0.7, +1.3, +3.8; -1.5, 0.0, +1.9,
+// +3.6; +3.0).
+constexpr int kNearPositions = 512;
+bool near_pass(const Model &m, int nseq, int n_kv) { return m.ep_world == 1 && nseq <= 2 && nseq * n_kv <= kNearPositions; }
+
+// Queue one pass for `nseq` sequences. Does not synchronise. near: see near_pass.
 // The order is crates/llamd-runtime/src/device.rs:486-655 (itself the CPU
 // order of crates/llamd-runtime/src/layer.rs:85-203, 230-304).
-void queue_token(Model &m, int nseq) {
+void queue_token(Model &m, int nseq, bool near) {
     const llamd_hparams &hp = m.hp;
     const int E = hp.n_embd, H = hp.n_head, HKV = hp.n_head_kv, hd = hp.head_dim;
     const int kvd = HKV * hd, qd = H * hd, nu = hp.n_expert_used, ffe = hp.n_ff_expert;
@@ -403,7 +413,7 @@ void queue_token(Model &m, int nseq) {
     // (option arith; the fused norm + router launch carries the router's tree, so the mask needs it on), the loads before
     // the dependency wait, the batch form of attention
     const int pf = (m.arith_fast && m.fuse_norm_router && !m.fuse_tails ? m.arith_fast : 0) | (m.early_loads ? kPassEarlyLoads : 0) |
-                   (m.attn_gqa ? kPassAttnGqa : 0);
+                   (m.attn_gqa && !near ? kPassAttnGqa : 0);
     const bool dense_gemm = m.dense_gemm && nseq >= m.dense_gemm && m.dense_fold_ready && !m.fuse_norm_qkv;
     int8_t *rm = dense_gemm ? m.head_rm.as<int8_t>() : nullptr;  // the GEMMs' operand, made with the quants
     bool rm_made = false;
@@ -790,8 +800,29 @@ bool ensure_folded(Model &m, int n, int prompt = 0, bool head = true) {
     return true;
 }
 
+// The graph of a pass over nseq sequences is the current one afterwards: recorded now unless it is there already. Two are
+// kept, for near contexts and for the rest; a graph recorded for another model, or another nseq, points at the wrong buffers.
+bool ensure_graph(Model &m, int nseq, bool near) {
+    if (g_graph_owner != m.id || m.graph_nseq != nseq) llamd_fwd_graph_destroy();
+    else if (m.graph_near != near) graph_swap();
+    g_graph_owner = m.id;
+    m.graph_nseq = nseq;
+    m.graph_near = near;
+    if (llamd_fwd_has_graph()) return true;
+    if (begin_capture_beside() != 0) return false;
+    const unsigned long long before = g_launches;
+    queue_token(m, nseq, near);
+    m.launches_per_pass = g_launches - before;
+    if (llamd_fwd_end_capture() != 0 || error_code() != 0) {
+        llamd_fwd_graph_destroy();
+        return false;
+    }
+    return true;
+}
+
 int run(Model &m, const int32_t *tokens, const int32_t *positions, int nseq, int32_t *out_tokens) {
     const llamd_hparams &hp = m.hp;
+    int n_kv = 0;
     if (nseq < 1 || nseq > m.max_seq) {
         m.err = "forward: nseq outside 1..max_seq";
         return -1;
@@ -807,7 +838,9 @@ int run(Model &m, const int32_t *tokens, const int32_t *positions, int nseq, int
         }
         m.h_meta[2 * s] = tokens[s];
         m.h_meta[2 * s + 1] = positions[s];
+        if (positions[s] + 1 > n_kv) n_kv = positions[s] + 1;
     }
+    const bool near = near_pass(m, nseq, n_kv);
     if (!check_ready(m)) return -1;
     if (m.resident) mega_prepare(m);  // (uploads a pointer table: not inside a capture)
     if (!ensure_folded(m, nseq)) return -1;
@@ -817,24 +850,10 @@ int run(Model &m, const int32_t *tokens, const int32_t *positions, int nseq, int
         return -1;
     }
     if (m.use_graph && !m.trace) {
-        // a graph recorded for another model, or another nseq, points at the wrong buffers
-        if (!llamd_fwd_has_graph() || g_graph_owner != m.id || m.graph_nseq != nseq) {
-            llamd_fwd_graph_destroy();
-            if (llamd_fwd_begin_capture() != 0) return -1;
-            const unsigned long long before = g_launches;
-            queue_token(m, nseq);
-            m.launches_per_pass = g_launches - before;
-            if (llamd_fwd_end_capture() != 0 || error_code() != 0) {
-                llamd_fwd_graph_destroy();
-                return -1;
-            }
-            g_graph_owner = m.id;
-            m.graph_nseq = nseq;
-        }
-        if (llamd_fwd_graph_launch() != 0) return -1;
+        if (!ensure_graph(m, nseq, near) || llamd_fwd_graph_launch() != 0) return -1;
     } else {
         const unsigned long long before = g_launches;
-        queue_token(m, nseq);
+        queue_token(m, nseq, near);
         m.launches_per_pass = g_launches - before;
     }
     if (cudaMemcpyAsync(m.h_out, m.out_token.p, (size_t)nseq * 4, cudaMemcpyDeviceToHost, stream()) != cudaSuccess) {
@@ -1511,7 +1530,7 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
             // the shape allows; the rows of earlier positions read before the dependency wait -- earlier passes wrote them)
             attention_rope_quant(p.q.as<float>(), wqn, p.k.as<float>(), wkn, p.v.as<float>(), l.kc.p, l.vc.p, p.attn.as<float>(),
                                  p.scores.as<float>(), H, HKV, hd, meta, m.rope_tab.as<float>(), hp.rms_eps, m.max_kv, T, m.kv16, nullptr, nullptr,
-                                 (m.early_loads ? kPassEarlyLoads : 0) | (m.attn_gqa ? kPassAttnGqa : 0));
+                                 (m.early_loads ? kPassEarlyLoads : 0) | (m.attn_gqa && !near_pass(m, T, n_kv_max) ? kPassAttnGqa : 0));
         } else if (multi_seq && m.kv16) {
             llamd_fwd_qk_norm_rope_store_kv16(p.q.as<float>(), wqn, p.k.as<float>(), wkn, p.v.as<float>(), l.kc.p, l.vc.p, H, HKV, hd, meta,
                                               m.rope_tab.as<float>(), hp.rms_eps, T, m.max_kv);
@@ -1876,19 +1895,8 @@ int llamd_model_decode(llamd_model *h, int32_t first_token, int32_t start_pos, i
     m->h_meta[1] = start_pos;
     LLAMD_TRY(cudaMemcpyAsync(m->meta.p, m->h_meta, 8, cudaMemcpyHostToDevice, stream()), "decode meta H2D");
     LLAMD_TRY(cudaMemsetAsync(m->tok_count.p, 0, 4, stream()), "decode counter reset");
-    if (m->use_graph && (!llamd_fwd_has_graph() || g_graph_owner != m->id || m->graph_nseq != 1)) {
-        llamd_fwd_graph_destroy();
-        if (llamd_fwd_begin_capture() != 0) return -1;
-        const unsigned long long before = g_launches;
-        queue_token(*m, 1);
-        m->launches_per_pass = g_launches - before;
-        if (llamd_fwd_end_capture() != 0 || error_code() != 0) {
-            llamd_fwd_graph_destroy();
-            return -1;
-        }
-        g_graph_owner = m->id;
-        m->graph_nseq = 1;
-    }
+    auto near_at = [&](int i) { return near_pass(*m, 1, start_pos + i + 1); };
+    if (m->use_graph && (!ensure_graph(*m, 1, near_at(n - 1)) || !ensure_graph(*m, 1, near_at(0)))) return -1;  // (both, if the positions cross)
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     int rc = 0;
     if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess || cudaEventRecord(e0, stream()) != cudaSuccess) {
@@ -1897,9 +1905,9 @@ int llamd_model_decode(llamd_model *h, int32_t first_token, int32_t start_pos, i
     }
     for (int i = 0; rc == 0 && i < n; i++) {
         if (m->use_graph) {
-            if (llamd_fwd_graph_launch() != 0) rc = -1;
+            if (!ensure_graph(*m, 1, near_at(i)) || llamd_fwd_graph_launch() != 0) rc = -1;
         } else {
-            queue_token(*m, 1);
+            queue_token(*m, 1, near_at(i));
         }
     }
     if (rc == 0 && cudaEventRecord(e1, stream()) != cudaSuccess) {

@@ -2275,7 +2275,7 @@ static void attention_rope_launch(const float *q, const float *wq, const float *
     const size_t smem_ga = (size_t)(ratio * hd + 2 * kAttTile * (hd + 4) + (ratio + 1) * hd + hd) * sizeof(float);
     const size_t smem_gb = (size_t)((size_t)ratio * cap + 2 * kPvTile * (hd / kSplit)) * sizeof(float);
     // (values, measured, 48 layers at position ~520: 8 sequences 814.7 -> 1044.8 tok/s, 4 sequences 641.8 -> 717.2, 2 sequences
-    // 456.2 -> 439.7, so from four sequences on; the scores from one on)
+    // 456.2 -> 439.7, so from four sequences on; the scores wherever the pass asks for it: near_pass in model.cu)
     const bool gqa = (flags & kPassAttnGqa) && !(flags & 4) && ratio == kGqaMax && hd / kSplit == 32 && smem_ga <= 200 * 1024;
     if (gqa) {
         static size_t conf_ga[2] = {0, 0};

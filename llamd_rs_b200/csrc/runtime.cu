@@ -23,6 +23,8 @@ static int g_err = 0;
 static std::string g_err_msg;
 static cudaGraph_t g_graph = nullptr;
 static cudaGraphExec_t g_graph_exec = nullptr;
+static cudaGraph_t g_kept_graph = nullptr;  // kept beside the current one (graph_swap)
+static cudaGraphExec_t g_kept_exec = nullptr;
 static void *g_scratch[8] = {};
 static size_t g_scratch_bytes[8] = {};
 
@@ -203,6 +205,28 @@ void *scratch(int slot, size_t bytes) {
     return g_scratch[slot];
 }
 
+static void destroy_current_graph() {
+    if (g_graph_exec) cudaGraphExecDestroy(g_graph_exec);
+    if (g_graph) cudaGraphDestroy(g_graph);
+    g_graph_exec = nullptr;
+    g_graph = nullptr;
+}
+// The current graph and the one kept beside it change places (either may be none).
+void graph_swap() {
+    cudaGraph_t g = g_graph;
+    cudaGraphExec_t e = g_graph_exec;
+    g_graph = g_kept_graph;
+    g_graph_exec = g_kept_exec;
+    g_kept_graph = g;
+    g_kept_exec = e;
+}
+// llamd_fwd_begin_capture that leaves the kept graph alone.
+int begin_capture_beside() {
+    destroy_current_graph();
+    LLAMD_TRY(cudaStreamBeginCapture(stream(), cudaStreamCaptureModeThreadLocal), "begin capture");
+    return 0;
+}
+
 // Pinned, device-visible host memory of this library's own, kept and grown per slot (0: a call's inputs, 1: its results).
 // A host-facing call copies through it instead of handing the driver pageable memory: the driver's own staging of a
 // pageable copy, or the result copy's wait for it, cost several microseconds of a call that takes a dozen.
@@ -378,8 +402,7 @@ int llamd_fwd_timer_stop(float *ms_out) {
 
 int llamd_fwd_begin_capture(void) {
     llamd_fwd_graph_destroy();
-    LLAMD_TRY(cudaStreamBeginCapture(stream(), cudaStreamCaptureModeThreadLocal), "begin capture");
-    return 0;
+    return begin_capture_beside();
 }
 int llamd_fwd_end_capture(void) {
     cudaGraph_t g = nullptr;
@@ -409,10 +432,9 @@ int llamd_fwd_graph_launch(void) {
 }
 int llamd_fwd_has_graph(void) { return g_graph_exec ? 1 : 0; }
 void llamd_fwd_graph_destroy(void) {
-    if (g_graph_exec) cudaGraphExecDestroy(g_graph_exec);
-    if (g_graph) cudaGraphDestroy(g_graph);
-    g_graph_exec = nullptr;
-    g_graph = nullptr;
+    destroy_current_graph();
+    graph_swap();
+    destroy_current_graph();
 }
 
 }  // extern "C"

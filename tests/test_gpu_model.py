@@ -508,3 +508,34 @@ def test_folded_copies_leave_room_for_a_tile(tight):
         assert took == 0 if tight else took > 0
     finally:
         gm.free()
+
+
+@pytest.mark.parametrize("kv16", [0, 1])
+def test_near_and_far_contexts(kv16):
+    """The scores launch changes with the context (one sequence at 512 positions, two at 256), and each kind has its graph: the
+    same tokens and logits as the per-head launches on both sides of the line, across it inside one decode call, and back."""
+    from llamd_rs_b200 import synth
+    from llamd_rs_b200.model import CudaModel
+
+    hp = dict(synth.TINY, n_layer=1, n_head=8, n_head_kv=1, head_dim=128)
+    gm = CudaModel.load_batched(hp, synth.make_model(hp, seed=9), max_kv=640, max_seq=2)
+    try:
+        if kv16:
+            gm.set_option("kv_f16", 1)
+        toks = synth.token_ids(600, hp["n_vocab"], 3, "near").tolist()
+        gm.prefill(toks, 0)
+        runs = []
+        for gqa, graph in ((0, True), (1, True), (1, False)):
+            gm.set_option("attn_gqa", gqa)
+            gm.use_graph = graph
+            got = [gm.decode(toks[505], 505, 16)[0].tolist(), gm.logits()[0].view(np.uint32).tolist()]
+            for pos in (3, 510, 511, 512, 513, 90, 599):
+                got += [gm.forward(toks[pos], pos), gm.logits()[0].view(np.uint32).tolist()]
+            for a, b in ((255, 10), (256, 10), (7, 254), (511, 512)):
+                got += [gm.forward_batch([toks[a], toks[b]], [a, b]).tolist(), gm.logits(2).view(np.uint32).tolist()]
+            gm.prefill(toks[500:530], 500)  # (the rows that the decode call wrote)
+            runs.append(got)
+        assert runs[0] == runs[1] == runs[2]
+    finally:
+        gm.use_graph = True
+        gm.free()
