@@ -2009,8 +2009,17 @@ void llamd_fwd_matvec_q8_0(const void *w, const float *x, float *out, int blocks
     if (n_raw < 2) n_raw = raw_fit(225 * 1024);
     if (n_raw > kQ80MaxRaw) n_raw = kQ80MaxRaw;
     if (n_raw > chunks) n_raw = chunks;
-    const bool by_bulk = ctas <= (nseq == 1 ? kQ80MaxCtasOne : kQ80MaxCtas) && n_raw >= (chunks < 2 ? 1 : 2) && ((uintptr_t)w & 15) == 0 && ((uintptr_t)x & 15) == 0 &&
-                         q80_status_word() != nullptr;
+    const bool usable = ((uintptr_t)w & 15) == 0 && ((uintptr_t)x & 15) == 0 && q80_status_word() != nullptr;
+    const bool by_bulk = usable && ctas <= (nseq == 1 ? kQ80MaxCtasOne : kQ80MaxCtas) && n_raw >= (chunks < 2 ? 1 : 2);
+    // Activations too large to leave room for two raw chunks: half of the sequences at a time, while a launch is one wave of
+    // CTAs. us, thread per row / two launches: 4096 x 4864 for eight sequences 96 / 66, 5632 for seven 141 / 77, 8192 for six
+    // 203 / 111, 40 x 14336 for three 221 / 143; of two waves (9472 x 5632 for seven) 141 / 148.
+    if (usable && !by_bulk && nseq > 1 && ctas <= 148) {
+        const int n = (nseq + 1) / 2;
+        llamd_fwd_matvec_q8_0(w, x, out, blocks32, rows, n);
+        llamd_fwd_matvec_q8_0(w, x + (size_t)n * blocks32 * 32, out + (size_t)n * rows, blocks32, rows, nseq - n);
+        return;
+    }
     const size_t smem_bulk = smem + kQ80RingBytes + (size_t)n_raw * kQ80RawBytes;
     const dim3 grid(by_bulk ? ctas : (rows + 127) / 128);
 #define Q80_CASE(N)                                                                                                   \

@@ -204,10 +204,12 @@ def test_grouped_repeated_expert_and_bad_ids(be, orc, synth):
     (33, 96, 2),                  # three blocks: less than one chunk
     (256, 2080, 1),               # 65 blocks: eight chunks and one block more
     (64, 1024, 8),                # one chain warp per sequence
-    (40, 14336, 3),               # activations too large to sit beside the staged weights: the thread-per-row form
+    (40, 14336, 3),               # activations too large to sit beside the staged weights: two launches
     (4744, 768, 1),               # more CTAs than SMs: the smaller ring, two CTAs per SM
     (70, 8224, 1), (70, 4128, 5), # 33 and 17 chunks through a ring of fewer
     (18976, 96, 2),               # past the line where the thread-per-row form takes over for several sequences
+    (40, 4640, 8), (40, 5632, 7), (70, 25600, 2),  # activations that leave no room for the ring: two launches
+    (4768, 4640, 8),              # ... but the thread-per-row form beyond one wave of CTAs
 ])
 def test_q8_0_matvec_is_bit_exact(be, orc, synth, rows, k, nseq):
     w = synth.q8_0_blocks(rows * k // 32, 51, "q80mv", rows, k)
