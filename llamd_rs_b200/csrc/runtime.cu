@@ -138,7 +138,7 @@ static bool build_exp_table(cudaStream_t s) {
         uint32_t *d_in = nullptr, *d_ds = nullptr;
         std::vector<uint32_t> ds(n_exc, 0xFFFFFFFFu);
         if (cudaMalloc(&d_in, n_exc * 4) == cudaSuccess && cudaMalloc(&d_ds, n_exc * 4) == cudaSuccess &&
-            cudaMemcpy(d_in, in.data(), n_exc * 4, cudaMemcpyHostToDevice) == cudaSuccess) {
+            cudaMemcpyAsync(d_in, in.data(), n_exc * 4, cudaMemcpyHostToDevice, s) == cudaSuccess) {  // (s does not wait for the default stream)
             exp_window_kernel<<<148 * 4, 256, 0, s>>>(d_in, (uint32_t)n_exc, d_ds);
             if (cudaMemcpyAsync(ds.data(), d_ds, n_exc * 4, cudaMemcpyDeviceToHost, s) == cudaSuccess && cudaStreamSynchronize(s) == cudaSuccess) {
                 uint32_t worst = 0;
@@ -316,7 +316,9 @@ void *llamd_cuda_upload(const void *host, size_t bytes) {
         set_error(cudaGetLastError(), "upload cudaMalloc");
         return nullptr;
     }
-    if (bytes && cudaMemcpy(d, host, bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
+    // (a copy from pageable memory returns when its last bytes are staged, not when they have arrived, and the library's stream
+    // does not wait for the default one)
+    if (bytes && (cudaMemcpy(d, host, bytes, cudaMemcpyHostToDevice) != cudaSuccess || cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess)) {
         set_error(cudaGetLastError(), "upload cudaMemcpy");
         cudaFree(d);
         return nullptr;

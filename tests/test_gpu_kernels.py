@@ -221,6 +221,26 @@ def test_q8_0_matvec_is_bit_exact(be, orc, synth, rows, k, nseq):
         assert_bit_equal(got[s], want, f"q8_0 {rows}x{k} sequence {s}")
 
 
+def test_uploaded_weights_are_complete(be, synth):
+    """An upload's last bytes are on the device when the repacking launch reads them, however busy the bus is."""
+    import torch
+
+    rows, blocks32 = 4096, 8
+    w = synth.q8_0_blocks(rows * blocks32, 71, "upload")
+    want = w.reshape(-1, 34)[:, 2:].view(np.int8).astype(np.float32) * w.reshape(-1, 34)[:, :2].copy().view(np.float16).astype(np.float32)
+    want = want.reshape(-1).view(np.uint32)
+    zeros = np.zeros_like(w)
+    host, side = torch.empty(256 << 20, dtype=torch.uint8, pin_memory=True), torch.cuda.Stream()
+    dev = torch.empty_like(host, device="cuda")
+    for i in range(20):
+        be.Q80Weights.upload(zeros, rows, blocks32)  # (whatever the device memory held is gone)
+        with torch.cuda.stream(side):
+            dev.copy_(host, non_blocking=True)
+        dw = be.Q80Weights.upload(w, rows, blocks32)
+        side.synchronize()
+        assert np.array_equal(dw.dequantize().reshape(-1).view(np.uint32), want), f"upload {i}"
+
+
 # ---- many tokens at once: the prefill kernels --------------------------------
 @pytest.mark.parametrize("ntok", [1, 7, 8, 9, 37])
 def test_matvec_tokens_equals_per_token_matvec(be, orc, synth, ntok):
