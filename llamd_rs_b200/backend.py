@@ -10,6 +10,7 @@ This module is for tests, the bench and Python users; the compiled host side
 from __future__ import annotations
 
 import ctypes as C
+import math
 import threading
 from dataclasses import dataclass
 
@@ -67,7 +68,7 @@ class _ResultPool:
     ordinary new array costs a page fault per 4 KB and a copy through the driver's staging (0.2 ms for the four rows of
     logits of a 151936-token vocabulary). At most LIMIT bytes are pinned, KEEP of them while nobody holds them; beyond that,
     and below MIN, a result is an ordinary array."""
-    MIN, KEEP, LIMIT = 1 << 15, 64 << 20, 256 << 20
+    MIN, KEEP, LIMIT = (128 << 10) + 1, 64 << 20, 256 << 20  # (up to 128 KB the library's own staging is quicker)
 
     def __init__(self):
         self.lock = threading.RLock()  # (re-entrant: a garbage collection inside may give a block back)
@@ -75,7 +76,7 @@ class _ResultPool:
         self.idle = self.total = 0
 
     def empty(self, shape) -> np.ndarray:
-        n = 4 * int(np.prod(shape))
+        n = 4 * math.prod(shape)
         if n < self.MIN:
             return np.empty(shape, dtype=np.float32)
         size = 1 << (n - 1).bit_length()

@@ -288,33 +288,33 @@ int llamd_cuda_quantize_q8k(const float *x, int nblocks, int8_t *qs, float *d, i
 }
 
 // Host-facing products: x in, out back, one synchronise. Inputs of up to kStageBytes go through pinned memory of the
-// library's own; results of up to kDirectBytes are stored there by the kernel itself (a warp's rows are 16-byte PCIe
-// writes, which is quicker than a copy of its own only while they are few), larger ones are copied, straight into `out` if that is
-// pinned (llamd_cuda_host_alloc). 512 x 2048 for one sequence: 29.9 us a call through pageable copies, 24.9 now (the two kernels
-// are 8 of them).
-constexpr size_t kStageBytes = 1 << 20, kDirectBytes = 16 << 10;
+// library's own; results of up to kDirectBytes are stored there by the kernel itself, larger ones are copied, straight into
+// `out` if that is pinned (llamd_cuda_host_alloc). Without pinned memory both go as pageable copies. us a call, repeated / with
+// new weights and activations, Q6_K rows of 2048: result through a pageable copy, a pinned copy of its own, stored by the kernel,
+// copied into a pinned array: 8 KB 34.7/60.3, 32.3/57.4, 30.1/53.5, 32.6/64.2; 32 KB 39.9/63.8, 36.9/66.7, 27.8/58.1, 36.7/67.4;
+// 128 KB 48.7/81.0, 45.5/77.6, 39.7/71.2, 41.1/78.5; 256 KB 75.8/119.8, 69.8/121.3, 69.4/122.8, 60.0/106.1.
+constexpr size_t kStageBytes = 1 << 20, kDirectBytes = 128 << 10;
 static int stage_x(const float *x, size_t bytes, float **d_x, bool read_once) {
-    if (bytes > kStageBytes) {
-        *d_x = (float *)scratch(4, bytes);
-        if (!*d_x) return -1;
-        LLAMD_TRY(cudaMemcpyAsync(*d_x, x, bytes, cudaMemcpyHostToDevice, stream()), "x H2D");
-        return 0;
-    }
-    float *h = (float *)host_stage(0, bytes);  // (free: every call that fills it waits for its own work)
-    if (!h) return -1;
-    memcpy(h, x, bytes);
+    float *h = bytes <= kStageBytes ? (float *)host_stage(0, bytes) : nullptr;  // (free: every call that fills it waits for its own work)
+    if (h) memcpy(h, x, bytes);
     *d_x = h;
-    if (read_once) return 0;  // one kernel reads it once, over PCIe
+    if (h && read_once) return 0;  // one kernel reads it once, over PCIe
     *d_x = (float *)scratch(4, bytes);
     if (!*d_x) return -1;
-    LLAMD_TRY(cudaMemcpyAsync(*d_x, h, bytes, cudaMemcpyHostToDevice, stream()), "x H2D");
+    LLAMD_TRY(cudaMemcpyAsync(*d_x, h ? h : x, bytes, cudaMemcpyHostToDevice, stream()), "x H2D");
     return 0;
 }
+// where the kernel puts a call's results: staging (then *staged), or device memory
+static float *out_buffer(size_t bytes, bool *staged) {
+    void *p = bytes <= kDirectBytes ? host_stage(1, bytes) : nullptr;
+    *staged = p != nullptr;
+    return (float *)(p ? p : scratch(2, bytes));
+}
 // after the launches: the results to the caller, and the call's synchronise
-static int finish_out(const float *d_out, float *out, size_t bytes) {
-    if (bytes > kDirectBytes) LLAMD_TRY(cudaMemcpyAsync(out, d_out, bytes, cudaMemcpyDeviceToHost, stream()), "out D2H");
+static int finish_out(const float *d_out, float *out, size_t bytes, bool staged) {
+    if (!staged) LLAMD_TRY(cudaMemcpyAsync(out, d_out, bytes, cudaMemcpyDeviceToHost, stream()), "out D2H");
     if (llamd_fwd_sync() != 0) return -1;
-    if (bytes <= kDirectBytes) memcpy(out, d_out, bytes);  // (d_out is host memory)
+    if (staged) memcpy(out, d_out, bytes);
     return 0;
 }
 
@@ -324,21 +324,23 @@ int llamd_cuda_matvec_q6k_f32(const void *d_w, const float *x, float *out, int b
     float *d_x;
     int8_t *d_q = (int8_t *)scratch(0, nseq * k);
     float *d_d = (float *)scratch(1, (size_t)nseq * blocks * sizeof(float));
-    float *d_out = (float *)(out_bytes <= kDirectBytes ? host_stage(1, out_bytes) : scratch(2, out_bytes));
+    bool staged;
+    float *d_out = out_buffer(out_bytes, &staged);
     if (!d_q || !d_d || !d_out || stage_x(x, nseq * k * sizeof(float), &d_x, true)) return -1;
     llamd_fwd_quantize(d_x, d_q, d_d, nseq * blocks);
     llamd_fwd_matvec_batch(d_w, d_q, d_d, d_out, blocks, rows, nseq);
-    return finish_out(d_out, out, out_bytes);
+    return finish_out(d_out, out, out_bytes, staged);
 }
 
 int llamd_cuda_matvec_q8_0_f32(const void *d_w, const float *x, float *out, int blocks32, int rows, int nseq) {
     if (!d_w || !x || !out || blocks32 <= 0 || rows <= 0 || nseq < 1 || nseq > LLAMD_MAX_SEQ) return -1;
     const size_t k = (size_t)blocks32 * 32, out_bytes = (size_t)nseq * rows * sizeof(float);
     float *d_x;
-    float *d_out = (float *)(out_bytes <= kDirectBytes ? host_stage(1, out_bytes) : scratch(2, out_bytes));
+    bool staged;
+    float *d_out = out_buffer(out_bytes, &staged);
     if (!d_out || stage_x(x, nseq * k * sizeof(float), &d_x, false)) return -1;  // (every CTA reads all of x)
     llamd_fwd_matvec_q8_0(d_w, d_x, d_out, blocks32, rows, nseq);
-    if (finish_out(d_out, out, out_bytes) != 0) return -1;
+    if (finish_out(d_out, out, out_bytes, staged) != 0) return -1;
     if (llamd_fwd_matvec_q8_0_status() != 0) {
         set_error_msg("matvec_q8_0: a bulk copy of the weights did not arrive within its limit; rows are missing");
         return -1;

@@ -229,7 +229,8 @@ int begin_capture_beside() {
 
 // Pinned, device-visible host memory of this library's own, kept and grown per slot (0: a call's inputs, 1: its results).
 // A host-facing call copies through it instead of handing the driver pageable memory: the driver's own staging of a
-// pageable copy, or the result copy's wait for it, cost several microseconds of a call that takes a dozen.
+// pageable copy, or the result copy's wait for it, cost several microseconds of a call that takes a dozen. Null, and no error,
+// when there is no pinned memory to be had: the caller hands over its own.
 void *host_stage(int slot, size_t bytes) {
     static void *buf[2] = {nullptr, nullptr};
     static size_t have[2] = {0, 0};
@@ -241,9 +242,8 @@ void *host_stage(int slot, size_t bytes) {
         have[slot] = 0;
     }
     const size_t want = bytes < 65536 ? 65536 : bytes;
-    cudaError_t e = cudaHostAlloc(&buf[slot], want, cudaHostAllocMapped);
-    if (e != cudaSuccess) {
-        set_error(e, "host staging");
+    if (cudaHostAlloc(&buf[slot], want, cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();
         return buf[slot] = nullptr;
     }
     have[slot] = want;

@@ -241,6 +241,22 @@ def test_uploaded_weights_are_complete(be, synth):
         assert np.array_equal(dw.dequantize().reshape(-1).view(np.uint32), want), f"upload {i}"
 
 
+@pytest.mark.parametrize("rows,nseq", [(32768, 1), (32769, 1), (4096, 8), (4097, 8)])
+def test_results_on_both_sides_of_the_staging_limit(be, orc, synth, rows, nseq):
+    """Results of up to 128 KB are stored into the library's own host memory, larger ones copied into the caller's array; earlier
+    arrays keep their values."""
+    k = 256
+    w6, w8 = synth.q6k_blocks(rows, 61, "stage"), synth.q8_0_blocks(rows * 8, 61, "stage")
+    x = synth.normal_f32(2 * nseq * k, 61, "stage.x").reshape(2, -1)
+    d6, d8 = be.DeviceWeights.upload(w6, rows, 1), be.Q80Weights.upload(w8, rows, 8)
+    got = [(d6.matvec_f32(v, nseq), d8.matvec_f32(v, nseq)) for v in x]
+    for v, (a, b) in zip(x, got):
+        for s in range(nseq):
+            xs = v[s * k:(s + 1) * k]
+            assert_bit_equal(a[s], orc.matvec_q6k(w6, xs, k, rows), f"q6k sequence {s}")
+            assert_bit_equal(b[s], orc.matvec_dequant(orc.Q8_0, w8, xs, k, rows), f"q8_0 sequence {s}")
+
+
 # ---- many tokens at once: the prefill kernels --------------------------------
 @pytest.mark.parametrize("ntok", [1, 7, 8, 9, 37])
 def test_matvec_tokens_equals_per_token_matvec(be, orc, synth, ntok):
