@@ -65,45 +65,82 @@ class _Block:
 
 class _ResultPool:
     """Pinned memory for large result arrays: the device copies straight into the array that the caller gets, where an
-    ordinary new array costs a page fault per 4 KB and a copy through the driver's staging (0.2 ms for the four rows of
-    logits of a 151936-token vocabulary). At most LIMIT bytes are pinned, KEEP of them while nobody holds them; beyond that,
-    and below MIN, a result is an ordinary array."""
-    MIN, KEEP, LIMIT = (128 << 10) + 1, 64 << 20, 256 << 20  # (up to 128 KB the library's own staging is quicker)
+    ordinary new array costs a page fault per 4 KB and a copy through the driver's staging (logits of 8 rows of a
+    151936-token vocabulary: 100 us, 740 as an ordinary array).
+
+    Pinning costs more than one result saves (2 ms and more a block), so a block once pinned is kept, and there are at most
+    PER_SIZE of each power of two from MIN to MAX, 32 MB in all: a caller that holds its results gets ordinary arrays beyond
+    those, and so does every result below MIN (the library's own staging is quicker) or above MAX. A model has the blocks for
+    its logits pinned when it is made (reserve), a product on its size's first results. release_idle() gives back what nobody
+    holds; freeing the last model does."""
+    MIN, MAX, PER_SIZE = (128 << 10) + 1, 8 << 20, 2
 
     def __init__(self):
         self.lock = threading.RLock()  # (re-entrant: a garbage collection inside may give a block back)
-        self.free = {}                 # size -> pointers
-        self.idle = self.total = 0
+        self.free = {}                 # size -> pointers of idle blocks
+        self.made = {}                 # size -> blocks there are, idle or lent
+        self.users = 0                 # who reserved and has not released
 
     def empty(self, shape) -> np.ndarray:
         n = 4 * math.prod(shape)
-        if n < self.MIN:
+        if not self.MIN <= n <= self.MAX:
             return np.empty(shape, dtype=np.float32)
         size = 1 << (n - 1).bit_length()
         ptr = None
         with self.lock:
-            have = self.free.get(size)
-            if have:
-                ptr = have.pop()
-                self.idle -= size
-            elif self.total + size <= self.LIMIT:
-                self.total += size
-                ptr = lib().llamd_cuda_host_alloc(size)
-                if not ptr:
-                    self.total -= size
+            idle = self.free.get(size)
+            if idle:
+                ptr = idle.pop()
+            else:
+                ptr = self._make(size)
         if not ptr:
             return np.empty(shape, dtype=np.float32)
         b = _Block(self, ptr, size)
         b.__array_interface__ = {"data": (ptr, False), "typestr": "<f4", "shape": tuple(shape), "version": 3}
         return np.asarray(b)
 
+    def _make(self, size):
+        if self.made.get(size, 0) >= self.PER_SIZE:
+            return None
+        ptr = self.pin(size)
+        if ptr:
+            self.made[size] = self.made.get(size, 0) + 1
+        return ptr
+
+    def reserve(self, least, most):
+        """Pins the blocks that results of `least` to `most` bytes take, for a user that says when it is done (release)."""
+        with self.lock:
+            self.users += 1
+            size = 1 << (max(least, self.MIN) - 1).bit_length()
+            while size <= self.MAX and size < 2 * most:
+                while (ptr := self._make(size)):
+                    self.free.setdefault(size, []).append(ptr)
+                size *= 2
+
+    def release(self):
+        with self.lock:
+            self.users -= 1
+            if self.users:
+                return
+        self.release_idle()
+
     def give_back(self, ptr, size):
         with self.lock:
-            if self.idle + size <= self.KEEP:
-                self.free.setdefault(size, []).append(ptr)
-                self.idle += size
-                return
-            self.total -= size
+            self.free.setdefault(size, []).append(ptr)
+
+    def release_idle(self):
+        with self.lock:
+            idle, self.free = self.free, {}
+            for size, ptrs in idle.items():
+                self.made[size] -= len(ptrs)
+        for ptrs in idle.values():
+            for ptr in ptrs:
+                self.unpin(ptr)
+
+    def pin(self, size):
+        return lib().llamd_cuda_host_alloc(size)
+
+    def unpin(self, ptr):
         lib().llamd_cuda_host_free(ptr)
 
 

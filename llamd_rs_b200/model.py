@@ -148,6 +148,7 @@ class CudaModel:
         if not self._h:
             raise backend.Other("model create failed: " + backend._last_error())
         self._use_graph = True
+        backend.results.reserve(4 * h.n_vocab, 4 * h.n_vocab * max_seq)  # (what logits() returns)
 
     # -- loading -----------------------------------------------------------
     @classmethod
@@ -461,6 +462,7 @@ class CudaModel:
         if getattr(self, "_h", None):
             self._L.llamd_model_free(self._h)
             self._h = None
+            backend.results.release()
 
     def __del__(self):
         try:

@@ -246,3 +246,87 @@ def test_every_model_option_is_documented():
     missing_i = [n for n in names if f"`{n}`" not in integ]
     assert not missing_h, f"options not described in the header: {missing_h}"
     assert not missing_i, f"options not named in INTEGRATION.md: {missing_i}"
+
+
+def test_result_pool_is_bounded_and_reuses_its_blocks():
+    """The pool of pinned result arrays over ordinary memory: a block per size once its array is gone, at most PER_SIZE pinned
+    however many results are held, none outside its sizes, idle ones given back on request; from several threads."""
+    import ctypes
+    import gc
+    import threading
+
+    from llamd_rs_b200.backend import _ResultPool
+
+    class Pool(_ResultPool):
+        def __init__(self):
+            super().__init__()
+            self.pinned, self.pins, self.most = {}, 0, 0
+
+        def pin(self, size):
+            buf = ctypes.create_string_buffer(size)
+            self.pinned[ctypes.addressof(buf)] = buf
+            self.pins += 1
+            self.most = max(self.most, sum(len(b) for b in self.pinned.values()))
+            return ctypes.addressof(buf)
+
+        def unpin(self, ptr):
+            del self.pinned[ptr]
+
+    pool = Pool()
+    vocab = 151936
+    for rows in (1, 8, 13):  # dropped at once: one block each
+        for _ in range(10):
+            a = pool.empty((rows, vocab))
+            assert a.shape == (rows, vocab) and a.dtype == np.float32 and a.flags.writeable
+            a[...] = rows
+            del a
+    assert pool.pins == 2  # (8 and 13 rows share a size)
+    before = pool.pins
+    for n in (1, 100, pool.MIN // 4 - 1, pool.MAX // 4 + 1, 128 * vocab):  # not its sizes
+        assert pool.empty((n,)).flags.owndata
+    assert pool.pins == before
+    held = [pool.empty((2, vocab)) for _ in range(20)]  # held: PER_SIZE pinned, the rest ordinary, all of them apart
+    assert pool.pins == before + pool.PER_SIZE
+    for i, a in enumerate(held):
+        a[...] = i
+    assert all((a == i).all() for i, a in enumerate(held))
+    view = held[0][1, 5:9]
+    assert held[0].base is not None
+    held = None
+    gc.collect()
+    pool.release_idle()
+    assert len(pool.pinned) == 1 and (view == 0).all()  # the block that a view still uses
+    del view
+    gc.collect()
+    pool.release_idle()
+    assert not pool.pinned and not any(pool.made.values())
+
+    pool.reserve(4 * vocab, 160 * 4 * vocab)  # a model: its logits pin nothing, another model's end leaves its blocks
+    pool.reserve(4 * 512, 4 * 512)
+    before = pool.pins
+    assert sorted(pool.free) == [1 << 20, 2 << 20, 4 << 20, 8 << 20]
+    pool.release()
+    a, b = pool.empty((8, vocab)), pool.empty((9, vocab))
+    assert pool.pins == before and not a.flags.owndata and not b.flags.owndata
+    del a, b
+    gc.collect()
+    pool.release()
+    assert not pool.pinned
+
+    def work(seed):
+        rng = np.random.default_rng(seed)
+        for _ in range(200):
+            n = int(rng.integers(1, 9))
+            a, b = pool.empty((n, 40000)), pool.empty((n, 40000))
+            a[...], b[...] = seed, -seed
+            assert (a == seed).all() and (b == -seed).all()
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in range(1, 5)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    gc.collect()
+    assert pool.most <= 32 << 20
+    pool.release_idle()
+    assert not pool.pinned
