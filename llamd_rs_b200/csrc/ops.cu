@@ -2091,7 +2091,8 @@ template <class KVT>
 static void qk_norm_rope_launch(int cls, const char *what, float *q, const float *wq, float *k, const float *wk, const float *v, KVT *kc, KVT *vc, int n_head,
                                 int n_head_kv, int hd, const int32_t *meta, const float *rope_tab, float eps, int n, int kv_stride) {
     const int n_vec = n * (n_head + n_head_kv);
-    if (n_vec >= 1024 && hd % 4 == 0 && hd <= 256)
+    // (that form reads the vectors 16 bytes at a time)
+    if (n_vec >= 1024 && hd % 4 == 0 && hd <= 256 && (((uintptr_t)q | (uintptr_t)k) & 15) == 0)
         launch_kc(cls, what, norm_rope_rows_kernel<KVT>, dim3((n_vec + kRopeVecs - 1) / kRopeVecs), dim3(256), kRopeVecs * (hd + 4) * sizeof(float), q, wq, k,
                   wk, v, kc, vc, n_head, n_head_kv, hd, meta, rope_tab, eps, kv_stride, n_vec);
     else

@@ -207,6 +207,55 @@ def test_router_matvec_logits_are_bit_exact(ops, orc, synth):
     assert bit_equal(ops.matvec_f32(w, x), np.stack([orc.matvec_dequant(orc.F32, w, x[s], k, ne) for s in range(3)]))
 
 
+@pytest.mark.parametrize("hd,heads,kv_heads,n,shift,kv16,own_caches,norms", [
+    (128, 7, 1, 129, 0, 0, False, "qk"),   # 1032 vectors: the last CTA holds 8
+    (64, 6, 2, 128, 0, 1, False, "qk"),    # 1024, binary16 cache
+    (256, 4, 2, 171, 0, 0, True, "q"),     # a cache per sequence, keys not normed
+    (20, 6, 2, 131, 0, 1, True, ""),       # no norm weights
+    (128, 7, 1, 129, 4, 0, False, "qk"),   # queries and keys off the 16-byte boundary
+    (128, 7, 1, 127, 0, 0, False, "k"),    # 1016: a CTA per head
+])
+def test_norm_rope_of_many_vectors(ops, orc, synth, hd, heads, kv_heads, n, shift, kv16, own_caches, norms):
+    """QK-norm, RoPE and the K/V store of a tile on both sides of the line where a CTA takes 32 vectors: queries, keys and cache
+    rows against the oracle, the other cache rows untouched."""
+    from llamd_rs_b200.backend import DevBuf, sync
+    from llamd_rs_b200._lib import lib
+
+    q, k, v = (synth.normal_f32(n * h * hd, 91, "many", what).reshape(n, h * hd) for what, h in (("q", heads), ("k", kv_heads), ("v", kv_heads)))
+    w = {c: synth.normal_f32(hd, 91, "many.w", c) if c in norms else None for c in "qk"}
+    max_kv, first = 160, 3
+    pos = np.array([(7 * i) % max_kv if own_caches else first + i for i in range(n)], np.int32)
+    rows = np.arange(n) * max_kv + pos if own_caches else pos  # of a cache
+    want = {}
+    for c, x, h in (("q", q, heads), ("k", k, kv_heads)):
+        if w[c] is not None:
+            x = orc.mul(orc.rms_norm(x.reshape(-1, hd), 1e-6).ravel(), np.tile(w[c], n * h))
+        want[c] = np.asarray(orc.rope(np.asarray(x, np.float32).reshape(n, h * hd), pos.tolist(), hd, 1e7)).reshape(n, h * hd)
+
+    def moved(x):  # `shift` bytes into a buffer
+        b = DevBuf.from_array(np.concatenate([np.zeros(shift // 4, np.float32), x.ravel()]))
+        return b, b.ptr + shift
+
+    (bq, pq), (bk, pk) = moved(q), moved(k)
+    dv, tab = DevBuf.from_array(v), DevBuf.from_array(ops.rope_table(max_kv, hd, 1e7))
+    dw = {c: DevBuf.from_array(x) if x is not None else None for c, x in w.items()}
+    meta = DevBuf.from_array(np.stack([np.zeros(n, np.int32), pos], 1))
+    n_rows = (n if own_caches else 1) * max_kv
+    elem = np.float16 if kv16 else np.float32
+    cache = [DevBuf.zeroed(n_rows * kv_heads * hd * np.dtype(elem).itemsize) for _ in range(2)]
+    args = [pq, dw["q"].ptr if dw["q"] else None, pk, dw["k"].ptr if dw["k"] else None, dv.ptr, cache[0].ptr, cache[1].ptr, heads, kv_heads, hd,
+            meta.ptr, tab.ptr, 1e-6, n] + ([max_kv] if own_caches else [])
+    getattr(lib(), "llamd_fwd_qk_norm_rope_store" + ("" if own_caches else "_tile") + ("_kv16" if kv16 else ""))(*args)
+    sync()
+    assert bit_equal(bq.download_f32(shift // 4 + q.size)[shift // 4:].reshape(q.shape), want["q"])
+    assert bit_equal(bk.download_f32(shift // 4 + k.size)[shift // 4:].reshape(k.shape), want["k"])
+    for buf, x in ((cache[0], want["k"]), (cache[1], v)):
+        full = np.zeros((n_rows, kv_heads * hd), elem)
+        full[rows] = x.astype(elem)
+        got = buf.download_f32(buf.nbytes // 4).view(elem).reshape(full.shape)
+        assert np.array_equal(got.view(np.uint8), full.view(np.uint8))
+
+
 @pytest.mark.parametrize("rows,k,ntok", [(128, 2048, 37), (8, 256, 1), (50, 100, 19), (33, 68, 16), (33, 772, 129), (128, 640, 593)])
 def test_matmul_f32_tokens(ops, orc, synth, rows, k, ntok):
     """The tile form of the f32 matvec: every output is the same -0.0-seeded left-to-right sum."""
