@@ -214,6 +214,8 @@ struct MatvecPlans {
     // L2 instead of reading them from HBM again. Produced by slot_order_launch; must be complete when the ids are.
     const int32_t *slot_order;
 };
+// llamd_fwd_matmul_f32_tokens; w_ready: no launch in front on the stream writes w (a model's weights).
+void matmul_f32_tokens(const float *w, const float *x, float *out, int k, int rows, int ntok, bool w_ready);
 // A tile's scatter plan, pairs in any order within an expert. One small launch.
 void moe_plan_launch(const int32_t *ids, int npair, int n_expert, int n_used, int32_t *gstart, int32_t *gcount, int32_t *ptoken, int32_t *pslot);
 // order[] = the slots 0..n_slots-1 sorted by ids[slot]. One small launch.

@@ -4,7 +4,7 @@
 // The sum over i is one chain per output element and stays one: a lane owns a row and walks i in order for two or four
 // tokens whose chains take turns. 2048 dependent adds are 4.6 us at 1.9 GHz whatever else happens, so everything else has
 // to fit beside them: the copies of the operands (chunks of 128 columns, 4 or 5 in flight, by warps of their own, the
-// weights' first ones before the dependency wait), the shared loads and the multiplies (a register set ahead of the adds).
+// weights' first ones before the dependency wait where the caller says that no launch in front writes them), the shared loads and the multiplies (a register set ahead of the adds).
 // Bound by instruction issue of the adding warps, and by L2 for many tokens. The router logits of a tile (128 experts x
 // 2048 columns) are the user, us with a 2x2 patch of chains per thread (16 tokens a CTA, one 64-column chunk ahead) / now:
 // 8 to 64 tokens 36.7 / 14.6, 128 36.7 / 21, 512 37.5 / 24.6, 2000 83 / 84.
@@ -27,7 +27,7 @@ constexpr int kFS = kFK + 4;  // shared-memory row stride: 16-byte aligned, neig
 // grid (row tiles, token tiles). Adding warp v owns tokens TPW*v .. +TPW-1 of its CTA's tile, lane r row r.
 template <int TPW, int kFWarps, int kFStages>
 __global__ void __launch_bounds__(32 * (kFWarps + kFLoaders)) matmul_f32_tokens_kernel(const float *__restrict__ w, const float *__restrict__ x, float *__restrict__ out,
-                                                                         int k, int rows, int ntok) {
+                                                                         int k, int rows, int ntok, int w_ready) {
     constexpr int kTok = TPW * kFWarps;
     extern __shared__ __align__(16) float sm[];  // [kFStages][kFR + kTok][kFS]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -48,8 +48,9 @@ __global__ void __launch_bounds__(32 * (kFWarps + kFLoaders)) matmul_f32_tokens_
         };
         const float *ws = w + (size_t)r0 * k, *xs = x + (size_t)t0 * k;
         const int nw = min(kFR, rows - r0), nx = min(kTok, ntok - t0);
+        if (!w_ready) pdl_wait();
         for (int ch = 0; ch < kFStages - 1 && ch < n_chunks; ch++) rows_of(ch, ws, nw, 0);
-        pdl_wait();
+        if (w_ready) pdl_wait();
         for (int ch = 0; ch < kFStages - 1; ch++) {
             if (ch < n_chunks) rows_of(ch, xs, nx, kFR);
             cp_async_commit();  // (the weights above join the first group)
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(32 * (kFWarps + kFLoaders)) matmul_f32_tokens_
 }
 
 template <int TPW, int kFWarps, int kFStages>
-void matmul_f32_tokens_launch(const float *w, const float *x, float *out, int k, int rows, int ntok) {
+void matmul_f32_tokens_launch(const float *w, const float *x, float *out, int k, int rows, int ntok, bool w_ready) {
     constexpr int kTok = TPW * kFWarps, kSmem = kFStages * (kFR + kTok) * kFS * 4 + 256;  // (+ what the last loads run past)
     static bool configured = false;
     if (!configured) {
@@ -150,7 +151,7 @@ void matmul_f32_tokens_launch(const float *w, const float *x, float *out, int k,
         configured = true;
     }
     launch_kc(PDL_ROUTER, "matmul_f32_tokens", matmul_f32_tokens_kernel<TPW, kFWarps, kFStages>, dim3((rows + kFR - 1) / kFR, (ntok + kTok - 1) / kTok), dim3(32 * (kFWarps + kFLoaders)), kSmem,
-              w, x, out, k, rows, ntok);
+              w, x, out, k, rows, ntok, (int)w_ready);
 }
 
 }  // namespace
@@ -158,7 +159,7 @@ void matmul_f32_tokens_launch(const float *w, const float *x, float *out, int k,
 
 using namespace llamd;
 
-extern "C" void llamd_fwd_matmul_f32_tokens(const float *w, const float *x, float *out, int k, int rows, int ntok) {
+void llamd::matmul_f32_tokens(const float *w, const float *x, float *out, int k, int rows, int ntok, bool w_ready) {
     if (ntok <= 0 || rows <= 0) return;
     if (k < 4 || k % 4) {
         set_error_msg("matmul_f32_tokens: k must be a positive multiple of 4");
@@ -170,9 +171,12 @@ extern "C" void llamd_fwd_matmul_f32_tokens(const float *w, const float *x, floa
     // CTAs than SMs (2000 tokens 96 and 84 us, but 300 tokens 24 and 37: two on some SMs, none on others).
     const long long ctas = (long long)((rows + kFR - 1) / kFR) * ((ntok + 15) / 16);
     if (ntok <= 128)
-        matmul_f32_tokens_launch<2, 2, 5>(w, x, out, k, rows, ntok);
+        matmul_f32_tokens_launch<2, 2, 5>(w, x, out, k, rows, ntok, w_ready);
     else if (ctas <= 148)
-        matmul_f32_tokens_launch<4, 4, 5>(w, x, out, k, rows, ntok);
+        matmul_f32_tokens_launch<4, 4, 5>(w, x, out, k, rows, ntok, w_ready);
     else
-        matmul_f32_tokens_launch<4, 4, 4>(w, x, out, k, rows, ntok);
+        matmul_f32_tokens_launch<4, 4, 4>(w, x, out, k, rows, ntok, w_ready);
+}
+extern "C" void llamd_fwd_matmul_f32_tokens(const float *w, const float *x, float *out, int k, int rows, int ntok) {
+    matmul_f32_tokens(w, x, out, k, rows, ntok, false);
 }

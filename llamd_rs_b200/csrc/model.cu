@@ -34,7 +34,6 @@ void llamd_fwd_attention_tile(const float *q, const float *kc, const float *vc, 
                               int hd, const int32_t *meta, int max_kv, int ntok);
 void llamd_fwd_attention_prefill(const float *q, const float *kc, const float *vc, float *out, float *scores, int n_head, int n_head_kv,
                                  int hd, const int32_t *meta, int max_kv, int ntok, int n_kv_max);
-void llamd_fwd_matmul_f32_tokens(const float *w, const float *x, float *out, int k, int rows, int ntok);
 void llamd_fwd_norm_router(const float *w, const float *x, const float *residual, float *x_out, const float *w_norm, float *xn_out,
                            int8_t *qs, float *d, int k, float eps, int n_expert, int n_used, float *logits, int32_t *ids, float *weights,
                            float *probs, unsigned int *counter, int nseq);
@@ -560,7 +559,7 @@ void queue_token(Model &m, int nseq, bool near) {
                                      hp.rms_eps, nseq, pf);
             mark(LLAMD_PH_FFN_NORM);
             if (nseq > kRouterRowsMax) {
-                llamd_fwd_matmul_f32_tokens(l.ffn_gate_inp.as<float>(), m.xb.as<float>(), m.router_logits.as<float>(), E, hp.n_expert, nseq);
+                matmul_f32_tokens(l.ffn_gate_inp.as<float>(), m.xb.as<float>(), m.router_logits.as<float>(), E, hp.n_expert, nseq, true);
                 llamd_fwd_router(m.router_logits.as<float>(), hp.n_expert, nu, m.expert_ids.as<int32_t>(), m.expert_w.as<float>(), nullptr, nseq);
             } else {
                 llamd_fwd_router_matvec(l.ffn_gate_inp.as<float>(), m.xb.as<float>(), E, hp.n_expert, nu, m.router_logits.as<float>(),
@@ -1583,7 +1582,7 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
         add_rms_norm_quant_flags(x, p.xb2.as<float>(), x, l.ffn_norm.as<float>(), p.xb.as<float>(), p.aq.as<int8_t>(), p.ad.as<float>(),
                                      E, hp.rms_eps, T, 0, small || ep ? nullptr : rm);
         if (m.prefill_attn && T > kRouterRowsMax) {
-            llamd_fwd_matmul_f32_tokens(l.ffn_gate_inp.as<float>(), p.xb.as<float>(), p.logits.as<float>(), E, ne, T);
+            matmul_f32_tokens(l.ffn_gate_inp.as<float>(), p.xb.as<float>(), p.logits.as<float>(), E, ne, T, true);
             llamd_fwd_router(p.logits.as<float>(), ne, nu, p.ids.as<int32_t>(), p.w.as<float>(), nullptr, T);
         } else {
             llamd_fwd_router_matvec(l.ffn_gate_inp.as<float>(), p.xb.as<float>(), E, ne, nu, p.logits.as<float>(), p.ids.as<int32_t>(),

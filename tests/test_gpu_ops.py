@@ -268,6 +268,28 @@ def test_matmul_f32_tokens(ops, orc, synth, rows, k, ntok):
     assert np.all(np.signbit(z)), "an all -0.0 sum keeps its sign: no padding term enters a chain"
 
 
+@pytest.mark.parametrize("ntok", [5, 300])
+def test_matmul_f32_tokens_of_a_launch_in_front(ops, synth, ntok):
+    """The matrix may be what the launch in front on the stream writes: the same bits as with a wait between the two."""
+    from llamd_rs_b200.backend import DevBuf, sync
+    from llamd_rs_b200._lib import lib
+
+    k0, k, rows = 4096, 512, 96
+    w0, x0 = (DevBuf.from_array(synth.normal_f32(n * k0, 92, "front", n, std=0.02)) for n in (k, rows))
+    x, w, out = DevBuf.from_array(synth.normal_f32(ntok * k, 92, "front.x")), DevBuf(rows * k * 4), DevBuf(ntok * rows * 4)
+    got = []
+    for wait in (True, False, False, False):
+        lib().llamd_fwd_memset(w.ptr, 0, w.nbytes)
+        sync()
+        lib().llamd_fwd_matmul_f32_tokens(w0.ptr, x0.ptr, w.ptr, k0, k, rows)  # w [rows][k]
+        if wait:
+            sync()
+        lib().llamd_fwd_matmul_f32_tokens(w.ptr, x.ptr, out.ptr, k, rows, ntok)
+        sync()
+        got.append(out.download_f32(ntok * rows))
+    assert np.any(got[0] != 0) and all(bit_equal(got[0], g) for g in got[1:])
+
+
 def test_silu_mul_and_quant(ops, orc, synth):
     g = synth.normal_f32(8 * 768, 6, "g") * np.float32(3.0)
     u = synth.normal_f32(8 * 768, 6, "u")
