@@ -19,6 +19,7 @@
 // an accumulator that started at +0.0 leaves it unchanged, so every token's
 // chain is exactly the chain over its own positions.
 #include "common.cuh"
+#include "packed_f32.cuh"
 #include "quant.cuh"
 
 namespace llamd {
@@ -34,27 +35,10 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Two chains per instruction: packed f32 multiply, and the add as an fma with 1.0 in a value the compiler cannot see (a packed
-// multiply feeding a packed add is contracted into one fma, which rounds once where the reference rounds twice). The FP32 pipe
-// does as many operations a cycle either way, but at two a scalar instruction left no issue slots for the shared-memory
-// loads: us a 512-token piece of a 2000-token prompt, scalar / packed: scores 199 / 181, values 214 / 200.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul_add2(f32x2 a, f32x2 b, f32x2 s, f32x2 one) {  // s + a*b, each rounded
-    f32x2 r;
-    asm("{\n\t.reg .b64 t;\n\tmul.rn.f32x2 t, %1, %2;\n\tfma.rn.f32x2 %0, t, %4, %3;\n\t}" : "=l"(r) : "l"(a), "l"(b), "l"(s), "l"(one));
-    return r;
-}
-constexpr f32x2 kOne2 = 0x3F8000003F800000ull;  // passed to the kernels as a parameter
+// Two chains per instruction (packed_f32.cuh). The FP32 pipe does as many operations a cycle either way, but at two a scalar
+// instruction left no issue slots for the shared-memory loads: us a 512-token piece of a 2000-token prompt, scalar / packed:
+// scores 199 / 181, values 214 / 200.
+__device__ __forceinline__ f32x2 mul_add2(f32x2 a, f32x2 b, f32x2 s, f32x2 one) { return add2(s, mul2(a, b), one); }  // s + a*b, each rounded
 
 constexpr int kST = 64;  // tokens per CTA of the score kernel
 constexpr int kSP = 64;  // positions per CTA of the score kernel

@@ -25,6 +25,7 @@
 //   grouped  grid (row tiles, experts), 4 warps: one fold, then all of the expert's tokens;
 //   dense    a fixed number of resident CTAs (8 warps) split the (row tile, 64-token chunk)
 //            items evenly; a CTA folds a row tile once for the consecutive chunks it owns.
+#include "packed_f32.cuh"
 #include "q6k_layout.cuh"
 
 namespace llamd {
@@ -57,33 +58,8 @@ struct GemmParams {
     // each exactly what fold_row_tile leaves in shared memory (A fragments, then the 16 x nb block scales)
     const uint8_t *folded[3];
     long long fold_tile_bytes;
-    unsigned long long one;  // 1.0f twice (see gemm_add2)
+    f32x2 one;  // kOne2
 };
-
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 gemm_pack(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 gemm_unpack(f32x2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 gemm_mul2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 gemm_fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-// s + t, rounded once, as an fma with 1.0 in a value the compiler cannot see: a packed multiply feeding a packed add is
-// contracted into one fma, which rounds once where the reference rounds twice.
-__device__ __forceinline__ f32x2 gemm_add2(f32x2 s, f32x2 t, f32x2 one) { return gemm_fma2(t, one, s); }
 
 // Ask L2 for the tiles that hold the 16 x nb blocks starting at block `unit0` (a hint: nothing waits on it).
 __device__ __forceinline__ void prefetch_row_tile(const uint8_t *w, size_t unit0, int live_rows, int nb) {
@@ -423,22 +399,20 @@ __global__ void __launch_bounds__(128, HOIST ? 3 : 5) q6k_gemm_grouped_kernel(co
 // s_b (coalesced 16-byte loads; the next block's wait in registers meanwhile), 16-byte pieces swizzled by the token so that
 // the MMA's fragment reads meet 32 banks. At the end the eight residues' sums meet in s_b and are added in order.
 template <int NT>
-__device__ __forceinline__ void mma_group(const GemmParams &p, int j, int row0, int rows, int first, int count, int n0, const uint4 *s_frag,
-                                          const float *s_d, uint32_t *s_b, float *s_ad, int tid) {
-    const int nb = p.nb, rp = tid >> 5, lane = tid & 31;
+__device__ __forceinline__ void folded_tiles(const GemmParams &p, int j, int row0, int n0, const uint4 *s_frag, const float *s_d, uint32_t *s_b,
+                                             float *s_ad, int tid) {
+    const int nb = p.nb, rp = tid >> 5, lane = tid & 31, rows = p.rows[j], count = p.n_tokens;
     const int g4 = lane >> 2, q4 = lane & 3;
-    auto pair_of = [&](int tok) { return first + min(n0 + tok, count - 1); };
+    auto token = [&](int tok) { return min(n0 + tok, count - 1); };
     for (int i = tid; i < NT * 8 * nb; i += 128) {  // the group's activation scales, [block][token]
-        const int tok = i / nb, b = i - tok * nb, pr = pair_of(tok);
-        s_ad[b * (8 * kGroupTiles) + tok] = __ldg(p.ad + (long long)(p.act_map ? p.act_map[pr] : pr) * nb + b);
+        const int tok = i / nb, b = i - tok * nb;
+        s_ad[b * (8 * kGroupTiles) + tok] = __ldg(p.ad + (long long)token(tok) * nb + b);
     }
     const uint4 *src[NT];
     uint4 st[NT];
 #pragma unroll
     for (int t = 0; t < NT; t++) {
-        const int pr = pair_of(t * 8 + g4);
-        const long long it = p.act_map ? p.act_map[pr] : pr;
-        src[t] = reinterpret_cast<const uint4 *>(p.aq_rm + (size_t)it * nb * 64) + rp * 4 + q4;
+        src[t] = reinterpret_cast<const uint4 *>(p.aq_rm + (size_t)token(t * 8 + g4) * nb * 64) + rp * 4 + q4;
         st[t] = __ldg(src[t]);
     }
     uint32_t *mine = s_b + rp * (kTeamWords / 4);
@@ -462,8 +436,8 @@ __device__ __forceinline__ void mma_group(const GemmParams &p, int j, int row0, 
 #pragma unroll
         for (int t = 0; t < NT; t++) {
             const f32x2 a = *reinterpret_cast<const f32x2 *>(s_ad + b * (8 * kGroupTiles) + t * 8 + 2 * q4);
-            dsc[t][0] = gemm_mul2(gemm_pack(d0, d0), a);
-            dsc[t][1] = gemm_mul2(gemm_pack(d1, d1), a);
+            dsc[t][0] = mul2(pack2(d0, d0), a);
+            dsc[t][1] = mul2(pack2(d1, d1), a);
         }
         const uint4 *fr = s_frag + ((size_t)(b * 8 + 2 * rp) * 2) * 32 + (lane ^ (lane >> 3) ^ (b & 7));
 #pragma unroll
@@ -479,9 +453,9 @@ __device__ __forceinline__ void mma_group(const GemmParams &p, int j, int row0, 
                 mma_s8<0x4B400000>(cl, al, b0w, b1w);
 #pragma unroll
                 for (int h = 0; h < 2; h++) {  // rows g4 and g4 + 8, tokens 2 q4 and 2 q4 + 1
-                    const f32x2 hi = gemm_add2(gemm_pack(__int_as_float(ch[2 * h]), __int_as_float(ch[2 * h + 1])), off, one);
-                    const f32x2 lo = gemm_add2(gemm_pack(__int_as_float(cl[2 * h]), __int_as_float(cl[2 * h + 1])), off, one);
-                    sum[t][rr][h] = gemm_add2(sum[t][rr][h], gemm_mul2(dsc[t][h], gemm_fma2(hi, c64, lo)), one);
+                    const f32x2 hi = add2(pack2(__int_as_float(ch[2 * h]), __int_as_float(ch[2 * h + 1])), off, one);
+                    const f32x2 lo = add2(pack2(__int_as_float(cl[2 * h]), __int_as_float(cl[2 * h + 1])), off, one);
+                    sum[t][rr][h] = add2(sum[t][rr][h], mul2(dsc[t][h], fma2(hi, c64, lo)), one);
                 }
             }
         }
@@ -498,10 +472,10 @@ __device__ __forceinline__ void mma_group(const GemmParams &p, int j, int row0, 
             for (int h = 0; h < 2; h++) {
                 float *x = s_x + ((t - t0) * 8 + q4) * 16 + g4 + 8 * h;  // (token 2 q4 + e has place q4 + 4 e)
                 if (rp == 0) {
-                    const float2 v = gemm_unpack(gemm_add2(sum[t][0][h], sum[t][1][h], one));
+                    const float2 v = unpack2(add2(sum[t][0][h], sum[t][1][h], one));
                     x[0] = v.x, x[4 * 16] = v.y;
                 } else {
-                    const float2 v = gemm_unpack(sum[t][0][h]), u = gemm_unpack(sum[t][1][h]);
+                    const float2 v = unpack2(sum[t][0][h]), u = unpack2(sum[t][1][h]);
                     x += (2 * rp - 1) * 256;
                     x[0] = v.x, x[4 * 16] = v.y, x[256] = u.x, x[256 + 4 * 16] = u.y;
                 }
@@ -516,23 +490,11 @@ __device__ __forceinline__ void mma_group(const GemmParams &p, int j, int row0, 
 #pragma unroll
             for (int r = 1; r < 7; r++) y = __fadd_rn(y, x[r * 256]);
             const int n = n0 + t * 8 + 2 * (place & 3) + (place >> 2);
-            if (n < count && row0 + row < rows) {
-                long long o = p.out_map ? p.out_map[first + n] : first + n;
-                float *out = p.out[j];
-                if (p.out_tab) {  // the rows of a pair go to the GPU the pair's token lives on (plain peer stores)
-                    out = p.out_tab[o / p.out_div];
-                    o %= p.out_div;
-                }
-                out[o * rows + row0 + row] = y;
-            }
+            if (n < count && row0 + row < rows) p.out[j][(size_t)n * rows + row0 + row] = y;
         }
     }
 }
 
-template <int NT>
-__device__ __forceinline__ void folded_tiles(const GemmParams &p, int j, int row0, int t, const uint4 *s_frag, const float *s_d, uint32_t *s_b, float *s_ad, int tid) {
-    mma_group<NT>(p, j, row0, p.rows[j], 0, p.n_tokens, t * 8, s_frag, s_d, s_b, s_ad, tid);
-}
 static_assert(7 * 256 * 4 <= kTeamWords * 4, "the residues' sums of two tiles fit where the activations were");
 
 __host__ __device__ inline size_t folded_smem_bytes(int nb) {
@@ -561,10 +523,10 @@ __global__ void __launch_bounds__(128, 3) q6k_gemm_folded_kernel(const GemmParam
     for (int g = 0, t = 0; g < groups; g++) {  // as few equal groups as kGroupTiles allows
         const int nt = (tiles - t + groups - g - 1) / (groups - g);
         switch (nt) {
-        case 1: folded_tiles<1>(p, j, rt * kGemmRows, t, s_frag, s_d, s_b, s_ad, tid); break;
-        case 2: folded_tiles<2>(p, j, rt * kGemmRows, t, s_frag, s_d, s_b, s_ad, tid); break;
-        case 3: folded_tiles<3>(p, j, rt * kGemmRows, t, s_frag, s_d, s_b, s_ad, tid); break;
-        default: folded_tiles<4>(p, j, rt * kGemmRows, t, s_frag, s_d, s_b, s_ad, tid); break;
+        case 1: folded_tiles<1>(p, j, rt * kGemmRows, t * 8, s_frag, s_d, s_b, s_ad, tid); break;
+        case 2: folded_tiles<2>(p, j, rt * kGemmRows, t * 8, s_frag, s_d, s_b, s_ad, tid); break;
+        case 3: folded_tiles<3>(p, j, rt * kGemmRows, t * 8, s_frag, s_d, s_b, s_ad, tid); break;
+        default: folded_tiles<4>(p, j, rt * kGemmRows, t * 8, s_frag, s_d, s_b, s_ad, tid); break;
         }
         t += nt;
     }
@@ -783,7 +745,7 @@ void llamd::gemm_tokens_folded3(const void *f0, const void *f1, const void *f2, 
     p.aq_rm = (const uint32_t *)aq_rm;
     p.ad = ad;
     p.n_tokens = ntok;
-    p.one = 0x3F8000003F800000ull;
+    p.one = kOne2;
     const size_t smem = folded_smem_bytes(blocks);
     if (blocks < 1 || smem > 220 * 1024) {
         set_error_msg("q6k gemm: blocks per row must be 1..24");

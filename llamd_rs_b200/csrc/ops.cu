@@ -10,6 +10,7 @@
 
 #include <vector>
 
+#include "packed_f32.cuh"
 #include "q6k_layout.cuh"
 #include "quant.cuh"
 #include "pos_sum.cuh"
@@ -340,11 +341,6 @@ constexpr int kQ80ChunkBlocks = 8;
 constexpr int kQ80Producers = 224;   // 7 warps
 constexpr int kQ80MaxRaw = 32;       // raw chunks in flight
 constexpr int kQ80RingBytes = 2 * kQ80ChunkBlocks * 32 * 32 * 4, kQ80RawBytes = kQ80ChunkBlocks * kQ80TileBytes;
-__device__ __forceinline__ unsigned long long q80_mul2(unsigned long long w, unsigned long long x) {
-    unsigned long long r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(w), "l"(x));
-    return r;
-}
 template <int NSEQ>
 __global__ void __launch_bounds__(kQ80Producers + 32 * NSEQ) matvec_q8_0_bulk_kernel(const uint8_t *__restrict__ tiled, const float *__restrict__ x,
                                                                                      float *__restrict__ out, int blocks, int rows, int n_raw, int *status) {
@@ -468,7 +464,7 @@ __global__ void __launch_bounds__(kQ80Producers + 32 * NSEQ) matvec_q8_0_bulk_ke
                 };
                 auto products = [&](ulonglong2 (&o)[4]) {
 #pragma unroll
-                    for (int j = 0; j < 4; j++) o[j].x = q80_mul2(wv[j].x, xv[j].x), o[j].y = q80_mul2(wv[j].y, xv[j].y);
+                    for (int j = 0; j < 4; j++) o[j].x = mul2(wv[j].x, xv[j].x), o[j].y = mul2(wv[j].y, xv[j].y);
                 };
                 fetch(0);
                 products(pr);
@@ -1426,54 +1422,54 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
         pdl_wait();
     }
     if (ROPE) {
-    // ---- QK-norm (crates/llamd-runtime/src/layer.rs:62-79) and RoPE (crates/llamd-cpu/src/lib.rs:158-209) of the kv head's
-    // query heads (adjacent in q_raw) and, where needed, of the new key
-    const int n_vec = ratio + (need_k ? 1 : 0);
-    for (int i = tid; i < n_vec * hd; i += blockDim.x) {
-        const float x = i < ratio * hd ? q_raw[((size_t)seq * n_head + h0) * hd + i] : k_raw[((size_t)seq * n_head_kv + kvh) * hd + i - ratio * hd];
-        s_raw[i] = x;
-        tile[i] = __fmul_rn(x, x);  // (no cached tile is in place yet)
-    }
-    __syncthreads();
-    {
-        // vector v's sum of squares is walked in order by lane v / 8 of warp v % 8: the chains run side by side
-        const int warp = tid >> 5, lane = tid & 31, v = lane * 8 + warp;
-        if (lane < 2 && v < n_vec && (v < ratio ? wq != nullptr : wk != nullptr)) {
-            const float sum = chain_sum(tile + v * hd, hd, 0.0f);
-            s_scale[v] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)hd), eps)));
+        // ---- QK-norm (crates/llamd-runtime/src/layer.rs:62-79) and RoPE (crates/llamd-cpu/src/lib.rs:158-209) of the kv head's
+        // query heads (adjacent in q_raw) and, where needed, of the new key
+        const int n_vec = ratio + (need_k ? 1 : 0);
+        for (int i = tid; i < n_vec * hd; i += blockDim.x) {
+            const float x = i < ratio * hd ? q_raw[((size_t)seq * n_head + h0) * hd + i] : k_raw[((size_t)seq * n_head_kv + kvh) * hd + i - ratio * hd];
+            s_raw[i] = x;
+            tile[i] = __fmul_rn(x, x);  // (no cached tile is in place yet)
         }
-    }
-    __syncthreads();
-    for (int idx = tid; idx < n_vec * half; idx += blockDim.x) {
-        const int v = idx / half, i = idx - v * half;
-        const bool is_k = v == ratio;
-        const float *sx = s_raw + v * hd;
-        const float *w = is_k ? wk : wq;
-        float a = sx[i], b = sx[i + half];
-        if (w) {
-            const float nsc = s_scale[v];
-            a = __fmul_rn(__fmul_rn(a, nsc), w[i]);
-            b = __fmul_rn(__fmul_rn(b, nsc), w[i + half]);
+        __syncthreads();
+        {
+            // vector v's sum of squares is walked in order by lane v / 8 of warp v % 8: the chains run side by side
+            const int warp = tid >> 5, lane = tid & 31, v = lane * 8 + warp;
+            if (lane < 2 && v < n_vec && (v < ratio ? wq != nullptr : wk != nullptr)) {
+                const float sum = chain_sum(tile + v * hd, hd, 0.0f);
+                s_scale[v] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)hd), eps)));
+            }
         }
-        const float2 cs = *reinterpret_cast<const float2 *>(rope_tab + ((size_t)pos * half + i) * 2);
-        const float o0 = __fsub_rn(__fmul_rn(a, cs.y), __fmul_rn(b, cs.x));
-        const float o1 = __fadd_rn(__fmul_rn(a, cs.x), __fmul_rn(b, cs.y));
-        if (!is_k) {
-            sq[v * hd + i] = o0;
-            sq[v * hd + i + half] = o1;
-        } else {
-            KVT t0, t1;  // as the cache holds it (a binary16 cache rounds here, once)
-            KvIo<KVT>::st(&t0, o0);
-            KvIo<KVT>::st(&t1, o1);
-            sk[i] = (float)t0;
-            sk[i + half] = (float)t1;
-            krow[i] = t0;
-            krow[i + half] = t1;
-            const float *vs = v_raw + ((size_t)seq * n_head_kv + kvh) * hd;
-            KvIo<KVT>::st(vrow + i, vs[i]);
-            KvIo<KVT>::st(vrow + i + half, vs[i + half]);
+        __syncthreads();
+        for (int idx = tid; idx < n_vec * half; idx += blockDim.x) {
+            const int v = idx / half, i = idx - v * half;
+            const bool is_k = v == ratio;
+            const float *sx = s_raw + v * hd;
+            const float *w = is_k ? wk : wq;
+            float a = sx[i], b = sx[i + half];
+            if (w) {
+                const float nsc = s_scale[v];
+                a = __fmul_rn(__fmul_rn(a, nsc), w[i]);
+                b = __fmul_rn(__fmul_rn(b, nsc), w[i + half]);
+            }
+            const float2 cs = *reinterpret_cast<const float2 *>(rope_tab + ((size_t)pos * half + i) * 2);
+            const float o0 = __fsub_rn(__fmul_rn(a, cs.y), __fmul_rn(b, cs.x));
+            const float o1 = __fadd_rn(__fmul_rn(a, cs.x), __fmul_rn(b, cs.y));
+            if (!is_k) {
+                sq[v * hd + i] = o0;
+                sq[v * hd + i + half] = o1;
+            } else {
+                KVT t0, t1;  // as the cache holds it (a binary16 cache rounds here, once)
+                KvIo<KVT>::st(&t0, o0);
+                KvIo<KVT>::st(&t1, o1);
+                sk[i] = (float)t0;
+                sk[i + half] = (float)t1;
+                krow[i] = t0;
+                krow[i + half] = t1;
+                const float *vs = v_raw + ((size_t)seq * n_head_kv + kvh) * hd;
+                KvIo<KVT>::st(vrow + i, vs[i]);
+                KvIo<KVT>::st(vrow + i + half, vs[i + half]);
+            }
         }
-    }
     } else {
         for (int i = tid; i < ratio * hd; i += blockDim.x) sq[i] = q_raw[((size_t)seq * n_head + h0) * hd + i];
     }
