@@ -539,3 +539,71 @@ def test_near_and_far_contexts(kv16):
     finally:
         gm.use_graph = True
         gm.free()
+
+
+@pytest.mark.parametrize("kv16", [0, 1])
+def test_automatic_tiles_equal_sequential_decode(kv16):
+    """prefill_tile never set: one tile up to 2048 tokens, two equal ones beyond, attention 512 tokens at a time. Tokens, logits and
+    K/V rows are those of one token after the other, from position 0 and behind a context; and on the tile GEMMs alone for the
+    lengths that otherwise run on the decode pass's launches."""
+    from llamd_rs_b200 import synth
+    from llamd_rs_b200.model import CudaModel
+
+    hp = synth.TINY
+    gm = CudaModel.load_batched(hp, synth.make_model(hp, seed=7), max_kv=2112, max_seq=1)
+    try:
+        if kv16:
+            gm.set_option("kv_f16", 1)
+        toks = synth.token_ids(2049, hp["n_vocab"], 5, "automatic tile").tolist()
+        ends, want = (37, 57, 193, 512, 513, 1025, 2048, 2049), {}
+        for pos, t in enumerate(toks):
+            tok = gm.forward(t, pos)
+            if pos + 1 in ends:
+                want[pos + 1] = tok, gm.logits()[0].view(np.uint32).copy()
+        rows = [[x.view(np.uint32).copy() for x in gm.read_kv(il, len(toks))] for il in range(hp["n_layer"])]
+        kvd = hp["n_head_kv"] * hp["head_dim"]
+        for gemm_only in (False, True):
+            gm.set_option("matvec_batch_max", 8 if gemm_only else 56)
+            gm.set_option("dense_gemm", 0 if gemm_only else 8)
+            for end in ends:
+                for base in (0, 20):
+                    gm.prefill(toks[:base] or toks[:1], 0)
+                    tok = gm.prefill(toks[base:end], base)
+                    what = f"{end - base} tokens from {base}, GEMMs only: {gemm_only}"
+                    assert tok == want[end][0] and np.array_equal(gm.logits()[0].view(np.uint32), want[end][1]), what
+                    for il in range(hp["n_layer"]):
+                        for got, ref in zip(gm.read_kv(il, end), rows[il]):
+                            assert np.array_equal(got.view(np.uint32), ref[:end * kvd]), what
+    finally:
+        gm.free()
+
+
+def test_tile_gemms_equal_sequential_decode_at_wide_rows():
+    """The benchmark's widths (8 blocks in, 16 out of attention, heads of 128, eight to a kv head, 8 experts of 16 used): the tile
+    GEMMs without folded copies against one token after the other."""
+    from llamd_rs_b200 import synth
+    from llamd_rs_b200.model import CudaModel
+
+    hp = dict(synth.QWEN3MOE_30B, n_layer=1, n_expert=16, n_vocab=1024)
+    gm = CudaModel.load_batched(hp, synth.make_model(hp, seed=7), max_kv=320, max_seq=1)
+    try:
+        toks = synth.token_ids(300, hp["n_vocab"], 5, "wide rows").tolist()
+        ends, want = (9, 40, 65, 300), {}
+        for pos, t in enumerate(toks):
+            tok = gm.forward(t, pos)
+            if pos + 1 in ends:
+                want[pos + 1] = tok, gm.logits()[0].view(np.uint32).copy()
+        rows = [x.view(np.uint32).copy() for x in gm.read_kv(0, len(toks))]
+        kvd = hp["n_head_kv"] * hp["head_dim"]
+        for line, dense in ((8, 0), (56, 8)):
+            gm.set_option("matvec_batch_max", line)
+            gm.set_option("dense_gemm", dense)
+            for end in ends:
+                tok = gm.prefill(toks[:end], 0)
+                what = f"{end} tokens, matvec launches up to {line}"
+                assert tok == want[end][0] and np.array_equal(gm.logits()[0].view(np.uint32), want[end][1]), what
+                assert all(np.array_equal(g.view(np.uint32), r[:end * kvd]) for g, r in zip(gm.read_kv(0, end), rows)), what
+                if end <= 65:
+                    assert gm.verify(toks[:end], 0)[-1] == tok, what
+    finally:
+        gm.free()
