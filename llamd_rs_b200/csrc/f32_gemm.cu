@@ -5,9 +5,9 @@
 // tokens whose chains take turns. 2048 dependent adds are 4.6 us at 1.9 GHz whatever else happens, so everything else has
 // to fit beside them: the copies of the operands (chunks of 128 columns, 4 or 5 in flight, by warps of their own, the
 // weights' first ones before the dependency wait where the caller says that no launch in front writes them), the shared loads and the multiplies (a register set ahead of the adds).
-// Bound by instruction issue of the adding warps, and by L2 for many tokens. The router logits of a tile (128 experts x
-// 2048 columns) are the user, us with a 2x2 patch of chains per thread (16 tokens a CTA, one 64-column chunk ahead) / now:
-// 8 to 64 tokens 36.7 / 14.6, 128 36.7 / 21, 512 37.5 / 24.6, 2000 83 / 84.
+// Bound by instruction issue of the adding warps, and by L2 for many tokens; where the CTAs are more than two per SM a 2x2
+// patch of chains per thread is quicker (matmul_f32_patch_kernel). The router logits of a tile (128 experts x 2048 columns) are
+// the user, us with patches / this: 8 to 64 tokens 37.0 / 15 to 18, 128 37.0 / 22.9, 512 37.0 / 25.0, 1000 53.4 / 44.4, 2000 80.1 / 85.3.
 #include "common.cuh"
 
 namespace llamd {
@@ -139,6 +139,84 @@ __global__ void __launch_bounds__(32 * (kFWarps + kFLoaders)) matmul_f32_tokens_
     }
 }
 
+// The same for many CTAs: a thread owns a 2x2 patch of outputs (two tokens x two rows) and walks i in order for its four
+// accumulators; a CTA stages 64 columns of 16 tokens and 32 rows (double-buffered), every staged value feeds two chains. The copies
+// and the multiplies stand between the adds, which costs a lone CTA twice the time; eight of them on an SM hide it.
+// grid (row tiles, token tiles), 128 threads. Thread (ty, tx) = (tid / 16, tid % 16) owns tokens 2ty, 2ty+1 and rows tx, tx+16.
+constexpr int kPT = 16, kPK = 64, kPS = kPK + 4;
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, int bytes) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+__global__ void __launch_bounds__(128) matmul_f32_patch_kernel(const float *__restrict__ w, const float *__restrict__ x, float *__restrict__ out, int k,
+                                                               int rows, int ntok) {
+    __shared__ __align__(16) float sX[2][kPT][kPS];
+    __shared__ __align__(16) float sW[2][kFR][kPS];
+    pdl_trigger();
+    pdl_wait();
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    const int r0 = blockIdx.x * kFR, t0 = blockIdx.y * kPT;
+    auto stage = [&](int k0, int buf) {
+        // 16-byte pieces: (16 + 32) rows x 16 pieces = 768, six per thread
+        for (int idx = tid; idx < (kPT + kFR) * (kPK / 4); idx += 128) {
+            const int r = idx >> 4, c = idx & 15;
+            const int col = k0 + 4 * c;
+            const int bytes = col < k ? 16 : 0;  // k is a multiple of 4
+            if (r < kPT) {
+                const int t = t0 + r;
+                cp_async16(&sX[buf][r][4 * c], x + (size_t)min(t, ntok - 1) * k + min(col, k - 4), t < ntok ? bytes : 0);
+            } else {
+                const int row = r0 + r - kPT;
+                cp_async16(&sW[buf][r - kPT][4 * c], w + (size_t)min(row, rows - 1) * k + min(col, k - 4), row < rows ? bytes : 0);
+            }
+        }
+        cp_async_commit();
+    };
+    float acc[2][2] = {{-0.0f, -0.0f}, {-0.0f, -0.0f}};
+    const int n_chunks = (k + kPK - 1) / kPK;
+    stage(0, 0);
+    for (int ch = 0; ch < n_chunks; ch++) {
+        const int buf = ch & 1;
+        if (ch + 1 < n_chunks) {
+            stage((ch + 1) * kPK, buf ^ 1);
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
+        }
+        __syncthreads();
+        const int n4 = min(kPK, k - ch * kPK) >> 2;  // no padding terms: a chain holds exactly its k products
+#pragma unroll 4
+        for (int c4 = 0; c4 < n4; c4++) {
+            float4 a[2], b[2];
+#pragma unroll
+            for (int i = 0; i < 2; i++) a[i] = *reinterpret_cast<const float4 *>(&sX[buf][2 * ty + i][4 * c4]);
+#pragma unroll
+            for (int j = 0; j < 2; j++) b[j] = *reinterpret_cast<const float4 *>(&sW[buf][tx + 16 * j][4 * c4]);
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    float s = acc[i][j];
+                    s = __fadd_rn(s, __fmul_rn(b[j].x, a[i].x));
+                    s = __fadd_rn(s, __fmul_rn(b[j].y, a[i].y));
+                    s = __fadd_rn(s, __fmul_rn(b[j].z, a[i].z));
+                    s = __fadd_rn(s, __fmul_rn(b[j].w, a[i].w));
+                    acc[i][j] = s;
+                }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int t = t0 + 2 * ty + i;
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int row = r0 + tx + 16 * j;
+            if (t < ntok && row < rows) out[(size_t)t * rows + row] = acc[i][j];
+        }
+    }
+}
+
 template <int TPW, int kFWarps, int kFStages>
 void matmul_f32_tokens_launch(const float *w, const float *x, float *out, int k, int rows, int ntok, bool w_ready) {
     constexpr int kTok = TPW * kFWarps, kSmem = kFStages * (kFR + kTok) * kFS * 4 + 256;  // (+ what the last loads run past)
@@ -165,17 +243,21 @@ void llamd::matmul_f32_tokens(const float *w, const float *x, float *out, int k,
         set_error_msg("matmul_f32_tokens: k must be a positive multiple of 4");
         return;
     }
-    // Few tokens: two warps of two tokens, so that a warp has nearly an SM to itself. More: four of four, or the CTAs' reads of
-    // the matrix become the limit (2048 columns of 32 rows each: 128 tokens 21 us this way and 24 that, 512 tokens 33 and 25).
-    // Five chunks in flight fill an SM with one such CTA; four let two share it, which is worth it only once there are more
-    // CTAs than SMs (2000 tokens 96 and 84 us, but 300 tokens 24 and 37: two on some SMs, none on others).
-    const long long ctas = (long long)((rows + kFR - 1) / kFR) * ((ntok + 15) / 16);
-    if (ntok <= 128)
+    // Small products: two warps of two tokens, so that a warp has nearly an SM to itself, while such CTAs are two per SM at most.
+    // More: four of four, or the CTAs' reads of the matrix become the limit; five chunks in flight fill an SM with one such CTA,
+    // four let two share it, which is worth it only once there are more CTAs than SMs. Beyond two of those per SM, the patches.
+    // us at 2048 columns, two of two / four of four / patches: 128 rows, 128 tokens 22.9 / 24.8 / 37.0; 256 rows, 128 tokens 23.9 /
+    // 24.9 / 37.0; 1024 rows, 64 tokens 43.9 / 25.1 / 37.0, 128 tokens 85 / 44 / 53; 300 tokens - / 104 / 98, 2000 - / 568 / 496.
+    const int row_tiles = (rows + kFR - 1) / kFR;
+    const long long small = (long long)row_tiles * ((ntok + 3) / 4), ctas = (long long)row_tiles * ((ntok + 15) / 16);
+    if (small <= 2 * 148)
         matmul_f32_tokens_launch<2, 2, 5>(w, x, out, k, rows, ntok, w_ready);
     else if (ctas <= 148)
         matmul_f32_tokens_launch<4, 4, 5>(w, x, out, k, rows, ntok, w_ready);
-    else
+    else if (ctas <= 2 * 148)
         matmul_f32_tokens_launch<4, 4, 4>(w, x, out, k, rows, ntok, w_ready);
+    else
+        launch_k("matmul_f32_patch", matmul_f32_patch_kernel, dim3(row_tiles, (ntok + kPT - 1) / kPT), dim3(128), 0, w, x, out, k, rows, ntok);
 }
 extern "C" void llamd_fwd_matmul_f32_tokens(const float *w, const float *x, float *out, int k, int rows, int ntok) {
     matmul_f32_tokens(w, x, out, k, rows, ntok, false);

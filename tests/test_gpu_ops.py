@@ -256,7 +256,8 @@ def test_norm_rope_of_many_vectors(ops, orc, synth, hd, heads, kv_heads, n, shif
         assert np.array_equal(got.view(np.uint8), full.view(np.uint8))
 
 
-@pytest.mark.parametrize("rows,k,ntok", [(128, 2048, 37), (8, 256, 1), (50, 100, 19), (33, 68, 16), (33, 772, 129), (128, 640, 593)])
+@pytest.mark.parametrize("rows,k,ntok", [(128, 2048, 37), (8, 256, 1), (50, 100, 19), (33, 68, 16), (33, 772, 129), (128, 640, 593),
+                                         (33, 260, 592), (33, 260, 593), (65, 324, 1180), (65, 324, 1601)])
 def test_matmul_f32_tokens(ops, orc, synth, rows, k, ntok):
     """The tile form of the f32 matvec: every output is the same -0.0-seeded left-to-right sum."""
     w = synth.normal_f32(rows * k, 5, "mm.w", rows, k, std=0.02).reshape(rows, k)
