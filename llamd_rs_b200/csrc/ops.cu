@@ -591,7 +591,7 @@ __global__ void norm_rope_kernel(float *__restrict__ xq, const float *__restrict
 // sums of squares side by side, a vector per lane, where a CTA per head kept one thread of 64 at work on a chain of its own
 // that nothing shortens. Bound by the traffic of q (read and written once) and one chain of hd adds. 36 heads of 128, us per
 // head / this: 512 tokens 22.9 / 13.4, 2000 tokens 78 / 36.
-constexpr int kRopeVecs = 32;
+constexpr int kRopeVecs = 32, kRopeRows = 4096;
 template <class KVT>
 __global__ void __launch_bounds__(256) norm_rope_rows_kernel(float *__restrict__ xq, const float *__restrict__ wq, float *__restrict__ xk,
                                                              const float *__restrict__ wk, const float *__restrict__ v_src, KVT *__restrict__ kc,
@@ -2080,15 +2080,16 @@ void llamd_fwd_k_norm_rope_store(float *k, const float *w, const float *v, float
     launch_k("k_norm_rope_store", norm_rope_kernel<float>, dim3(n_head_kv, nseq), dim3(hd / 2), hd * sizeof(float), nullptr, nullptr, k, w, v, kc,
              vc, 0, n_head_kv, hd, meta, 0, rope_tab, eps, max_kv);
 }
-// Query heads and key heads in one launch: QK-norm, RoPE, and the KV store. From 1024 vectors on (28 tokens of 36 heads: the
-// heads then no longer all fit the chip at once) 32 of them per CTA.
+// Query heads and key heads in one launch: QK-norm, RoPE, and the KV store. From kRopeRows vectors on, where the heads of a CTA
+// each come in waves, 32 of them per CTA. us, a CTA per head / this: vectors of 128, 1044 of them 4.2 / 7.2, 3096 6.2 / 7.2, 4104
+// 8.2 / 7.4, 8208 12.3 / 8.2; of 64, 4096 6.2 / 6.2, 4608 8.2 / 6.2; of 256, 6156 12.3 / 13.0, 8208 14.4 / 14.1.
 }
 template <class KVT>
 static void qk_norm_rope_launch(int cls, const char *what, float *q, const float *wq, float *k, const float *wk, const float *v, KVT *kc, KVT *vc, int n_head,
                                 int n_head_kv, int hd, const int32_t *meta, const float *rope_tab, float eps, int n, int kv_stride) {
     const int n_vec = n * (n_head + n_head_kv);
     // (that form reads the vectors 16 bytes at a time)
-    if (n_vec >= 1024 && hd % 4 == 0 && hd <= 256 && (((uintptr_t)q | (uintptr_t)k) & 15) == 0)
+    if (n_vec >= (hd <= 128 ? kRopeRows : 2 * kRopeRows) && hd % 4 == 0 && hd <= 256 && (((uintptr_t)q | (uintptr_t)k) & 15) == 0)
         launch_kc(cls, what, norm_rope_rows_kernel<KVT>, dim3((n_vec + kRopeVecs - 1) / kRopeVecs), dim3(256), kRopeVecs * (hd + 4) * sizeof(float), q, wq, k,
                   wk, v, kc, vc, n_head, n_head_kv, hd, meta, rope_tab, eps, kv_stride, n_vec);
     else

@@ -208,12 +208,12 @@ def test_router_matvec_logits_are_bit_exact(ops, orc, synth):
 
 
 @pytest.mark.parametrize("hd,heads,kv_heads,n,shift,kv16,own_caches,norms", [
-    (128, 7, 1, 129, 0, 0, False, "qk"),   # 1032 vectors: the last CTA holds 8
-    (64, 6, 2, 128, 0, 1, False, "qk"),    # 1024, binary16 cache
-    (256, 4, 2, 171, 0, 0, True, "q"),     # a cache per sequence, keys not normed
-    (20, 6, 2, 131, 0, 1, True, ""),       # no norm weights
-    (128, 7, 1, 129, 4, 0, False, "qk"),   # queries and keys off the 16-byte boundary
-    (128, 7, 1, 127, 0, 0, False, "k"),    # 1016: a CTA per head
+    (128, 7, 1, 513, 0, 0, False, "qk"),   # 4104 vectors: the last CTA holds 8
+    (64, 6, 2, 512, 0, 1, False, "qk"),    # 4096, binary16 cache
+    (256, 12, 4, 513, 0, 0, True, "q"),    # 8208, a cache per sequence, keys not normed
+    (20, 30, 10, 131, 0, 1, True, ""),     # 5240, no norm weights
+    (128, 7, 1, 513, 4, 0, False, "qk"),   # queries and keys off the 16-byte boundary
+    (128, 7, 1, 511, 0, 0, False, "k"),    # 4088: a CTA per head
 ])
 def test_norm_rope_of_many_vectors(ops, orc, synth, hd, heads, kv_heads, n, shift, kv16, own_caches, norms):
     """QK-norm, RoPE and the K/V store of a tile on both sides of the line where a CTA takes 32 vectors: queries, keys and cache
@@ -223,7 +223,7 @@ def test_norm_rope_of_many_vectors(ops, orc, synth, hd, heads, kv_heads, n, shif
 
     q, k, v = (synth.normal_f32(n * h * hd, 91, "many", what).reshape(n, h * hd) for what, h in (("q", heads), ("k", kv_heads), ("v", kv_heads)))
     w = {c: synth.normal_f32(hd, 91, "many.w", c) if c in norms else None for c in "qk"}
-    max_kv, first = 160, 3
+    max_kv, first = (160 if own_caches else 520), 3
     pos = np.array([(7 * i) % max_kv if own_caches else first + i for i in range(n)], np.int32)
     rows = np.arange(n) * max_kv + pos if own_caches else pos  # of a cache
     want = {}
