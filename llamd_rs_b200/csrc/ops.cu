@@ -311,11 +311,11 @@ __global__ void __launch_bounds__(128) matvec_q8_0_kernel(const uint8_t *__restr
 
 // The same result with the row's work spread over a CTA, fed by bulk copies. Above, one thread unpacks, converts, multiplies
 // and adds every element of its row alone and is bound by its own instruction latency (~20 cycles per element). Here a CTA
-// owns 32 rows: seven producer warps turn 8 blocks (256 columns) of the 32 rows into f32 weights d*q in shared memory while
-// one chain warp per sequence (lane = row) walks acc = acc + w*x over the previous 256 columns: only the add is on the
-// dependent chain (~4 cycles per element). The raw blocks come as one bulk copy per chunk (cp.async.bulk, 32 rows x 256
-// columns are one contiguous run of the tiled layout), n_raw chunks ahead, the first ones before anything else happens; the
-// producers convert from shared memory. With one sequence the producers
+// owns 32 rows: seven producer warps turn a chunk of 8 blocks (256 columns; 4 blocks where shared memory is short) of the 32
+// rows into f32 weights d*q in shared memory while one chain warp per sequence (lane = row) walks acc = acc + w*x over the
+// chunk before: only the add is on the dependent chain (~4 cycles per element). The raw blocks come as one bulk copy per
+// chunk (cp.async.bulk, 32 rows of a chunk are one contiguous run of the tiled layout), n_raw chunks ahead, the first ones
+// before anything else happens; the producers convert from shared memory. With one sequence the producers
 // store the products (d*q)*x, so the chain warp's loop is a shared load and the dependent add alone; with more, each has
 // a chain warp that multiplies ahead of its adds. Bound by those chains (2048 dependent adds are 4.3 us at 1.9 GHz).
 // 4096 x 2048, 1 / 2 / 4 / 8 sequences: 13.8 / 26.2 / 27.5 / 37.9 us with the activations staged a load at a time and the
@@ -337,35 +337,33 @@ __device__ __forceinline__ bool q80_mbar_wait(uint64_t *bar, uint32_t parity) {
     }
     return false;
 }
-constexpr int kQ80ChunkBlocks = 8;
 constexpr int kQ80Producers = 224;   // 7 warps
 constexpr int kQ80MaxRaw = 32;       // raw chunks in flight
-constexpr int kQ80RingBytes = 2 * kQ80ChunkBlocks * 32 * 32 * 4, kQ80RawBytes = kQ80ChunkBlocks * kQ80TileBytes;
-template <int NSEQ>
+template <int NSEQ, int CB>  // CB: blocks per chunk
 __global__ void __launch_bounds__(kQ80Producers + 32 * NSEQ) matvec_q8_0_bulk_kernel(const uint8_t *__restrict__ tiled, const float *__restrict__ x,
                                                                                      float *__restrict__ out, int blocks, int rows, int n_raw, int *status) {
     extern __shared__ __align__(16) float smem_f[];
     __shared__ __align__(8) uint64_t s_bar[kQ80MaxRaw];
     __shared__ int s_fail;
     constexpr bool kProd = NSEQ == 1;                         // the ring holds products w*x instead of weights
-    // ring: [2][64 column quads][32 rows][4]: a lane (= row) reads four consecutive columns with one 16-byte load, and the
+    // ring: [2][8 CB column quads][32 rows][4]: a lane (= row) reads four consecutive columns with one 16-byte load, and the
     // 32 lanes' loads are one conflict-free 512-byte run (a scalar load per column cost the chain warp 16 issue slots per
     // 16 adds and ran at ~7 cycles per add instead of ~4.4)
     float *s_w = smem_f;
-    float *sx = smem_f + 2 * kQ80ChunkBlocks * 32 * 32;       // [NSEQ][k]
+    float *sx = smem_f + 2 * CB * 32 * 32;       // [NSEQ][k]
     const int k = blocks * 32, tid = threadIdx.x;
-    uint8_t *s_raw = reinterpret_cast<uint8_t *>(sx + (size_t)NSEQ * k);  // [n_raw][8 blocks][1088]: the tiles as they lie in memory
+    uint8_t *s_raw = reinterpret_cast<uint8_t *>(sx + (size_t)NSEQ * k);  // [n_raw][CB blocks][1088]: the tiles as they lie in memory
     const bool producer = tid < kQ80Producers;
-    const int n_chunks = (blocks + kQ80ChunkBlocks - 1) / kQ80ChunkBlocks;
+    const int n_chunks = (blocks + CB - 1) / CB;
     const uint8_t *tile0 = tiled + (size_t)blockIdx.x * blocks * kQ80TileBytes;  // this CTA's 32 rows, block 0
     auto request = [&](int ch) {  // one thread
-        const uint32_t bytes = (uint32_t)min(kQ80ChunkBlocks, blocks - ch * kQ80ChunkBlocks) * kQ80TileBytes;  // (1088 = 68 x 16)
+        const uint32_t bytes = (uint32_t)min(CB, blocks - ch * CB) * kQ80TileBytes;  // (1088 = 68 x 16)
         const int slot = ch % n_raw;
         const uint32_t bar = q80_smem_u32(&s_bar[slot]);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                         q80_smem_u32(s_raw + (size_t)slot * kQ80RawBytes)),
-                     "l"(tile0 + (size_t)ch * kQ80RawBytes), "r"(bytes), "r"(bar)
+                         q80_smem_u32(s_raw + (size_t)slot * (CB * kQ80TileBytes))),
+                     "l"(tile0 + (size_t)ch * (CB * kQ80TileBytes)), "r"(bytes), "r"(bar)
                      : "memory");
     };
     if (tid == 0) {
@@ -396,21 +394,21 @@ __global__ void __launch_bounds__(kQ80Producers + 32 * NSEQ) matvec_q8_0_bulk_ke
         }
     }
     __syncthreads();  // (the barriers are initialised, the activations staged)
-    constexpr int kItems = kQ80ChunkBlocks * 64;                        // (block, half, row): 16 weights each
-    constexpr int kPer = (kItems + kQ80Producers - 1) / kQ80Producers;  // 3
+    constexpr int kItems = CB * 64;                        // (block, half, row): 16 weights each
+    constexpr int kPer = (kItems + kQ80Producers - 1) / kQ80Producers;  
     auto convert_chunk = [&](int ch) -> bool {
         if (!q80_mbar_wait(&s_bar[ch % n_raw], (uint32_t)(ch / n_raw) & 1)) return false;
-        float4 *dst = reinterpret_cast<float4 *>(s_w + (ch & 1) * (kQ80ChunkBlocks * 32 * 32));
+        float4 *dst = reinterpret_cast<float4 *>(s_w + (ch & 1) * (CB * 32 * 32));
 #pragma unroll
         for (int u = 0; u < kPer; u++) {
             const int item = tid + u * kQ80Producers;
             const int bl = item >> 6, h = (item >> 5) & 1, r = item & 31;
-            if (item < kItems && ch * kQ80ChunkBlocks + bl < blocks) {
-                const uint8_t *t = s_raw + (size_t)(ch % n_raw) * kQ80RawBytes + (size_t)bl * kQ80TileBytes;
+            if (item < kItems && ch * CB + bl < blocks) {
+                const uint8_t *t = s_raw + (size_t)(ch % n_raw) * (CB * kQ80TileBytes) + (size_t)bl * kQ80TileBytes;
                 const uint4 raw = *(reinterpret_cast<const uint4 *>(t + 512 * h) + r);
                 const float d = f16_bits_to_f32(*(reinterpret_cast<const uint16_t *>(t + 1024) + r));
                 const uint32_t ws[4] = {raw.x ^ 0x80808080u, raw.y ^ 0x80808080u, raw.z ^ 0x80808080u, raw.w ^ 0x80808080u};
-                const float4 *xs = reinterpret_cast<const float4 *>(sx + (ch * kQ80ChunkBlocks + bl) * 32 + h * 16);
+                const float4 *xs = reinterpret_cast<const float4 *>(sx + (ch * CB + bl) * 32 + h * 16);
 #pragma unroll
                 for (int g = 0; g < 4; g++) {
                     // q as f32 without the converter unit: the byte q + 128 dropped into the mantissa of 2^23 is 2^23 + 128 + q
@@ -440,8 +438,8 @@ __global__ void __launch_bounds__(kQ80Producers + 32 * NSEQ) matvec_q8_0_bulk_ke
             if (tid == 0 && !s_fail && ch + n_raw < n_chunks) request(requested = ch + n_raw);
             if (ch + 1 < n_chunks && !s_fail && !convert_chunk(ch + 1)) s_fail = 1;
         } else {
-            const float4 *w = reinterpret_cast<const float4 *>(s_w + (ch & 1) * (kQ80ChunkBlocks * 32 * 32)) + lane;
-            const int nq = min(kQ80ChunkBlocks, blocks - ch * kQ80ChunkBlocks) * 8;  // column quads: a multiple of 8
+            const float4 *w = reinterpret_cast<const float4 *>(s_w + (ch & 1) * (CB * 32 * 32)) + lane;
+            const int nq = min(CB, blocks - ch * CB) * 8;  // column quads: a multiple of 8
             if (kProd) {
                 // two register sets of 16 products alternate; a set is re-loaded right after it has been added
                 float4 a0 = w[0], a1 = w[32], a2 = w[64], a3 = w[96], b0 = w[128], b1 = w[160], b2 = w[192], b3 = w[224];
@@ -456,7 +454,7 @@ __global__ void __launch_bounds__(kQ80Producers + 32 * NSEQ) matvec_q8_0_bulk_ke
             } else {
                 // the products of 16 columns (packed: w and x of neighbouring columns are register pairs as they lie) and the
                 // loads of the 16 after them do not depend on the adds that they are scheduled among
-                const ulonglong2 *w2 = reinterpret_cast<const ulonglong2 *>(w), *xs = reinterpret_cast<const ulonglong2 *>(sx + (size_t)seq * k + ch * kQ80ChunkBlocks * 32);
+                const ulonglong2 *w2 = reinterpret_cast<const ulonglong2 *>(w), *xs = reinterpret_cast<const ulonglong2 *>(sx + (size_t)seq * k + ch * CB * 32);
                 ulonglong2 wv[4], xv[4], pr[4];
                 auto fetch = [&](int q0) {
 #pragma unroll
@@ -1968,9 +1966,10 @@ void llamd::norm_router_flags(const float *w, const float *x, const float *resid
 }
 extern "C" {
 
-// Measured, this form / thread per row: 20000 x 4096 (625 CTAs) 57 / 86 us for one sequence, 137 / 120 for four (one CTA
-// per SM beside their activations); 20000 x 1056 21 / 26 and 33 / 35.
-constexpr int kQ80MaxCtasOne = 148 * 8, kQ80MaxCtas = 148 * 4;
+// Measured with one sequence, this form / thread per row, weights from HBM and from L2: 20000 x 2048 (625 CTAs) 32.7 / 42.5 and
+// 30.8 / 26.7 us, 30000 x 2048 41.0 / 43.1 and 41.0 / 26.8, 20000 x 4096 57.3 / 84.2 and 55.3 / 51.4; with four, 20000 x 4096 137 /
+// 120.
+constexpr int kQ80MaxCtasOne = 148 * 5, kQ80MaxCtas = 148 * 4;
 static int *g_q80_status = nullptr;
 static int *q80_status_word() {  // mapped host memory: reading it after a synchronise costs no copy
     if (!g_q80_status) {
@@ -1989,6 +1988,21 @@ int llamd_fwd_matvec_q8_0_status(void) {
     if (cudaStreamSynchronize(stream()) != cudaSuccess) return -1;
     return *(volatile int *)g_q80_status;
 }
+}
+template <int N, int CB>
+static void q80_bulk_launch(int ctas, size_t smem, const uint8_t *t, const float *x, float *out, int blocks32, int rows, int n_raw) {
+    static size_t configured = 0;
+    if (smem > configured) {
+        if (cudaFuncSetAttribute(matvec_q8_0_bulk_kernel<N, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+            set_error_msg("matvec_q8_0: shared memory attribute");
+            return;
+        }
+        configured = smem;
+    }
+    launch_kc(PDL_OTHER, "matvec_q8_0_bulk", matvec_q8_0_bulk_kernel<N, CB>, dim3(ctas), dim3(kQ80Producers + 32 * N), smem, t, x, out, blocks32, rows, n_raw,
+              q80_status_word());
+}
+extern "C" {
 void llamd_fwd_matvec_q8_0(const void *w, const float *x, float *out, int blocks32, int rows, int nseq) {
     const size_t smem = (size_t)nseq * blocks32 * 32 * sizeof(float);
     if (nseq < 1 || nseq > LLAMD_MAX_SEQ || smem > 200 * 1024 || rows <= 0 || blocks32 <= 0) {
@@ -1996,14 +2010,21 @@ void llamd_fwd_matvec_q8_0(const void *w, const float *x, float *out, int blocks
         return;
     }
     const uint8_t *t = (const uint8_t *)w;
-    // The CTA-per-32-rows form: 64 KiB of converted weights and at least two raw chunks beside the activations. Its CTAs are
-    // bound by their chains, so where they do not all fit at one per SM the raw ring gives way to a second CTA per SM. It
-    // wins while they are a few waves; beyond that the thread-per-row form's deeper occupancy does (lm_head).
-    const int ctas = (rows + 31) / 32, chunks = (blocks32 + kQ80ChunkBlocks - 1) / kQ80ChunkBlocks;
-    auto raw_fit = [&](size_t budget) { return budget < smem + kQ80RingBytes ? 0 : (int)((budget - smem - kQ80RingBytes) / kQ80RawBytes); };
-    int n_raw = ctas > 148 ? raw_fit(111 * 1024) : 0;
-    if (n_raw < 2) n_raw = raw_fit(225 * 1024);
+    // The CTA-per-32-rows form: 64 KiB of converted weights (two chunks of 8 blocks) and at least two raw chunks beside the
+    // activations. Its CTAs are bound by their chains, so where they do not all fit at one per SM the raw ring gives way to a
+    // second CTA per SM, and where that is not enough the chunks are halved. It wins while they are a few waves; beyond that
+    // the thread-per-row form's deeper occupancy does (lm_head). us of 9472 x 4096 for 2 / 3 / 4 sequences, whole chunks at one
+    // CTA per SM / halved ones at two: 55.4 / 57.4 / 55.4, 39.2 / 41.2 / 47.3; of 9472 x 2048 for 4: 30.9, 26.8.
+    const int ctas = (rows + 31) / 32;
+    auto raw_fit = [&](size_t budget, int cb) {
+        const size_t used = smem + (size_t)2 * cb * 32 * 32 * 4;
+        return budget < used ? 0 : (int)((budget - used) / (cb * kQ80TileBytes));
+    };
+    int cb = 8, n_raw = ctas > 148 ? raw_fit(111 * 1024, 8) : 0;
+    if (ctas > 148 && n_raw < 2 && (n_raw = raw_fit(111 * 1024, 4)) >= 2) cb = 4;
+    if (n_raw < 2) n_raw = raw_fit(225 * 1024, 8);
     if (n_raw > kQ80MaxRaw) n_raw = kQ80MaxRaw;
+    const int chunks = (blocks32 + cb - 1) / cb;
     if (n_raw > chunks) n_raw = chunks;
     const bool usable = ((uintptr_t)w & 15) == 0 && ((uintptr_t)x & 15) == 0 && q80_status_word() != nullptr;
     const bool by_bulk = usable && ctas <= (nseq == 1 ? kQ80MaxCtasOne : kQ80MaxCtas) && n_raw >= (chunks < 2 ? 1 : 2);
@@ -2016,21 +2037,14 @@ void llamd_fwd_matvec_q8_0(const void *w, const float *x, float *out, int blocks
         llamd_fwd_matvec_q8_0(w, x + (size_t)n * blocks32 * 32, out + (size_t)n * rows, blocks32, rows, nseq - n);
         return;
     }
-    const size_t smem_bulk = smem + kQ80RingBytes + (size_t)n_raw * kQ80RawBytes;
-    const dim3 grid(by_bulk ? ctas : (rows + 127) / 128);
+    const size_t smem_bulk = smem + (size_t)2 * cb * 32 * 32 * 4 + (size_t)n_raw * cb * kQ80TileBytes;
+    const dim3 grid((rows + 127) / 128);
 #define Q80_CASE(N)                                                                                                   \
     case N: {                                                                                                          \
         static size_t configured = 0;                                                                                  \
         if (by_bulk) {                                                                                                 \
-            static size_t configured_bulk = 0;                                                                         \
-            if (smem_bulk > configured_bulk) {                                                                         \
-                if (cudaFuncSetAttribute(matvec_q8_0_bulk_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bulk) != cudaSuccess) { \
-                    set_error_msg("matvec_q8_0: shared memory attribute");                                             \
-                    return;                                                                                            \
-                }                                                                                                      \
-                configured_bulk = smem_bulk;                                                                           \
-            }                                                                                                          \
-            launch_kc(PDL_OTHER, "matvec_q8_0_bulk", matvec_q8_0_bulk_kernel<N>, grid, dim3(kQ80Producers + 32 * N), smem_bulk, t, x, out, blocks32, rows, n_raw, q80_status_word()); \
+            if (cb == 4) q80_bulk_launch<N, 4>(ctas, smem_bulk, t, x, out, blocks32, rows, n_raw);                      \
+            else q80_bulk_launch<N, 8>(ctas, smem_bulk, t, x, out, blocks32, rows, n_raw);                              \
             break;                                                                                                     \
         }                                                                                                              \
         if (smem > 48 * 1024 && smem > configured) {                                                                   \

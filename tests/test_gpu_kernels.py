@@ -210,6 +210,8 @@ def test_grouped_repeated_expert_and_bad_ids(be, orc, synth):
     (18976, 96, 2),               # past the line where the thread-per-row form takes over for several sequences
     (40, 4640, 8), (40, 5632, 7), (70, 25600, 2),  # activations that leave no room for the ring: two launches
     (4768, 4640, 8),              # ... but the thread-per-row form beyond one wave of CTAs
+    (4768, 4096, 2), (4768, 4128, 3), (4800, 2080, 4),  # two CTAs per SM with halved chunks, the last of them ragged
+    (23712, 64, 1),               # past the line where the thread-per-row form takes over for one sequence
 ])
 def test_q8_0_matvec_is_bit_exact(be, orc, synth, rows, k, nseq):
     w = synth.q8_0_blocks(rows * k // 32, 51, "q80mv", rows, k)
