@@ -75,7 +75,7 @@ class _ResultPool:
     quicker) or above MAX. A model has the blocks for its logits pinned when it is made (reserve), a product on its size's
     first results. release_idle() gives back what nobody
     holds; freeing the last model does."""
-    MIN, MAX, PER_SIZE = (128 << 10) + 1, 8 << 20, 4
+    MIN, MAX, PER_SIZE = (64 << 10) + 1, 8 << 20, 4
 
     def __init__(self):
         self.lock = threading.RLock()  # (re-entrant: a garbage collection inside may give a block back)

@@ -290,10 +290,10 @@ int llamd_cuda_quantize_q8k(const float *x, int nblocks, int8_t *qs, float *d, i
 // Host-facing products: x in, out back, one synchronise. Inputs of up to kStageBytes go through pinned memory of the
 // library's own; results of up to kDirectBytes are stored there by the kernel itself, larger ones are copied, straight into
 // `out` if that is pinned (llamd_cuda_host_alloc). Without pinned memory both go as pageable copies. us a call, repeated / with
-// new weights and activations, Q6_K rows of 2048: result through a pageable copy, a pinned copy of its own, stored by the kernel,
-// copied into a pinned array: 8 KB 34.7/60.3, 32.3/57.4, 30.1/53.5, 32.6/64.2; 32 KB 39.9/63.8, 36.9/66.7, 27.8/58.1, 36.7/67.4;
-// 128 KB 48.7/81.0, 45.5/77.6, 39.7/71.2, 41.1/78.5; 256 KB 75.8/119.8, 69.8/121.3, 69.4/122.8, 60.0/106.1.
-constexpr size_t kStageBytes = 1 << 20, kDirectBytes = 128 << 10;
+// new weights and activations, Q6_K rows of 2048, result stored by the kernel / copied into a pinned array of the pool: 48 KB
+// 30.2/49.4 and 35.7/62.8, 64 KB 33.1/51.4 and 35.6/59.7, 96 KB 40.7/57.8 and 36/66, 128 KB 45.2/65.4 and 39.0/64.4; pageable
+// copies 39.9/63.8 at 32 KB, 48.7/81.0 at 128.
+constexpr size_t kStageBytes = 1 << 20, kDirectBytes = 64 << 10;
 static int stage_x(const float *x, size_t bytes, float **d_x, bool read_once) {
     float *h = bytes <= kStageBytes ? (float *)host_stage(0, bytes) : nullptr;  // (free: every call that fills it waits for its own work)
     if (h) memcpy(h, x, bytes);
