@@ -257,8 +257,9 @@ class CudaModel:
 
     @property
     def prefill_tile(self) -> int:
-        """Tokens per prefill tile. Until it is set, the library cuts a prompt into equal tiles of up to 2048 tokens on one
-        GPU; the results do not depend on it."""
+        """Tokens per prefill tile, 512 until it is set: what several GPUs then use, and one GPU where memory is short. With
+        memory to spare one GPU cuts a prompt into equal tiles of up to 2048 tokens until it is set. The results do not depend
+        on it."""
         return getattr(self, "_prefill_tile", 512)
 
     @prefill_tile.setter
