@@ -318,6 +318,11 @@ static int finish_out(const float *d_out, float *out, size_t bytes, bool staged)
     return 0;
 }
 
+// From this many sequences on a host-facing product of up to 24 blocks a row runs on the integer tensor path, which folds a weight
+// once for all of them (the same bits). us in the kernel, matvec / GEMM: 151936 x 2048, 2 sequences 78 / 82, 3: 143 / 83, 8: 296 / 86;
+// 5120 x 2048, 3: 7.1 / 6.5, 8: 13.7 / 7.2; 2048 x 4096, 3: 5.9 / 6.8, 4: 6.8 / 7.4, 8: 12.1 / 6.9.
+constexpr int kGemmSeqs = 3;
+
 int llamd_cuda_matvec_q6k_f32(const void *d_w, const float *x, float *out, int blocks, int rows, int nseq) {
     if (!d_w || !x || !out || blocks <= 0 || rows <= 0 || nseq < 1 || nseq > LLAMD_MAX_SEQ) return -1;
     const size_t k = (size_t)blocks * 256, out_bytes = (size_t)nseq * rows * sizeof(float);
@@ -326,9 +331,12 @@ int llamd_cuda_matvec_q6k_f32(const void *d_w, const float *x, float *out, int b
     float *d_d = (float *)scratch(1, (size_t)nseq * blocks * sizeof(float));
     bool staged;
     float *d_out = out_buffer(out_bytes, &staged);
-    if (!d_q || !d_d || !d_out || stage_x(x, nseq * k * sizeof(float), &d_x, true)) return -1;
-    llamd_fwd_quantize(d_x, d_q, d_d, nseq * blocks);
-    llamd_fwd_matvec_batch(d_w, d_q, d_d, d_out, blocks, rows, nseq);
+    const bool gemm = nseq >= kGemmSeqs && blocks <= 24;
+    int8_t *d_rm = gemm ? (int8_t *)scratch(5, nseq * k) : nullptr;
+    if (!d_q || !d_d || !d_out || (gemm && !d_rm) || stage_x(x, nseq * k * sizeof(float), &d_x, true)) return -1;
+    quantize_rm(d_x, d_q, d_d, nseq * blocks, d_rm);
+    if (gemm) llamd_fwd_gemm_tokens(d_w, nullptr, nullptr, d_rm, d_d, d_out, nullptr, nullptr, blocks, rows, 0, 0, nseq);
+    else llamd_fwd_matvec_batch(d_w, d_q, d_d, d_out, blocks, rows, nseq);
     return finish_out(d_out, out, out_bytes, staged);
 }
 

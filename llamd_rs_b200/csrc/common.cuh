@@ -264,10 +264,10 @@ void matvec_grouped_pa_owned(const MatvecPlans &pl, const void *w, const int32_t
 void moe_group_owned(const int32_t *ids, int n_expert, int n_used, int nseq, int32_t *gstart, int32_t *gcount, int32_t *ptoken,
                      int32_t *pslot, int32_t *work, int32_t *n_work, int own_lo, int own_hi);
 // The grouped expert GEMM with its output rows scattered over several GPUs: row block o goes to out_tab[o / out_div],
-// local row block o % out_div (out_tab null: everything into oa / ob).
+// local row block o % out_div (out_tab null: everything into oa / ob). pairs: how many the plan holds about (0: unknown).
 void expert_gemm_scatter(const void *wa, const void *wb, const int32_t *gstart, const int32_t *gcount, const int32_t *act_map,
                          const int32_t *pslot, const void *aq_rm, const float *ad, float *oa, float *ob, int blocks, int rows, int n_expert,
-                         float *const *out_tab, int out_div, const void *fa = nullptr, const void *fb = nullptr);
+                         int pairs, float *const *out_tab = nullptr, int out_div = 1, const void *fa = nullptr, const void *fb = nullptr);
 // Pre-folded expert matrices (prefill): every (expert, 16-row tile) folded once into the integer MMA's operand order and
 // kept (2 bytes per weight); fa / fb above name such copies of wa / wb.
 size_t expert_fold_tile_bytes(int blocks);

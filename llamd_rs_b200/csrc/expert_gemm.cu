@@ -1,5 +1,6 @@
-// Q6_K x Q8_K for MANY tokens on the integer tensor path: the grouped expert
-// GEMM of prefill (and the QKV / attn_out projections of a prefill tile).
+// Q6_K x Q8_K for several tokens on the integer tensor path: the grouped expert
+// matmuls of prompts, drafts and batches, and the dense projections and the
+// output matrix of the same passes.
 //
 // The reference's arithmetic (crates/llamd-quant/src/dot.rs:138-196) keeps, per
 // (row, token, block b, residue r = element mod 8), the integer
@@ -8,461 +9,299 @@
 // That fixes the shape of the tensor-core formulation: each (b, r) is its own
 // 32-deep contraction whose result needs its own f32 scaling, so the MMA is
 //     D[16 rows x 8 tokens] = A[16 x 32] * B[32 x 8]     (mma.sync m16n8k32, s8 x s8 -> s32)
-// with A = scale[g]*w folded per row and B = the token's Q8_K bytes of that
-// residue. scale*w needs 13 bits, so A is split exactly into hi = U >> 6 and
-// lo = U & 63 (two MMAs, aux = 64*hi + lo). Integer results are exact in any
-// order; the f32 tail runs in the reference's order inside each thread (a
-// thread owns all eight residues of its four (row, token) outputs), so the
-// result is bit-identical to the scalar loop and to the dp4a matvec kernels.
+// with A = U = scale[g]*w folded per row and B = the token's Q8_K bytes of that
+// residue. U needs 13 bits, so 4U is split exactly into its high byte (signed)
+// and its low byte (unsigned): two MMAs, aux = 64*hi + lo/4. Integer results are
+// exact in any order; the f32 tail runs in the reference's order, so the result
+// is bit-identical to the scalar loop and to the dp4a matvec kernels.
 // This mirrors the role of crates/llamd-vulkan/shaders/q6k_expert_cm.comp
 // (cooperative-matrix s8 GEMM with f32 scaling per 16-K group).
 //
-// A CTA owns 16 weight rows of one matrix/expert at a time: it folds and splits
-// those rows once into shared memory in MMA fragment order, then each warp walks
-// token tiles of 8. Activations are read as residue-major words (one 32-bit word
-// = the four bytes of one MMA k-quad) prepared by q8k_residue_major_kernel.
-// Two launch shapes share the code:
-//   grouped  grid (row tiles, experts), 4 warps: one fold, then all of the expert's tokens;
-//   dense    a fixed number of resident CTAs (8 warps) split the (row tile, 64-token chunk)
-//            items evenly; a CTA folds a row tile once for the consecutive chunks it owns.
+// What it costs is instruction issue: the packed codes have to become operands (some 40 instructions per 512 weights and warp)
+// and every 128 sums need 2 MMAs (10 cycles each, which keep the FP32 pipe from issuing) and 8 packed FP32 instructions.
+// The operands are made in registers by the lane that multiplies with them -- the weight layout gives every lane its own words
+// (q6k_layout.cuh) -- and used for all the token tiles at hand. Three forms, by tokens per group:
+//   q6k_gemm_few_kernel     up to 16: a warp folds all residues of its blocks, one or two tiles;
+//   q6k_gemm_kernel         four warps, a residue pair each, share 16 rows and up to 8 tiles;
+//   q6k_gemm_shared_kernel  short rows and many tokens: rows folded into shared memory once for four warps.
+// us for 128 experts, gate and up (2 x 768 x 2048) / down (2048 x 768), 8 experts per token, before (every row tile folded into
+// shared memory, a warp per token tile) and now: 32 tokens 200 / 101, 114 / 58; 128: 243 / 119, 141 / 82; 512: 360 / 180, 257 / 164; 2048:
+// 910 / 465, 795 / 465.
 #include "packed_f32.cuh"
 #include "q6k_layout.cuh"
 
 namespace llamd {
 
 constexpr int kGemmRows = 16;
-constexpr int kTokStride = 68;  // words per staged token row: 16-byte aligned, conflict-free fragment reads
-constexpr int kChunkTiles = 8;  // token tiles per dense work item
-constexpr int kGroupTiles = 4;  // token tiles that the four warps of the folded kernel take together
-constexpr int kTeamWords = 4 * kGroupTiles * 8 * 16;  // their staged activations: 4 warps x 32 tokens x one residue pair's 16 words
 
 struct GemmParams {
     const uint8_t *w[3];  // tiled Q6_K; up to three matrices that share the activations
     float *out[3];
     int rows[3];
-    int tile_begin[3];    // first row tile (blockIdx.x) of each matrix
+    int tile_begin[3];    // first blockIdx.x of each matrix
     int njobs;
     int nb;               // blocks per row
-    const uint32_t *aq_rm;  // activations, residue-major words: [index][nb][8 residues][8 words]
+    int row_tiles;        // row tiles per CTA
+    int raw_bytes;        // shared memory for their blocks
+    const uint32_t *aq_rm;  // activations in operand order (t32_place): [index][nb][64 words]
     const float *ad;        // [index][nb]
     // token groups: group e = pairs [gstart[e], gstart[e]+gcount[e]); pair p reads activation act_map[p] and writes
-    // output row block out_map[p]. gstart == null: one group of n_tokens pairs. maps == null: identity.
+    // output row block out_map[p]. gstart == null: one group of n_tokens pairs, cut into runs of run_tiles token tiles
+    // (blockIdx.y). maps == null: identity.
     const int32_t *gstart, *gcount, *act_map, *out_map;
-    int n_tokens;
+    int n_tokens, run_tiles;
     long long expert_units;  // blocks between consecutive experts in w
-    int prefetch_ahead;      // grouped kernel: CTA i asks L2 for the weights of CTA i + prefetch_ahead (0: off)
+    int prefetch_ahead;      // grouped: CTA i asks L2 for the weights of CTA i + prefetch_ahead (0: off)
     // expert parallelism: output row block o lives on GPU o / out_div, at local row block o % out_div (null: out[j])
     float *const *out_tab;
     int out_div;
-    // pre-folded copies of the matrices (grouped kernel; null: fold from w): [expert][row tile] images of fold_tile_bytes,
-    // each exactly what fold_row_tile leaves in shared memory (A fragments, then the 16 x nb block scales)
+    // copies of the matrices kept folded (null: fold from w): [expert][row tile] images of fold_tile_bytes, see fold_image
     const uint8_t *folded[3];
     long long fold_tile_bytes;
     f32x2 one;  // kOne2
 };
 
-// Ask L2 for the tiles that hold the 16 x nb blocks starting at block `unit0` (a hint: nothing waits on it).
-__device__ __forceinline__ void prefetch_row_tile(const uint8_t *w, size_t unit0, int live_rows, int nb) {
-    const size_t t_lo = unit0 >> 5, t_hi = (unit0 + (size_t)min(live_rows, kGemmRows) * nb - 1) >> 5;
-    const uint8_t *src = w + t_lo * kTileBytes;
-    const uint32_t bytes = (uint32_t)((t_hi - t_lo + 1) * kTileBytes);  // 6720 = 16 * 420
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+struct Quad { uint32_t v[4]; };
+__device__ __forceinline__ void opaque(Quad &q, uint32_t c) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) asm volatile("mov.u32 %0, %1;" : "=r"(q.v[i]) : "r"(c));
+}
+template <bool UNSIGNED>
+__device__ __forceinline__ void mma_8(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, const Quad &q) {
+    if (UNSIGNED)
+        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+                     : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+                     : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(q.v[0]), "r"(q.v[1]), "r"(q.v[2]), "r"(q.v[3]));
+    else
+        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+                     : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+                     : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(q.v[0]), "r"(q.v[1]), "r"(q.v[2]), "r"(q.v[3]));
 }
 
-template <int C = 0>  // what the sums land on
-__device__ __forceinline__ void mma_s8(int (&c)[4], const uint4 &a, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-                 : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
-                 : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1), "r"(C));
+__device__ __forceinline__ void copy_async16(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+// ... through L1: the CTAs of an SM read the same activations, and in L2 a few tokens' lines are too few for all SMs
+__device__ __forceinline__ void copy_async16_l1(uint32_t dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Natural-order Q8_K quants -> residue-major words (t32_element order), one thread per word.
+__device__ __forceinline__ f32x2 add2x(f32x2 a, f32x2 b) {  // a + b where no product is an operand, see packed_f32.cuh
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// Natural-order Q8_K quants -> operand order, one thread per word.
 __global__ void q8k_residue_major_kernel(const int8_t *__restrict__ aq, uint32_t *__restrict__ rm, size_t nblocks) {
     pdl_trigger();
     pdl_wait();
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (i >= nblocks * 64) return;
     const size_t blk = i >> 6;
-    const int r = (int)(i >> 3) & 7, j = (int)i & 7;
+    const int r = t32_place_r((int)i & 63), j = t32_place_j((int)i & 63);
     const uint8_t *src = reinterpret_cast<const uint8_t *>(aq) + blk * 256;
     rm[i] = (uint32_t)src[t32_element(r, j, 0)] | ((uint32_t)src[t32_element(r, j, 1)] << 8) | ((uint32_t)src[t32_element(r, j, 2)] << 16) |
             ((uint32_t)src[t32_element(r, j, 3)] << 24);
 }
 
-// ---- fold the scales into the weights, split hi/lo, store in fragment order ----
-// One thread per (row, block, half): residues 4h..4h+3 of the block are 6 of its 12 code chunks, fetched with
-// coalesced 16-byte loads (consecutive threads = consecutive blocks of the tile), all issued before any is used.
-//
-// Two weights of one scale group are folded by ONE 32-bit multiply-add: with q = w + 32 in [0, 63],
-//     (q0 | q1 << 16) * sc + (C | C << 16),  C = 16384 - 32*sc
-// is, as an integer, sum_i (sc*(q_i - 32) + 16384) << 16i, and every term lies in [12288, 20480], so the two 16-bit
-// fields hold V_i = U_i + 16384 with no carry between them. 16384 is a multiple of 64*256: V & 63 = U & 63 and the
-// low byte of V >> 6 is the two's-complement byte of U >> 6.
-struct FoldItem {
-    uint32_t S[24];  // six 16-byte code chunks: residues 4h..4h+3 of one block
-    uint4 scw;       // its 16 scales
-    float d;
-    int rb, half;    // row_local * nb + block, which half; rb < 0: nothing to do
-};
-
-__device__ __forceinline__ void fold_load(FoldItem &f, const uint8_t *__restrict__ w, size_t unit0, int live_rows, int nb, int it) {
-    const int n_units = kGemmRows * nb;
-    f.rb = -1;
-    if (it >= 2 * n_units) return;
-    f.half = it >= n_units ? 1 : 0;
-    f.rb = it - f.half * n_units;
-    f.scw = make_uint4(0, 0, 0, 0);
-    f.d = 0.0f;
-    if (f.rb / nb < live_rows) {
-        const size_t unit = unit0 + f.rb;
-        const uint8_t *tile = w + (unit >> 5) * kTileBytes;
-        const int sl = (int)(unit & 31);
-        const uint4 *cp = reinterpret_cast<const uint4 *>(tile) + sl + f.half * 6 * 32;
-#pragma unroll
-        for (int c = 0; c < 6; c++) {
-            const uint4 v = __ldg(cp + c * 32);
-            f.S[4 * c + 0] = v.x; f.S[4 * c + 1] = v.y; f.S[4 * c + 2] = v.z; f.S[4 * c + 3] = v.w;
-        }
-        f.scw = __ldg(reinterpret_cast<const uint4 *>(tile + kTileScaleOff) + sl);
-        f.d = f16_bits_to_f32(__ldg(reinterpret_cast<const uint16_t *>(tile + kTileDOff) + sl));
-    } else {
-        // a row past the matrix: with zero scales the fold below yields hi = lo = 0 whatever the codes
-#pragma unroll
-        for (int c = 0; c < 24; c++) f.S[c] = 0;
-    }
-}
-
-__device__ __forceinline__ void fold_store(const FoldItem &f, int nb, uint4 *s_frag, float *s_d) {
-    if (f.rb < 0) return;
-    const int row_l = f.rb / nb, b = f.rb - row_l * nb;
-    if (f.half == 0) s_d[f.rb] = f.d;
-    uint32_t sc[16], crep[16];
-    {
-        const uint32_t ws[4] = {f.scw.x, f.scw.y, f.scw.z, f.scw.w};
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const int v = (int)(int8_t)(ws[i >> 2] >> (8 * (i & 3)));
-            sc[i] = (uint32_t)v;
-            crep[i] = (uint32_t)(16384 - 32 * v) * 0x00010001u;
-        }
-    }
-#pragma unroll
-    for (int rl = 0; rl < 4; rl++) {
-        const int r = 4 * f.half + rl;
-#pragma unroll
-        for (int m = 0; m < 2; m++) {
-            const uint32_t s0 = f.S[6 * rl + 3 * m], s1 = f.S[6 * rl + 3 * m + 1], s2 = f.S[6 * rl + 3 * m + 2];
-            // the stored byte is (q ^ 0x20) << 2; the fourth word's codes are the low bit pairs of the other three
-            uint32_t qb[4];
-            qb[0] = ((s0 >> 2) & 0x3F3F3F3Fu) ^ 0x20202020u;
-            qb[1] = ((s1 >> 2) & 0x3F3F3F3Fu) ^ 0x20202020u;
-            qb[2] = ((s2 >> 2) & 0x3F3F3F3Fu) ^ 0x20202020u;
-            qb[3] = (((s0 << 4) & 0x30303030u) | ((s1 << 2) & 0x0C0C0C0Cu) | (s2 & 0x03030303u)) ^ 0x20202020u;
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int jw = 4 * m + i;  // bytes 0,1 of word jw belong to scale group 2jw, bytes 2,3 to 2jw+1
-                const uint32_t v01 = __byte_perm(qb[i], 0u, 0x4140) * sc[2 * jw] + crep[2 * jw];
-                const uint32_t v23 = __byte_perm(qb[i], 0u, 0x4342) * sc[2 * jw + 1] + crep[2 * jw + 1];
-                const uint32_t lo = __byte_perm(v01, v23, 0x6420) & 0x3F3F3F3Fu;
-                const uint32_t hi = __byte_perm(v01 >> 6, v23 >> 6, 0x6420);
-                // fragment word q of lane L: row = L/4 + 8(q&1), word jw = L%4 + 4(q>>1).
-                // Lane L's 16 bytes sit in slot L ^ (L >> 3) ^ (b & 7): the threads of a warp here write the same jw
-                // of neighbouring rows and blocks, and the swizzle spreads them over all eight 16-byte bank groups
-                // (the readers of one fragment still touch 32 distinct slots).
-                const int L = (row_l & 7) * 4 + (jw & 3), q = (row_l >> 3) + 2 * (jw >> 2);
-                const int P = L ^ (L >> 3) ^ (b & 7);
-                reinterpret_cast<uint32_t *>(s_frag + ((size_t)(b * 8 + r) * 2 + 0) * 32 + P)[q] = hi;
-                reinterpret_cast<uint32_t *>(s_frag + ((size_t)(b * 8 + r) * 2 + 1) * 32 + P)[q] = lo;
-            }
-        }
-    }
-}
-
-// HOIST: two items per thread and trip, the loads of both in flight before either is folded (more registers).
-template <int THREADS, bool HOIST>
-__device__ __forceinline__ void fold_row_tile(const uint8_t *__restrict__ w, size_t unit0, int live_rows, int nb, uint4 *s_frag, float *s_d,
-                                              int tid) {
-    const int n_items = 2 * kGemmRows * nb;
-    if (HOIST) {
-        for (int base = 0; base < n_items; base += 2 * THREADS) {
-            FoldItem fa, fb;
-            fold_load(fa, w, unit0, live_rows, nb, base + tid);
-            fold_load(fb, w, unit0, live_rows, nb, base + THREADS + tid);
-            fold_store(fa, nb, s_frag, s_d);
-            fold_store(fb, nb, s_frag, s_d);
-        }
-    } else {
-        for (int base = 0; base < n_items; base += THREADS) {
-            FoldItem fa;
-            fold_load(fa, w, unit0, live_rows, nb, base + tid);
-            fold_store(fa, nb, s_frag, s_d);
-        }
-    }
-}
-
-// ---- token tiles of 8 against the folded row tile ----
-// Warp `warp` of `nwarps` takes tiles tile_lo + warp, + nwarps, ... below tile_hi. Per block b the warp copies its
-// 8 tokens' 256 activation bytes into its own buffer with coalesced 16-byte loads; the next block's bytes wait in
-// registers meanwhile.
-template <int DEPTH>
-__device__ __forceinline__ void mma_token_tiles(const GemmParams &p, int j, int row0, int rows, int first, int count, int tile_lo, int tile_hi,
-                                                const uint4 *s_frag, const float *s_d, uint32_t *s_b, int warp, int nwarps, int lane) {
-    const int nb = p.nb;
-    const int g4 = lane >> 2, q4 = lane & 3;
-    const int m0 = g4, m1 = g4 + 8;
-    for (int tn = tile_lo + warp; tn < tile_hi; tn += nwarps) {
-        const int n0 = tn * 8;
-        // the two tokens whose outputs this lane owns
-        const int pa0 = first + min(n0 + 2 * q4, count - 1), pa1 = first + min(n0 + 2 * q4 + 1, count - 1);
-        const long long ia0 = p.act_map ? p.act_map[pa0] : pa0, ia1 = p.act_map ? p.act_map[pa1] : pa1;
-        // staging: 8 tokens x 16 pieces of 16 bytes = 128 pieces, four per lane
-        const uint4 *src[4];
-        int dsto[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int chunk = lane + 32 * i;
-            const int tok = chunk >> 4, c16 = chunk & 15;
-            const int pt = first + min(n0 + tok, count - 1);
-            const long long it = p.act_map ? p.act_map[pt] : pt;
-            src[i] = reinterpret_cast<const uint4 *>(p.aq_rm + (size_t)it * nb * 64) + c16;
-            dsto[i] = tok * kTokStride + c16 * 4;
-        }
-        float sums[4][8];
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int r = 0; r < 8; r++) sums[i][r] = 0.0f;
-        // The tokens' activation bytes of the next DEPTH blocks wait in registers. (DEPTH 3-4 was measured: no faster than
-        // 1 -- the warps wait on the tile's own copy, on shared-memory and MMA latency and on fixed-latency dependencies
-        // in equal parts, at 12 warps per SM -- so the kernels use 1 and keep their registers.)
-        uint4 st[DEPTH][4];
-        float an[DEPTH][2];
-#pragma unroll
-        for (int s = 0; s < DEPTH; s++) {
-            if (s < nb) {
-#pragma unroll
-                for (int i = 0; i < 4; i++) st[s][i] = __ldg(src[i] + (size_t)s * 16);
-                an[s][0] = __ldg(p.ad + ia0 * nb + s);
-                an[s][1] = __ldg(p.ad + ia1 * nb + s);
-            }
-        }
-        for (int b0 = 0; b0 < nb; b0 += DEPTH) {
-#pragma unroll
-            for (int s = 0; s < DEPTH; s++) {
-                const int b = b0 + s;
-                if (b >= nb) break;
-#pragma unroll
-                for (int i = 0; i < 4; i++) *reinterpret_cast<uint4 *>(s_b + dsto[i]) = st[s][i];
-                __syncwarp();
-                const float a0 = an[s][0], a1 = an[s][1];
-                if (b + DEPTH < nb) {
-#pragma unroll
-                    for (int i = 0; i < 4; i++) st[s][i] = __ldg(src[i] + (size_t)(b + DEPTH) * 16);
-                    an[s][0] = __ldg(p.ad + ia0 * nb + b + DEPTH);
-                    an[s][1] = __ldg(p.ad + ia1 * nb + b + DEPTH);
-                }
-                const float d0 = s_d[m0 * nb + b], d1 = s_d[m1 * nb + b];
-                const float dsc[4] = {__fmul_rn(d0, a0), __fmul_rn(d0, a1), __fmul_rn(d1, a0), __fmul_rn(d1, a1)};
-                const uint4 *fr = s_frag + (size_t)b * 8 * 2 * 32 + (lane ^ (lane >> 3) ^ (b & 7));
-                const uint32_t *bt = s_b + g4 * kTokStride + q4;
-#pragma unroll
-                for (int r = 0; r < 8; r++) {
-                    const uint4 ah = fr[(r * 2 + 0) * 32], al = fr[(r * 2 + 1) * 32];
-                    const uint32_t b0w = bt[r * 8], b1w = bt[r * 8 + 4];
-                    int ch[4], cl[4];
-                    mma_s8(ch, ah, b0w, b1w);
-                    mma_s8(cl, al, b0w, b1w);
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        // aux = 64*hi + lo as a float, exactly (|aux| < 2^24). Two routes share the work between pipes:
-                        // the int->float converter (a quarter-rate unit), and an arithmetic route for the fourth output:
-                        // |hi|, |lo| < 2^22, so adding them to 1.5*2^23 as integers and subtracting the constant as floats
-                        // converts each exactly, and 64*fh + fl is exact because the sum is representable.
-                        float aux;
-                        if (i < 3) {
-                            aux = (float)(ch[i] * 64 + cl[i]);
-                        } else {
-                            const float fh = __fsub_rn(__int_as_float(0x4B400000 + ch[i]), 12582912.0f);
-                            const float fl = __fsub_rn(__int_as_float(0x4B400000 + cl[i]), 12582912.0f);
-                            aux = __fmaf_rn(fh, 64.0f, fl);
-                        }
-                        sums[i][r] = __fadd_rn(sums[i][r], __fmul_rn(dsc[i], aux));
-                    }
-                }
-                __syncwarp();
-            }
-        }
-        // y = ((((((s0+s1)+s2)+s3)+s4)+s5)+s6)+s7, then scatter
-        float tot[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            float t = sums[i][0];
-#pragma unroll
-            for (int r = 1; r < 8; r++) t = __fadd_rn(t, sums[i][r]);
-            tot[i] = t;
-        }
-        const bool v0 = n0 + 2 * q4 < count, v1 = n0 + 2 * q4 + 1 < count;
-        long long o0 = p.out_map ? p.out_map[pa0] : pa0, o1 = p.out_map ? p.out_map[pa1] : pa1;
-        float *out0 = p.out[j], *out1 = p.out[j];
-        if (p.out_tab) {  // the rows of a pair go to the GPU the pair's token lives on (plain peer stores)
-            if (v0) out0 = p.out_tab[o0 / p.out_div];
-            if (v1) out1 = p.out_tab[o1 / p.out_div];
-            o0 %= p.out_div;
-            o1 %= p.out_div;
-        }
-        if (row0 + m0 < rows) {
-            if (v0) out0[o0 * rows + row0 + m0] = tot[0];
-            if (v1) out1[o1 * rows + row0 + m0] = tot[1];
-        }
-        if (row0 + m1 < rows) {
-            if (v0) out0[o0 * rows + row0 + m1] = tot[2];
-            if (v1) out1[o1 * rows + row0 + m1] = tot[3];
-        }
-    }
-}
-
-// Shared memory: [nb][8 residues][hi, lo][32 lanes] x 16 B of A fragments, [16 rows][nb] f32 of d, one staging
-// buffer of 8 x kTokStride words per warp.
-__host__ __device__ inline size_t gemm_smem_bytes(int nb, int threads) {
-    return (size_t)nb * 8 * 2 * 32 * 16 + (size_t)kGemmRows * nb * 4 + (size_t)(threads / 32) * 8 * kTokStride * 4;
-}
-
-__device__ __forceinline__ int job_of_tile(const GemmParams &p, int rt) {
+__device__ __forceinline__ int job_of_tile(const GemmParams &p, int x) {
     int j = 0;
-    if (p.njobs > 1 && rt >= p.tile_begin[1]) j = 1;
-    if (p.njobs > 2 && rt >= p.tile_begin[2]) j = 2;
+    if (p.njobs > 1 && x >= p.tile_begin[1]) j = 1;
+    if (p.njobs > 2 && x >= p.tile_begin[2]) j = 2;
     return j;
 }
 
-// grid (row tiles of all jobs, groups). HOIST (long rows): three CTAs per SM fit anyway, spend registers on loads
-// in flight; short rows: keep registers low so that five CTAs fit.
-template <bool HOIST>
-__global__ void __launch_bounds__(128, HOIST ? 3 : 5) q6k_gemm_grouped_kernel(const GemmParams p) {
-    extern __shared__ __align__(16) uint8_t smem[];
-    const int nb = p.nb;
-    uint4 *s_frag = reinterpret_cast<uint4 *>(smem);
-    float *s_d = reinterpret_cast<float *>(smem + (size_t)nb * 8 * 2 * 32 * 16);
-    pdl_trigger();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0 && p.prefetch_ahead > 0) {
-        // the weights of the CTA that will take this one's place on the SM start their trip from HBM now
-        const long long lin = (long long)blockIdx.y * gridDim.x + blockIdx.x + p.prefetch_ahead;
-        if (lin < (long long)gridDim.x * gridDim.y) {
-            const int px = (int)(lin % gridDim.x), pe = (int)(lin / gridDim.x);
-            const int pj = job_of_tile(p, px);
-            const int prow0 = (px - p.tile_begin[pj]) * kGemmRows;
-            if (p.folded[pj]) {
-                const int tiles_j = (p.rows[pj] + kGemmRows - 1) / kGemmRows;
-                const uint8_t *src = p.folded[pj] + ((size_t)pe * tiles_j + (size_t)(px - p.tile_begin[pj])) * (size_t)p.fold_tile_bytes;
-                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"((uint32_t)p.fold_tile_bytes) : "memory");
-            } else
-            prefetch_row_tile(p.w[pj], (size_t)pe * (size_t)(p.gstart ? p.expert_units : 0) + (size_t)prow0 * nb, p.rows[pj] - prow0, nb);
-        }
+// ---- the A operand: scale times weight, split into bytes ----
+// Two weights of one scale group are folded by ONE 32-bit multiply-add: with q = w + 32 in [0, 63],
+//     (4*q0 | 4*q2 << 16) * sc + (C | C << 16),  C = 32768 - 128*sc
+// is, as an integer, sum_i (4*U_i + 32768) << 16i, and every term lies in [16384, 49152], so the two 16-bit fields hold
+// 4*U_i + 32768 with no carry between them: the low byte is 4*(U & 63), the high byte (U >> 6) + 128.
+struct Fold {
+    uint32_t mask, sc[4], c[4];  // 0x00FC00FC; a lane's four scales of one row: groups 2q, 2q+1, 2q+8, 2q+9
+};
+__device__ __forceinline__ void fold_scales(Fold &f, uint32_t packed) {
+    asm("mov.u32 %0, 0x00FC00FC;" : "=r"(f.mask));  // (in a register: a LOP3 takes one immediate)
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        f.sc[i] = (uint32_t)(int)(int8_t)(packed >> (8 * i));
+        f.c[i] = f.sc[i] * (uint32_t)(-128 * 0x00010001) + 0x80008000u;
     }
-    pdl_wait();
-    const int j = job_of_tile(p, blockIdx.x);
-    const int rows = p.rows[j];
-    const int row0 = ((int)blockIdx.x - p.tile_begin[j]) * kGemmRows;
-    const int e = blockIdx.y;
-    const int first = p.gstart ? p.gstart[e] : 0;
-    const int count = p.gstart ? p.gcount[e] : p.n_tokens;
-    if (count <= 0) return;
-    const size_t unit0 = (size_t)e * (size_t)(p.gstart ? p.expert_units : 0) + (size_t)row0 * nb;
-    if (p.folded[j]) {
-        // the tile was folded when the model was loaded: its image comes straight into place, 16 bytes per request, and
-        // the CTA's time goes to the MMAs instead of to turning Q6_K blocks into operands again
-        const int tiles_j = (rows + kGemmRows - 1) / kGemmRows;
-        const uint8_t *src = p.folded[j] + ((size_t)e * tiles_j + (size_t)(row0 / kGemmRows)) * (size_t)p.fold_tile_bytes;
-        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem);
-        const int n16 = (int)(p.fold_tile_bytes >> 4);
-        for (int i = tid; i < n16; i += 128)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (uint32_t)i), "l"(src + 16 * (size_t)i) : "memory");
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-    } else {
-        fold_row_tile<128, HOIST>(p.w[j], unit0, rows - row0, nb, s_frag, s_d, tid);
+}
+__device__ __forceinline__ uint32_t and_xor(uint32_t a, uint32_t m, uint32_t x) {  // (a & m) ^ x; written out it becomes two instructions
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0x78;" : "=r"(r) : "r"(x), "r"(a), "r"(m));
+    return r;
+}
+// A lane's words of one row and residue pair: s = the quad's three stored words. Operand registers `reg` and reg + 2 of both
+// residues (words j = q and q + 4). Bytes 0 and 2 of a word share a scale, as do bytes 1 and 3.
+__device__ __forceinline__ void fold_quad(const uint32_t (&s)[3], const Fold &f, int reg, uint32_t (&hi)[2][4], uint32_t (&lo)[2][4]) {
+    // the fourth word's codes are the low bit pairs of the other three (what else is in it the mask takes away)
+    const uint32_t w01 = ((s[0] << 6) & 0xC0C0C0C0u) | ((s[1] << 4) & ~0xC0C0C0C0u);
+    const uint32_t w3 = (w01 & 0xF0F0F0F0u) | ((s[2] << 2) & ~0xF0F0F0F0u);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint32_t w = i < 3 ? s[i < 3 ? i : 0] : w3;
+        const int half = i & 1;
+        const uint32_t ve = and_xor(w, f.mask, 0x00800080u) * f.sc[2 * half] + f.c[2 * half];
+        const uint32_t vo = and_xor(w >> 8, f.mask, 0x00800080u) * f.sc[2 * half + 1] + f.c[2 * half + 1];
+        hi[i >> 1][reg + 2 * half] = __byte_perm(ve, vo, 0x7351) ^ 0x80808080u;
+        lo[i >> 1][reg + 2 * half] = __byte_perm(ve, vo, 0x6240);
     }
-    __syncthreads();
-    uint32_t *s_b = reinterpret_cast<uint32_t *>(s_d + kGemmRows * nb) + (size_t)warp * 8 * kTokStride;
-    mma_token_tiles<1>(p, j, row0, rows, first, count, 0, (count + 7) >> 3, s_frag, s_d, s_b, warp, 4, lane);
 }
 
-// ---- few tokens against one matrix kept folded (the dense matrices and the head of a batch): four warps, a residue pair each
-// mma_token_tiles gives a warp whole token tiles, so 8 tokens keep one warp of a CTA at work, and every warp reads every
-// fragment (1 KB of shared memory a residue). Here the four warps of a CTA take up to 32 tokens together: each reads only
-// its own residues' fragments, once for all of them. The tail is packed, two tokens per instruction: the MMAs accumulate onto
-// 1.5 * 2^23, so that hi and lo come out as floats with that offset, and 64*hi + lo is exact because |aux| < 2^24. The image's
-// copy starts before the dependency wait. Bound by the image (2 bytes per weight); us, a warp per tile / this: QKV of 8
-// sequences 10.3 / 5.7, output projection 14.3 / 6.7, head 142 / 127; 32 sequences 13.5 / 10.7, 14.8 / 9.4, 196 / 180. For many tokens the
-// kernels above are quicker (2048: 906 us against 1024, gate and up), which spend less on staging and exchanging.
-// Warp rp owns residues 2rp and 2rp + 1. Per block it copies its 16 words of every token into its own part of
-// s_b (coalesced 16-byte loads; the next block's wait in registers meanwhile), 16-byte pieces swizzled by the token so that
-// the MMA's fragment reads meet 32 banks. At the end the eight residues' sums meet in s_b and are added in order.
-template <int NT>
-__device__ __forceinline__ void folded_tiles(const GemmParams &p, int j, int row0, int n0, const uint4 *s_frag, const float *s_d, uint32_t *s_b,
-                                             float *s_ad, int tid) {
-    const int nb = p.nb, rp = tid >> 5, lane = tid & 31, rows = p.rows[j], count = p.n_tokens;
-    const int g4 = lane >> 2, q4 = lane & 3;
-    auto token = [&](int tok) { return min(n0 + tok, count - 1); };
-    for (int i = tid; i < NT * 8 * nb; i += 128) {  // the group's activation scales, [block][token]
-        const int tok = i / nb, b = i - tok * nb;
-        s_ad[b * (8 * kGroupTiles) + tok] = __ldg(p.ad + (long long)token(tok) * nb + b);
-    }
-    const uint4 *src[NT];
-    uint4 st[NT];
+// The weights of the CTA that will take this one's place on the SM start their trip from HBM now.
+template <bool FOLDED = false>
+__device__ __forceinline__ void prefetch_ahead(const GemmParams &p, int ahead) {
+    if (threadIdx.x || ahead <= 0) return;
+    const long long lin = (long long)blockIdx.y * gridDim.x + blockIdx.x + ahead;
+    const int px = (int)(lin % gridDim.x), pe = (int)(lin / gridDim.x), pj = job_of_tile(p, px);
+    if (pe >= (int)gridDim.y || p.gcount[pe] <= 0) return;
+    const int pt = (px - p.tile_begin[pj]) * p.row_tiles;
+    const size_t u0 = (size_t)pe * (size_t)p.expert_units + (size_t)pt * kGemmRows * p.nb;
+    const size_t a = u0 >> 5, z = (u0 + (size_t)min(p.row_tiles * kGemmRows, p.rows[pj] - pt * kGemmRows) * p.nb - 1) >> 5;
+    const uint8_t *src = FOLDED ? p.folded[pj] + ((size_t)pe * ((p.rows[pj] + kGemmRows - 1) / kGemmRows) + pt) * (size_t)p.fold_tile_bytes
+                                : p.w[pj] + a * kTileBytes;
+    const uint32_t bytes = FOLDED ? (uint32_t)p.fold_tile_bytes : (uint32_t)((z - a + 1) * kTileBytes);
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
+struct RowTile {
+    int j, row0, live;   // matrix, first row, rows that exist (<= 16)
+    uint32_t raw;        // shared-memory address of the tile that holds block `unit0` and the ones behind it, or of the image
+    int unit0;           // block of (row0, 0), counted from that tile's first
+};
+
+// The operands of one block of a row tile, made by the lane that multiplies with them. u: block of the lane's row g4 + 8h,
+// counted from the tile at `raw`.
+__device__ __forceinline__ void fold_block(uint32_t raw, int u, int rp, int q4, const uint32_t (&word_off)[3], int h, uint32_t (&hi)[2][4],
+                                           uint32_t (&lo)[2][4], float &d) {
+    const uint32_t tile = raw + (uint32_t)(u >> 5) * kTileBytes, sl = (uint32_t)(u & 31), at = tile + 16u * (uint32_t)t32_slot((int)sl);
+    uint32_t s[3], sc;
+    uint16_t db;
 #pragma unroll
-    for (int t = 0; t < NT; t++) {
-        src[t] = reinterpret_cast<const uint4 *>(p.aq_rm + (size_t)token(t * 8 + g4) * nb * 64) + rp * 4 + q4;
-        st[t] = __ldg(src[t]);
+    for (int i = 0; i < 3; i++) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(s[i]) : "r"(at + word_off[i]));
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sc) : "r"(at + kTileScaleOff + 4u * (uint32_t)q4));
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(db) : "r"(tile + kTileDOff + 2u * sl));
+    Fold f;
+    fold_scales(f, sc);
+    fold_quad(s, f, h, hi, lo);
+    d = f16_bits_to_f32(db);
+}
+__device__ __forceinline__ void fold_offsets(int rp, int q4, uint32_t (&word_off)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) word_off[i] = (uint32_t)((3 * rp + ((3 * q4 + i) >> 2)) * 512 + ((3 * q4 + i) & 3) * 4);
+}
+// The image of a folded row tile: [block][rp][hi of residue 2rp, of 2rp + 1, lo of both][lane] x 16 bytes, then the 16 x nb
+// block scales as floats.
+constexpr int kImageBlockBytes = 4 * 4 * 512;
+
+// NT token tiles from tile0 on against one row tile: warp rp owns residues 2rp and 2rp + 1; their sums meet in shared memory at
+// the end and are added in order.
+template <int NT, int SLOTS, bool FOLDED>
+__device__ __forceinline__ void team_tiles(const GemmParams &p, const RowTile &rt, int first, int count, int tile0, uint32_t s_ring, float *s_ring_f,
+                                           float *s_ad, int ad_stride, int tid) {
+    constexpr int D = SLOTS / NT;  // blocks of activations on their way
+    const int nb = p.nb, rp = tid >> 5, lane = tid & 31, rows = p.rows[rt.j];
+    const int g4 = lane >> 2, q4 = lane & 3, n0 = tile0 * 8;
+    __syncthreads();  // (the ring and the scales of the tiles before are no longer read)
+    auto act = [&](int tok) -> unsigned {
+        const int pt = first + min(n0 + tok, count - 1);
+        return p.act_map ? (unsigned)p.act_map[pt] : (unsigned)pt;
+    };
+    // A lane copies the 16 bytes that it will itself multiply with: word q4 and q4 + 4 of its residues, token g4 of the tile.
+    const uint32_t ring = s_ring + (uint32_t)(rp * SLOTS * 512 + lane * 16);
+    const uint4 *src[NT];
+#pragma unroll
+    for (int t = 0; t < NT; t++) src[t] = reinterpret_cast<const uint4 *>(p.aq_rm) + (size_t)act(t * 8 + g4) * nb * 16 + rp * 4 + q4;
+    // (places without a token are left as they are: their sums go nowhere, and one line read by every lane of the GPU is slow)
+    const bool last_live = n0 + (NT - 1) * 8 + g4 < count;
+    auto request = [&](int b, int slot) {
+        if (b < nb) {
+#pragma unroll
+            for (int t = 0; t < NT; t++)
+                if (t + 1 < NT || last_live) copy_async16(ring + (uint32_t)((slot * NT + t) * 512), src[t] + (size_t)b * 16);
+        }
+        copy_commit();
+    };
+#pragma unroll
+    for (int s = 0; s < D; s++) request(s, s);
+    for (int i = tid; i < NT * 8 * nb; i += 128) {  // the tiles' activation scales, [block][token]
+        const int tok = i / nb, b = i - tok * nb;
+        s_ad[b * ad_stride + tok] = __ldg(p.ad + (size_t)act(tok) * nb + b);
     }
-    uint32_t *mine = s_b + rp * (kTeamWords / 4);
-    const int key = (g4 >> 1) & 3;
-    uint32_t *put = mine + g4 * 16 + 4 * (q4 ^ key);
     f32x2 sum[NT][2][2];
 #pragma unroll
     for (int t = 0; t < NT; t++) sum[t][0][0] = sum[t][0][1] = sum[t][1][0] = sum[t][1][1] = 0ull;
-    const f32x2 one = p.one, off = 0xCB400000CB400000ull, c64 = 0x4280000042800000ull;  // -1.5 * 2^23 and 64.0, twice
+    // -(1.5 * 2^29 + 1.5 * 2^21), twice: see the tail
+    const f32x2 one = p.one, off = 0xCE40C000CE40C000ull;
+    const int u[2] = {rt.unit0 + min(g4, rt.live - 1) * nb, rt.unit0 + min(g4 + 8, rt.live - 1) * nb};
+    uint32_t word_off[3];
+    fold_offsets(rp, q4, word_off);
+    Quad qh, ql;
+    opaque(qh, 0x4E400000u);
+    opaque(ql, 0x4A400000u);
+    copy_wait<D>();  // the weights' copies came before the ring's
     __syncthreads();
+    int slot = 0;
     for (int b = 0; b < nb; b++) {
+        uint32_t hi[2][4], lo[2][4];
+        f32x2 d[2];
+        if (FOLDED) {
+            const uint32_t at = rt.raw + (uint32_t)(b * kImageBlockBytes + rp * 2048 + lane * 16);
 #pragma unroll
-        for (int t = 0; t < NT; t++) *reinterpret_cast<uint4 *>(put + t * 128) = st[t];
-        __syncwarp();
-        if (b + 1 < nb) {
+            for (int rr = 0; rr < 2; rr++) {
+                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(hi[rr][0]), "=r"(hi[rr][1]), "=r"(hi[rr][2]), "=r"(hi[rr][3]) : "r"(at + rr * 512));
+                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(lo[rr][0]), "=r"(lo[rr][1]), "=r"(lo[rr][2]), "=r"(lo[rr][3]) : "r"(at + 1024 + rr * 512));
+            }
 #pragma unroll
-            for (int t = 0; t < NT; t++) st[t] = __ldg(src[t] + (size_t)(b + 1) * 16);
+            for (int h = 0; h < 2; h++) {
+                float df;
+                asm volatile("ld.shared.f32 %0, [%1];" : "=f"(df) : "r"(rt.raw + (uint32_t)(nb * kImageBlockBytes + ((g4 + 8 * h) * nb + b) * 4)));
+                d[h] = pack2(df, df);
+            }
+        } else {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                float df;
+                fold_block(rt.raw, u[h] + b, rp, q4, word_off, h, hi, lo, df);
+                d[h] = pack2(df, df);
+            }
         }
-        const float d0 = s_d[g4 * nb + b], d1 = s_d[(g4 + 8) * nb + b];
-        f32x2 dsc[NT][2];
+        copy_wait<D - 1>();
 #pragma unroll
         for (int t = 0; t < NT; t++) {
-            const f32x2 a = *reinterpret_cast<const f32x2 *>(s_ad + b * (8 * kGroupTiles) + t * 8 + 2 * q4);
-            dsc[t][0] = mul2(pack2(d0, d0), a);
-            dsc[t][1] = mul2(pack2(d1, d1), a);
-        }
-        const uint4 *fr = s_frag + ((size_t)(b * 8 + 2 * rp) * 2) * 32 + (lane ^ (lane >> 3) ^ (b & 7));
+            uint32_t bw[4];
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(bw[0]), "=r"(bw[1]), "=r"(bw[2]), "=r"(bw[3])
+                         : "r"(ring + (uint32_t)((slot * NT + t) * 512)));
+            const f32x2 a = *reinterpret_cast<const f32x2 *>(s_ad + b * ad_stride + t * 8 + 2 * q4);
+            const f32x2 dsc[2] = {mul2(d[0], a), mul2(d[1], a)};
 #pragma unroll
-        for (int rr = 0; rr < 2; rr++) {
-            const uint4 ah = fr[(rr * 2 + 0) * 32], al = fr[(rr * 2 + 1) * 32];
-            const uint32_t *bt = mine + g4 * 16 + q4;
-            const int o0 = 4 * ((2 * rr) ^ key), o1 = 4 * ((2 * rr + 1) ^ key);
-#pragma unroll
-            for (int t = 0; t < NT; t++) {
-                const uint32_t b0w = bt[t * 128 + o0], b1w = bt[t * 128 + o1];
+            for (int rr = 0; rr < 2; rr++) {
+                // The sums land on 1.5 * 2^29 (whose last place is 64) and on 1.5 * 2^21 (last place 1/4), so that they come
+                // out as the floats 64*hi and lo/4 with that offset. Both differences below are exact: multiples of 64
+                // below 2^25, and |aux| < 2^24.
                 int ch[4], cl[4];
-                mma_s8<0x4B400000>(ch, ah, b0w, b1w);
-                mma_s8<0x4B400000>(cl, al, b0w, b1w);
+                mma_8<false>(ch, hi[rr], bw[2 * rr], bw[2 * rr + 1], qh);
+                mma_8<true>(cl, lo[rr], bw[2 * rr], bw[2 * rr + 1], ql);
 #pragma unroll
                 for (int h = 0; h < 2; h++) {  // rows g4 and g4 + 8, tokens 2 q4 and 2 q4 + 1
-                    const f32x2 hi = add2(pack2(__int_as_float(ch[2 * h]), __int_as_float(ch[2 * h + 1])), off, one);
-                    const f32x2 lo = add2(pack2(__int_as_float(cl[2 * h]), __int_as_float(cl[2 * h + 1])), off, one);
-                    sum[t][rr][h] = add2(sum[t][rr][h], mul2(dsc[t][h], fma2(hi, c64, lo)), one);
+                    const f32x2 x = add2x(pack2(__int_as_float(ch[2 * h]), __int_as_float(ch[2 * h + 1])), off);
+                    const f32x2 aux = add2x(pack2(__int_as_float(cl[2 * h]), __int_as_float(cl[2 * h + 1])), x);
+                    sum[t][rr][h] = add2(sum[t][rr][h], mul2(dsc[h], aux), one);
                 }
             }
         }
-        __syncwarp();
+        request(b + D, slot);
+        slot = slot + 1 == D ? 0 : slot + 1;
     }
-    // y = ((((((s0+s1)+s2)+s3)+s4)+s5)+s6)+s7, two tiles at a time: [7 terms][16 token places][16 rows]
-    float *s_x = reinterpret_cast<float *>(s_b);
+    // y = ((((((s0+s1)+s2)+s3)+s4)+s5)+s6)+s7, two tiles at a time: [7 terms][16 token places][16 rows] where the ring was
+    float *s_x = s_ring_f;
 #pragma unroll
     for (int t0 = 0; t0 < NT; t0 += 2) {
         __syncthreads();
@@ -475,9 +314,9 @@ __device__ __forceinline__ void folded_tiles(const GemmParams &p, int j, int row
                     const float2 v = unpack2(add2(sum[t][0][h], sum[t][1][h], one));
                     x[0] = v.x, x[4 * 16] = v.y;
                 } else {
-                    const float2 v = unpack2(sum[t][0][h]), u = unpack2(sum[t][1][h]);
+                    const float2 v = unpack2(sum[t][0][h]), w = unpack2(sum[t][1][h]);
                     x += (2 * rp - 1) * 256;
-                    x[0] = v.x, x[4 * 16] = v.y, x[256] = u.x, x[256 + 4 * 16] = u.y;
+                    x[0] = v.x, x[4 * 16] = v.y, x[256] = w.x, x[256 + 4 * 16] = w.y;
                 }
             }
         }
@@ -490,97 +329,429 @@ __device__ __forceinline__ void folded_tiles(const GemmParams &p, int j, int row
 #pragma unroll
             for (int r = 1; r < 7; r++) y = __fadd_rn(y, x[r * 256]);
             const int n = n0 + t * 8 + 2 * (place & 3) + (place >> 2);
-            if (n < count && row0 + row < rows) p.out[j][(size_t)n * rows + row0 + row] = y;
+            if (n < count && row < rt.live) {
+                long long o = p.out_map ? p.out_map[first + n] : first + n;
+                float *out = p.out[rt.j];
+                if (p.out_tab) {  // the rows of a pair go to the GPU the pair's token lives on (plain peer stores)
+                    out = p.out_tab[o / p.out_div];
+                    o %= p.out_div;
+                }
+                out[o * rows + rt.row0 + row] = y;
+            }
         }
     }
 }
 
-static_assert(7 * 256 * 4 <= kTeamWords * 4, "the residues' sums of two tiles fit where the activations were");
-
-__host__ __device__ inline size_t folded_smem_bytes(int nb) {
-    return (size_t)nb * 8 * 2 * 32 * 16 + (size_t)kGemmRows * nb * 4 + (size_t)kTeamWords * 4 + (size_t)nb * 8 * kGroupTiles * 4;
+// A lane's four outputs: rows g4 (ya) and g4 + 8 (yb) of the row tile, tokens n and n + 1 of the group.
+__device__ __forceinline__ void store_pair(const GemmParams &p, int j, int row0, int live, int first, int count, int n, int g4, float2 ya, float2 yb) {
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        if (n + e >= count) continue;
+        long long o = p.out_map ? p.out_map[first + n + e] : first + n + e;
+        float *out = p.out[j];
+        if (p.out_tab) {  // the rows of a pair go to the GPU the pair's token lives on (plain peer stores)
+            out = p.out_tab[o / p.out_div];
+            o %= p.out_div;
+        }
+        out += o * p.rows[j] + row0;
+        if (g4 < live) out[g4] = e ? ya.y : ya.x;
+        if (g4 + 8 < live) out[g4 + 8] = e ? yb.y : yb.x;
+    }
 }
-// grid (row tiles of all jobs), one group of n_tokens
-__global__ void __launch_bounds__(128, 3) q6k_gemm_folded_kernel(const GemmParams p) {
+
+// ---- few tokens per group ----
+// Up to 8 NT tokens against one row tile, one warp per BW blocks of the rows: a warp folds all eight residues of its blocks, so
+// that a block's scales, addresses and token scales are prepared once for eight residues and not for two. The products of the
+// tail wait in registers; then the warps add theirs in block order, each to the sums that the warp before it left in shared
+// memory, and the last one adds the eight residues. DIRECT (short rows): one warp has all the blocks of its own row tile.
+// us, a residue pair per warp / this: the head for 8 tokens 95 / 86; down of 128 experts, 32 tokens 72 / 58, 128: 94 / 82. (Groups of 8
+// blocks a row: no gain, 130 / 131 for gate and up of 64 tokens, the products' registers cost the occupancy.)
+template <int NT>
+struct Sums {
+    f32x2 v[NT][8][2];  // [token tile][residue][rows g4, g4 + 8] x tokens 2 q4, 2 q4 + 1
+};
+template <int NT, int BW, bool DIRECT>
+__device__ __forceinline__ void few_tiles(const GemmParams &p, const RowTile &rt, int first, int count, int tile0, uint32_t s_act, float *s_x, int w,
+                                          int nw, int lane) {
+    const int nb = p.nb;
+    const int g4 = lane >> 2, q4 = lane & 3, n0 = tile0 * 8, b0 = w * BW;
+    auto act = [&](int tok) -> unsigned {
+        const int pt = first + min(n0 + tok, count - 1);
+        return p.act_map ? (unsigned)p.act_map[pt] : (unsigned)pt;
+    };
+    // this warp's blocks of the tokens: a lane copies the 16 bytes per residue pair that it will itself multiply with
+    const uint32_t mine = s_act + (uint32_t)(lane * 16);
+    float ad[NT][2][BW];
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(p.aq_rm) + ((size_t)act(t * 8 + g4) * nb + b0) * 16 + q4;
+        if (n0 + t * 8 + g4 < count) {  // (places without a token are left as they are: their sums go nowhere)
+#pragma unroll
+            for (int i = 0; i < BW; i++)
+                if (b0 + i < nb) {
+#pragma unroll
+                    for (int rp = 0; rp < 4; rp++) copy_async16_l1(mine + (uint32_t)(((t * BW + i) * 4 + rp) * 512), src + i * 16 + rp * 4);
+                }
+        }
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const float *a = p.ad + (size_t)act(t * 8 + 2 * q4 + e) * nb + b0;
+#pragma unroll
+            for (int i = 0; i < BW; i++) ad[t][e][i] = __ldg(a + min(i, nb - 1 - b0));
+        }
+    }
+    copy_commit();
+    const f32x2 one = p.one, off = 0xCE40C000CE40C000ull;  // -(1.5 * 2^29 + 1.5 * 2^21), twice: see team_tiles
+    const int u[2] = {rt.unit0 + min(g4, rt.live - 1) * nb + b0, rt.unit0 + min(g4 + 8, rt.live - 1) * nb + b0};
+    uint32_t word_off[3];
+    fold_offsets(0, q4, word_off);
+    Quad qh, ql;
+    opaque(qh, 0x4E400000u);
+    opaque(ql, 0x4A400000u);
+    copy_wait<0>();
+    __syncthreads();  // everyone's pieces of the weights
+    Sums<NT> sums, prod[DIRECT ? 1 : BW];
+#pragma unroll
+    for (int t = 0; t < NT; t++)
+#pragma unroll
+        for (int r = 0; r < 8; r++) sums.v[t][r][0] = sums.v[t][r][1] = 0ull;
+#pragma unroll
+    for (int i = 0; i < BW; i++) {
+        if (b0 + i < nb) {
+            uint32_t at[2];
+            Fold f[2];
+            f32x2 dsc[NT][2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint32_t tile = rt.raw + (uint32_t)((u[h] + i) >> 5) * kTileBytes, sl = (uint32_t)((u[h] + i) & 31);
+                at[h] = tile + 16u * (uint32_t)t32_slot((int)sl);
+                uint32_t sc;
+                uint16_t db;
+                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sc) : "r"(at[h] + kTileScaleOff + 4u * (uint32_t)q4));
+                asm volatile("ld.shared.u16 %0, [%1];" : "=h"(db) : "r"(tile + kTileDOff + 2u * sl));
+                fold_scales(f[h], sc);
+                const float d = f16_bits_to_f32(db);
+#pragma unroll
+                for (int t = 0; t < NT; t++) dsc[t][h] = mul2(pack2(d, d), pack2(ad[t][0][i], ad[t][1][i]));
+            }
+#pragma unroll
+            for (int rp = 0; rp < 4; rp++) {
+                uint32_t hi[2][4], lo[2][4];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    uint32_t s[3];
+#pragma unroll
+                    for (int c = 0; c < 3; c++) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(s[c]) : "r"(at[h] + word_off[c] + (uint32_t)(rp * 1536)));
+                    fold_quad(s, f[h], h, hi, lo);
+                }
+#pragma unroll
+                for (int t = 0; t < NT; t++) {
+                    uint32_t bw[4];
+                    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(bw[0]), "=r"(bw[1]), "=r"(bw[2]), "=r"(bw[3])
+                                 : "r"(mine + (uint32_t)(((t * BW + i) * 4 + rp) * 512)));
+#pragma unroll
+                    for (int rr = 0; rr < 2; rr++) {
+                        int ch[4], cl[4];
+                        mma_8<false>(ch, hi[rr], bw[2 * rr], bw[2 * rr + 1], qh);
+                        mma_8<true>(cl, lo[rr], bw[2 * rr], bw[2 * rr + 1], ql);
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const f32x2 x = add2x(pack2(__int_as_float(ch[2 * h]), __int_as_float(ch[2 * h + 1])), off);
+                            const f32x2 y = mul2(dsc[t][h], add2x(pack2(__int_as_float(cl[2 * h]), __int_as_float(cl[2 * h + 1])), x));
+                            if (DIRECT) sums.v[t][2 * rp + rr][h] = add2(sums.v[t][2 * rp + rr][h], y, one);
+                            else prod[DIRECT ? 0 : i].v[t][2 * rp + rr][h] = y;
+                        }
+                    }
+                }
+            }
+        }
+    }
+    f32x2 *x = reinterpret_cast<f32x2 *>(s_x) + lane;  // [token tile][residue][rows][lane]
+    if (!DIRECT) {
+        for (int ww = 0; ww < nw; ww++) {
+            if (ww == w) {
+                if (ww > 0) {
+#pragma unroll
+                    for (int k = 0; k < NT * 16; k++) sums.v[k >> 4][(k >> 1) & 7][k & 1] = x[k * 32];
+                }
+#pragma unroll
+                for (int i = 0; i < BW; i++)
+                    if (b0 + i < nb) {
+#pragma unroll
+                        for (int k = 0; k < NT * 16; k++)
+                            sums.v[k >> 4][(k >> 1) & 7][k & 1] = add2(sums.v[k >> 4][(k >> 1) & 7][k & 1], prod[DIRECT ? 0 : i].v[k >> 4][(k >> 1) & 7][k & 1], one);
+                    }
+                if (ww + 1 < nw) {
+#pragma unroll
+                    for (int k = 0; k < NT * 16; k++) x[k * 32] = sums.v[k >> 4][(k >> 1) & 7][k & 1];
+                }
+            }
+            if (ww + 1 < nw) __syncthreads();
+        }
+    }
+    if (DIRECT || w == nw - 1) {
+        // y = ((((((s0+s1)+s2)+s3)+s4)+s5)+s6)+s7
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+            f32x2 y[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                y[h] = sums.v[t][0][h];
+#pragma unroll
+                for (int r = 1; r < 8; r++) y[h] = add2(y[h], sums.v[t][r][h], one);
+            }
+            store_pair(p, rt.j, rt.row0, rt.live, first, count, n0 + t * 8 + 2 * q4, g4, unpack2(y[0]), unpack2(y[1]));
+        }
+    }
+}
+
+// grid (row_tiles-sized pieces of all jobs, groups or runs of tokens). Shared memory: the CTA's blocks as they are in memory
+// | four warps' rings of activation fragments, SLOTS x 512 bytes each | activation scales [nb][8 MAXT].
+template <int MAXT, int SLOTS, int MINB, bool FOLDED>
+__global__ void __launch_bounds__(128, MINB) q6k_gemm_kernel(const GemmParams p) {
+    static_assert(SLOTS / MAXT >= 2, "a block is read while the next is on its way");
+    static_assert(SLOTS * 2048 >= 7 * 256 * 4, "the residues' sums of two tiles fit where the activations were");
     extern __shared__ __align__(16) uint8_t smem[];
     const int nb = p.nb, tid = threadIdx.x;
-    uint4 *s_frag = reinterpret_cast<uint4 *>(smem);
-    float *s_d = reinterpret_cast<float *>(smem + (size_t)nb * 8 * 2 * 32 * 16);
-    uint32_t *s_b = reinterpret_cast<uint32_t *>(s_d + kGemmRows * nb);
-    float *s_ad = reinterpret_cast<float *>(s_b + kTeamWords);
-    const int j = job_of_tile(p, blockIdx.x), rt = (int)blockIdx.x - p.tile_begin[j];
-    const uint8_t *src = p.folded[j] + (size_t)rt * (size_t)p.fold_tile_bytes;
-    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem);
-    const int n16 = (int)(p.fold_tile_bytes >> 4);
-    for (int i = tid; i < n16; i += 128)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (uint32_t)i), "l"(src + 16 * (size_t)i) : "memory");
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    const int j = job_of_tile(p, blockIdx.x);
+    const int row_a = ((int)blockIdx.x - p.tile_begin[j]) * kGemmRows * p.row_tiles, live = min(p.row_tiles * kGemmRows, p.rows[j] - row_a);
     pdl_trigger();
-    pdl_wait();
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    // (the first barrier of a group stands between everyone's pieces of the image and their first use)
-    const int tiles = (p.n_tokens + 7) >> 3, groups = (tiles + kGroupTiles - 1) / kGroupTiles;
-    for (int g = 0, t = 0; g < groups; g++) {  // as few equal groups as kGroupTiles allows
-        const int nt = (tiles - t + groups - g - 1) / (groups - g);
-        switch (nt) {
-        case 1: folded_tiles<1>(p, j, rt * kGemmRows, t * 8, s_frag, s_d, s_b, s_ad, tid); break;
-        case 2: folded_tiles<2>(p, j, rt * kGemmRows, t * 8, s_frag, s_d, s_b, s_ad, tid); break;
-        case 3: folded_tiles<3>(p, j, rt * kGemmRows, t * 8, s_frag, s_d, s_b, s_ad, tid); break;
-        default: folded_tiles<4>(p, j, rt * kGemmRows, t * 8, s_frag, s_d, s_b, s_ad, tid); break;
+    int first = 0, tile_lo = 0, count = p.n_tokens, tile_hi;
+    size_t unit0 = (size_t)row_a * nb;
+    if (p.gstart) {
+        pdl_wait();
+        prefetch_ahead<FOLDED>(p, p.prefetch_ahead);
+        first = p.gstart[blockIdx.y];
+        count = p.gcount[blockIdx.y];
+        if (count <= 0) return;
+        unit0 += (size_t)blockIdx.y * (size_t)p.expert_units;
+        tile_hi = (count + 7) >> 3;
+    } else {
+        tile_lo = (int)blockIdx.y * p.run_tiles;
+        tile_hi = min((count + 7) >> 3, tile_lo + p.run_tiles);
+    }
+    const size_t t_lo = unit0 >> 5, t_hi = (unit0 + (size_t)live * nb - 1) >> 5;
+    const uint32_t s_raw = (uint32_t)__cvta_generic_to_shared(smem);
+    {
+        const uint8_t *src = p.w[j] + t_lo * kTileBytes;
+        int n16 = (int)(t_hi - t_lo + 1) * (kTileBytes / 16);
+        if (FOLDED) {
+            const int tiles_j = (p.rows[j] + kGemmRows - 1) / kGemmRows;
+            src = p.folded[j] + ((p.gstart ? (size_t)blockIdx.y * tiles_j : 0) + (size_t)(row_a / kGemmRows)) * (size_t)p.fold_tile_bytes;
+            n16 = (int)(p.fold_tile_bytes >> 4);
         }
-        t += nt;
+        for (int i = tid; i < n16; i += 128) copy_async16(s_raw + 16u * (uint32_t)i, src + 16 * (size_t)i);
+        copy_commit();
+    }
+    if (!p.gstart) pdl_wait();
+    float *s_ring = reinterpret_cast<float *>(smem + p.raw_bytes), *s_ad = s_ring + SLOTS * 512;
+    for (int r0 = 0; r0 < live; r0 += kGemmRows) {
+        const RowTile rt = {j, row_a + r0, min(kGemmRows, live - r0), s_raw, (int)(unit0 - (t_lo << 5)) + r0 * nb};
+        const int tiles = tile_hi - tile_lo, groups = (tiles + MAXT - 1) / MAXT;
+        for (int g = 0, t = tile_lo; g < groups; g++) {  // as few equal groups as MAXT allows
+            const int nt = (tile_hi - t + groups - g - 1) / (groups - g);
+#define LLAMD_TEAM(N)                                                                                                               \
+    if constexpr (N <= MAXT) {                                                                                                      \
+        if (nt == N) team_tiles<N, SLOTS, FOLDED>(p, rt, first, count, t, s_raw + (uint32_t)p.raw_bytes, s_ring, s_ad, 8 * MAXT, tid);       \
+    }
+            LLAMD_TEAM(1) LLAMD_TEAM(2) LLAMD_TEAM(3) LLAMD_TEAM(4) LLAMD_TEAM(5) LLAMD_TEAM(6) LLAMD_TEAM(7) LLAMD_TEAM(8)
+#undef LLAMD_TEAM
+            t += nt;
+        }
     }
 }
 
-// Folds every (expert, row tile) of one matrix once and keeps the image: grid (row tiles, experts).
+// grid as q6k_gemm_kernel's; a warp per BW blocks of a row tile, or (DIRECT) a warp per row tile, four row tiles a CTA.
+// Shared memory: the blocks | the warps' activations, NT x BW x 2 KB each | the sums on their way from warp to warp.
+template <int NT, int BW, bool DIRECT, int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) q6k_gemm_few_kernel(const GemmParams p) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int nb = p.nb, tid = threadIdx.x, w = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    const int j = job_of_tile(p, blockIdx.x);
+    const int row_a = ((int)blockIdx.x - p.tile_begin[j]) * kGemmRows * p.row_tiles, live = min(p.row_tiles * kGemmRows, p.rows[j] - row_a);
+    int first = 0, tile_lo = 0, count = p.n_tokens, tile_hi;
+    size_t unit0 = (size_t)row_a * nb;
+    pdl_trigger();
+    if (p.gstart) {
+        pdl_wait();
+        prefetch_ahead(p, p.prefetch_ahead);
+        first = p.gstart[blockIdx.y];
+        count = p.gcount[blockIdx.y];
+        if (count <= 0) return;
+        unit0 += (size_t)blockIdx.y * (size_t)p.expert_units;
+        tile_hi = (count + 7) >> 3;
+    } else {
+        tile_lo = (int)blockIdx.y * p.run_tiles;
+        tile_hi = min((count + 7) >> 3, tile_lo + p.run_tiles);
+    }
+    const size_t t_lo = unit0 >> 5, t_hi = (unit0 + (size_t)live * nb - 1) >> 5;
+    const uint32_t s_raw = (uint32_t)__cvta_generic_to_shared(smem);
+    {
+        const uint8_t *src = p.w[j] + t_lo * kTileBytes;
+        const int n16 = (int)(t_hi - t_lo + 1) * (kTileBytes / 16);
+        for (int i = tid; i < n16; i += blockDim.x) copy_async16(s_raw + 16u * (uint32_t)i, src + 16 * (size_t)i);
+        copy_commit();
+    }
+    if (!p.gstart) pdl_wait();
+    const uint32_t s_act = s_raw + (uint32_t)p.raw_bytes + (uint32_t)(w * NT * BW * 2048);
+    float *s_x = reinterpret_cast<float *>(smem + p.raw_bytes + nw * NT * BW * 2048);
+    const int r0 = DIRECT ? min(w * kGemmRows, ((live - 1) / kGemmRows) * kGemmRows) : 0;  // (a warp without a row tile repeats the last one)
+    const RowTile rt = {j, row_a + r0, min(kGemmRows, live - r0), s_raw, (int)(unit0 - (t_lo << 5)) + r0 * nb};
+    for (int t = tile_lo; t < tile_hi; t += NT) {
+        if (NT == 1 || tile_hi - t > 1) few_tiles<NT, BW, DIRECT>(p, rt, first, count, t, s_act, s_x, DIRECT ? 0 : w, nw, lane);
+        else few_tiles<1, BW, DIRECT>(p, rt, first, count, t, s_act, s_x, DIRECT ? 0 : w, nw, lane);
+        if (!DIRECT && t + NT < tile_hi) __syncthreads();  // (the sums' place is free again)
+    }
+}
+
+// ---- short rows, many tokens per group ----
+// With four blocks a row and less, a token group's preparation in q6k_gemm_kernel is as long as its products (down of 2048 tokens
+// 519 us, here 465; 768: 236 / 226; 512: 164 / 180). Here a CTA folds its 16 rows
+// into shared memory once, in operand order, and each of its warps takes token tiles of its own, all residues of them.
+constexpr int kTokStride = 80;  // words per staged token: 16-byte aligned, fragment reads in 32 banks
+__global__ void __launch_bounds__(128, 5) q6k_gemm_shared_kernel(const GemmParams p) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int nb = p.nb, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g4 = lane >> 2, q4 = lane & 3;
+    uint4 *s_frag = reinterpret_cast<uint4 *>(smem);  // [block][residue][hi, lo][lane]
+    float *s_d = reinterpret_cast<float *>(smem + (size_t)nb * 8 * 2 * 32 * 16);
+    uint32_t *s_b = reinterpret_cast<uint32_t *>(s_d + kGemmRows * nb) + warp * 8 * kTokStride;
+    const int j = job_of_tile(p, blockIdx.x), row0 = ((int)blockIdx.x - p.tile_begin[j]) * kGemmRows, rows = p.rows[j];
+    pdl_trigger();
+    pdl_wait();
+    prefetch_ahead(p, p.prefetch_ahead);
+    const int first = p.gstart[blockIdx.y], count = p.gcount[blockIdx.y], live = min(kGemmRows, rows - row0);
+    if (count <= 0) return;
+    const size_t unit0 = (size_t)blockIdx.y * (size_t)p.expert_units + (size_t)row0 * nb;
+    for (int it = tid; it < 2 * kGemmRows * nb; it += 128) {  // a thread: half of a (row, block)
+        const int half = it >= kGemmRows * nb ? 1 : 0, rb = it - half * kGemmRows * nb, row = rb / nb, b = rb - row * nb;
+        const size_t unit = unit0 + (size_t)min(row, live - 1) * nb + b;
+        const uint8_t *tile = p.w[j] + (unit >> 5) * kTileBytes;
+        const uint4 *cp = reinterpret_cast<const uint4 *>(tile) + t32_slot((int)(unit & 31));
+        uint32_t S[24];
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            const uint4 v = __ldg(cp + (6 * half + c) * 32);
+            S[4 * c] = v.x, S[4 * c + 1] = v.y, S[4 * c + 2] = v.z, S[4 * c + 3] = v.w;
+        }
+        const uint4 sc = __ldg(cp + kTileScaleOff / 16);
+        if (half == 0) s_d[rb] = f16_bits_to_f32(__ldg(reinterpret_cast<const uint16_t *>(tile + kTileDOff) + (unit & 31)));
+        const uint32_t scw[4] = {sc.x, sc.y, sc.z, sc.w};
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            Fold f;
+            fold_scales(f, scw[q]);
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const int quad = 4 * k + q;
+                const uint32_t words[3] = {S[3 * quad], S[3 * quad + 1], S[3 * quad + 2]};
+                uint32_t hi[2][4], lo[2][4];
+                fold_quad(words, f, 0, hi, lo);
+                // Lane L's 16 bytes sit in slot L ^ (L >> 3) ^ (b & 7): the threads of a warp here write the same word of
+                // neighbouring rows and blocks, and the swizzle spreads them over all eight 16-byte bank groups.
+                const int L = (row & 7) * 4 + q, P = L ^ (L >> 3) ^ (b & 7);
+#pragma unroll
+                for (int rr = 0; rr < 2; rr++) {
+                    uint32_t *at = reinterpret_cast<uint32_t *>(s_frag + (size_t)((b * 8 + 4 * half + 2 * k + rr) * 2) * 32 + P) + (row >> 3);
+                    at[0] = hi[rr][0], at[2] = hi[rr][2];
+                    at[128] = lo[rr][0], at[130] = lo[rr][2];
+                }
+            }
+        }
+    }
+    __syncthreads();
+    const f32x2 one = p.one;
+    const Quad zero = {{0, 0, 0, 0}};
+    for (int n0 = warp * 8; n0 < count; n0 += 32) {
+        auto act = [&](int tok) -> size_t {
+            const int pt = first + min(n0 + tok, count - 1);
+            return p.act_map ? (size_t)p.act_map[pt] : (size_t)pt;
+        };
+        const float *ad0 = p.ad + act(2 * q4) * nb, *ad1 = p.ad + act(2 * q4 + 1) * nb;
+        const uint4 *src[4];  // staging: 8 tokens x 16 pieces of 16 bytes, four per lane
+#pragma unroll
+        for (int i = 0; i < 4; i++) src[i] = reinterpret_cast<const uint4 *>(p.aq_rm) + act((lane >> 4) + 2 * i) * nb * 16 + (lane & 15);
+        uint32_t *put = s_b + (lane >> 4) * kTokStride + (lane & 15) * 4;
+        f32x2 sum[8][2];
+#pragma unroll
+        for (int r = 0; r < 8; r++) sum[r][0] = sum[r][1] = 0ull;
+        uint4 st[4];  // the next block's bytes wait in registers
+#pragma unroll
+        for (int i = 0; i < 4; i++) st[i] = __ldg(src[i]);
+        f32x2 a = pack2(__ldg(ad0), __ldg(ad1));
+        for (int b = 0; b < nb; b++) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) *reinterpret_cast<uint4 *>(put + 2 * i * kTokStride) = st[i];
+            __syncwarp();
+            const float d0 = s_d[g4 * nb + b], d1 = s_d[(g4 + 8) * nb + b];
+            const f32x2 dsc[2] = {mul2(pack2(d0, d0), a), mul2(pack2(d1, d1), a)};
+            if (b + 1 < nb) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) st[i] = __ldg(src[i] + (size_t)(b + 1) * 16);
+                a = pack2(__ldg(ad0 + b + 1), __ldg(ad1 + b + 1));
+            }
+            const uint4 *fr = s_frag + (size_t)b * 8 * 2 * 32 + (lane ^ (lane >> 3) ^ (b & 7));
+#pragma unroll
+            for (int rp = 0; rp < 4; rp++) {
+                const uint4 bw = *reinterpret_cast<const uint4 *>(s_b + g4 * kTokStride + rp * 16 + q4 * 4);
+#pragma unroll
+                for (int rr = 0; rr < 2; rr++) {
+                    const uint4 h4 = fr[((2 * rp + rr) * 2 + 0) * 32], l4 = fr[((2 * rp + rr) * 2 + 1) * 32];
+                    const uint32_t ah[4] = {h4.x, h4.y, h4.z, h4.w}, al[4] = {l4.x, l4.y, l4.z, l4.w};
+                    int ch[4], cl[4];
+                    mma_8<false>(ch, ah, rr ? bw.z : bw.x, rr ? bw.w : bw.y, zero);
+                    mma_8<true>(cl, al, rr ? bw.z : bw.x, rr ? bw.w : bw.y, zero);
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {  // (|aux| < 2^24: exact as a float)
+                        const f32x2 aux = pack2((float)(ch[2 * h] * 64 + (cl[2 * h] >> 2)), (float)(ch[2 * h + 1] * 64 + (cl[2 * h + 1] >> 2)));
+                        sum[2 * rp + rr][h] = add2(sum[2 * rp + rr][h], mul2(dsc[h], aux), one);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        f32x2 y[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            y[h] = sum[0][h];
+#pragma unroll
+            for (int r = 1; r < 8; r++) y[h] = add2(y[h], sum[r][h], one);
+        }
+        store_pair(p, j, row0, live, first, count, n0 + 2 * q4, g4, unpack2(y[0]), unpack2(y[1]));
+    }
+}
+
+// Folds every (expert, row tile) of one matrix once and keeps the image: grid (row tiles, experts), a warp per residue pair.
 __global__ void __launch_bounds__(128) q6k_prefold_kernel(const uint8_t *__restrict__ w, uint8_t *__restrict__ dst, int rows, int nb,
                                                           long long expert_units, long long tile_bytes) {
     extern __shared__ __align__(16) uint8_t smem[];
-    uint4 *s_frag = reinterpret_cast<uint4 *>(smem);
-    float *s_d = reinterpret_cast<float *>(smem + (size_t)nb * 8 * 2 * 32 * 16);
-    const int tid = threadIdx.x, row0 = blockIdx.x * kGemmRows, e = blockIdx.y;
-    for (int i = tid; i < kGemmRows * nb; i += 128) s_d[i] = 0.0f;  // (rows past the matrix: fold_store leaves their scales alone)
+    const int tid = threadIdx.x, rp = tid >> 5, lane = tid & 31, g4 = lane >> 2, q4 = lane & 3, row0 = blockIdx.x * kGemmRows;
+    const int live = min(kGemmRows, rows - row0);
+    const size_t unit0 = (size_t)blockIdx.y * (size_t)expert_units + (size_t)row0 * nb;
+    const size_t t_lo = unit0 >> 5, t_hi = (unit0 + (size_t)live * nb - 1) >> 5;
+    const uint32_t s_raw = (uint32_t)__cvta_generic_to_shared(smem);
+    const int n16 = (int)(t_hi - t_lo + 1) * (kTileBytes / 16);
+    for (int i = tid; i < n16; i += 128) copy_async16(s_raw + 16u * (uint32_t)i, w + t_lo * kTileBytes + 16 * (size_t)i);
+    copy_commit();
+    copy_wait<0>();
     __syncthreads();
-    fold_row_tile<128, false>(w, (size_t)e * (size_t)expert_units + (size_t)row0 * nb, rows - row0, nb, s_frag, s_d, tid);
-    __syncthreads();
-    uint4 *out = reinterpret_cast<uint4 *>(dst + ((size_t)e * gridDim.x + blockIdx.x) * (size_t)tile_bytes);
-    const int n16 = (int)(tile_bytes >> 4);
-    for (int i = tid; i < n16; i += 128) out[i] = reinterpret_cast<const uint4 *>(smem)[i];
-}
-
-// One group of n_tokens tokens; gridDim.x resident CTAs share the (row tile, chunk of kChunkTiles token tiles) items,
-// CTA c taking the contiguous range [c*items/grid, (c+1)*items/grid) in row-tile-major order.
-__global__ void __launch_bounds__(256, 2) q6k_gemm_dense_kernel(const GemmParams p, int total_row_tiles) {
-    extern __shared__ __align__(16) uint8_t smem[];
-    const int nb = p.nb;
-    uint4 *s_frag = reinterpret_cast<uint4 *>(smem);
-    float *s_d = reinterpret_cast<float *>(smem + (size_t)nb * 8 * 2 * 32 * 16);
-    pdl_trigger();
-    pdl_wait();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    uint32_t *s_b = reinterpret_cast<uint32_t *>(s_d + kGemmRows * nb) + (size_t)warp * 8 * kTokStride;
-    const int n_tiles = (p.n_tokens + 7) >> 3;
-    const int n_chunks = (n_tiles + kChunkTiles - 1) / kChunkTiles;
-    const long long items = (long long)total_row_tiles * n_chunks;
-    const long long it_lo = items * blockIdx.x / gridDim.x, it_hi = items * (blockIdx.x + 1) / gridDim.x;
-    int cur_rt = -1, j = 0, row0 = 0;
-    for (long long it = it_lo; it < it_hi; it++) {
-        const int rt = (int)(it / n_chunks), ch = (int)(it - (long long)rt * n_chunks);
-        if (rt != cur_rt) {
-            __syncthreads();  // every warp is done with the previous row tile's fragments
-            cur_rt = rt;
-            j = job_of_tile(p, rt);
-            row0 = (rt - p.tile_begin[j]) * kGemmRows;
-            if (tid == 0 && (long long)(rt + 1) * n_chunks < it_hi) {  // this CTA's next row tile
-                const int nj = job_of_tile(p, rt + 1);
-                const int nrow0 = (rt + 1 - p.tile_begin[nj]) * kGemmRows;
-                prefetch_row_tile(p.w[nj], (size_t)nrow0 * nb, p.rows[nj] - nrow0, nb);
-            }
-            fold_row_tile<256, false>(p.w[j], (size_t)row0 * nb, p.rows[j] - row0, nb, s_frag, s_d, tid);
-            __syncthreads();
+    uint8_t *out = dst + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * (size_t)tile_bytes;
+    uint32_t word_off[3];
+    fold_offsets(rp, q4, word_off);
+    for (int b = 0; b < nb; b++) {
+        uint32_t hi[2][4], lo[2][4];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            float d;
+            const int m = g4 + 8 * h;
+            fold_block(s_raw, (int)(unit0 - (t_lo << 5)) + min(m, live - 1) * nb + b, rp, q4, word_off, h, hi, lo, d);
+            if (rp == 0 && q4 == 0) reinterpret_cast<float *>(out + (size_t)nb * kImageBlockBytes)[m * nb + b] = m < live ? d : 0.0f;
         }
-        mma_token_tiles<1>(p, j, row0, p.rows[j], 0, p.n_tokens, ch * kChunkTiles, min(n_tiles, (ch + 1) * kChunkTiles), s_frag, s_d, s_b, warp, 8,
-                        lane);
+        uint4 *o = reinterpret_cast<uint4 *>(out + (size_t)b * kImageBlockBytes + rp * 2048) + lane;
+#pragma unroll
+        for (int rr = 0; rr < 2; rr++) {
+            o[rr * 32] = make_uint4(hi[rr][0], hi[rr][1], hi[rr][2], hi[rr][3]);
+            o[64 + rr * 32] = make_uint4(lo[rr][0], lo[rr][1], lo[rr][2], lo[rr][3]);
+        }
     }
 }
 
@@ -588,67 +759,108 @@ __global__ void __launch_bounds__(256, 2) q6k_gemm_dense_kernel(const GemmParams
 
 using namespace llamd;
 
-static void gemm_launch(GemmParams &p, int n_groups) {
-    const int threads = n_groups > 1 || p.gstart ? 128 : 256;
-    const size_t smem = gemm_smem_bytes(p.nb, threads);
-    if (p.nb < 1 || smem > 220 * 1024) {
-        set_error_msg("q6k gemm: blocks per row must be 1..24");
-        return;
+// KERNEL: one launch configuration remembers its own limits
+template <auto KERNEL>
+static void gemm_launch_k(GemmParams &p, int n_groups, int threads, size_t smem) {
+    static size_t configured = 0;
+    if (smem > 48 * 1024 && smem > configured) {
+        cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        configured = smem;
     }
-    int tiles = 0;
+    int grid_x = 0;
     for (int i = 0; i < p.njobs; i++) {
-        p.tile_begin[i] = tiles;
-        tiles += (p.rows[i] + kGemmRows - 1) / kGemmRows;
+        p.tile_begin[i] = grid_x;
+        grid_x += (p.rows[i] + kGemmRows * p.row_tiles - 1) / (kGemmRows * p.row_tiles);
     }
-    if (threads == 128) {
-        if (n_groups > 65535) {
-            set_error_msg("q6k gemm: too many groups");
-            return;
-        }
-        const bool hoist = p.nb > 4;
-        auto kernel = hoist ? q6k_gemm_grouped_kernel<true> : q6k_gemm_grouped_kernel<false>;
-        static size_t configured[2] = {0, 0};
-        if (smem > 48 * 1024 && smem > configured[hoist]) {
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            configured[hoist] = smem;
-        }
-        static int cached_nb = -1, cached_slots = 0;
-        if (cached_nb != p.nb) {
+    if (p.gstart) {
+        static size_t cached_smem = 0;
+        static int cached_slots = 0;
+        if (cached_smem != smem) {
             int dev = 0, sms = 0, per_sm = 0;
             cudaGetDevice(&dev);
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, smem);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KERNEL, threads, smem);
             cached_slots = sms * (per_sm > 0 ? per_sm : 1);
-            cached_nb = p.nb;
+            cached_smem = smem;
         }
         p.prefetch_ahead = cached_slots;
-        launch_k("q6k_gemm_grouped", kernel, dim3(tiles, n_groups), dim3(128), smem, p);
+    }
+    launch_kc(p.gstart ? PDL_OTHER : PDL_MATVEC, "q6k_gemm", KERNEL, dim3(grid_x, n_groups), dim3(threads), smem, p);
+}
+template <int MAXT, int SLOTS, int MINB, bool FOLDED>
+static void gemm_launch_t(GemmParams &p, int n_groups) {
+    gemm_launch_k<q6k_gemm_kernel<MAXT, SLOTS, MINB, FOLDED>>(p, n_groups, 128, (size_t)p.raw_bytes + (size_t)SLOTS * 2048 + (size_t)p.nb * 8 * MAXT * 4);
+}
+template <int NT, int BW, bool DIRECT, int THREADS, int MINB>
+static void gemm_launch_few(GemmParams &p, int n_groups) {
+    const int warps = DIRECT ? p.row_tiles : (p.nb + BW - 1) / BW;
+    gemm_launch_k<q6k_gemm_few_kernel<NT, BW, DIRECT, THREADS, MINB>>(p, n_groups, 32 * warps, (size_t)p.raw_bytes + (size_t)warps * NT * BW * 2048 + NT * 4096);
+}
+
+static void shared_launch(GemmParams &p, int n_groups) {
+    p.row_tiles = 1;
+    gemm_launch_k<q6k_gemm_shared_kernel>(p, n_groups, 128, (size_t)p.nb * 8 * 2 * 32 * 16 + (size_t)kGemmRows * p.nb * 4 + 4 * 8 * kTokStride * 4);
+}
+
+// Shared memory for `units` consecutive blocks: whole tiles, one more where they need not start with one.
+static int raw_tile_bytes(int units, bool aligned) {
+    return (aligned && units % 32 == 0 ? units / 32 : (units + 30) / 32 + 1) * kTileBytes;
+}
+
+// n_groups > 0: that many token groups of about `tokens` each. 0: one group of p.n_tokens.
+static void gemm_launch(GemmParams &p, int n_groups, int tokens) {
+    // (24 blocks a row: what the rings and the blocks of 16 rows leave of an SM's shared memory)
+    if (p.nb < 1 || p.nb > 24) {
+        set_error_msg("q6k gemm: blocks per row must be 1..24");
         return;
     }
-    static size_t configured = 0;
-    if (smem > 48 * 1024 && smem > configured) {
-        cudaFuncSetAttribute(q6k_gemm_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        configured = smem;
+    if (n_groups > 65535) {
+        set_error_msg("q6k gemm: too many groups");
+        return;
     }
-    // as many CTAs as stay resident at once (per shared-memory size: cached)
-    static int cached_nb = -1, cached_slots = 0;
-    if (cached_nb != p.nb) {
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, q6k_gemm_dense_kernel, 256, smem);
-        cached_slots = sms * (per_sm > 0 ? per_sm : 1);
-        cached_nb = p.nb;
+    const bool folded = p.folded[0] != nullptr;
+    p.one = kOne2;
+    const int tiles = (tokens + 7) / 8;
+    const bool direct = !folded && p.nb <= 3 && tokens <= 16, few = direct || (!folded && !p.gstart && tiles <= 1);
+    p.row_tiles = direct ? 4 : folded || few || p.nb >= 6 ? 1 : (p.nb >= 3 ? 2 : 4);
+    p.fold_tile_bytes = (long long)expert_fold_tile_bytes(p.nb);
+    p.raw_bytes = folded ? (int)p.fold_tile_bytes : raw_tile_bytes(p.row_tiles * kGemmRows * p.nb, !n_groups || p.expert_units % 32 == 0);
+    if (!n_groups) {
+        p.run_tiles = tiles <= 8 ? tiles : 8;
+        n_groups = (tiles + p.run_tiles - 1) / p.run_tiles;
+        if (n_groups > 65535) {
+            set_error_msg("q6k gemm: too many tokens");
+            return;
+        }
     }
-    const int n_tiles = (p.n_tokens + 7) / 8, n_chunks = (n_tiles + kChunkTiles - 1) / kChunkTiles;
-    const long long items = (long long)tiles * n_chunks;
-    const int grid = (int)(items < cached_slots ? items : cached_slots);
-    launch_k("q6k_gemm_dense", q6k_gemm_dense_kernel, dim3(grid), dim3(256), smem, p, tiles);
+    // The lines lie where the forms' times cross, see there; MAXT and the CTAs per SM by us of gate and up: 64 tokens (half a tile per
+    // expert) <2, 4, 6> 124, <4, 8, 5> 136; 512 (four) <8, 16, 3> 257, <6, 12, 4> 267, <4, 8, 4> 285; down of 512 <6, 12, 4> 164, <8, 16, 3> 179.
+    if (folded) {
+        if (tiles <= 4) gemm_launch_t<4, 8, 2, true>(p, n_groups);
+        else gemm_launch_t<8, 16, 2, true>(p, n_groups);
+    } else if (direct) {
+        if (tiles <= 1) gemm_launch_few<1, 3, true, 128, 5>(p, n_groups);
+        else gemm_launch_few<2, 3, true, 128, 3>(p, n_groups);
+    } else if (few) {
+        if (p.nb <= 8) gemm_launch_few<1, 2, false, 128, 4>(p, n_groups);
+        else if (p.nb <= 16) gemm_launch_few<1, 2, false, 256, 2>(p, n_groups);
+        else gemm_launch_few<1, 2, false, 384, 1>(p, n_groups);
+    } else if (p.gstart && p.nb <= 4 && tokens > 40) {
+        shared_launch(p, n_groups);
+    } else if (tiles <= 1) {
+        gemm_launch_t<2, 4, 6, false>(p, n_groups);
+    } else if (tiles <= 3) {
+        gemm_launch_t<4, 8, 4, false>(p, n_groups);
+    } else if (p.nb <= 4) {
+        gemm_launch_t<6, 12, 4, false>(p, n_groups);
+    } else {
+        gemm_launch_t<8, 16, 3, false>(p, n_groups);
+    }
 }
 
 extern "C" {
 
-// Q8_K quants [nblocks][256] (natural order) -> the residue-major words the GEMM reads.
+// Q8_K quants [nblocks][256] (natural order) -> the operand-order words the GEMM reads.
 void llamd_fwd_q8k_residue_major(const int8_t *aq, void *aq_rm, size_t nblocks) {
     if (!nblocks) return;
     const size_t n = nblocks * 64;
@@ -669,7 +881,7 @@ void llamd_fwd_gemm_tokens(const void *w0, const void *w1, const void *w2, const
     p.aq_rm = (const uint32_t *)aq_rm;
     p.ad = ad;
     p.n_tokens = ntok;
-    gemm_launch(p, 1);
+    gemm_launch(p, 0, ntok);
 }
 
 // Expert-major grouped GEMM over the scatter plan (gstart/gcount per expert, pairs sorted by expert):
@@ -678,46 +890,46 @@ void llamd_fwd_gemm_tokens(const void *w0, const void *w1, const void *w2, const
 void llamd_fwd_expert_gemm(const void *wa, const void *wb, const int32_t *gstart, const int32_t *gcount, const int32_t *act_map,
                            const int32_t *pslot, const void *aq_rm, const float *ad, float *oa, float *ob, int blocks, int rows,
                            int n_expert) {
-    expert_gemm_scatter(wa, wb, gstart, gcount, act_map, pslot, aq_rm, ad, oa, ob, blocks, rows, n_expert, nullptr, 1, nullptr, nullptr);
+    expert_gemm_scatter(wa, wb, gstart, gcount, act_map, pslot, aq_rm, ad, oa, ob, blocks, rows, n_expert, 0, nullptr, 1);
 }
 
 }  // extern "C"
 
-size_t llamd::expert_fold_tile_bytes(int blocks) { return (size_t)blocks * 8 * 2 * 32 * 16 + (size_t)kGemmRows * blocks * 4; }
+size_t llamd::expert_fold_tile_bytes(int blocks) { return (size_t)blocks * kImageBlockBytes + (size_t)kGemmRows * blocks * 4; }
 size_t llamd::expert_fold_bytes(int blocks, int rows, int n_expert) {
     return expert_fold_tile_bytes(blocks) * (size_t)((rows + kGemmRows - 1) / kGemmRows) * (size_t)n_expert;
 }
 void llamd::expert_prefold(const void *w, void *dst, int blocks, int rows, int n_expert) {
-    const size_t tile_bytes = expert_fold_tile_bytes(blocks);
+    if (n_expert > 65535 || n_expert < 1 || rows < 1 || blocks < 1 || blocks > 24) {
+        set_error_msg("expert prefold: 1..65535 experts, rows positive, 1..24 blocks per row");
+        return;
+    }
+    const size_t smem = (size_t)raw_tile_bytes(kGemmRows * blocks, false);
     static size_t configured = 0;
-    if (tile_bytes > 48 * 1024 && tile_bytes > configured) {
-        if (cudaFuncSetAttribute(q6k_prefold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_bytes) != cudaSuccess) {
+    if (smem > 48 * 1024 && smem > configured) {
+        if (cudaFuncSetAttribute(q6k_prefold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
             set_error_msg("expert prefold: shared memory attribute");
             return;
         }
-        configured = tile_bytes;
+        configured = smem;
     }
-    if (n_expert > 65535 || n_expert < 1 || rows < 1) {
-        set_error_msg("expert prefold: 1..65535 experts, rows positive");
-        return;
-    }
-    launch_k("q6k_prefold", q6k_prefold_kernel, dim3((rows + kGemmRows - 1) / kGemmRows, n_expert), dim3(128), tile_bytes, (const uint8_t *)w,
-             (uint8_t *)dst, rows, blocks, (long long)rows * blocks, (long long)tile_bytes);
+    launch_k("q6k_prefold", q6k_prefold_kernel, dim3((rows + kGemmRows - 1) / kGemmRows, n_expert), dim3(128), smem, (const uint8_t *)w,
+             (uint8_t *)dst, rows, blocks, (long long)rows * blocks, (long long)expert_fold_tile_bytes(blocks));
 }
 
 void llamd::expert_gemm_scatter(const void *wa, const void *wb, const int32_t *gstart, const int32_t *gcount, const int32_t *act_map,
                                 const int32_t *pslot, const void *aq_rm, const float *ad, float *oa, float *ob, int blocks, int rows,
-                                int n_expert, float *const *out_tab, int out_div, const void *fa, const void *fb) {
+                                int n_expert, int pairs, float *const *out_tab, int out_div, const void *fa, const void *fb) {
     if (out_tab && (wb || out_div < 1)) {
         set_error_msg("expert gemm: scattered outputs take one matrix and a positive row-block count per GPU");
         return;
     }
+    if (n_expert < 1) return;
     GemmParams p = {};
     p.out_tab = out_tab;
     p.out_div = out_div;
     p.w[0] = (const uint8_t *)wa; p.w[1] = (const uint8_t *)wb;
     p.folded[0] = (const uint8_t *)fa; p.folded[1] = wb ? (const uint8_t *)fb : nullptr;
-    p.fold_tile_bytes = (long long)expert_fold_tile_bytes(blocks);
     p.out[0] = oa; p.out[1] = ob;
     p.rows[0] = rows; p.rows[1] = rows;
     p.njobs = wb ? 2 : 1;
@@ -726,18 +938,16 @@ void llamd::expert_gemm_scatter(const void *wa, const void *wb, const int32_t *g
     p.ad = ad;
     p.gstart = gstart; p.gcount = gcount; p.act_map = act_map; p.out_map = pslot;
     p.expert_units = (long long)rows * blocks;
-    gemm_launch(p, n_expert);
+    gemm_launch(p, n_expert, pairs > 0 ? (pairs + n_expert - 1) / n_expert : 64);
 }
 
 // Up to three matrices kept folded (expert_prefold with one "expert" each) against ntok activations: out_i[ntok][rows_i].
-// A CTA copies its row tile's image and multiplies (q6k_gemm_folded_kernel); 2 bytes per weight whatever
-// ntok is, where the matvec repeats its integer work per sequence. Same results as llamd_fwd_gemm_tokens.
+// 2 bytes per weight and no folding. Same results as llamd_fwd_gemm_tokens.
 void llamd::gemm_tokens_folded3(const void *f0, const void *f1, const void *f2, const void *aq_rm, const float *ad, float *o0, float *o1,
                                 float *o2, int blocks, int rows0, int rows1, int rows2, int ntok) {
     if (ntok < 1) return;
     GemmParams p = {};
     p.folded[0] = (const uint8_t *)f0; p.folded[1] = (const uint8_t *)f1; p.folded[2] = (const uint8_t *)f2;
-    p.fold_tile_bytes = (long long)expert_fold_tile_bytes(blocks);
     p.out[0] = o0; p.out[1] = o1; p.out[2] = o2;
     p.rows[0] = rows0; p.rows[1] = rows1; p.rows[2] = rows2;
     p.njobs = f2 ? 3 : (f1 ? 2 : 1);
@@ -745,23 +955,7 @@ void llamd::gemm_tokens_folded3(const void *f0, const void *f1, const void *f2, 
     p.aq_rm = (const uint32_t *)aq_rm;
     p.ad = ad;
     p.n_tokens = ntok;
-    p.one = kOne2;
-    const size_t smem = folded_smem_bytes(blocks);
-    if (blocks < 1 || smem > 220 * 1024) {
-        set_error_msg("q6k gemm: blocks per row must be 1..24");
-        return;
-    }
-    static size_t configured = 0;
-    if (smem > 48 * 1024 && smem > configured) {
-        cudaFuncSetAttribute(q6k_gemm_folded_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        configured = smem;
-    }
-    int tiles = 0;
-    for (int i = 0; i < p.njobs; i++) {
-        p.tile_begin[i] = tiles;
-        tiles += (p.rows[i] + kGemmRows - 1) / kGemmRows;
-    }
-    launch_kc(PDL_MATVEC, "q6k_gemm_folded", q6k_gemm_folded_kernel, dim3(tiles), dim3(128), smem, p);
+    gemm_launch(p, 0, ntok);
 }
 void llamd::gemm_tokens_folded(const void *folded, const void *aq_rm, const float *ad, float *out, int blocks, int rows, int ntok) {
     gemm_tokens_folded3(folded, nullptr, nullptr, aq_rm, ad, out, nullptr, nullptr, blocks, rows, 0, 0, ntok);

@@ -101,8 +101,9 @@ __global__ void act_f16_rm_kernel(const int8_t *__restrict__ aq, const float *__
     const __half h1 = __float2half_rn(v);
     const __half h2 = __float2half_rn(__fsub_rn(v, __half2float(h1)));
     __half *row = out + (blk * 8 + r) * 64;
-    row[j * 4 + k] = h1;
-    row[32 + j * 4 + k] = h2;
+    const int kk = 2 * (k & 1) + (k >> 1);  // the bytes of one scale group side by side, as the weights are folded
+    row[j * 4 + kk] = h1;
+    row[32 + j * 4 + kk] = h2;
 }
 
 __device__ __forceinline__ int tc_job_of_tile(const TcParams &p, int rt) {
@@ -225,26 +226,23 @@ __global__ void __launch_bounds__(256, 2) q6k_gemm_tc_kernel(const TcParams p) {
     const uint32_t sA_u = smem_u32(sA), sB_u = smem_u32(sB);
     const int sw = row & 7;
     // the four 16-byte pieces this thread writes in a stage's A tile: row = [U >> 6: words jw 0..7 | (U & 63)/64: words jw 0..7],
-    // 8 bytes per word; this thread owns jw = 4m .. 4m+3
-    const uint32_t a_off[4] = {(uint32_t)(row * 128 + (((2 * m + 0) ^ sw) << 4)), (uint32_t)(row * 128 + (((2 * m + 1) ^ sw) << 4)),
-                               (uint32_t)(row * 128 + (((4 + 2 * m + 0) ^ sw) << 4)), (uint32_t)(row * 128 + (((4 + 2 * m + 1) ^ sw) << 4))};
+    // 8 bytes per word; this thread owns jw = 2m, 2m+1, 2m+4, 2m+5 (two quads of every residue pair)
+    const uint32_t a_off[4] = {(uint32_t)(row * 128 + (((m + 0) ^ sw) << 4)), (uint32_t)(row * 128 + (((m + 2) ^ sw) << 4)),
+                               (uint32_t)(row * 128 + (((4 + m + 0) ^ sw) << 4)), (uint32_t)(row * 128 + (((4 + m + 2) ^ sw) << 4))};
     const bool bcopy[2] = {n_pad * 8 > tid, n_pad * 8 > tid + 256};
     bool ok = true;
     // where block b of this thread's row sits: tile base + its slot
     auto block_ptr = [&](int b) -> const uint8_t * {
         const size_t unit = unit_row + b;
-        return wj + (unit >> 5) * kTileBytes + (unit & 31) * 16;
+        return wj + (unit >> 5) * kTileBytes + t32_slot((int)(unit & 31)) * 16;
     };
     const uint8_t *tb = live ? block_ptr(0) : wj;
-    // code words of the next stage (Sn) and of the one after it (Sn2): two stages of L2 latency are covered
-    uint32_t Sn[3] = {0, 0, 0}, Sn2[3] = {0, 0, 0};
+    // code words of the current residue pair (Sn) and of the next one (Sn2): two stages of L2 latency are covered
+    uint32_t Sn[6] = {0, 0, 0, 0, 0, 0}, Sn2[6] = {0, 0, 0, 0, 0, 0};
     uint2 scn = make_uint2(0, 0);
     if (live) {
 #pragma unroll
-        for (int x = 0; x < 3; x++) {
-            Sn[x] = __ldg(reinterpret_cast<const uint32_t *>(tb + (m ? TC_WOFF(3 + x) : TC_WOFF(x))));
-            Sn2[x] = __ldg(reinterpret_cast<const uint32_t *>(tb + (m ? TC_WOFF(6 + 3 + x) : TC_WOFF(6 + x))));
-        }
+        for (int x = 0; x < 6; x++) Sn2[x] = __ldg(reinterpret_cast<const uint32_t *>(tb + (m ? TC_WOFF(6 + x) : TC_WOFF(x))));
         scn = __ldg(reinterpret_cast<const uint2 *>(tb + kTileScaleOff + 8 * m));
     }
     // the B tiles of stages 0 and 1 start their trip now; stage s issues the copy for stage s+2
@@ -285,45 +283,53 @@ __global__ void __launch_bounds__(256, 2) q6k_gemm_tc_kernel(const TcParams p) {
             else asm volatile("cp.async.commit_group;" ::: "memory");  // keep one group per stage so that the count below holds
 
             if (r == 3) load_d(b);  // the previous block's drain (at r == 1) is done with the old value
-            // ---- this thread's 16 weights: MMA words jw = 4m .. 4m+3 of residue r of block (row, b) ----
-            const uint32_t S0 = Sn[0], S1 = Sn[1], S2 = Sn[2];
+            // ---- this thread's 16 weights: MMA words 2m, 2m+1, 2m+4, 2m+5 of residue r of block (row, b) ----
             if (r == 0) {
                 const uint32_t ws[2] = {scn.x, scn.y};
 #pragma unroll
                 for (int i = 0; i < 8; i++) sc[i] = (int)(int8_t)(ws[i >> 2] >> (8 * (i & 3)));
             }
-            Sn[0] = Sn2[0]; Sn[1] = Sn2[1]; Sn[2] = Sn2[2];
-            if (live) {  // the words of stage s+2: two stages of work hide their latency
-                if (r < 6) {
+            if ((r & 1) == 0) {
 #pragma unroll
-                    for (int x = 0; x < 3; x++)
-                        Sn2[x] = __ldg(reinterpret_cast<const uint32_t *>(tb + (m ? TC_WOFF(6 * (r + 2) + 3 + x) : TC_WOFF(6 * (r + 2) + x))));
-                } else if (b + 1 < nb) {
+                for (int x = 0; x < 6; x++) Sn[x] = Sn2[x];
+            }
+            if (live) {  // the words of the next residue pair: two stages of work hide their latency
+                if ((r & 1) == 0 && r < 6) {
 #pragma unroll
-                    for (int x = 0; x < 3; x++)
-                        Sn2[x] = __ldg(reinterpret_cast<const uint32_t *>(tb_next + (m ? TC_WOFF(6 * (r - 6) + 3 + x) : TC_WOFF(6 * (r - 6) + x))));
+                    for (int x = 0; x < 6; x++)
+                        Sn2[x] = __ldg(reinterpret_cast<const uint32_t *>(tb + (m ? TC_WOFF(6 * (r + 2) + 6 + x) : TC_WOFF(6 * (r + 2) + x))));
+                } else if (r == 6 && b + 1 < nb) {
+#pragma unroll
+                    for (int x = 0; x < 6; x++) Sn2[x] = __ldg(reinterpret_cast<const uint32_t *>(tb_next + (m ? TC_WOFF(6 + x) : TC_WOFF(x))));
                 }
                 if (r == 4 && b + 1 < nb) scn = __ldg(reinterpret_cast<const uint2 *>(tb_next + kTileScaleOff + 8 * m));  // used from the next block's r == 0
             }
             uint32_t ahi[8], alo[8];
             if (live) {
-                // The stored byte is 4*(q-32) mod 256; ^0x80 makes it 4q. The fourth word's codes are the low bit pairs of
-                // the other three.
-                uint32_t ub[4];
-                ub[0] = (S0 & 0xFCFCFCFCu) ^ 0x80808080u;
-                ub[1] = (S1 & 0xFCFCFCFCu) ^ 0x80808080u;
-                ub[2] = (S2 & 0xFCFCFCFCu) ^ 0x80808080u;
-                ub[3] = (((S0 << 6) & 0xC0C0C0C0u) | ((S1 << 4) & 0x30303030u) | ((S2 << 2) & 0x0C0C0C0Cu)) ^ 0x80808080u;
+                // The stored byte is 4*(q-32) mod 256; ^0x80 makes it 4q. A quad's fourth word is the low bit pairs of the
+                // other three; an even residue takes its quads' words 0 and 1, an odd one words 2 and 3.
+                uint32_t ub[4];  // words 2m, 2m+1, 2m+4, 2m+5
+#pragma unroll
+                for (int ql = 0; ql < 2; ql++) {
+                    const uint32_t S0 = Sn[3 * ql], S1 = Sn[3 * ql + 1], S2 = Sn[3 * ql + 2];
+                    if ((r & 1) == 0) {
+                        ub[ql] = (S0 & 0xFCFCFCFCu) ^ 0x80808080u;
+                        ub[2 + ql] = (S1 & 0xFCFCFCFCu) ^ 0x80808080u;
+                    } else {
+                        ub[ql] = (S2 & 0xFCFCFCFCu) ^ 0x80808080u;
+                        ub[2 + ql] = (((S0 << 6) & 0xC0C0C0C0u) | ((S1 << 4) & 0x30303030u) | ((S2 << 2) & 0x0C0C0C0Cu)) ^ 0x80808080u;
+                    }
+                }
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     // Two weights per multiply-add. With the bytes spread into 16-bit fields, x - 0x00800080 is, as an
                     // integer, sum_i 4*(q_i - 32) << 16i, so sc*(x - 0x00800080) + 0x80008000 holds 4*U_i + 32768
                     // (U = sc*(q-32), in [16512, 49152]) in each field with no carry between them: the high byte is
-                    // (U >> 6) + 128, the low byte 4*(U & 63). Bytes 0,1 of word i belong to scale group 2i, bytes 2,3 to 2i+1.
+                    // (U >> 6) + 128, the low byte 4*(U & 63). Bytes 0 and 2 of word j belong to scale group 2j, bytes 1 and 3 to 2j+1.
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
-                        const uint32_t x = __byte_perm(ub[i], 0u, h ? 0x4342 : 0x4140);
-                        const uint32_t v = (x - 0x00800080u) * (uint32_t)sc[2 * i + h] + 0x80008000u;
+                        const uint32_t x = __byte_perm(ub[i], 0u, h ? 0x4341 : 0x4240);
+                        const uint32_t v = (x - 0x00800080u) * (uint32_t)sc[4 * (i & 1) + 2 * (i >> 1) + h] + 0x80008000u;
                         // bytes under the exponent of 1024: (1024 + byte) as f16, two per register
                         const uint32_t bh = __byte_perm(v, 0x64646464u, 0x4341), bl = __byte_perm(v, 0x64646464u, 0x4240);
                         const __half2 hh = __hsub2(*reinterpret_cast<const __half2 *>(&bh), __half2half2(__ushort_as_half(0x6480)));  // - 1152: U >> 6

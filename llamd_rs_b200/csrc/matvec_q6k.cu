@@ -15,10 +15,11 @@
 // floor(256/blocks) whole rows. The per-unit f32 products go through shared
 // memory to the threads that walk the ordered sums.
 //
-// Activation staging: for block b and residue r the shared-memory image holds
-// eight word pairs (lo, hi): word j carries bytes a[e(r,j,0..3)] and lo / hi
-// keep bytes 0-1 / 2-3 only, so dp4a(W4_j, lo) and dp4a(W4_j, hi) are the two
-// per-group pair products (times 4, since W4 = 4*(q-32)).
+// Activation staging: for block b the shared-memory image holds 64 word pairs,
+// in the order of the weights' quads: word j of residue r carries bytes
+// a[e(r,j,0..3)] and the pair keeps bytes 0 and 2 / bytes 1 and 3 only, so a
+// dp4a of W4_j with each is the pair product of one scale group (times 4, since
+// W4 = 4*(q-32)).
 #include "q6k_layout.cuh"
 #include "quant.cuh"
 
@@ -196,7 +197,7 @@ __global__ void __launch_bounds__(kThreads, NSEQ == 1 ? 3 : (NSEQ == 2 ? 2 : 1))
     if (active) {
         const size_t unit = (size_t)expert_off + (size_t)(row0 + row_l) * nb + b;
         const uint8_t *tile = job.w + (unit >> 5) * kTileBytes;
-        const int sl = (int)(unit & 31);
+        const int sl = t32_slot((int)(unit & 31));
         const uint4 *cp = reinterpret_cast<const uint4 *>(tile) + sl;
 #pragma unroll
         for (int c = 0; c < 12; c++) {
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(kThreads, NSEQ == 1 ? 3 : (NSEQ == 2 ? 2 : 1))
             S[4 * c + 3] = v.w;
         }
         scw = __ldg(reinterpret_cast<const uint4 *>(tile + kTileScaleOff) + sl);
-        dbits = __ldg(reinterpret_cast<const uint16_t *>(tile + kTileDOff) + sl);
+        dbits = __ldg(reinterpret_cast<const uint16_t *>(tile + kTileDOff) + (unit & 31));
     }
 
     // Ungrouped: the weight loads above do not depend on the previous kernel and
@@ -325,7 +326,7 @@ __global__ void __launch_bounds__(kThreads, NSEQ == 1 ? 3 : (NSEQ == 2 ? 2 : 1))
         }
     }
     __syncthreads();
-    // ... then the residue-major (lo, hi) image
+    // ... then the image of word pairs
     {
         const int nitems = NSEQ * nb * 64;  // (s, b, r, j)
         for (int i = tid; i < nitems; i += kThreads) {
@@ -333,9 +334,9 @@ __global__ void __launch_bounds__(kThreads, NSEQ == 1 ? 3 : (NSEQ == 2 ? 2 : 1))
             const int8_t *src = s_nat + sb * 256;
             const uint32_t b0 = (uint8_t)src[t32_element(r, jj, 0)], b1 = (uint8_t)src[t32_element(r, jj, 1)];
             const uint32_t b2 = (uint8_t)src[t32_element(r, jj, 2)], b3 = (uint8_t)src[t32_element(r, jj, 3)];
-            uint32_t *dst = s_act + sb * kActBlockWords + r * 16 + jj * 2;
-            dst[0] = b0 | (b1 << 8);
-            dst[1] = (b2 << 16) | (b3 << 24);
+            uint32_t *dst = s_act + sb * kActBlockWords + t32_place(r, jj) * 2;
+            dst[0] = b0 | (b2 << 16);
+            dst[1] = (b1 << 8) | (b3 << 24);
         }
     }
     __syncthreads();  // s_nat is dead from here: s_ex may be written
@@ -354,26 +355,25 @@ __global__ void __launch_bounds__(kThreads, NSEQ == 1 ? 3 : (NSEQ == 2 ? 2 : 1))
 #pragma unroll
             for (int r = 0; r < 8; r++) aux[s][r] = 0;
 #pragma unroll
-        for (int r = 0; r < 8; r++) {
+        for (int quad = 0; quad < 16; quad++) {
+            const int r = 2 * (quad >> 2), q = quad & 3;
+            uint32_t w4[4];
+            unpack_quad(S[3 * quad], S[3 * quad + 1], S[3 * quad + 2], w4);
 #pragma unroll
-            for (int m = 0; m < 2; m++) {
-                uint32_t w4[4];
-                unpack_quad(S[6 * r + 3 * m], S[6 * r + 3 * m + 1], S[6 * r + 3 * m + 2], w4);
-#pragma unroll
-                for (int s = 0; s < NSEQ; s++) {
-                    const uint4 *ap = reinterpret_cast<const uint4 *>(s_act + (s * nb + b) * kActBlockWords + r * 16 + m * 8);
-                    const uint4 a01 = ap[0], a23 = ap[1];
-                    int acc = aux[s][r];
-                    acc += sc[8 * m + 0] * __dp4a((int)w4[0], (int)a01.x, 0);
-                    acc += sc[8 * m + 1] * __dp4a((int)w4[0], (int)a01.y, 0);
-                    acc += sc[8 * m + 2] * __dp4a((int)w4[1], (int)a01.z, 0);
-                    acc += sc[8 * m + 3] * __dp4a((int)w4[1], (int)a01.w, 0);
-                    acc += sc[8 * m + 4] * __dp4a((int)w4[2], (int)a23.x, 0);
-                    acc += sc[8 * m + 5] * __dp4a((int)w4[2], (int)a23.y, 0);
-                    acc += sc[8 * m + 6] * __dp4a((int)w4[3], (int)a23.z, 0);
-                    acc += sc[8 * m + 7] * __dp4a((int)w4[3], (int)a23.w, 0);
-                    aux[s][r] = acc;
-                }
+            for (int s = 0; s < NSEQ; s++) {
+                const uint4 *ap = reinterpret_cast<const uint4 *>(s_act + (s * nb + b) * kActBlockWords + quad * 8);
+                const uint4 a01 = ap[0], a23 = ap[1];
+                int a0 = aux[s][r], a1 = aux[s][r + 1];
+                a0 += sc[4 * q + 0] * __dp4a((int)w4[0], (int)a01.x, 0);
+                a0 += sc[4 * q + 1] * __dp4a((int)w4[0], (int)a01.y, 0);
+                a0 += sc[4 * q + 2] * __dp4a((int)w4[1], (int)a01.z, 0);
+                a0 += sc[4 * q + 3] * __dp4a((int)w4[1], (int)a01.w, 0);
+                a1 += sc[4 * q + 0] * __dp4a((int)w4[2], (int)a23.x, 0);
+                a1 += sc[4 * q + 1] * __dp4a((int)w4[2], (int)a23.y, 0);
+                a1 += sc[4 * q + 2] * __dp4a((int)w4[3], (int)a23.z, 0);
+                a1 += sc[4 * q + 3] * __dp4a((int)w4[3], (int)a23.w, 0);
+                aux[s][r] = a0;
+                aux[s][r + 1] = a1;
             }
         }
         const float dw = f16_bits_to_f32(dbits);

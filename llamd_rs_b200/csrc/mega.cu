@@ -128,7 +128,7 @@ struct MvUnit {
 };
 __device__ __forceinline__ void mv_load(MvUnit &u, const uint8_t *w, size_t unit) {
     const uint8_t *tile = w + (unit >> 5) * kTileBytes;
-    const int sl = (int)(unit & 31);
+    const int sl = t32_slot((int)(unit & 31));
     const uint4 *cp = reinterpret_cast<const uint4 *>(tile) + sl;
 #pragma unroll
     for (int c = 0; c < 12; c++) {
@@ -139,7 +139,7 @@ __device__ __forceinline__ void mv_load(MvUnit &u, const uint8_t *w, size_t unit
         u.S[4 * c + 3] = v.w;
     }
     u.scw = __ldg(reinterpret_cast<const uint4 *>(tile + kTileScaleOff) + sl);
-    u.dbits = __ldg(reinterpret_cast<const uint16_t *>(tile + kTileDOff) + sl);
+    u.dbits = __ldg(reinterpret_cast<const uint16_t *>(tile + kTileDOff) + (unit & 31));
 }
 // the unit's eight (d_w * d_a) * aux products into the exchange buffer, column `col`
 __device__ __forceinline__ void mv_compute(const MvUnit &u, const uint32_t *s_act_blk, float adv, float *s_ex, int col) {
@@ -153,40 +153,36 @@ __device__ __forceinline__ void mv_compute(const MvUnit &u, const uint32_t *s_ac
 #pragma unroll
     for (int r = 0; r < 8; r++) aux[r] = 0;
 #pragma unroll
-    for (int r = 0; r < 8; r++) {
-#pragma unroll
-        for (int m = 0; m < 2; m++) {
-            uint32_t w4[4];
-            unpack_quad(u.S[6 * r + 3 * m], u.S[6 * r + 3 * m + 1], u.S[6 * r + 3 * m + 2], w4);
-            const uint4 *ap = reinterpret_cast<const uint4 *>(s_act_blk + r * 16 + m * 8);
-            const uint4 a01 = ap[0], a23 = ap[1];
-            int acc = aux[r];
-            acc += sc[8 * m + 0] * __dp4a((int)w4[0], (int)a01.x, 0);
-            acc += sc[8 * m + 1] * __dp4a((int)w4[0], (int)a01.y, 0);
-            acc += sc[8 * m + 2] * __dp4a((int)w4[1], (int)a01.z, 0);
-            acc += sc[8 * m + 3] * __dp4a((int)w4[1], (int)a01.w, 0);
-            acc += sc[8 * m + 4] * __dp4a((int)w4[2], (int)a23.x, 0);
-            acc += sc[8 * m + 5] * __dp4a((int)w4[2], (int)a23.y, 0);
-            acc += sc[8 * m + 6] * __dp4a((int)w4[3], (int)a23.z, 0);
-            acc += sc[8 * m + 7] * __dp4a((int)w4[3], (int)a23.w, 0);
-            aux[r] = acc;
-        }
+    for (int quad = 0; quad < 16; quad++) {
+        const int r = 2 * (quad >> 2), q = quad & 3;
+        uint32_t w4[4];
+        unpack_quad(u.S[3 * quad], u.S[3 * quad + 1], u.S[3 * quad + 2], w4);
+        const uint4 *ap = reinterpret_cast<const uint4 *>(s_act_blk + quad * 8);
+        const uint4 a01 = ap[0], a23 = ap[1];
+        aux[r] += sc[4 * q + 0] * __dp4a((int)w4[0], (int)a01.x, 0);
+        aux[r] += sc[4 * q + 1] * __dp4a((int)w4[0], (int)a01.y, 0);
+        aux[r] += sc[4 * q + 2] * __dp4a((int)w4[1], (int)a01.z, 0);
+        aux[r] += sc[4 * q + 3] * __dp4a((int)w4[1], (int)a01.w, 0);
+        aux[r + 1] += sc[4 * q + 0] * __dp4a((int)w4[2], (int)a23.x, 0);
+        aux[r + 1] += sc[4 * q + 1] * __dp4a((int)w4[2], (int)a23.y, 0);
+        aux[r + 1] += sc[4 * q + 2] * __dp4a((int)w4[3], (int)a23.z, 0);
+        aux[r + 1] += sc[4 * q + 3] * __dp4a((int)w4[3], (int)a23.w, 0);
     }
     const float dsc = __fmul_rn(f16_bits_to_f32(u.dbits), adv);
 #pragma unroll
     for (int r = 0; r < 8; r++) s_ex[r * kMegaExStride + col] = __fmul_rn(dsc, (float)(aux[r] >> 2));
 }
 
-// natural-order Q8_K bytes of `nblk` blocks -> the residue-major (lo, hi) image the units read
+// natural-order Q8_K bytes of `nblk` blocks -> the (even bytes, odd bytes) image the units read
 __device__ __forceinline__ void build_act_image(const int8_t *s_nat, uint32_t *s_act, int nblk) {
     for (int i = threadIdx.x; i < nblk * 64; i += kMegaThreads) {
         const int jj = i & 7, r = (i >> 3) & 7, sb = i >> 6;
         const int8_t *src = s_nat + sb * 256;
         const uint32_t b0 = (uint8_t)src[t32_element(r, jj, 0)], b1 = (uint8_t)src[t32_element(r, jj, 1)];
         const uint32_t b2 = (uint8_t)src[t32_element(r, jj, 2)], b3 = (uint8_t)src[t32_element(r, jj, 3)];
-        uint32_t *dst = s_act + sb * kMegaActWords + r * 16 + jj * 2;
-        dst[0] = b0 | (b1 << 8);
-        dst[1] = (b2 << 16) | (b3 << 24);
+        uint32_t *dst = s_act + sb * kMegaActWords + t32_place(r, jj) * 2;
+        dst[0] = b0 | (b2 << 16);
+        dst[1] = (b1 << 8) | (b3 << 24);
     }
 }
 
@@ -921,7 +917,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_mega_kernel(const __gr
             const size_t unit = (size_t)token * eb + (i >> 8);
             const int e = i & 255;
             const float d = f16_bits_to_f32(*reinterpret_cast<const uint16_t *>(p.tok_embd + t32_d_offset(unit)));
-            const float sc = (float)(int8_t)p.tok_embd[t32_scale_offset(unit) + (e >> 4)];
+            const float sc = (float)(int8_t)p.tok_embd[t32_scale_offset(unit, e >> 4)];
             sx0[i] = __fmul_rn(__fmul_rn(d, sc), (float)t32_weight(p.tok_embd, unit, e));
         }
     }

@@ -144,8 +144,8 @@ struct Model {
     Buf tok_embd, output_norm, output, rope_tab;
     // scratch (crates/llamd-runtime/src/device.rs:407-434)
     Buf x, xb, xb2, q, k, v, attn, aq, ad, aq2, ad2, router_logits, router_probs, expert_ids, expert_w;
-    Buf head_fold, head_rm;  // the output matrix folded for the integer GEMM (option "head_gemm"); a batch's activations in the GEMM's operand order
-    bool head_fold_ready = false, head_fold_failed = false;
+    Buf head_rm, aq2_rm;     // a batch's activations in the GEMM's operand order, and its experts' (decode pass)
+    Buf plan;                // ... and its scatter plan: gstart, gcount [n_expert], ptoken, pslot [max_seq * n_expert_used]
     Buf slot_order;          // [max_seq * n_expert_used] a batch's (sequence, slot) pairs sorted by expert (decode pass, 8 sequences and more)
     Buf e_gate, e_up, e_down, logits, amax_v, amax_i, out_token, meta;
     Buf trace_x, trace_ids;  // [n_layer][max_seq][n_embd], [n_layer][max_seq][n_used]
@@ -206,10 +206,10 @@ struct Model {
                              // copies of their matrices (as "head_gemm"; +2 bytes per weight of the four matrices of every layer); 0: never
     Buf dense_fold;          // the folded projections of all layers
     bool dense_fold_ready = false, dense_fold_failed = false;
-    bool prompt_no_dense = false, prompt_no_head = false;  // a prompt found too little memory free to make these copies (a batch may still)
-    int head_gemm = 4;       // option "head_gemm" = n: from n sequences per pass the output projection runs on the integer GEMM over a folded
-                             // copy of the matrix (2 bytes per weight once per pass, where the matvec repeats its integer work per sequence;
-                             // +0.6 GB for a 151936 x 2048 matrix, made at the first such pass); 0: never
+    bool prompt_no_dense = false;  // a prompt found too little memory free to make these copies (a batch may still)
+    int head_gemm = 4;       // option "head_gemm" = n: from n sequences per pass the output projection runs on the integer GEMM, which folds a
+                             // weight once for all of them where the matvec repeats its integer work per sequence; 0: never. us for
+                             // 151936 x 2048, matvec / GEMM: 1 sequence 46 / 81, 3: 143 / 83, 8: 296 / 86
     int fuse_norm_router_max = 2;  // option "fuse_norm_router_max": the fused norm + router launch serves passes of fewer sequences than this.
                                    // Measured, tok/s aggregate, fused / separate: 1 sequence 281.3 / 275.7 (when it was built), 2: 460.5 / 485.0,
                                    // 4: 727.1 / 736.8, 8: 1112.5 / 1149.2, 24: 1644.5 / 1718.7, 48: 1876.2 / 1941.4
@@ -393,6 +393,15 @@ void queue_token_resident(Model &m) {
 constexpr int kNearPositions = 512;
 bool near_pass(const Model &m, int nseq, int n_kv) { return m.ep_world == 1 && nseq <= 2 && nseq * n_kv <= kNearPositions; }
 
+// From how many tokens (sequences of a pass, tokens of a tile) on the experts run as a grouped GEMM over the scatter plan instead
+// of a matvec per (token, expert): it folds an expert's weights once for all its tokens, the matvec repeats its integer work
+// for each. us a layer (plan or slot order, gate and up, down) of 128 experts of 768 x 2048, 8 per token, matvec / GEMM: 16 tokens
+// 106 / 135, 24: 153 / 163, 32: 197 / 171, 40: 240 / 183, 64: 382 / 195. The GEMM's rows are up to 24 blocks.
+constexpr int kExpertGemmMin = 27;
+bool expert_gemm_pass(const Model &m, int n) {
+    return n >= kExpertGemmMin && m.ep_world == 1 && m.hp.n_embd <= 24 * 256 && m.hp.n_ff_expert <= 24 * 256 && m.hp.n_expert <= 1024;
+}
+
 // Queue one pass for `nseq` sequences. Does not synchronise. near: see near_pass.
 // The order is crates/llamd-runtime/src/device.rs:486-655 (itself the CPU
 // order of crates/llamd-runtime/src/layer.rs:85-203, 230-304).
@@ -413,7 +422,13 @@ void queue_token(Model &m, int nseq, bool near) {
     // the dependency wait, the batch form of attention
     const int pf = (m.arith_fast && m.fuse_norm_router && !m.fuse_tails ? m.arith_fast : 0) | (m.early_loads ? kPassEarlyLoads : 0) |
                    (m.attn_gqa && !near ? kPassAttnGqa : 0);
+    // (the fused launch repeats the norm in each of its n_expert / 4 CTAs per sequence; it wins for a single sequence, where a
+    // launch boundary is what it saves, and loses from two sequences on -- m.fuse_norm_router_max -- where the norm as a
+    // launch of its own and the router rows behind it cost less; the `fast` arithmetic's router tree lives in the fused kernel)
+    const bool fuse_nr = m.fuse_norm_router && (size_t)6 * E * sizeof(float) <= 200 * 1024 && E % 256 == 0 && hp.n_expert <= 4 * E &&
+                         (nseq < m.fuse_norm_router_max || m.arith_fast);
     const bool dense_gemm = m.dense_gemm && nseq >= m.dense_gemm && m.dense_fold_ready && !m.fuse_norm_qkv;
+    const bool experts_gemm = expert_gemm_pass(m, nseq) && !fuse_nr && !m.fuse_tails && !m.fuse_silu_down;
     int8_t *rm = dense_gemm ? m.head_rm.as<int8_t>() : nullptr;  // the GEMMs' operand, made with the quants
     bool rm_made = false;
     size_t n_marks = 0;
@@ -456,11 +471,6 @@ void queue_token(Model &m, int nseq, bool near) {
     // where the residual stream lives: m.x, or m.xb after a fused norm + router launch (which may not write in place: its
     // other CTAs still read the old stream); the combine that opens the next layer moves it back to m.x
     const float *x_res = x;
-    // (the fused launch repeats the norm in each of its n_expert / 4 CTAs per sequence; it wins for a single sequence, where a
-    // launch boundary is what it saves, and loses from two sequences on -- m.fuse_norm_router_max -- where the norm as a
-    // launch of its own and the router rows behind it cost less; the `fast` arithmetic's router tree lives in the fused kernel)
-    const bool fuse_nr = m.fuse_norm_router && (size_t)6 * E * sizeof(float) <= 200 * 1024 && E % 256 == 0 && hp.n_expert <= 4 * E &&
-                         (nseq < m.fuse_norm_router_max || m.arith_fast);
     for (int il = 0; il < hp.n_layer; il++) {
         Layer &l = m.layers[il];
         // Attention norm, f32 and Q8_K in one pass (Q, K and V read the same
@@ -556,7 +566,7 @@ void queue_token(Model &m, int nseq, bool near) {
             mark(LLAMD_PH_FFN_NORM);
         } else {
             add_rms_norm_quant_flags(x, m.xb2.as<float>(), x, l.ffn_norm.as<float>(), m.xb.as<float>(), m.aq.as<int8_t>(), m.ad.as<float>(), E,
-                                     hp.rms_eps, nseq, pf);
+                                     hp.rms_eps, nseq, pf, experts_gemm ? m.head_rm.as<int8_t>() : nullptr);
             mark(LLAMD_PH_FFN_NORM);
             if (nseq > kRouterRowsMax) {
                 matmul_f32_tokens(l.ffn_gate_inp.as<float>(), m.xb.as<float>(), m.router_logits.as<float>(), E, hp.n_expert, nseq, true);
@@ -607,6 +617,24 @@ void queue_token(Model &m, int nseq, bool near) {
                                 cudaMemcpyDeviceToDevice, stream());
             continue;
         }
+        if (experts_gemm) {
+            // many sequences: an expert's weights folded once for all that chose it (the same bits)
+            int32_t *gstart = m.plan.as<int32_t>(), *gcount = gstart + hp.n_expert, *ptoken = gcount + hp.n_expert, *pslot = ptoken + m.max_seq * nu;
+            moe_plan_launch(m.expert_ids.as<int32_t>(), nseq * nu, hp.n_expert, nu, gstart, gcount, ptoken, pslot);
+            expert_gemm_scatter(l.gate_exps.p, l.up_exps.p, gstart, gcount, ptoken, pslot, m.head_rm.p, m.ad.as<float>(), m.e_gate.as<float>(),
+                                m.e_up.as<float>(), eb, ffe, hp.n_expert, nseq * nu);
+            mark(LLAMD_PH_GATE_UP);
+            silu_mul_quant_rm(m.e_gate.as<float>(), m.e_up.as<float>(), nullptr, m.aq2.as<int8_t>(), m.ad2.as<float>(), nseq * nu * ffe,
+                              m.aq2_rm.as<int8_t>());
+            mark(LLAMD_PH_SILU);
+            expert_gemm_scatter(l.down_exps.p, nullptr, gstart, gcount, pslot, pslot, m.aq2_rm.p, m.ad2.as<float>(), m.e_down.as<float>(), nullptr,
+                                ffe / 256, E, hp.n_expert, nseq * nu);
+            mark(LLAMD_PH_DOWN);
+            if (m.trace)
+                cudaMemcpyAsync(m.trace_ids.as<int32_t>() + (size_t)il * m.max_seq * nu, m.expert_ids.p, (size_t)nseq * nu * sizeof(int32_t),
+                                cudaMemcpyDeviceToDevice, stream());
+            continue;
+        }
         MatvecPlans gu = plan_experts(m, l.down_exps, m.expert_ids.as<int32_t>(), nseq * nu);
         // a batch's slots in expert order, so that the sequences that chose the same expert read it side by side (one small
         // launch; measured worth it from 8 sequences on)
@@ -648,15 +676,16 @@ void queue_token(Model &m, int nseq, bool near) {
                             cudaMemcpyDeviceToDevice, stream());
     }
     // the last layer's combine, fused with the output norm
-    const bool head_gemm = m.head_gemm && nseq >= m.head_gemm && m.head_fold_ready;
+    const bool head_gemm = m.head_gemm && nseq >= m.head_gemm;
     combine_rms_norm_quant_wait(plan_ep_wait(), x_res, m.e_down.as<float>(), m.expert_w.as<float>(), nu, x, m.output_norm.as<float>(), nullptr,
                                 m.aq.as<int8_t>(), m.ad.as<float>(), E, hp.rms_eps, nseq, pf,
                                 head_gemm ? m.head_rm.as<int8_t>() : nullptr);
     trace_x(hp.n_layer - 1);
     mark(LLAMD_PH_ATTN_NORM);
     if (head_gemm) {
-        // a batch: the folded matrix once for all the sequences, on the integer tensor path (the same bits)
-        gemm_tokens_folded(m.head_fold.p, m.head_rm.p, m.ad.as<float>(), m.logits.as<float>(), eb, hp.n_vocab, nseq);
+        // a batch: every weight folded once for all the sequences, on the integer tensor path (the same bits)
+        llamd_fwd_gemm_tokens(m.output.p ? m.output.p : m.tok_embd.p, nullptr, nullptr, m.head_rm.p, m.ad.as<float>(), m.logits.as<float>(), nullptr,
+                              nullptr, eb, hp.n_vocab, 0, 0, nseq);
     } else {
         // (the prefetch plan names where the next token starts)
         matvec_batch(plan_static(m, &m.layers[0].attn_q, &m.layers[0].attn_k, &m.layers[0].attn_v), m.output.p ? m.output.p : m.tok_embd.p,
@@ -733,12 +762,12 @@ size_t prefill_bytes(const Model &m, size_t T) {
     return T * per_token + scores + 30 * ((size_t)2 << 20);  // (30 buffers, 2 MB pages)
 }
 
-// The folded copies that a pass over n sequences, or a small tile of n tokens, multiplies with (options "dense_gemm" and
-// "head_gemm"), made once and not inside a capture; without the memory for them the matvec serves every pass. They stay, so
+// The folded copies that a pass over n sequences, or a small tile of n tokens, multiplies with (option "dense_gemm"), made once
+// and not inside a capture; without the memory for them the matvec serves every pass. They stay, so
 // a prompt or a draft (`prompt` tokens per tile that it may take) makes them only where a full tile's buffers fit beside them.
 // False: an error. The projections of a 48-layer model (1.9 GB, one allocation) cost the first prompt of 8 tokens or more 5 ms;
 // with four allocations per layer it was 66.
-bool ensure_folded(Model &m, int n, int prompt = 0, bool head = true) {
+bool ensure_folded(Model &m, int n, int prompt = 0) {
     const llamd_hparams &hp = m.hp;
     const int eb = hp.n_embd / 256, qd = hp.n_head * hp.head_dim, kvd = hp.n_head_kv * hp.head_dim;
     const bool clean = error_code() == 0;
@@ -775,23 +804,6 @@ bool ensure_folded(Model &m, int n, int prompt = 0, bool head = true) {
             if (!m.dense_fold_ready) {
                 m.dense_fold.release();
                 m.dense_fold_failed = true;
-                return false;
-            }
-        }
-    }
-    if (head && m.head_gemm && n >= m.head_gemm && !m.head_fold_ready && !m.head_fold_failed && !(prompt && m.prompt_no_head)) {
-        const size_t need = expert_fold_bytes(eb, hp.n_vocab, 1);
-        if (!room(need)) {
-            (prompt ? m.prompt_no_head : m.head_fold_failed) = true;
-        } else if (!m.head_fold.alloc(need)) {
-            failed(m.head_fold);
-            m.head_fold_failed = true;
-        } else {
-            expert_prefold(m.output.p ? m.output.p : m.tok_embd.p, m.head_fold.p, eb, hp.n_vocab, 1);
-            m.head_fold_ready = llamd_fwd_sync() == 0;
-            if (!m.head_fold_ready) {
-                m.head_fold.release();
-                m.head_fold_failed = true;
                 return false;
             }
         }
@@ -918,7 +930,7 @@ llamd_model *llamd_model_create(const llamd_hparams *hp, int max_kv, int max_seq
     f(m->x, E); f(m->xb, E); f(m->xb2, E); f(m->q, qd); f(m->k, kvd); f(m->v, kvd); f(m->attn, qd);
     ok = ok && m->aq.alloc(max_act * S);
     f(m->ad, max_act / 256);
-    ok = ok && m->aq2.alloc(nu * ffe * S) && m->head_rm.alloc(max_act * S);
+    ok = ok && m->aq2.alloc(nu * ffe * S) && m->head_rm.alloc(max_act * S) && m->aq2_rm.alloc(nu * ffe * S) && m->plan.alloc((2 * (size_t)hp->n_expert + 2 * nu * S) * 4);
     f(m->ad2, nu * ffe / 256);
     f(m->router_logits, hp->n_expert); f(m->router_probs, hp->n_expert);
     ok = ok && m->expert_ids.alloc(nu * 4 * S) && m->slot_order.alloc(nu * 4 * S);
@@ -970,7 +982,7 @@ void llamd_model_free(llamd_model *h) {
                        &l.ffn_gate_inp, &l.gate_exps, &l.up_exps, &l.down_exps, &l.gate_fold, &l.up_fold, &l.down_fold, &l.kc, &l.vc})
             b->release();
     for (Buf *b : {&m->tok_embd, &m->output_norm, &m->output, &m->rope_tab, &m->x, &m->xb, &m->xb2, &m->q, &m->k, &m->v, &m->attn,
-                   &m->aq, &m->ad, &m->aq2, &m->ad2, &m->router_logits, &m->router_probs, &m->expert_ids, &m->slot_order, &m->head_fold, &m->dense_fold, &m->head_rm, &m->expert_w, &m->e_gate,
+                   &m->aq, &m->ad, &m->aq2, &m->ad2, &m->router_logits, &m->router_probs, &m->expert_ids, &m->slot_order, &m->dense_fold, &m->head_rm, &m->aq2_rm, &m->plan, &m->expert_w, &m->e_gate,
                    &m->e_up, &m->e_down, &m->logits, &m->amax_v, &m->amax_i, &m->out_token, &m->meta, &m->trace_x, &m->trace_ids,
                    &m->tok_log, &m->tok_count, &m->router_counter, &m->tail_counter, &m->scores, &m->ids_all, &m->ad_all, &m->aq_all, &m->gate_all,
                    &m->up_all, &m->aq2_all, &m->ad2_all, &m->down_all, &m->recv_all, &m->ep_arrive, &m->ep_status, &m->ep_out_tab,
@@ -1011,11 +1023,7 @@ int llamd_model_set_tensor(llamd_model *h, int layer, int which, size_t first_bl
     if (which == LLAMD_T_TOK_EMBD || which == LLAMD_T_OUTPUT) {
         total = q6k_blocks_for(hp.n_vocab, E);
         ok = upload_q6k_slice(which == LLAMD_T_TOK_EMBD ? m->tok_embd : m->output, total, first_block, host, count);
-        if (m->head_fold_ready || m->head_fold_failed) {  // the folded copy of the output matrix is of the old bytes
-            if (g_graph_owner == m->id) llamd_fwd_graph_destroy();
-            m->head_fold.release();
-            m->head_fold_ready = m->head_fold_failed = false;
-        }
+        if (g_graph_owner == m->id) llamd_fwd_graph_destroy();  // (it names the matrix that served as the head)
     } else if (which == LLAMD_T_OUTPUT_NORM) {
         ok = count == E && upload_f32(m->output_norm, host, E);
     } else {
@@ -1455,14 +1463,15 @@ static int ep_tile_cap(const Model &m) {
 }
 
 // Up to kFoldedMax tokens the dense matrices run on the folded copies whatever the experts do, us folded / folding on the
-// way: QKV of 64 tokens 18.0 / 31, 128: 33 / 40, 160: 40 / 47, 250: 62 / 60.
+// way, QKV and output projection: 8 tokens 6.3 + 5.7 / 7.2 + 6.9, 32: 9.9 + 7.4 / 10.3 + 11.3, 64: 16.6 + 12.7 / 16.4 + 19.8, 192: 33.7 + 35.1 /
+// 34.2 + 32.4.
 constexpr int kFoldedMax = 192;
 static bool folded_tile(const Model &m, int T) { return m.ep_world == 1 && m.prefill_gemm == 1 && T <= kFoldedMax; }
 
-// A small tile of one sequence (a draft, a short turn, a prompt's rest) runs its matrices as a decode pass over as many
-// sequences does: the experts as grouped matvecs with the slots in expert order, the dense matrices on the folded copies.
-// The tile GEMMs fold every weight for 16-token MMA tiles that a handful of tokens leaves nearly empty. The line is where
-// a batch of sequences changes over, which was measured there (matvec_batch_max).
+// A small tile of one sequence (a draft, a short turn, a prompt's rest) runs as a decode pass over as many sequences does: its
+// attention by kv head, the experts of a handful of tokens as grouped matvecs with the slots in expert order
+// (expert_gemm_pass), the dense matrices on the folded copies. The line is where a batch of sequences changes over
+// (matvec_batch_max).
 static bool small_tile(const Model &m, int T, bool multi_seq) {
     return !multi_seq && m.ep_world == 1 && m.prefill_gemm == 1 && !m.prefold_ready && T <= m.matvec_batch_max;
 }
@@ -1480,6 +1489,7 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
     float *x = p.x.as<float>();
     const int max_items = T * nu / 8 + ne;
     const bool small = small_tile(m, T, multi_seq);
+    const bool few = small && !expert_gemm_pass(m, T);  // the experts as grouped matvecs
     const bool folded = folded_tile(m, T) && m.dense_gemm && T >= m.dense_gemm && m.dense_fold_ready;
     // up to three dense matrices of a small or folded tile against the activations in p.aq / p.ad
     auto small_dense = [&](const void *f0, const void *f1, const void *f2, const Buf &w0, const Buf &w1, const Buf &w2, const Buf &o0, const Buf &o1,
@@ -1497,7 +1507,7 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
     const Buf none;
     // the GEMMs' operand is made with the quants
     const bool exact_gemm = (m.prefill_gemm != 0 && m.prefill_gemm != 2) || m.ep_world > 1;
-    int8_t *rm = folded || (exact_gemm && !small) ? p.aq_rm.as<int8_t>() : nullptr;
+    int8_t *rm = folded || (exact_gemm && !few) ? p.aq_rm.as<int8_t>() : nullptr;
     llamd_fwd_embed_meta(m.tok_embd.p, meta, x, eb, T);
     for (int il = 0; il < hp.n_layer; il++) {
         Layer &l = m.layers[il];
@@ -1580,7 +1590,7 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
                                     qd / 256, E, 0, 0, T);
         }
         add_rms_norm_quant_flags(x, p.xb2.as<float>(), x, l.ffn_norm.as<float>(), p.xb.as<float>(), p.aq.as<int8_t>(), p.ad.as<float>(),
-                                     E, hp.rms_eps, T, 0, small || ep ? nullptr : rm);
+                                     E, hp.rms_eps, T, 0, few || ep ? nullptr : rm);
         if (m.prefill_attn && T > kRouterRowsMax) {
             matmul_f32_tokens(l.ffn_gate_inp.as<float>(), p.xb.as<float>(), p.logits.as<float>(), E, ne, T, true);
             llamd_fwd_router(p.logits.as<float>(), ne, nu, p.ids.as<int32_t>(), p.w.as<float>(), nullptr, T);
@@ -1605,19 +1615,19 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
             const bool pre = m.prefold_ready;
             expert_gemm_scatter(l.gate_exps.p, l.up_exps.p, p.gstart.as<int32_t>() + m.own_lo, p.gcount.as<int32_t>() + m.own_lo,
                                 p.ptoken.as<int32_t>(), p.pslot.as<int32_t>(), p.aq_all_rm.p, p.ad_all.as<float>(), p.gate_all.as<float>(),
-                                p.up_all.as<float>(), eb, ffe, n_local, nullptr, 1, pre ? l.gate_fold.p : nullptr, pre ? l.up_fold.p : nullptr);
+                                p.up_all.as<float>(), eb, ffe, n_local, T * nu, nullptr, 1, pre ? l.gate_fold.p : nullptr, pre ? l.up_fold.p : nullptr);
             // (every gathered pair, owned or not: the others' rows are never read)
             llamd_fwd_silu_mul_quant(p.gate_all.as<float>(), p.up_all.as<float>(), nullptr, p.aq2_all.as<int8_t>(), p.ad2_all.as<float>(),
                                      G * nu * ffe);
             llamd_fwd_q8k_residue_major(p.aq2_all.as<int8_t>(), p.aq2_all_rm.p, (size_t)G * nu * (ffe / 256));
             expert_gemm_scatter(l.down_exps.p, nullptr, p.gstart.as<int32_t>() + m.own_lo, p.gcount.as<int32_t>() + m.own_lo,
                                 p.pslot.as<int32_t>(), p.pslot.as<int32_t>(), p.aq2_all_rm.p, p.ad2_all.as<float>(), p.down.as<float>(), nullptr,
-                                ffe / 256, E, n_local, p.down_tab.as<float *>(), cap * nu);
+                                ffe / 256, E, n_local, T * nu, p.down_tab.as<float *>(), cap * nu);
             ep_signal_rows(m.ep_arrive_tab.as<unsigned int *>());
             ep_wait_rows(m.ep_arrive.as<unsigned int>(), (unsigned)W, m.ep_status.as<int>(), m.ep_poll_limit);
             continue;
         }
-        if (small) {
+        if (few) {
             MatvecPlans plan = {};
             if (m.sort_slots && T >= m.sort_slots) {
                 slot_order_launch(p.ids.as<int32_t>(), T * nu, ne, p.pslot.as<int32_t>());
@@ -1648,11 +1658,11 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
         } else if (gemm) {
             const bool pre = m.prefold_ready;
             expert_gemm_scatter(l.gate_exps.p, l.up_exps.p, p.gstart.as<int32_t>(), p.gcount.as<int32_t>(), p.ptoken.as<int32_t>(),
-                                p.pslot.as<int32_t>(), p.aq_rm.p, p.ad.as<float>(), p.gate.as<float>(), p.up.as<float>(), eb, ffe, ne, nullptr, 1,
+                                p.pslot.as<int32_t>(), p.aq_rm.p, p.ad.as<float>(), p.gate.as<float>(), p.up.as<float>(), eb, ffe, ne, T * nu, nullptr, 1,
                                 pre ? l.gate_fold.p : nullptr, pre ? l.up_fold.p : nullptr);
             silu_mul_quant_rm(p.gate.as<float>(), p.up.as<float>(), nullptr, p.aq2.as<int8_t>(), p.ad2.as<float>(), T * nu * ffe, p.aq2_rm.as<int8_t>());
             expert_gemm_scatter(l.down_exps.p, nullptr, p.gstart.as<int32_t>(), p.gcount.as<int32_t>(), p.pslot.as<int32_t>(),
-                                p.pslot.as<int32_t>(), p.aq2_rm.p, p.ad2.as<float>(), p.down.as<float>(), nullptr, ffe / 256, E, ne, nullptr, 1,
+                                p.pslot.as<int32_t>(), p.aq2_rm.p, p.ad2.as<float>(), p.down.as<float>(), nullptr, ffe / 256, E, ne, T * nu, nullptr, 1,
                                 pre ? l.down_fold.p : nullptr, nullptr);
         } else {
             llamd_fwd_expert_major(l.gate_exps.p, l.up_exps.p, p.work.as<int32_t>(), p.n_work.as<int32_t>(), max_items,
@@ -1668,16 +1678,11 @@ static void queue_prefill_tile(Model &m, int T, int n_kv_max, bool last, bool mu
         // the head for every token of the tile: combine + output norm + Q8_K per row, lm_head as a GEMM, greedy pick per row
         combine_rms_norm_quant_wait(WaitPlan{}, x, p.down.as<float>(), p.w.as<float>(), nu, x, m.output_norm.as<float>(), nullptr,
                                          p.aq.as<int8_t>(), p.ad.as<float>(), E, hp.rms_eps, T, 0, p.aq_rm.as<int8_t>());
-        const bool head_folded = folded_tile(m, T) && m.head_gemm && T >= m.head_gemm && m.head_fold_ready;
-        if (small && !head_folded) {
+        if (small && !(m.head_gemm && T >= m.head_gemm))
             matvec_batch(MatvecPlans{}, m.output.p ? m.output.p : m.tok_embd.p, p.aq.as<int8_t>(), p.ad.as<float>(), logits_out, eb, hp.n_vocab, T);
-        } else {
-            if (head_folded)
-                gemm_tokens_folded(m.head_fold.p, p.aq_rm.p, p.ad.as<float>(), logits_out, eb, hp.n_vocab, T);
-            else
-                llamd_fwd_gemm_tokens(m.output.p ? m.output.p : m.tok_embd.p, nullptr, nullptr, p.aq_rm.p, p.ad.as<float>(), logits_out, nullptr,
-                                      nullptr, eb, hp.n_vocab, 0, 0, T);
-        }
+        else
+            llamd_fwd_gemm_tokens(m.output.p ? m.output.p : m.tok_embd.p, nullptr, nullptr, p.aq_rm.p, p.ad.as<float>(), logits_out, nullptr, nullptr,
+                                  eb, hp.n_vocab, 0, 0, T);
         llamd_fwd_argmax(logits_out, hp.n_vocab, p.amax_v.as<float>(), p.amax_i.as<int32_t>(), p.out_tokens.as<int32_t>(), kArgmaxBlocks, T);
         return;
     }
@@ -1746,7 +1751,7 @@ int llamd_model_prefill(llamd_model *h, const int32_t *tokens, int n_tokens, int
             set_error(cudaGetLastError(), "prefill meta H2D");
             return -1;
         }
-        if (folded_tile(*m, T) && !ensure_folded(*m, T, full_tile(*m), false)) return -1;
+        if (folded_tile(*m, T) && !ensure_folded(*m, T, full_tile(*m))) return -1;
         queue_prefill_tile(*m, T, base_pos + t0 + T, t0 + T >= n_tokens);
     }
     if (cudaMemcpyAsync(m->h_out, m->out_token.p, 4, cudaMemcpyDeviceToHost, stream()) != cudaSuccess) return -1;

@@ -66,9 +66,9 @@ static ExpBinderRegistration s_exp_binder_registration;
 
 // ---- Q8_K: crates/llamd-quant/src/dot.rs:88-128 ---------------------------
 // One warp per 256-element block; lane l owns elements 8l..8l+7.
-// Produces qs[256] (natural order), d and optionally bsums[16], and optionally the quants residue-major as well, the GEMMs'
-// operand order: word j of residue r holds elements 32j + 8k + r, so lane l's byte r belongs at 32r + l, and a warp stores
-// eight runs of 32 bytes. (A launch of its own for that order cost 3 to 4 us four times a layer.)
+// Produces qs[256] (natural order), d and optionally bsums[16], and optionally the quants in the GEMMs' operand order as well
+// (t32_place, t32_element in q6k_layout.cuh): lane l holds byte k of word l / 4 of every residue, where k swaps the two bits
+// of l % 4. (A launch of its own for that order cost 3 to 4 us four times a layer.)
 __device__ __forceinline__ void q8k_quantize_block(const float v[8], int lane, int8_t *__restrict__ qs, float *__restrict__ d_out,
                                                    int16_t *__restrict__ bsums, int8_t *__restrict__ rm = nullptr) {
     // the SIGNED value at the largest magnitude, first such element
@@ -114,7 +114,8 @@ __device__ __forceinline__ void q8k_quantize_block(const float v[8], int lane, i
     *reinterpret_cast<uint2 *>(qs + lane * 8) = make_uint2(w0, w1);
     if (rm) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) rm[32 * i + lane] = (int8_t)q[i];
+        for (int i = 0; i < 8; i++)
+            rm[64 * (i >> 1) + 16 * ((lane >> 2) & 3) + 8 * (i & 1) + 4 * (lane >> 4) + 2 * (lane & 1) + ((lane >> 1) & 1)] = (int8_t)q[i];
     }
     if (lane == 0) *d_out = dd;
     if (bsums) {

@@ -16,22 +16,19 @@ __global__ void repack_q6k_kernel(const uint8_t *__restrict__ src, uint8_t *__re
     const size_t unit = dst_first + src_unit;
     const int t = threadIdx.x;
     if (t < 48) {
-        const int r = t / 6, m = (t % 6) / 3, i = t % 3;
+        const int quad = t / 3, i = t % 3;
         uint32_t word = 0;
         for (int k = 0; k < 4; k++) {
-            const uint32_t w4 = ((ggml_q6k_code(blk, t32_element(r, 4 * m + i, k)) ^ 0x20u) << 2) & 0xFFu;
-            const uint32_t w3 = ((ggml_q6k_code(blk, t32_element(r, 4 * m + 3, k)) ^ 0x20u) << 2) & 0xFFu;
+            const uint32_t w4 = ((ggml_q6k_code(blk, t32_element(t32_place_r(4 * quad + i), t32_place_j(4 * quad + i), k)) ^ 0x20u) << 2) & 0xFFu;
+            const uint32_t w3 = ((ggml_q6k_code(blk, t32_element(t32_place_r(4 * quad + 3), t32_place_j(4 * quad + 3), k)) ^ 0x20u) << 2) & 0xFFu;
             const uint32_t byte = (w4 & 0xFCu) | ((w3 >> (6 - 2 * i)) & 3u);
             word |= byte << (8 * k);
         }
         *reinterpret_cast<uint32_t *>(dst + t32_word_offset(unit, t)) = word;
-    } else if (t < 52) {
-        const int q = t - 48;
-        uint32_t word = 0;
-        for (int k = 0; k < 4; k++) word |= (uint32_t)blk[192 + 4 * q + k] << (8 * k);
-        *reinterpret_cast<uint32_t *>(dst + t32_scale_offset(unit) + 4 * q) = word;
-    } else if (t == 52) {
-        *reinterpret_cast<uint16_t *>(dst + t32_d_offset(unit)) = (uint16_t)(blk[208] | (blk[209] << 8));
+    } else {
+        const int g = t - 48;
+        dst[t32_scale_offset(unit, g)] = blk[192 + g];
+        if (g == 0) *reinterpret_cast<uint16_t *>(dst + t32_d_offset(unit)) = (uint16_t)(blk[208] | (blk[209] << 8));
     }
 }
 
@@ -53,7 +50,7 @@ __global__ void unpack_q6k_kernel(const uint8_t *__restrict__ tiled, uint8_t *__
             blk[128 + half * 32 + l] = (uint8_t)((c0 >> 4) | ((c1 >> 4) << 2) | ((c2 >> 4) << 4) | ((c3 >> 4) << 6));
         }
     }
-    for (int i = 0; i < 16; i++) blk[192 + i] = tiled[t32_scale_offset(unit) + i];
+    for (int i = 0; i < 16; i++) blk[192 + i] = tiled[t32_scale_offset(unit, i)];
     blk[208] = tiled[t32_d_offset(unit)];
     blk[209] = tiled[t32_d_offset(unit) + 1];
 }
@@ -67,7 +64,7 @@ __global__ void dequantize_q6k_kernel(const uint8_t *__restrict__ tiled, size_t 
     const size_t unit = first_unit + idx / LLAMD_QK_K;
     const int e = (int)(idx % LLAMD_QK_K);
     const float d = f16_bits_to_f32(*reinterpret_cast<const uint16_t *>(tiled + t32_d_offset(unit)));
-    const float sc = (float)(int8_t)tiled[t32_scale_offset(unit) + (e >> 4)];
+    const float sc = (float)(int8_t)tiled[t32_scale_offset(unit, e >> 4)];
     const float q = (float)t32_weight(tiled, unit, e);
     out[idx] = __fmul_rn(__fmul_rn(d, sc), q);
 }
@@ -86,7 +83,7 @@ __global__ void embed_meta_kernel(const uint8_t *__restrict__ tiled, const int32
     const size_t unit = (size_t)token * blocks + idx / LLAMD_QK_K;
     const int e = idx % LLAMD_QK_K;
     const float d = f16_bits_to_f32(*reinterpret_cast<const uint16_t *>(tiled + t32_d_offset(unit)));
-    const float sc = (float)(int8_t)tiled[t32_scale_offset(unit) + (e >> 4)];
+    const float sc = (float)(int8_t)tiled[t32_scale_offset(unit, e >> 4)];
     const float q = (float)t32_weight(tiled, unit, e);
     out[(size_t)seq * blocks * LLAMD_QK_K + idx] = __fmul_rn(__fmul_rn(d, sc), q);
 }
