@@ -7,13 +7,13 @@
 // cache the tile has already stored into. Nothing is re-associated: each
 // output element is one thread-private accumulator that walks its reduction
 // index in order with an unfused multiply and add. What changes against the
-// per-token kernels is only WHO holds the chains: a thread owns a 4x4 (scores)
+// per-token kernels is only WHO holds the chains: a thread owns an 8x4 (scores)
 // or 4x8 (output) patch of independent chains, so operands fetched from shared
 // memory are reused 4-8 times and the FP32 pipe, not memory, sets the pace.
 //
-//   tile_scores_kernel   S[t][p] = scale * (q_t . k_p)        64 tokens x 64 positions x one head per CTA
+//   tile_scores_kernel   S[t][p] = scale * (q_t . k_p)        64 tokens x 128 positions x one head per CTA
 //   tile_softmax_kernel  W[t][p] = exp(S - max) / sum          one warp per (token, head) row, in place
-//   tile_pv_kernel       out[t][d] = sum_p W[t][p] * v_p[d]    32 tokens x head_dim x one head per CTA
+//   tile_pv_kernel       out[t][d] = sum_p W[t][p] * v_p[d]    16 tokens x head_dim x one head per CTA
 //
 // A weight beyond a token's own position is staged as +0.0, and 0*v added to
 // an accumulator that started at +0.0 leaves it unchanged, so every token's
@@ -35,97 +35,120 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Two chains per instruction (packed_f32.cuh). The FP32 pipe does as many operations a cycle either way, but at two a scalar
-// instruction left no issue slots for the shared-memory loads: us a 512-token piece of a 2000-token prompt, scalar / packed:
-// scores 199 / 181, values 214 / 200.
+// Two chains per instruction (packed_f32.cuh). The FP32 pipe takes two cycles for a packed instruction, as for two scalar ones
+// (2.1 to 2.5 measured, with the operands' registers); what packing saves is issue. Scalar multiplies feeding packed adds, which
+// need no value twice, took as long for the scores and 4 % longer for the values; all scalar 6 and 10 % longer.
 __device__ __forceinline__ f32x2 mul_add2(f32x2 a, f32x2 b, f32x2 s, f32x2 one) { return add2(s, mul2(a, b), one); }  // s + a*b, each rounded
 
-constexpr int kST = 64;  // tokens per CTA of the score kernel
-constexpr int kSP = 64;  // positions per CTA of the score kernel
+constexpr int kST = 64;   // tokens per CTA of the score kernel
+constexpr int kSP = 128;  // positions per CTA of the score kernel
+constexpr int kSC = 32;   // columns of a stage
 
-// grid (position tiles, token tiles, heads), 256 threads.
-// Thread (ty, tx) = (tid / 16, tid % 16) owns tokens 4ty..4ty+3 and positions tx, tx+16, tx+32, tx+48 of the tile:
-// two token pairs, whose queries lie interleaved in shared memory, against four keys.
-__global__ void __launch_bounds__(256) tile_scores_kernel(const float *__restrict__ q, const float *__restrict__ kc, float *__restrict__ scores,
-                                                          int n_head, int n_head_kv, int hd, const int32_t *__restrict__ meta, int max_kv,
-                                                          int ntok, f32x2 one) {
+// grid (position tiles, token tiles, heads), 256 threads. Warp w owns tokens 8w..8w+7 of the tile, its lane l positions 2l, 2l+1,
+// 64+2l, 65+2l: two position pairs, whose keys lie interleaved in shared memory, against eight queries, which lie there with every
+// value twice, so that both operands of a packed instruction are loaded as they are (made twice in registers, a quarter of what
+// the FP32 pipe issued were moves). Bound by that pipe, 79 % busy, 70 % of the load unit. The columns come in stages of 32, two in
+// shared memory and the next on its way in registers: rows of all columns left one warp in four of what fits, and took longer
+// than the moves had. us of the four 512-token pieces of a 1999-token prompt (4x4 patches with moves / this): 56 141 226 309 /
+// 61 140 218 277.
+template <int HD>
+__global__ void __launch_bounds__(256, 2) tile_scores_kernel(const float *__restrict__ q, const float *__restrict__ kc, float *__restrict__ scores,
+                                                             int n_head, int n_head_kv, const int32_t *__restrict__ meta, int max_kv, int ntok,
+                                                             f32x2 one) {
+    constexpr int S = 2 * kSC + 4;  // row stride: 16-byte aligned, neighbouring rows in different bank groups
+    constexpr int C4 = kSC / 4, kStage = (kST + kSP / 2) * S;
     extern __shared__ __align__(16) float sm[];
     __shared__ int s_pos[kST];
     pdl_trigger();
     pdl_wait();
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int p0 = blockIdx.x * kSP, t0 = blockIdx.y * kST, h = blockIdx.z;
     if (tid < kST) s_pos[tid] = (t0 + tid < ntok) ? meta[2 * (t0 + tid) + 1] : -1;
     __syncthreads();
     int maxpos = -1;
     for (int i = 0; i < kST; i++) maxpos = max(maxpos, s_pos[i]);
     if (p0 > maxpos) return;
-    const int S = hd + 4;  // row stride: 16-byte aligned, rows 4 apart fall into different bank groups
-    const int SQ = 2 * hd + 4;  // ... of a token pair: (even, odd) for every column
-    float *sQ = sm, *sK = sm + (kST / 2) * SQ;
-    const int hd4 = hd >> 2, kv_dim = n_head_kv * hd, kvh = h / (n_head / n_head_kv);
-    for (int idx = tid; idx < kST * hd4; idx += 256) {
-        const int r = idx / hd4, c = idx - r * hd4;
-        const int p = p0 + r;
-        cp_async16(sK + r * S + 4 * c, kc + (size_t)min(p, maxpos) * kv_dim + (size_t)kvh * hd + 4 * c, p <= maxpos ? 16 : 0);
+    int wpos = -1;  // the last position of this warp's tokens: in front of the tile (or no tokens left), it only brings its share
+    for (int i = 0; i < 8; i++) wpos = max(wpos, s_pos[8 * warp + i]);
+    const int kv_dim = n_head_kv * HD;
+    // What this thread brings of a stage: rows tid / 8 and 32 further of the position pairs, the same rows of the queries, four
+    // columns of each. (A position past the last scores like the last one, a token past the end likewise; neither is stored.)
+    const int r = tid / C4, c = tid % C4;
+    const float *kh = kc + (size_t)(h / (n_head / n_head_kv)) * HD + 4 * c, *qh = q + (size_t)h * HD + 4 * c;
+    const float *src[6];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int p = p0 + 2 * (r + 32 * u);
+        src[3 * u] = kh + (size_t)min(p, maxpos) * kv_dim;
+        src[3 * u + 1] = kh + (size_t)min(p + 1, maxpos) * kv_dim;
+        src[3 * u + 2] = qh + (size_t)min(t0 + r + 32 * u, ntok - 1) * n_head * HD;
     }
-    cp_async_commit();
-    for (int idx = tid; idx < (kST / 2) * hd4; idx += 256) {
-        const int r = idx / hd4, c = idx - r * hd4, t = t0 + 2 * r;
-        const float4 *q0 = reinterpret_cast<const float4 *>(q + ((size_t)min(t, ntok - 1) * n_head + h) * hd) + c;
-        const float4 *q1 = reinterpret_cast<const float4 *>(q + ((size_t)min(t + 1, ntok - 1) * n_head + h) * hd) + c;
-        const float4 a = *q0, b = *q1;  // (a token past the end scores like the last one; its rows are not stored)
-        float4 *d = reinterpret_cast<float4 *>(sQ + r * SQ + 8 * c);
-        d[0] = make_float4(a.x, b.x, a.y, b.y);
-        d[1] = make_float4(a.z, b.z, a.w, b.w);
-    }
-    cp_async_wait<0>();
-    __syncthreads();
-    f32x2 acc[2][4];
+    float4 in[6];
+    auto load = [&](int s) {
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+        for (int u = 0; u < 6; u++) in[u] = *reinterpret_cast<const float4 *>(src[u] + s * kSC);
+    };
+    auto store = [&](int s) {
+        float *sQ = sm + (s & 1) * kStage, *sK = sQ + kST * S;
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0ull;
-    const float *qb = sQ + (ty * 2) * SQ, *kb = sK + tx * S;
-#pragma unroll 2
-    for (int d4 = 0; d4 < hd4; d4++) {
-        ulonglong2 a[2][2];
-        float4 b[4];
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-            a[i][0] = *reinterpret_cast<const ulonglong2 *>(qb + i * SQ + 8 * d4);
-            a[i][1] = *reinterpret_cast<const ulonglong2 *>(qb + i * SQ + 8 * d4 + 4);
+        for (int u = 0; u < 2; u++) {
+            const float4 a = in[3 * u], b = in[3 * u + 1], x = in[3 * u + 2];
+            float4 *k = reinterpret_cast<float4 *>(sK + (r + 32 * u) * S + 8 * c), *d = reinterpret_cast<float4 *>(sQ + (r + 32 * u) * S + 8 * c);
+            k[0] = make_float4(a.x, b.x, a.y, b.y);
+            k[1] = make_float4(a.z, b.z, a.w, b.w);
+            d[0] = make_float4(x.x, x.x, x.y, x.y);
+            d[1] = make_float4(x.z, x.z, x.w, x.w);
         }
+    };
+    f32x2 acc[8][2];
 #pragma unroll
-        for (int j = 0; j < 4; j++) b[j] = *reinterpret_cast<const float4 *>(kb + j * 16 * S + 4 * d4);
+    for (int i = 0; i < 8; i++) acc[i][0] = acc[i][1] = 0ull;
+    load(0);
+    store(0);
+    __syncthreads();
+#pragma unroll 1
+    for (int s = 0; s < HD / kSC; s++) {
+        if (s + 1 < HD / kSC) load(s + 1);
+        const float *qb = sm + (s & 1) * kStage + (warp * 8) * S, *kb = sm + (s & 1) * kStage + (kST + lane) * S;
+        if (p0 <= wpos) {
+#pragma unroll 4
+            for (int d2 = 0; d2 < kSC / 2; d2++) {  // two columns at a time
+                ulonglong2 b[2];
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
+                for (int j = 0; j < 2; j++) b[j] = *reinterpret_cast<const ulonglong2 *>(kb + j * 32 * S + 4 * d2);
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const float k = c == 0 ? b[j].x : c == 1 ? b[j].y : c == 2 ? b[j].z : b[j].w;
-                const f32x2 kk = pack2(k, k);
+                for (int i = 0; i < 8; i++) {
+                    const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(qb + i * S + 4 * d2);
 #pragma unroll
-                for (int i = 0; i < 2; i++) acc[i][j] = mul_add2(c & 1 ? a[i][c >> 1].y : a[i][c >> 1].x, kk, acc[i][j], one);
+                    for (int j = 0; j < 2; j++) acc[i][j] = mul_add2(a.y, b[j].y, mul_add2(a.x, b[j].x, acc[i][j], one), one);
+                }
             }
         }
+        if (s + 1 < HD / kSC) {
+            store(s + 1);  // (the last readers of these rows passed the barrier in front of this stage)
+            __syncthreads();
+        }
     }
-    const float scale = __fdiv_rn(1.0f, __fsqrt_rn((float)hd));
+    const float scale = __fdiv_rn(1.0f, __fsqrt_rn((float)HD));
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int t = t0 + ty * 4 + i, pos = s_pos[ty * 4 + i];
+    for (int i = 0; i < 8; i++) {
+        const int t = t0 + warp * 8 + i, pos = s_pos[warp * 8 + i];
         float *row = scores + ((size_t)t * n_head + h) * max_kv;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int p = p0 + j * 16 + tx;
-            const float2 v = unpack2(acc[i >> 1][j]);
-            if (p <= pos) row[p] = __fmul_rn(i & 1 ? v.y : v.x, scale);
+        for (int j = 0; j < 2; j++) {
+            const int p = p0 + 64 * j + 2 * lane;
+            const float2 v = unpack2(acc[i][j]), l = make_float2(__fmul_rn(v.x, scale), __fmul_rn(v.y, scale));
+            if (p < pos) *reinterpret_cast<float2 *>(row + p) = l;
+            else if (p == pos) row[p] = l.x;
         }
     }
 }
 
 // One warp per (token, head) row: the logits become the softmax weights e*inv in place. The rows' sums are walked side by
-// side by the first warp, a lane per row (a warp per chain is one lane's adds at a whole warp's issue; the kernel is bound by
-// issue, most of it the exponentials): with a warp per chain a prompt of 1999 tokens took 0.5 % longer.
+// side by the first warp, a lane per row (a warp per chain is one lane's adds at a whole warp's issue): with a warp per chain a
+// prompt of 1999 tokens took 0.5 % longer. Bound by the issue of the exponentials and by latency (three CTAs of rows fill the shared
+// memory): four positions a lane at a time instead of one, with the shorter exponential, took the four
+// pieces of a 1999-token prompt from 35 65 98 140 to 28 50 75 102 us.
 // Dynamic shared memory: [warps][n_cap] floats, n_cap = 4 mod 32 (the lanes' 16-byte reads meet different banks).
 __global__ void tile_softmax_kernel(float *__restrict__ scores, const int32_t *__restrict__ meta, int n_head, int max_kv, int ntok, int n_cap) {
     extern __shared__ __align__(16) float sm[];
@@ -137,14 +160,23 @@ __global__ void tile_softmax_kernel(float *__restrict__ scores, const int32_t *_
     const int n = row < rows ? min(meta[2 * (row / n_head) + 1] + 1, n_cap) : 0;
     float *sl = sm + (size_t)warp * n_cap;
     float *g = scores + (size_t)row * max_kv;
+    // (four positions a lane at a time; rows are whole 16-byte pieces, and what lies beyond the row's positions counts for nothing)
     float lmax = -INFINITY;
-    for (int p = lane; p < n; p += 32) {
-        const float l = g[p];
-        sl[p] = l;
-        lmax = fmaxf(lmax, l);
+    for (int p = 4 * lane; p < n; p += 128) {
+        float4 l = *reinterpret_cast<const float4 *>(g + p);
+        if (p + 1 >= n) l.y = -INFINITY;
+        if (p + 2 >= n) l.z = -INFINITY;
+        if (p + 3 >= n) l.w = -INFINITY;
+        *reinterpret_cast<float4 *>(sl + p) = l;
+        lmax = fmaxf(fmaxf(fmaxf(l.x, l.y), fmaxf(l.z, l.w)), lmax);
     }
     for (int off = 16; off > 0; off >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, off));
-    for (int p = lane; p < n; p += 32) sl[p] = ref_expf(__fsub_rn(sl[p], lmax));
+    for (int p = 4 * lane; p < n; p += 128) {
+        float4 *l = reinterpret_cast<float4 *>(sl + p);
+        float e[4] = {l->x, l->y, l->z, l->w};
+        ref_expf4(e, lmax);
+        *l = make_float4(e[0], e[1], e[2], e[3]);
+    }
     __syncthreads();
     if (warp == 0 && lane < warps) {
         const int r = blockIdx.x * warps + lane;
@@ -152,95 +184,87 @@ __global__ void tile_softmax_kernel(float *__restrict__ scores, const int32_t *_
     }
     __syncthreads();
     const float inv = s_inv[warp];
-    for (int p = lane; p < n; p += 32) g[p] = __fmul_rn(sl[p], inv);
+    for (int p = 4 * lane; p < n; p += 128) {
+        const float4 e = *reinterpret_cast<const float4 *>(sl + p);
+        *reinterpret_cast<float4 *>(g + p) = make_float4(__fmul_rn(e.x, inv), __fmul_rn(e.y, inv), __fmul_rn(e.z, inv), __fmul_rn(e.w, inv));
+    }
 }
 
-constexpr int kOT = 32;  // tokens per CTA of the output kernel
-constexpr int kOP = 32;  // positions per staged tile
+constexpr int kOT = 16;  // tokens per CTA of the output kernel
+constexpr int kOP = 16;  // positions per staged tile
 constexpr int kWS = kOP + 4;
 
-// grid (token tiles, heads), 128 threads. Thread (ty, tx) = (tid / 16, tid % 16) owns tokens 4ty..4ty+3 and the
-// output columns 64g + 4tx .. +3 for g < HD/64.
+// grid (heads, token tiles), HD threads. Thread (ty, tx) = (tid / (HD/4), tid % (HD/4)) owns tokens 4ty..4ty+3 and the output
+// columns 4tx..4tx+3. Bound by the FP32 pipe, 82 % busy while a CTA is there. A CTA is one warp per scheduler and 16 tokens: the
+// 1024 CTAs of a 512-token piece are seven to an SM, all at once, and 99 % of that many; with two warps to a CTA a scheduler
+// got three or four of them, with 32 tokens an SM three or four CTAs, and the others waited a fifth of the time. The longest tokens
+// of all heads start first. us of the four pieces of a 1999-token prompt (32 tokens, 4x8 patches / this): 72 161 251 332 /
+// 54 136 218 289.
 template <int HD>
-__global__ void __launch_bounds__(128) tile_pv_kernel(const float *__restrict__ w, const float *__restrict__ vc, float *__restrict__ out, int n_head,
-                                                      int n_head_kv, const int32_t *__restrict__ meta, int max_kv, int ntok, f32x2 one) {
-    constexpr int G = HD / 64, HD4 = HD / 4;
-    __shared__ __align__(16) float sW[2][kOT][kWS];
-    __shared__ __align__(16) float sV[2][kOP][HD];
+__global__ void __launch_bounds__(HD) tile_pv_kernel(const float *__restrict__ w, const float *__restrict__ vc, float *__restrict__ out, int n_head,
+                                                     int n_head_kv, const int32_t *__restrict__ meta, int max_kv, int ntok, f32x2 one) {
+    constexpr int HD4 = HD / 4;
+    __shared__ __align__(16) float sW[3][kOT][kWS];
+    __shared__ __align__(16) float sV[3][kOP][HD];
     __shared__ int s_pos[kOT];
     pdl_trigger();
     pdl_wait();
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-    const int t0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kOT, h = blockIdx.y;  // the longest tiles start first
+    const int tid = threadIdx.x, ty = tid / HD4, tx = tid % HD4;
+    const int t0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kOT, h = blockIdx.x;  // the longest tiles start first
     if (tid < kOT) s_pos[tid] = (t0 + tid < ntok) ? meta[2 * (t0 + tid) + 1] : -1;
     __syncthreads();
     int maxpos = -1;
     for (int i = 0; i < kOT; i++) maxpos = max(maxpos, s_pos[i]);
     const int kv_dim = n_head_kv * HD, kvh = h / (n_head / n_head_kv);
-    const float *vb = vc + (size_t)kvh * HD;
+    const float *vb = vc + (size_t)kvh * HD + 4 * tx;
+    const int wr = (tid >> 2) % kOT, wp = 4 * (tid & 3), wpos = s_pos[wr];  // four weights of a stage: token wr, positions wp..
+    const float *wrow = w + ((size_t)min(t0 + wr, ntok - 1) * n_head + h) * max_kv + wp;
     auto stage = [&](int pt, int buf) {
-        for (int idx = tid; idx < kOT * (kOP / 4); idx += 128) {
-            const int r = idx / (kOP / 4), c = idx - r * (kOP / 4);
-            const int p = pt * kOP + 4 * c;
-            const int valid = max(0, min(4, s_pos[r] - p + 1));
-            const float *src = valid ? w + ((size_t)(t0 + r) * n_head + h) * max_kv + p : w;
-            cp_async16(&sW[buf][r][4 * c], src, 4 * valid);
+        if (tid < 4 * kOT) {
+            const int valid = max(0, min(4, wpos - (pt * kOP + wp) + 1));
+            cp_async16(&sW[buf][wr][wp], valid ? wrow + pt * kOP : w, 4 * valid);
         }
-        for (int idx = tid; idx < kOP * HD4; idx += 128) {
-            const int r = idx / HD4, c = idx - r * HD4;
-            const int p = pt * kOP + r;
-            cp_async16(&sV[buf][r][4 * c], vb + (size_t)min(p, maxpos) * kv_dim + 4 * c, p <= maxpos ? 16 : 0);
+#pragma unroll
+        for (int u = 0; u < kOP / 4; u++) {
+            const int r = ty + 4 * u, p = pt * kOP + r;
+            cp_async16(&sV[buf][r][4 * tx], vb + (size_t)min(p, maxpos) * kv_dim, p <= maxpos ? 16 : 0);
         }
-        cp_async_commit();
     };
-    f32x2 acc[4][G * 2];
+    f32x2 acc[4][2];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int c = 0; c < G * 2; c++) acc[i][c] = 0ull;
+    for (int i = 0; i < 4; i++) acc[i][0] = acc[i][1] = 0ull;
     const int n_pt = maxpos / kOP + 1;  // maxpos >= 0: the tile holds at least one token
     stage(0, 0);
-    for (int pt = 0; pt < n_pt; pt++) {
-        const int buf = pt & 1;
-        if (pt + 1 < n_pt) {
-            stage(pt + 1, buf ^ 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-#pragma unroll 2
+    cp_async_commit();
+    if (n_pt > 1) stage(1, 1);
+    cp_async_commit();
+    for (int pt = 0, buf = 0; pt < n_pt; pt++, buf = buf == 2 ? 0 : buf + 1) {
+        cp_async_wait<1>();
+        __syncthreads();  // stage pt is there, and everyone is done with stage pt - 1, whose place stage pt + 2 takes
+        if (pt + 2 < n_pt) stage(pt + 2, buf == 0 ? 2 : buf - 1);
+        cp_async_commit();
+#pragma unroll
         for (int p4 = 0; p4 < kOP / 4; p4++) {
             float4 wv[4];
 #pragma unroll
             for (int i = 0; i < 4; i++) wv[i] = *reinterpret_cast<const float4 *>(&sW[buf][ty * 4 + i][4 * p4]);
 #pragma unroll
             for (int c = 0; c < 4; c++) {
-                ulonglong2 v[G];
-#pragma unroll
-                for (int g = 0; g < G; g++) v[g] = *reinterpret_cast<const ulonglong2 *>(&sV[buf][4 * p4 + c][64 * g + 4 * tx]);
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(&sV[buf][4 * p4 + c][4 * tx]);
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     const float wi = c == 0 ? wv[i].x : c == 1 ? wv[i].y : c == 2 ? wv[i].z : wv[i].w;
                     const f32x2 ww = pack2(wi, wi);
-#pragma unroll
-                    for (int g = 0; g < G; g++) {
-                        acc[i][2 * g] = mul_add2(ww, v[g].x, acc[i][2 * g], one);
-                        acc[i][2 * g + 1] = mul_add2(ww, v[g].y, acc[i][2 * g + 1], one);
-                    }
+                    acc[i][0] = mul_add2(ww, v.x, acc[i][0], one);
+                    acc[i][1] = mul_add2(ww, v.y, acc[i][1], one);
                 }
             }
         }
-        __syncthreads();
     }
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int t = t0 + ty * 4 + i;
-        if (t < ntok) {
-#pragma unroll
-            for (int g = 0; g < G; g++)
-                *reinterpret_cast<ulonglong2 *>(out + ((size_t)t * n_head + h) * HD + 64 * g + 4 * tx) = make_ulonglong2(acc[i][2 * g], acc[i][2 * g + 1]);
-        }
+        if (t < ntok) *reinterpret_cast<ulonglong2 *>(out + ((size_t)t * n_head + h) * HD + 4 * tx) = make_ulonglong2(acc[i][0], acc[i][1]);
     }
 }
 
@@ -264,14 +288,13 @@ void llamd_fwd_attention_prefill(const float *q, const float *kc, const float *v
         llamd_fwd_attention_tile(q, kc, vc, out, scores, n_head, n_head_kv, hd, meta, max_kv, ntok);
         return;
     }
-    const size_t smem_s = (size_t)(kST / 2 * (2 * hd + 4) + kSP * (hd + 4)) * sizeof(float);
-    static size_t conf_s = 0;
-    if (smem_s > 48 * 1024 && smem_s > conf_s) {
-        cudaFuncSetAttribute(tile_scores_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_s);
-        conf_s = smem_s;
-    }
-    launch_k("tile_scores", tile_scores_kernel, dim3((n_kv_max + kSP - 1) / kSP, (ntok + kST - 1) / kST, n_head), dim3(256), smem_s, q, kc, scores,
-             n_head, n_head_kv, hd, meta, max_kv, ntok, kOne2);
+    constexpr size_t smem_s = 2 * (kST + kSP / 2) * (2 * kSC + 4) * sizeof(float);
+    static bool conf_s = false;
+    if (!conf_s)
+        conf_s = cudaFuncSetAttribute(tile_scores_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_s) == cudaSuccess &&
+                 cudaFuncSetAttribute(tile_scores_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_s) == cudaSuccess;
+    launch_k("tile_scores", hd == 64 ? tile_scores_kernel<64> : tile_scores_kernel<128>, dim3((n_kv_max + kSP - 1) / kSP, (ntok + kST - 1) / kST, n_head),
+             dim3(256), smem_s, q, kc, scores, n_head, n_head_kv, meta, max_kv, ntok, kOne2);
     int warps = (int)((200 * 1024) / ((size_t)n_cap * 4));
     warps = warps > 8 ? 8 : warps;
     const size_t smem_m = (size_t)warps * n_cap * sizeof(float);
@@ -282,10 +305,10 @@ void llamd_fwd_attention_prefill(const float *q, const float *kc, const float *v
     }
     const int rows = ntok * n_head;
     launch_k("tile_softmax", tile_softmax_kernel, dim3((rows + warps - 1) / warps), dim3(32 * warps), smem_m, scores, meta, n_head, max_kv, ntok, n_cap);
-    const dim3 grid((ntok + kOT - 1) / kOT, n_head);
+    const dim3 grid(n_head, (ntok + kOT - 1) / kOT);
     if (hd == 64)
-        launch_k("tile_pv", tile_pv_kernel<64>, grid, dim3(128), 0, (const float *)scores, vc, out, n_head, n_head_kv, meta, max_kv, ntok, kOne2);
+        launch_k("tile_pv", tile_pv_kernel<64>, grid, dim3(hd), 0, (const float *)scores, vc, out, n_head, n_head_kv, meta, max_kv, ntok, kOne2);
     else
-        launch_k("tile_pv", tile_pv_kernel<128>, grid, dim3(128), 0, (const float *)scores, vc, out, n_head, n_head_kv, meta, max_kv, ntok, kOne2);
+        launch_k("tile_pv", tile_pv_kernel<128>, grid, dim3(hd), 0, (const float *)scores, vc, out, n_head, n_head_kv, meta, max_kv, ntok, kOne2);
 }
 }

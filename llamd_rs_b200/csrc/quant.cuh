@@ -30,24 +30,66 @@ __device__ __forceinline__ bool exp_needs_lookup(float x, double yd, uint32_t wi
     return frac - (0x10000000u - window) < 2u * window;  // |frac - 2^28| < window
 }
 
-__device__ __forceinline__ float ref_expf(float x) {
-    const double yd = exp((double)x);
-    float y = __double2float_rn(yd);
+// e^x in double for a float x: x = k ln2 + r with k = round(x / ln2), taken by the rounding of an addition, ln2 in two parts
+// (Cody and Waite), for e^r the polynomial of degree 10 that equals it at the eleven Chebyshev nodes of |r| <= ln2 / 2 (relative
+// error 3.3e-16, a unit in the last place of a double), and k into the exponent. Half the instructions of CUDA's exp((double)x).
+// The result is rounded to f32 behind it, and the table below is made with this very function. Inputs whose float result is 0 or
+// infinite are cut to where it still is; a NaN comes out as one.
+__device__ __forceinline__ double exp_f64(float x) {
+    x = x < -110.0f ? -110.0f : x > 100.0f ? 100.0f : x;
+    const double xd = (double)x, shift = 6755399441055744.0;  // 1.5 * 2^52: the sum's last place is 1
+    const double t = __fma_rn(xd, 1.4426950408889634, shift), k = __dsub_rn(t, shift);
+    const double r = __fma_rn(k, -5.497923018708371e-14, __fma_rn(k, -0.6931471805598903, xd));  // (the first part has 42 bits: k times it is exact)
+    double p = __fma_rn(r, 2.762635725527078e-07, 2.7640180812804505e-06);
+    p = __fma_rn(p, r, 2.480150434696448e-05);
+    p = __fma_rn(p, r, 0.00019841170270400204);
+    p = __fma_rn(p, r, 0.0013888888932488625);
+    p = __fma_rn(p, r, 0.008333333385667814);
+    p = __fma_rn(p, r, 0.04166666666657314);
+    p = __fma_rn(p, r, 0.16666666666554406);
+    p = __fma_rn(p, r, 0.5000000000000006);
+    p = __fma_rn(p, r, 1.0000000000000067);
+    p = __fma_rn(p, r, 1.0);
+    return __hiloint2double(__double2hiint(p) + (__double2loint(t) << 20), __double2loint(p));
+}
+
+__device__ __forceinline__ float exp_exception(float x, float y) {  // the listed result for x, or y
     const uint32_t *keys = c_exp_keys;
-    if (keys && exp_needs_lookup(x, yd, c_exp_window)) {
-        const uint32_t b = __float_as_uint(x), mask = c_exp_mask;
-        uint32_t h = (b * 2654435761u) >> 8 & mask;
-        for (int probe = 0; probe < 64; probe++) {  // (a table at most a quarter full: runs are short)
-            const uint32_t k = __ldg(keys + h);
-            if (k == 0) break;
-            if (k == b) {
-                y = __uint_as_float(__ldg(c_exp_vals + h));
-                break;
-            }
-            h = (h + 1) & mask;
-        }
+    const uint32_t b = __float_as_uint(x), mask = c_exp_mask;
+    uint32_t h = (b * 2654435761u) >> 8 & mask;
+    for (int probe = 0; probe < 64; probe++) {  // (a table at most a quarter full: runs are short)
+        const uint32_t k = __ldg(keys + h);
+        if (k == 0) break;
+        if (k == b) return __uint_as_float(__ldg(c_exp_vals + h));
+        h = (h + 1) & mask;
     }
     return y;
+}
+
+__device__ __forceinline__ float ref_expf(float x) {
+    const double yd = exp_f64(x);
+    const float y = __double2float_rn(yd);
+    return c_exp_keys && exp_needs_lookup(x, yd, c_exp_window) ? exp_exception(x, y) : y;
+}
+
+// v[i] = ref_expf(v[i] - m): four side by side, and one branch for all of their exceptions
+__device__ __forceinline__ void ref_expf4(float v[4], float m) {
+    float y[4];
+    bool look[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        v[i] = __fsub_rn(v[i], m);
+        const double yd = exp_f64(v[i]);
+        y[i] = __double2float_rn(yd);
+        look[i] = exp_needs_lookup(v[i], yd, c_exp_window);
+    }
+    if (c_exp_keys && (look[0] || look[1] || look[2] || look[3])) {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (look[i]) y[i] = exp_exception(v[i], y[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] = y[i];
 }
 
 void register_exp_binder(void (*bind)(const uint32_t *, const uint32_t *, uint32_t, uint32_t));

@@ -41,10 +41,10 @@ static uint32_t *g_exp_keys_dev = nullptr, *g_exp_vals_dev = nullptr;
 static long long g_exp_exceptions = -1;  // -1: no table (switched off, or it could not be built)
 static uint32_t g_exp_window = 0;        // the look-up window in use (0: every input is looked up)
 
-// out[i] = bits of (float)exp((double)x) for the float whose bits are first + i: the expression of ref_expf
+// out[i] = bits of (float)exp_f64(x) for the float whose bits are first + i: the expression of ref_expf
 __global__ void exp_scan_kernel(uint32_t first, uint32_t n, uint32_t *__restrict__ out) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        out[i] = __float_as_uint(__double2float_rn(exp((double)__uint_as_float(first + i))));
+        out[i] = __float_as_uint(__double2float_rn(exp_f64(__uint_as_float(first + i))));
 }
 
 // dist[i] = how far (in units of 2^-29 ulp) the double result for input bits in[i] lies from the midpoint of two
@@ -52,7 +52,7 @@ __global__ void exp_scan_kernel(uint32_t first, uint32_t n, uint32_t *__restrict
 __global__ void exp_window_kernel(const uint32_t *__restrict__ in, uint32_t n, uint32_t *__restrict__ dist) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float x = __uint_as_float(in[i]);
-        const uint32_t frac = (uint32_t)__double_as_longlong(exp((double)x)) & 0x1FFFFFFFu;
+        const uint32_t frac = (uint32_t)__double_as_longlong(exp_f64(x)) & 0x1FFFFFFFu;
         dist[i] = x < -87.0f ? 0u : (frac >= 0x10000000u ? frac - 0x10000000u : 0x10000000u - frac);
     }
 }
