@@ -28,6 +28,10 @@ namespace llamd {
 constexpr int kThreads = 256;
 constexpr int kActBlockWords = 132;  // 128 + 4 padding words: conflict-free 16-byte reads across blocks
 constexpr int kExStride = 257;
+// Rows of up to this many blocks are added up by one thread each: an odd stride, and a fifth of the instructions of a thread per
+// residue and eight shuffles. 64 slots of 2048 x 768, us: 19.7 / 16.5. (Eight blocks are 64 loads one after the other, with
+// eight rows in one bank: 35 / 46.)
+constexpr int kSerialTail = 3;
 
 struct MatvecJob {
     const uint8_t *w;  // tiled Q6_K
@@ -41,6 +45,7 @@ struct MatvecParams {
     int njobs;
     int ctas_per_slot;     // sum over jobs of ceil(rows / rows_per_cta)
     int nb;                // blocks per row
+    unsigned nb_inv;       // ceil(65536 / nb): x * nb_inv >> 16 is x / nb for x < 256 (a division in front of the loads is 0.05 us)
     int rows_per_cta;
     const int32_t *ids;    // [n_slots] expert ids, or null (ungrouped)
     int n_slots;           // 1 when ids is null; nseq*n_used for a batched grouped launch
@@ -103,6 +108,26 @@ __device__ __forceinline__ void peer_arrive(const PeerOutPlan &peer, unsigned in
     }
 }
 
+// The word pairs of word j = i / 4 in residues 2(i % 4) and the next of a block's activation image: residue r's pair is the bytes
+// r and 8+r of the block's bytes 32j..32j+15, and the same of the sixteen behind. l2: the bytes were written by peers. Every
+// thread makes two pairs from four words of global memory; through a copy in shared memory, byte by byte, it was three times
+// the instructions and a barrier more, which a launch of one wave waits for and three CTAs to an SM do not hide: 1 / 8 / 16
+// sequences' gate and up (8 slots each of 2 x 768 x 2048) 6.9 35.2 64.8 us before, 6.5 32.7 60.4 now. (A whole word
+// column per thread, two warps of eight at work, was slower than either.)
+template <bool EP>
+__device__ __forceinline__ void act_image_pair(const int8_t *block, uint32_t *image, int i, bool l2) {
+    const int j = i >> 2, r = 2 * (i & 3);
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(block) + 8 * j + (r >> 2);
+    uint32_t v[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) v[k] = EP && l2 ? __ldcg(src + 2 * k) : __ldg(src + 2 * k);
+    const uint32_t t = r & 2, even = t | (4 + t) << 8;  // bytes t of both operands, two bytes apart
+    uint32_t *dst = image + t32_place(r, j) * 2;
+    *reinterpret_cast<uint2 *>(dst) = make_uint2(__byte_perm(v[0], v[1], even) & 0x00FF00FFu, __byte_perm(v[2], v[3], even << 4) & 0xFF00FF00u);
+    *reinterpret_cast<uint2 *>(dst + 4) =
+        make_uint2(__byte_perm(v[0], v[1], even + 0x101u) & 0x00FF00FFu, __byte_perm(v[2], v[3], (even + 0x101u) << 4) & 0xFF00FF00u);
+}
+
 // EP: the expert-parallel forms (requests pushed by peers, rows stored to peers); kept out of the other instantiations.
 // EXTRA: the optional L2 prefetch plan and the SiLU tail. Both are off by default, and their code in the plain kernel
 // cost every launch ~0.3 us and lm_head 3 % of its bandwidth, so they too are an instantiation of their own.
@@ -132,7 +157,7 @@ __global__ void __launch_bounds__(kThreads, NSEQ == 1 ? 3 : (NSEQ == 2 ? 2 : 1))
     const int rows_here = min(p.rows_per_cta, job.rows - row0);
     const int tid = threadIdx.x;
     const bool active = tid < rows_here * nb;
-    const int row_l = tid / nb, b = tid - row_l * nb;
+    const int row_l = (int)((unsigned)tid * p.nb_inv >> 16), b = tid - row_l * nb;  // tid / nb
     // ungrouped launches may be cut into groups of NSEQ sequences, one "slot" per group (small matrices at batch > 1:
     // more CTAs for the same rows; the weights are re-read from L2)
     const int seq0 = (!MULTI && !p.ids) ? slot * NSEQ : 0;
@@ -221,16 +246,14 @@ __global__ void __launch_bounds__(kThreads, NSEQ == 1 ? 3 : (NSEQ == 2 ? 2 : 1))
         pdl_wait();  // the activations come from the launch in front
     }
     // ---- stage the activations ----------------------------------------
-    // natural order bytes first ...
+    // the image of word pairs from the Q8_K activations in global memory; where they are made here, natural order bytes first ...
     if (ACT == ACT_Q8K) {
         // (the block scales are read where they are used, straight from global memory: staging them here put a second
         // dependent round trip in front of the barrier and cost every launch ~0.4 us)
-        const int n16 = NSEQ * nb * 16;
-        for (int i = tid; i < n16; i += kThreads) {
-            const int s = i / (nb * 16), o = i - s * nb * 16;
+        for (int i = tid; i < NSEQ * nb * 32; i += kThreads) {
+            const int sb = i >> 5, s = NSEQ == 1 ? 0 : sb / nb;
             const long long a_idx = MULTI ? s_aidx[s] : (p.ids ? slot / p.act_div : seq0 + s);
-            const uint4 *src = reinterpret_cast<const uint4 *>(p.aq + a_idx * nb * 256) + o;
-            reinterpret_cast<uint4 *>(s_nat)[i] = (EP && p.dwait.counter) ? __ldcg(src) : __ldg(src);  // written by peers: from L2
+            act_image_pair<EP>(p.aq + (a_idx * nb + (sb - s * nb)) * 256, s_act + sb * kActBlockWords, i & 31, EP && p.dwait.counter);
         }
     } else if (ACT == ACT_NORM) {
         // ... made here from the residual stream: combine, norm (its sum of squares walked in order by one thread), weight,
@@ -325,9 +348,9 @@ __global__ void __launch_bounds__(kThreads, NSEQ == 1 ? 3 : (NSEQ == 2 ? 2 : 1))
             q8k_quantize_block(v, lane, s_nat + blk * 256, s_ad + blk, nullptr);
         }
     }
-    __syncthreads();
+    if (ACT != ACT_Q8K) __syncthreads();
     // ... then the image of word pairs
-    {
+    if (ACT != ACT_Q8K) {
         const int nitems = NSEQ * nb * 64;  // (s, b, r, j)
         for (int i = tid; i < nitems; i += kThreads) {
             const int jj = i & 7, r = (i >> 3) & 7, sb = i >> 6;
@@ -396,31 +419,46 @@ __global__ void __launch_bounds__(kThreads, NSEQ == 1 ? 3 : (NSEQ == 2 ? 2 : 1))
 
     // ---- ordered f32 tail ---------------------------------------------------
     // thread (row_l, r) adds the blocks in order; then the eight residues are
-    // added in order across the 8 adjacent lanes.
-    const int n_out = rows_here * 8;
-    for (int base = 0; base < n_out; base += kThreads) {
-        const int idx = base + tid;
-        const bool on = idx < n_out;
-        const int rl = idx >> 3, r = idx & 7;
+    // added in order across the 8 adjacent lanes. Short rows: one thread a row.
+    auto store = [&](int s, int rl, float total) {
+        // ungrouped: out[seq][rows]; grouped: out[slot][rows]
+        if (MULTI) {
+            if (s < count) job.out[(long long)s_oidx[s] * job.rows + row0 + rl] = total;
+        } else if (EP && p.peer.out_tab) {  // (grouped launches run one sequence per slot: s == 0)
+            p.peer.out_tab[slot / p.peer.div][(size_t)(slot % p.peer.div) * job.rows + row0 + rl] = total;
+        } else {
+            job.out[((long long)s + (p.ids ? slot : seq0)) * job.rows + row0 + rl] = total;
+        }
+    };
+    if (NSEQ == 1 && nb <= kSerialTail) {
+        if (tid < rows_here) {
+            const float *ex = s_ex + tid * nb;
+            float acc[8] = {};
+            for (int bb = 0; bb < nb; bb++)
 #pragma unroll
-        for (int s = 0; s < NSEQ; s++) {
-            float acc = 0.0f;
-            if (on) {
-                const float *ex = s_ex + (s * 8 + r) * kExStride + rl * nb;
-                for (int bb = 0; bb < nb; bb++) acc = __fadd_rn(acc, ex[bb]);
-            }
-            const int lane0 = (tid & 31) & ~7;
-            float total = __shfl_sync(0xffffffffu, acc, lane0);
+                for (int r = 0; r < 8; r++) acc[r] = __fadd_rn(acc[r], ex[r * kExStride + bb]);
 #pragma unroll
-            for (int rr = 1; rr < 8; rr++) total = __fadd_rn(total, __shfl_sync(0xffffffffu, acc, lane0 + rr));
-            // ungrouped: out[seq][rows]; grouped: out[slot][rows]
-            if (MULTI) {
-                if (on && r == 0 && s < count) job.out[(long long)s_oidx[s] * job.rows + row0 + rl] = total;
-            } else if (on && r == 0) {
-                if (EP && p.peer.out_tab)  // (grouped launches run one sequence per slot: s == 0)
-                    p.peer.out_tab[slot / p.peer.div][(size_t)(slot % p.peer.div) * job.rows + row0 + rl] = total;
-                else
-                    job.out[((long long)s + (p.ids ? slot : seq0)) * job.rows + row0 + rl] = total;
+            for (int r = 1; r < 8; r++) acc[0] = __fadd_rn(acc[0], acc[r]);
+            store(0, tid, acc[0]);
+        }
+    } else {
+        const int n_out = rows_here * 8;
+        for (int base = 0; base < n_out; base += kThreads) {
+            const int idx = base + tid;
+            const bool on = idx < n_out;
+            const int rl = idx >> 3, r = idx & 7;
+#pragma unroll
+            for (int s = 0; s < NSEQ; s++) {
+                float acc = 0.0f;
+                if (on) {
+                    const float *ex = s_ex + (s * 8 + r) * kExStride + rl * nb;
+                    for (int bb = 0; bb < nb; bb++) acc = __fadd_rn(acc, ex[bb]);
+                }
+                const int lane0 = (tid & 31) & ~7;
+                float total = __shfl_sync(0xffffffffu, acc, lane0);
+#pragma unroll
+                for (int rr = 1; rr < 8; rr++) total = __fadd_rn(total, __shfl_sync(0xffffffffu, acc, lane0 + rr));
+                if (on && r == 0) store(s, rl, total);
             }
         }
     }
@@ -550,6 +588,7 @@ void launch_matvec(int njobs, const void *const *w, float *const *out, const int
     MatvecParams p = {};
     p.njobs = njobs;
     p.nb = blocks;
+    p.nb_inv = (65536u + (unsigned)blocks - 1) / (unsigned)blocks;
     p.rows_per_cta = kThreads / blocks;
     int cta = 0;
     for (int i = 0; i < njobs; i++) {
@@ -654,6 +693,7 @@ void launch_matvec_multi(int njobs, const void *const *w, float *const *out, con
     MatvecParams p = {};
     p.njobs = njobs;
     p.nb = blocks;
+    p.nb_inv = (65536u + (unsigned)blocks - 1) / (unsigned)blocks;
     p.rows_per_cta = kThreads / blocks;
     int cta = 0;
     for (int i = 0; i < njobs; i++) {

@@ -85,3 +85,23 @@ def test_expert_forms_by_tokens_per_expert(embd, ffe):
                 assert got[s] == gm.forward(toks[s], 0) and np.array_equal(gm.logits()[0].view(np.uint32), rows[s]), f"sequence {s} of {n}"
     finally:
         gm.free()
+
+
+# blocks per row around the rows one thread adds up by itself (3); rows around what one CTA of 256 (row, block) units covers
+@pytest.mark.parametrize("blocks", [1, 2, 3, 4, 7, 24, 256])
+def test_matvec_tails(be, blocks):
+    """One activation: dense and grouped products, with quants of -128 and 127 and the largest weights, against the oracle."""
+    import oracle as orc
+    from llamd_rs_b200 import synth
+
+    k, per_cta = 256 * blocks, 256 // blocks
+    rng = np.random.default_rng(blocks)
+    for rows in sorted({1, per_cta, per_cta + 1, 2 * per_cta - 1}):
+        w = _largest(synth.q6k_blocks(2 * rows * blocks, 93, "tails", blocks, rows).copy(), rows * blocks // 2 + 1)
+        qs, d = rng.integers(-128, 128, k).astype(np.int8), rng.random(blocks, dtype=np.float32)
+        qs[:256] = np.where(qs[:256] < 0, -128, 127)
+        want = orc.matvec_q6k_q8k(w, qs, d, k, 2 * rows).view(np.uint32)
+        dw = be.DeviceWeights.upload(w, 2 * rows, blocks)
+        assert np.array_equal(dw.matvec(qs, d).view(np.uint32), want)
+        got = dw.matvec_grouped(qs, d, [1, 0, 1], rows).view(np.uint32)
+        assert np.array_equal(got, want.reshape(2, rows)[[1, 0, 1]])
