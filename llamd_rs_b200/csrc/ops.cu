@@ -1354,21 +1354,24 @@ __global__ void __launch_bounds__(256) attn_out_kernel(const float *__restrict__
 // 29.0 per head / 11.8 here, at 512 9.9 / 10.3; 128 sequences of 30 to 264 positions 34.2 (82.4 with eight CTAs each and one chain
 // per thread).
 constexpr int kGqaMax = 8;  // query heads per kv head these kernels hold
+constexpr int kGqaHead = 32 * kSplit;  // their head size
+constexpr int kGqaPvTile = 128;  // positions per V tile
 
 // ROPE: with the query's and the new key's norm and rotation and the K/V store, for the new token of a sequence. Otherwise for
 // the tokens of a small tile of one sequence: the queries are ready and every key is in the cache (kv_stride 0).
 template <class KVT, bool ROPE>
-__global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *__restrict__ q_raw, const float *__restrict__ wq,
+__global__ void __launch_bounds__(256, 3) attn_rope_scores_gqa_kernel(const float *__restrict__ q_raw, const float *__restrict__ wq,
                                                                    const float *__restrict__ k_raw, const float *__restrict__ wk,
                                                                    const float *__restrict__ v_raw, KVT *__restrict__ kc, KVT *__restrict__ vc,
-                                                                   float *__restrict__ scores, int n_head, int n_head_kv, int hd,
+                                                                   float *__restrict__ scores, int n_head, int n_head_kv,
                                                                    const int32_t *__restrict__ meta, int max_kv, int kv_stride,
                                                                    const float *__restrict__ rope_tab, float eps, int flags) {
     extern __shared__ __align__(16) float sm[];
-    const int stride = hd + 4, half = hd / 2, ratio = n_head / n_head_kv;
+    constexpr int hd = kGqaHead, stride = hd + 4, half = hd / 2, hd4 = hd / 4, per_tile4 = kAttTile * hd4;
+    const int ratio = n_head / n_head_kv;
     float *sq = sm;                               // [ratio][hd] the roped queries
-    float *tile = sq + ratio * hd;                // [2][kAttTile][stride]
-    float *s_raw = tile + 2 * kAttTile * stride;  // [ratio + 1][hd] raw queries, raw key
+    float *tile = sq + ratio * hd;                // [kAttTile][stride]
+    float *s_raw = tile + kAttTile * stride;  // [ratio + 1][hd] raw queries, raw key
     float *sk = s_raw + (ratio + 1) * hd;         // [hd] the roped new key, as the cache holds it
     __shared__ float s_scale[kGqaMax + 1];
     pdl_trigger();
@@ -1384,9 +1387,8 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
     KVT *vrow = vc + ((size_t)seq * kv_stride + pos) * kv_dim + (size_t)kvh * hd;
     const KVT *kb = kc + (size_t)seq * kv_stride * kv_dim + (size_t)kvh * hd;
     const float scale = __fdiv_rn(1.0f, __fsqrt_rn((float)hd));
-    const int hd4 = hd / 4, per_tile4 = kAttTile * hd4;
     const int n_tiles = (n_kv + kAttTile - 1) / kAttTile;
-    constexpr int kMaxLd = 8;
+    constexpr int kMaxLd = per_tile4 / 256;
     typename KvIo<KVT>::Raw reg[kMaxLd];
     auto fetch = [&](int ti) {
 #pragma unroll
@@ -1395,7 +1397,7 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
             const int r = idx / hd4, cc = idx - r * hd4;
             const int t = ti * kAttTile + r;
             reg[j] = typename KvIo<KVT>::Raw{};
-            if (idx < per_tile4 && (ROPE ? t < pos : t < n_kv)) reg[j] = KvIo<KVT>::raw4(kb + (size_t)t * kv_dim + 4 * cc);
+            if (ROPE ? t < pos : t < n_kv) reg[j] = KvIo<KVT>::raw4(kb + (size_t)t * kv_dim + 4 * cc);
         }
     };
     auto stash = [&](float *dst, int ti) {
@@ -1403,7 +1405,7 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
         for (int j = 0; j < kMaxLd; j++) {
             const int idx = tid + j * 256;
             const int r = idx / hd4, cc = idx - r * hd4;
-            if (idx < per_tile4 && (!ROPE || ti * kAttTile + r != pos)) {  // (the token's own row is written below, by other threads)
+            if (!ROPE || ti * kAttTile + r != pos) {  // (the token's own row is written below, by other threads)
                 *reinterpret_cast<float4 *>(dst + r * stride + 4 * cc) = KvIo<KVT>::wide4(reg[j]);
             }
         }
@@ -1473,9 +1475,8 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
     }
     __syncthreads();
     // ---- scores: (query head, position) pairs of the tile over the threads ----
-    int buf = 0;
-    for (int ti = c; ti < n_tiles; ti += split, buf ^= 1) {
-        float *cur = tile + buf * kAttTile * stride;
+    for (int ti = c; ti < n_tiles; ti += split) {
+        float *cur = tile;
         stash(cur, ti);
         if (ROPE && ti == ti_pos)
             for (int i = tid; i < hd; i += blockDim.x) cur[(pos - ti * kAttTile) * stride + i] = sk[i];
@@ -1488,7 +1489,7 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
             const float4 *kr = reinterpret_cast<const float4 *>(cur + r * stride), *qa = reinterpret_cast<const float4 *>(sq + j * hd), *qb = qa + hd4;
             float da = 0.0f, db = 0.0f;
             float4 k0 = kr[0], a0 = qa[0], b0 = qb[0];
-#pragma unroll 4
+#pragma unroll 2
             for (int d = 0; d < hd4; d++) {
                 const int dn = min(d + 1, hd4 - 1);
                 const float4 k1 = kr[dn], a1 = qa[dn], b1 = qb[dn];
@@ -1502,13 +1503,14 @@ __global__ void __launch_bounds__(256) attn_rope_scores_gqa_kernel(const float *
             out[0] = __fmul_rn(da, scale);
             out[max_kv] = __fmul_rn(db, scale);
         }
+        if (ti + split < n_tiles) __syncthreads();  // everyone is done with the tile
     }
 }
 
 // Softmax and weighted values for the query heads of one kv head: warp j is head j (ratio * hd / kSplit == 256 threads).
 template <class KVT>
-__global__ void __launch_bounds__(256) attn_out_gqa_kernel(const float *__restrict__ scores, const KVT *__restrict__ vc, float *__restrict__ out,
-                                                           int n_head, int n_head_kv, int hd, const int32_t *__restrict__ meta, int max_kv,
+__global__ void __launch_bounds__(256, 3) attn_out_gqa_kernel(const float *__restrict__ scores, const KVT *__restrict__ vc, float *__restrict__ out,
+                                                           int n_head, int n_head_kv, const int32_t *__restrict__ meta, int max_kv,
                                                            int kv_stride, int flags) {
     extern __shared__ __align__(16) float sm[];
     __shared__ float s_inv[kGqaMax];
@@ -1518,30 +1520,29 @@ __global__ void __launch_bounds__(256) attn_out_gqa_kernel(const float *__restri
     const int kvh = blockIdx.x, c = blockIdx.y, seq = blockIdx.z, tid = threadIdx.x;
     const int ratio = n_head / n_head_kv, h0 = kvh * ratio;
     const int n_kv = meta[2 * seq + 1] + 1, cap = (max_kv + 3) & ~3;
-    const int cols = hd / kSplit, cols4 = cols / 4;
+    constexpr int hd = kGqaHead, cols = hd / kSplit, cols4 = cols / 4, per_tile4 = kGqaPvTile * cols4;
     float *sl = sm;                 // [ratio][cap]
-    float *tile = sm + ratio * cap;  // [2][kPvTile][cols]
+    float *tile = sm + ratio * cap;  // [2][kGqaPvTile][cols]
     const int kv_dim = n_head_kv * hd;
     const KVT *vb = vc + (size_t)seq * kv_stride * kv_dim + (size_t)kvh * hd + (size_t)c * cols;
-    const int per_tile4 = kPvTile * cols4;
-    const int n_tiles = (n_kv + kPvTile - 1) / kPvTile;
-    constexpr int kMaxLd = 8;
+    const int n_tiles = (n_kv + kGqaPvTile - 1) / kGqaPvTile;
+    constexpr int kMaxLd = per_tile4 / 256;
     typename KvIo<KVT>::Raw reg[kMaxLd];
     auto fetch = [&](int ti) {
 #pragma unroll
         for (int j = 0; j < kMaxLd; j++) {
             const int idx = tid + j * 256;
             const int r = idx / cols4, cc = idx - r * cols4;
-            const int t = ti * kPvTile + r;
+            const int t = ti * kGqaPvTile + r;
             reg[j] = typename KvIo<KVT>::Raw{};
-            if (idx < per_tile4 && t < n_kv) reg[j] = KvIo<KVT>::raw4(vb + (size_t)t * kv_dim + 4 * cc);
+            if (t < n_kv) reg[j] = KvIo<KVT>::raw4(vb + (size_t)t * kv_dim + 4 * cc);
         }
     };
     auto stash = [&](float *dst) {
 #pragma unroll
         for (int j = 0; j < kMaxLd; j++) {
             const int idx = tid + j * 256;
-            if (idx < per_tile4) reinterpret_cast<float4 *>(dst)[idx] = KvIo<KVT>::wide4(reg[j]);
+            reinterpret_cast<float4 *>(dst)[idx] = KvIo<KVT>::wide4(reg[j]);
         }
     };
     if (early) {
@@ -1575,11 +1576,11 @@ __global__ void __launch_bounds__(256) attn_out_gqa_kernel(const float *__restri
     const float *slj = sl + (size_t)j * cap;
     float acc = 0.0f;
     for (int ti = 0; ti < n_tiles; ti++) {
-        float *cur = tile + (ti & 1) * kPvTile * cols;
+        float *cur = tile + (ti & 1) * kGqaPvTile * cols;
         stash(cur);
         __syncthreads();
         if (ti + 1 < n_tiles) fetch(ti + 1);
-        const int t0 = ti * kPvTile, cnt = min(kPvTile, n_kv - t0);
+        const int t0 = ti * kGqaPvTile, cnt = min(kGqaPvTile, n_kv - t0);
         int r = 0;
         if (cnt >= 16) {
             float pa[16], pb[16];
@@ -2293,11 +2294,11 @@ static void attention_rope_launch(const float *q, const float *wq, const float *
     }
     // One CTA per (kv head, ...) for all the query heads that share it (the decode pass asks for it)
     const int ratio = n_head / n_head_kv, cap = (max_kv + 3) & ~3;
-    const size_t smem_ga = (size_t)(ratio * hd + 2 * kAttTile * (hd + 4) + (ratio + 1) * hd + hd) * sizeof(float);
-    const size_t smem_gb = (size_t)((size_t)ratio * cap + 2 * kPvTile * (hd / kSplit)) * sizeof(float);
+    const size_t smem_ga = (size_t)(ratio * hd + kAttTile * (hd + 4) + (ratio + 1) * hd + hd) * sizeof(float);
+    const size_t smem_gb = (size_t)((size_t)ratio * cap + 2 * kGqaPvTile * (hd / kSplit)) * sizeof(float);
     // (values, measured, 48 layers at position ~520: 8 sequences 814.7 -> 1044.8 tok/s, 4 sequences 641.8 -> 717.2, 2 sequences
     // 456.2 -> 439.7, so from four sequences on; the scores wherever the pass asks for it: near_pass in model.cu)
-    const bool gqa = (flags & kPassAttnGqa) && !(flags & 4) && ratio == kGqaMax && hd / kSplit == 32 && smem_ga <= 200 * 1024;
+    const bool gqa = (flags & kPassAttnGqa) && !(flags & 4) && ratio == kGqaMax && hd == kGqaHead && smem_ga <= 200 * 1024;
     if (gqa) {
         static size_t conf_ga[2] = {0, 0};
         if (smem_ga > conf_ga[kv16]) {
@@ -2316,10 +2317,10 @@ static void attention_rope_launch(const float *q, const float *wq, const float *
         const dim3 grid(n_head_kv, split, nseq);
         if (kv16)
             launch_kc(PDL_ATTN, "attn_rope_scores_gqa", attn_rope_scores_gqa_kernel<__half, true>, grid, dim3(256), smem_ga, q, wq, k, wk, v, (__half *)kc,
-                      (__half *)vc, scores, n_head, n_head_kv, hd, meta, max_kv, max_kv, rope_tab, eps, flags);
+                      (__half *)vc, scores, n_head, n_head_kv, meta, max_kv, max_kv, rope_tab, eps, flags);
         else
             launch_kc(PDL_ATTN, "attn_rope_scores_gqa", attn_rope_scores_gqa_kernel<float, true>, grid, dim3(256), smem_ga, q, wq, k, wk, v, (float *)kc,
-                      (float *)vc, scores, n_head, n_head_kv, hd, meta, max_kv, max_kv, rope_tab, eps, flags);
+                      (float *)vc, scores, n_head, n_head_kv, meta, max_kv, max_kv, rope_tab, eps, flags);
     } else if (kv16) {
         launch_kc(PDL_ATTN, "attn_rope_scores", attn_rope_scores_kernel<__half>, dim3(n_head, kSplitT, nseq), dim3(256), smem_a, q, wq, k, wk, v,
                   (__half *)kc, (__half *)vc, scores, n_head, n_head_kv, hd, meta, max_kv, max_kv, rope_tab, eps, flags);
@@ -2340,10 +2341,10 @@ static void attention_rope_launch(const float *q, const float *wq, const float *
         }
         if (kv16)
             launch_kc(PDL_ATTN, "attn_out_gqa", attn_out_gqa_kernel<__half>, dim3(n_head_kv, kSplit, nseq), dim3(256), smem_gb, (const float *)scores,
-                      (const __half *)vc, out, n_head, n_head_kv, hd, meta, max_kv, max_kv, flags);
+                      (const __half *)vc, out, n_head, n_head_kv, meta, max_kv, max_kv, flags);
         else
             launch_kc(PDL_ATTN, "attn_out_gqa", attn_out_gqa_kernel<float>, dim3(n_head_kv, kSplit, nseq), dim3(256), smem_gb, (const float *)scores,
-                      (const float *)vc, out, n_head, n_head_kv, hd, meta, max_kv, max_kv, flags);
+                      (const float *)vc, out, n_head, n_head_kv, meta, max_kv, max_kv, flags);
         if (qs && qd) llamd_fwd_quantize(out, qs, qd, nseq * (n_head * hd / 256));
         return;
     }
@@ -2379,10 +2380,10 @@ void attention_meta_flags(const float *q, const void *kc, const void *vc, float 
 // of the same cache. n_kv_max bounds pos + 1 over the tokens. False: a shape they do not cover.
 bool attention_small_tile(const float *q, const void *kc, const void *vc, float *out, float *scores, int n_head, int n_head_kv, int hd,
                           const int32_t *meta, int n_kv_max, int ntok, bool kv16) {
-    if (n_head_kv <= 0 || n_head != kGqaMax * n_head_kv || hd != 32 * kSplit) return false;
+    if (n_head_kv <= 0 || n_head != kGqaMax * n_head_kv || hd != kGqaHead) return false;
     const int row = (n_kv_max + 3) & ~3;  // a row of scores
-    const size_t smem_a = (size_t)(kGqaMax * hd + 2 * kAttTile * (hd + 4) + (kGqaMax + 1) * hd + hd) * sizeof(float);
-    const size_t smem_b = (size_t)((size_t)kGqaMax * row + 2 * kPvTile * (hd / kSplit)) * sizeof(float);
+    const size_t smem_a = (size_t)(kGqaMax * hd + kAttTile * (hd + 4) + (kGqaMax + 1) * hd + hd) * sizeof(float);
+    const size_t smem_b = (size_t)((size_t)kGqaMax * row + 2 * kGqaPvTile * (hd / kSplit)) * sizeof(float);
     if (smem_b > 200 * 1024) return false;
     static size_t conf_a[2] = {0, 0}, conf_b[2] = {0, 0};
     if (smem_a > conf_a[kv16] || smem_b > conf_b[kv16]) {
@@ -2405,16 +2406,16 @@ bool attention_small_tile(const float *q, const void *kc, const void *vc, float 
     const dim3 grid_a(n_head_kv, split, ntok), grid_b(n_head_kv, kSplit, ntok);
     if (kv16) {
         launch_kc(PDL_ATTN, "attn_scores_small_tile", attn_rope_scores_gqa_kernel<__half, false>, grid_a, dim3(256), smem_a, q, (const float *)nullptr,
-                  (const float *)nullptr, (const float *)nullptr, (const float *)nullptr, (__half *)kc, (__half *)vc, scores, n_head, n_head_kv, hd, meta, row, 0,
+                  (const float *)nullptr, (const float *)nullptr, (const float *)nullptr, (__half *)kc, (__half *)vc, scores, n_head, n_head_kv, meta, row, 0,
                   (const float *)nullptr, 0.0f, 0);
         launch_kc(PDL_ATTN, "attn_out_small_tile", attn_out_gqa_kernel<__half>, grid_b, dim3(256), smem_b, (const float *)scores, (const __half *)vc, out, n_head,
-                  n_head_kv, hd, meta, row, 0, 0);
+                  n_head_kv, meta, row, 0, 0);
     } else {
         launch_kc(PDL_ATTN, "attn_scores_small_tile", attn_rope_scores_gqa_kernel<float, false>, grid_a, dim3(256), smem_a, q, (const float *)nullptr,
-                  (const float *)nullptr, (const float *)nullptr, (const float *)nullptr, (float *)kc, (float *)vc, scores, n_head, n_head_kv, hd, meta, row, 0,
+                  (const float *)nullptr, (const float *)nullptr, (const float *)nullptr, (float *)kc, (float *)vc, scores, n_head, n_head_kv, meta, row, 0,
                   (const float *)nullptr, 0.0f, 0);
         launch_kc(PDL_ATTN, "attn_out_small_tile", attn_out_gqa_kernel<float>, grid_b, dim3(256), smem_b, (const float *)scores, (const float *)vc, out, n_head,
-                  n_head_kv, hd, meta, row, 0, 0);
+                  n_head_kv, meta, row, 0, 0);
     }
     return true;
 }
