@@ -1513,7 +1513,6 @@ __global__ void __launch_bounds__(256, 3) attn_out_gqa_kernel(const float *__res
                                                            int n_head, int n_head_kv, const int32_t *__restrict__ meta, int max_kv,
                                                            int kv_stride, int flags) {
     extern __shared__ __align__(16) float sm[];
-    __shared__ float s_inv[kGqaMax];
     pdl_trigger();
     const bool early = (flags & kPassEarlyLoads) != 0;
     if (!early) pdl_wait();
@@ -1569,10 +1568,11 @@ __global__ void __launch_bounds__(256, 3) attn_out_gqa_kernel(const float *__res
         for (int off = 16; off > 0; off >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, off));
         for (int t = lane; t < n_kv; t += 32) slj[t] = ref_expf(__fsub_rn(slj[t], lmax));
         __syncwarp();
-        if (lane == 0) s_inv[j] = __fdiv_rn(1.0f, chain_sum(slj, n_kv, 0.0f));
+        float inv = lane == 0 ? __fdiv_rn(1.0f, chain_sum(slj, n_kv, 0.0f)) : 0.0f;
+        inv = __shfl_sync(0xffffffffu, inv, 0);
+        for (int t = lane; t < n_kv; t += 32) slj[t] = __fmul_rn(slj[t], inv);  // (once here, or once a column and lane below)
     }
-    __syncthreads();
-    const float inv = s_inv[j];
+    __syncwarp();
     const float *slj = sl + (size_t)j * cap;
     float acc = 0.0f;
     for (int ti = 0; ti < n_tiles; ti++) {
@@ -1584,19 +1584,24 @@ __global__ void __launch_bounds__(256, 3) attn_out_gqa_kernel(const float *__res
         int r = 0;
         if (cnt >= 16) {
             float pa[16], pb[16];
+            auto products = [&](float p[16], int r0) {
 #pragma unroll
-            for (int i = 0; i < 16; i++) pa[i] = __fmul_rn(__fmul_rn(slj[t0 + i], inv), cur[i * cols + lane]);
+                for (int i = 0; i < 16; i += 4) {
+                    const float4 e = *reinterpret_cast<const float4 *>(slj + t0 + r0 + i);
+                    p[i] = __fmul_rn(e.x, cur[(r0 + i) * cols + lane]), p[i + 1] = __fmul_rn(e.y, cur[(r0 + i + 1) * cols + lane]);
+                    p[i + 2] = __fmul_rn(e.z, cur[(r0 + i + 2) * cols + lane]), p[i + 3] = __fmul_rn(e.w, cur[(r0 + i + 3) * cols + lane]);
+                }
+            };
+            products(pa, 0);
             for (; r + 16 <= cnt; r += 16) {
-                const int rn = (r + 32 <= cnt) ? r + 16 : r;
-#pragma unroll
-                for (int i = 0; i < 16; i++) pb[i] = __fmul_rn(__fmul_rn(slj[t0 + rn + i], inv), cur[(rn + i) * cols + lane]);
+                products(pb, (r + 32 <= cnt) ? r + 16 : r);
 #pragma unroll
                 for (int i = 0; i < 16; i++) acc = __fadd_rn(acc, pa[i]);
 #pragma unroll
                 for (int i = 0; i < 16; i++) pa[i] = pb[i];
             }
         }
-        for (; r < cnt; r++) acc = __fadd_rn(acc, __fmul_rn(__fmul_rn(slj[t0 + r], inv), cur[r * cols + lane]));
+        for (; r < cnt; r++) acc = __fadd_rn(acc, __fmul_rn(slj[t0 + r], cur[r * cols + lane]));
     }
     out[((size_t)seq * n_head + h0 + j) * hd + (size_t)c * cols + lane] = acc;
 }
