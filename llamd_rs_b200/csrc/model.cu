@@ -396,8 +396,9 @@ bool near_pass(const Model &m, int nseq, int n_kv) { return m.ep_world == 1 && n
 // From how many tokens (sequences of a pass, tokens of a tile) on the experts run as a grouped GEMM over the scatter plan instead
 // of a matvec per (token, expert): it folds an expert's weights once for all its tokens, the matvec repeats its integer work
 // for each. us a layer (plan or slot order, gate and up, down) of 128 experts of 768 x 2048, 8 per token, matvec / GEMM: 16 tokens
-// 106 / 135, 24: 153 / 163, 32: 197 / 171, 40: 240 / 183, 64: 382 / 195. The GEMM's rows are up to 24 blocks.
-constexpr int kExpertGemmMin = 27;
+// 95 / 129, 24: 137 / 162, 28: 158 / 167, 30: 168 / 170, 32: 179 / 173, 40: 220 / 182, 64: 345 / 194. The GEMM's rows are up to 24
+// blocks.
+constexpr int kExpertGemmMin = 31;
 bool expert_gemm_pass(const Model &m, int n) {
     return n >= kExpertGemmMin && m.ep_world == 1 && m.hp.n_embd <= 24 * 256 && m.hp.n_ff_expert <= 24 * 256 && m.hp.n_expert <= 1024;
 }

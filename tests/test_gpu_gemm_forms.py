@@ -62,7 +62,7 @@ def test_grouped_token_counts(be, blocks):
 
 @pytest.mark.parametrize("embd,ffe", [(1280, 768), (512, 1536)])
 def test_expert_forms_by_tokens_per_expert(embd, ffe):
-    """64 experts, 4 per token: tiles of 26 to 400 tokens are 2 to 25 tokens per expert, where the experts go from matvecs over
+    """64 experts, 4 per token: tiles of 30 to 400 tokens are 2 to 25 tokens per expert, where the experts go from matvecs over
     the few-token forms to the teams; batches likewise. Tokens and logits are those of one token after the other."""
     from llamd_rs_b200 import synth
     from llamd_rs_b200.model import CudaModel
@@ -75,10 +75,10 @@ def test_expert_forms_by_tokens_per_expert(embd, ffe):
         for pos, t in enumerate(toks):
             want.append(gm.forward(t, pos))
             logits.append(gm.logits()[0].view(np.uint32).copy())
-        for n in (26, 27, 33, 100, 200, 400):
+        for n in (26, 30, 31, 33, 100, 200, 400):
             assert gm.prefill(toks[:n], 0) == want[n - 1] and np.array_equal(gm.logits()[0].view(np.uint32), logits[n - 1]), f"prompt of {n}"
             assert list(gm.verify(toks[:n], 0)) == want[:n], f"draft of {n}"
-        for n in (3, 4, 9, 26, 27, 56, 64):  # one position of n sequences
+        for n in (3, 4, 9, 30, 31, 56, 64):  # one position of n sequences
             got = gm.forward_batch(toks[:n], [0] * n)
             rows = gm.logits(n).view(np.uint32)
             for s in range(n):
