@@ -268,9 +268,9 @@ def run_prefill(args, m, hp, prompt, rank, world, backend, dist):
             "gpu_launches": int(L.llamd_fwd_launch_count() - launches0), "last_token": int(tok),
             "roofline": {"bound": "hbm", "achieved": wbytes / (ms.value / K * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": wbytes / (ms.value / K * 1e-3) / 1e9 / peak,
-                         # one ncu capture of the grouped GEMM read 1.006x its algorithmic bytes (pre-folded: 816.7 MB for the 811 MB of
+                         # one ncu capture of the expert GEMMs read 1.01x their algorithmic bytes (pre-folded: 816.7 MB for the 811 MB of
                          # gate+up images); the matmuls' weights are the pass's traffic to within that
-                         "traffic": 1.006 * hp["n_layer"] * (15482880 + 128 * 3 * 1290240 * (2.016 / 0.8203 if args.prefold else 1.0))
+                         "traffic": 1.01 * hp["n_layer"] * (15482880 + 128 * 3 * 1290240 * (2.016 / 0.8203 if args.prefold else 1.0))
                          if world == 1 else None,
                          "peak_source": peak_src,
                          "matmul_tops": tops, "matmul_frac_of_bf16_peak": tops / float(peaks.get("bf16_tflops_sustained", 1400.0)),

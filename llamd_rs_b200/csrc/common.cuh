@@ -232,7 +232,7 @@ void attention_meta_flags(const float *q, const void *kc, const void *vc, float 
 void norm_router_flags(const float *w, const float *x, const float *residual, float *x_out, const float *w_norm, float *xn_out, int8_t *qs,
                        float *d, int k, float eps, int n_expert, int n_used, float *logits, int32_t *ids, float *weights, float *probs,
                        unsigned int *counter, int nseq, int flags);
-// rm (here and below): the residue-major form of the quants as well, or null
+// rm (here and below): the quants in operand order (t32_place) as well, or null
 void quantize_rm(const float *x, int8_t *qs, float *d, int nblocks, int8_t *rm);
 void silu_mul_quant_rm(const float *gate, const float *up, float *out, int8_t *qs, float *d, int n, int8_t *rm);
 void rms_norm_quant_flags(const float *x, const float *w, float *out, int8_t *qs, float *d, int n, float eps, int nseq, int flags, int8_t *rm = nullptr);

@@ -161,7 +161,7 @@ struct Model {
         Buf gstart, gcount, ptoken, pslot, work, n_work;
         Buf logits_all, amax_v, amax_i, out_tokens;  // every token's logits and greedy pick (verification, wide batches)
         int32_t *h_out_tokens = nullptr;             // pinned [tile]
-        Buf aq_rm, aq2_rm;  // the GEMMs' view of aq / aq2: residue-major bytes (integer path) or two f16 terms per element (tcgen05 path)
+        Buf aq_rm, aq2_rm;  // the GEMMs' view of aq / aq2: operand-order bytes (integer path) or two f16 terms per element (tcgen05 path)
         int32_t *h_meta = nullptr;
         // Expert parallelism over peer memory: every rank's tile (activations, scales, routed ids) gathered here by the
         // ranks' own stores, [world][ep_cap] token rows; then this rank's share of the expert work over all of them.

@@ -311,7 +311,7 @@ void llamd::add_rms_norm_quant_flags(const float *x, const float *residual, floa
                     WaitPlan{}, flags);
 }
 
-// llamd_fwd_quantize with the residue-major form beside the natural one.
+// llamd_fwd_quantize with the operand-order form beside the natural one.
 void llamd::quantize_rm(const float *x, int8_t *qs, float *d, int nblocks, int8_t *rm) {
     if (nblocks <= 0) return;
     launch_kc(PDL_SMALL, "q8k_quantize", q8k_quantize_kernel, dim3((nblocks + 7) / 8), dim3(256), 0, x, qs, d, (int16_t *)nullptr, rm, nblocks);
