@@ -1508,8 +1508,11 @@ __global__ void __launch_bounds__(256, 3) attn_rope_scores_gqa_kernel(const floa
 }
 
 // Softmax and weighted values for the query heads of one kv head: warp j is head j (ratio * hd / kSplit == 256 threads).
-template <class KVT>
-__global__ void __launch_bounds__(256, 3) attn_out_gqa_kernel(const float *__restrict__ scores, const KVT *__restrict__ vc, float *__restrict__ out,
+// CTAS to an SM: three, with sixteen products ahead of a chain, or four with eight where the launch has more than three and a half to
+// an SM. us a pass, three / four: 128 sequences 19975 / 19868, a turn of 37 tokens (592 CTAs) 14546 / 14299; 32 sequences (512) 11985 /
+// 12016, 9 positions of a draft (144) 7440 / 7458.
+template <class KVT, int CTAS>
+__global__ void __launch_bounds__(256, CTAS) attn_out_gqa_kernel(const float *__restrict__ scores, const KVT *__restrict__ vc, float *__restrict__ out,
                                                            int n_head, int n_head_kv, const int32_t *__restrict__ meta, int max_kv,
                                                            int kv_stride, int flags) {
     extern __shared__ __align__(16) float sm[];
@@ -1573,6 +1576,7 @@ __global__ void __launch_bounds__(256, 3) attn_out_gqa_kernel(const float *__res
         for (int t = lane; t < n_kv; t += 32) slj[t] = __fmul_rn(slj[t], inv);  // (once here, or once a column and lane below)
     }
     __syncwarp();
+    constexpr int W = CTAS > 3 ? 8 : 16;  // products ahead of the chain
     const float *slj = sl + (size_t)j * cap;
     float acc = 0.0f;
     for (int ti = 0; ti < n_tiles; ti++) {
@@ -1582,28 +1586,37 @@ __global__ void __launch_bounds__(256, 3) attn_out_gqa_kernel(const float *__res
         if (ti + 1 < n_tiles) fetch(ti + 1);
         const int t0 = ti * kGqaPvTile, cnt = min(kGqaPvTile, n_kv - t0);
         int r = 0;
-        if (cnt >= 16) {
-            float pa[16], pb[16];
-            auto products = [&](float p[16], int r0) {
+        if (cnt >= W) {
+            float pa[W], pb[W];
+            auto products = [&](float p[W], int r0) {
 #pragma unroll
-                for (int i = 0; i < 16; i += 4) {
+                for (int i = 0; i < W; i += 4) {
                     const float4 e = *reinterpret_cast<const float4 *>(slj + t0 + r0 + i);
                     p[i] = __fmul_rn(e.x, cur[(r0 + i) * cols + lane]), p[i + 1] = __fmul_rn(e.y, cur[(r0 + i + 1) * cols + lane]);
                     p[i + 2] = __fmul_rn(e.z, cur[(r0 + i + 2) * cols + lane]), p[i + 3] = __fmul_rn(e.w, cur[(r0 + i + 3) * cols + lane]);
                 }
             };
             products(pa, 0);
-            for (; r + 16 <= cnt; r += 16) {
-                products(pb, (r + 32 <= cnt) ? r + 16 : r);
+            for (; r + W <= cnt; r += W) {
+                products(pb, (r + 2 * W <= cnt) ? r + W : r);
 #pragma unroll
-                for (int i = 0; i < 16; i++) acc = __fadd_rn(acc, pa[i]);
+                for (int i = 0; i < W; i++) acc = __fadd_rn(acc, pa[i]);
 #pragma unroll
-                for (int i = 0; i < 16; i++) pa[i] = pb[i];
+                for (int i = 0; i < W; i++) pa[i] = pb[i];
             }
         }
         for (; r < cnt; r++) acc = __fadd_rn(acc, __fmul_rn(slj[t0 + r], cur[r * cols + lane]));
     }
     out[((size_t)seq * n_head + h0 + j) * hd + (size_t)c * cols + lane] = acc;
+}
+template <class KVT>
+static auto gqa_out_kernel(dim3 grid) {
+    return 2 * grid.x * grid.y * grid.z > 7 * 148 ? attn_out_gqa_kernel<KVT, 4> : attn_out_gqa_kernel<KVT, 3>;
+}
+template <class KVT>
+static cudaError_t gqa_out_attribute() {  // (the batches' launch and the small tile's set the same)
+    const cudaError_t e = cudaFuncSetAttribute(attn_out_gqa_kernel<KVT, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(attn_out_gqa_kernel<KVT, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
 }
 
 // The attention-output launch with a cluster per 256-element block of its result (attn_out_kernel's quantizing tail).
@@ -2336,8 +2349,8 @@ static void attention_rope_launch(const float *q, const float *wq, const float *
     if (gqa && nseq >= 4 && smem_gb <= 200 * 1024) {
         static size_t conf_gb[2] = {0, 0};
         if (smem_gb > conf_gb[kv16]) {
-            const cudaError_t e = kv16 ? cudaFuncSetAttribute(attn_out_gqa_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024  /* (the small tile's launch sets the same) */)
-                                       : cudaFuncSetAttribute(attn_out_gqa_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024  /* (the small tile's launch sets the same) */);
+            const cudaError_t e = kv16 ? gqa_out_attribute<__half>()
+                                       : gqa_out_attribute<float>();
             if (e != cudaSuccess) {
                 set_error(e, "attention (output, per kv head) smem attribute");
                 return;
@@ -2345,10 +2358,10 @@ static void attention_rope_launch(const float *q, const float *wq, const float *
             conf_gb[kv16] = 200 * 1024;
         }
         if (kv16)
-            launch_kc(PDL_ATTN, "attn_out_gqa", attn_out_gqa_kernel<__half>, dim3(n_head_kv, kSplit, nseq), dim3(256), smem_gb, (const float *)scores,
+            launch_kc(PDL_ATTN, "attn_out_gqa", gqa_out_kernel<__half>(dim3(n_head_kv, kSplit, nseq)), dim3(n_head_kv, kSplit, nseq), dim3(256), smem_gb, (const float *)scores,
                       (const __half *)vc, out, n_head, n_head_kv, meta, max_kv, max_kv, flags);
         else
-            launch_kc(PDL_ATTN, "attn_out_gqa", attn_out_gqa_kernel<float>, dim3(n_head_kv, kSplit, nseq), dim3(256), smem_gb, (const float *)scores,
+            launch_kc(PDL_ATTN, "attn_out_gqa", gqa_out_kernel<float>(dim3(n_head_kv, kSplit, nseq)), dim3(n_head_kv, kSplit, nseq), dim3(256), smem_gb, (const float *)scores,
                       (const float *)vc, out, n_head, n_head_kv, meta, max_kv, max_kv, flags);
         if (qs && qd) llamd_fwd_quantize(out, qs, qd, nseq * (n_head * hd / 256));
         return;
@@ -2395,8 +2408,8 @@ bool attention_small_tile(const float *q, const void *kc, const void *vc, float 
         const cudaError_t e =
             kv16 ? cudaFuncSetAttribute(attn_rope_scores_gqa_kernel<__half, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a)
                  : cudaFuncSetAttribute(attn_rope_scores_gqa_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a);
-        const cudaError_t f = kv16 ? cudaFuncSetAttribute(attn_out_gqa_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)
-                                   : cudaFuncSetAttribute(attn_out_gqa_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        const cudaError_t f = kv16 ? gqa_out_attribute<__half>()
+                                   : gqa_out_attribute<float>();
         if (e != cudaSuccess || f != cudaSuccess) {
             set_error(e != cudaSuccess ? e : f, "attention (small tile) smem attribute");
             return true;
@@ -2413,13 +2426,13 @@ bool attention_small_tile(const float *q, const void *kc, const void *vc, float 
         launch_kc(PDL_ATTN, "attn_scores_small_tile", attn_rope_scores_gqa_kernel<__half, false>, grid_a, dim3(256), smem_a, q, (const float *)nullptr,
                   (const float *)nullptr, (const float *)nullptr, (const float *)nullptr, (__half *)kc, (__half *)vc, scores, n_head, n_head_kv, meta, row, 0,
                   (const float *)nullptr, 0.0f, 0);
-        launch_kc(PDL_ATTN, "attn_out_small_tile", attn_out_gqa_kernel<__half>, grid_b, dim3(256), smem_b, (const float *)scores, (const __half *)vc, out, n_head,
+        launch_kc(PDL_ATTN, "attn_out_small_tile", gqa_out_kernel<__half>(grid_b), grid_b, dim3(256), smem_b, (const float *)scores, (const __half *)vc, out, n_head,
                   n_head_kv, meta, row, 0, 0);
     } else {
         launch_kc(PDL_ATTN, "attn_scores_small_tile", attn_rope_scores_gqa_kernel<float, false>, grid_a, dim3(256), smem_a, q, (const float *)nullptr,
                   (const float *)nullptr, (const float *)nullptr, (const float *)nullptr, (float *)kc, (float *)vc, scores, n_head, n_head_kv, meta, row, 0,
                   (const float *)nullptr, 0.0f, 0);
-        launch_kc(PDL_ATTN, "attn_out_small_tile", attn_out_gqa_kernel<float>, grid_b, dim3(256), smem_b, (const float *)scores, (const float *)vc, out, n_head,
+        launch_kc(PDL_ATTN, "attn_out_small_tile", gqa_out_kernel<float>(grid_b), grid_b, dim3(256), smem_b, (const float *)scores, (const float *)vc, out, n_head,
                   n_head_kv, meta, row, 0, 0);
     }
     return true;

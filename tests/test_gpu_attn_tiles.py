@@ -22,3 +22,34 @@ def test_tile_edges(hd, n_head, n_head_kv, base, ntok, scale):
     got = ops.attention_prefill(q, k, v, pos, n_head, n_head_kv, hd, max_kv)
     want = ops.attention_prefill(q, k, v, pos, n_head, n_head_kv, hd, max_kv, tiled=False)
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("kv_f16", [False, True])
+def test_per_kv_head_forms_by_ctas(kv_f16):
+    """Tiles and batches on either side of 518 value CTAs (32 and 33 tokens at four kv heads), contexts around 8 and 16
+    positions and the value tile of 128: logits and tokens are those of one token after the other."""
+    from llamd_rs_b200 import synth
+    from llamd_rs_b200.model import CudaModel
+
+    hp = dict(synth.TINY, n_layer=1, n_embd=512, n_head=32, n_head_kv=4, head_dim=128, n_vocab=512)
+    gm = CudaModel.load_batched(hp, synth.make_model(hp, seed=6), max_kv=200, max_seq=40)
+    try:
+        if kv_f16:
+            gm.set_option("kv_f16", 1)
+        toks = synth.token_ids(180, hp["n_vocab"], 6, "ctas").tolist()
+        want, logits = [], []
+        for pos, t in enumerate(toks):
+            want.append(gm.forward(t, pos))
+            logits.append(gm.logits()[0].view(np.uint32).copy())
+        for base in (0, 100, 124):
+            for n in (9, 16, 17, 32, 33, 56):
+                assert list(gm.verify(toks[base : base + n], base)) == want[base : base + n], f"draft of {n} at {base}"
+                assert gm.prefill(toks[base : base + n], base) == want[base + n - 1], f"turn of {n} at {base}"
+                assert np.array_equal(gm.logits()[0].view(np.uint32), logits[base + n - 1]), f"turn of {n} at {base}"
+        for n in (32, 33, 40):  # every sequence behind the same context
+            for pos in range(20):
+                got = gm.forward_batch([toks[pos]] * n, [pos] * n)
+                rows = gm.logits(n).view(np.uint32)
+                assert list(got) == [want[pos]] * n and all(np.array_equal(r, logits[pos]) for r in rows), f"{n} sequences at {pos}"
+    finally:
+        gm.free()
