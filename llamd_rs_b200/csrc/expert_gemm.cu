@@ -764,7 +764,12 @@ template <auto KERNEL>
 static void gemm_launch_k(GemmParams &p, int n_groups, int threads, size_t smem) {
     static size_t configured = 0;
     if (smem > 48 * 1024 && smem > configured) {
-        cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) {
+            cudaGetLastError();  // (a refusal of this launch, not of the next one)
+            set_error(e, "q6k gemm: shared memory attribute");
+            return;
+        }
         configured = smem;
     }
     int grid_x = 0;

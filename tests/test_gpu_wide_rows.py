@@ -1,0 +1,43 @@
+"""Rows around the widest that the integer GEMM takes: models of one layer whose matrices have 23 to 32 blocks a row, tiles and
+batches against one token after the other. Everything is bit for bit."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _model(max_seq, **hp):
+    from llamd_rs_b200 import synth
+    from llamd_rs_b200.model import CudaModel
+
+    hp = dict(synth.TINY, n_layer=1, n_head_kv=2, head_dim=128, n_expert=4, **hp)
+    return CudaModel.load_batched(hp, synth.make_model(hp, seed=11), max_kv=200, max_seq=max_seq), hp
+
+
+def _one_by_one(gm, toks):
+    want, logits = [], []
+    for pos, t in enumerate(toks):
+        want.append(gm.forward(t, pos))
+        logits.append(gm.logits()[0].view(np.uint32).copy())
+    return want, logits
+
+
+def test_narrower_rows_after_a_refused_form():
+    """Folded rows of 24 blocks and more than 32 tokens, whether or not a form takes them, leave those of 23 as they were."""
+    from llamd_rs_b200 import backend, synth
+    from llamd_rs_b200._lib import lib
+
+    for blocks in (24, 23):
+        gm, hp = _model(1, n_embd=256 * blocks, n_head=2 * blocks)
+        try:
+            toks = synth.token_ids(33, hp["n_vocab"], 11, "wide").tolist()
+            want, logits = _one_by_one(gm, toks)
+            try:
+                got = gm.prefill(toks, 0)
+            except backend.Other:
+                assert blocks == 24
+                lib().llamd_fwd_last_error()
+                continue
+            assert got == want[-1] and np.array_equal(gm.logits()[0].view(np.uint32), logits[-1])
+        finally:
+            gm.free()
