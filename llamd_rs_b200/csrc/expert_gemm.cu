@@ -792,9 +792,14 @@ static void gemm_launch_k(GemmParams &p, int n_groups, int threads, size_t smem)
     }
     launch_kc(p.gstart ? PDL_OTHER : PDL_MATVEC, "q6k_gemm", KERNEL, dim3(grid_x, n_groups), dim3(threads), smem, p);
 }
+constexpr size_t kMaxSmem = 227 * 1024;  // what a CTA may have
+template <int MAXT, int SLOTS>
+static size_t team_smem(const GemmParams &p) {
+    return (size_t)p.raw_bytes + (size_t)SLOTS * 2048 + (size_t)p.nb * 8 * MAXT * 4;
+}
 template <int MAXT, int SLOTS, int MINB, bool FOLDED>
 static void gemm_launch_t(GemmParams &p, int n_groups) {
-    gemm_launch_k<q6k_gemm_kernel<MAXT, SLOTS, MINB, FOLDED>>(p, n_groups, 128, (size_t)p.raw_bytes + (size_t)SLOTS * 2048 + (size_t)p.nb * 8 * MAXT * 4);
+    gemm_launch_k<q6k_gemm_kernel<MAXT, SLOTS, MINB, FOLDED>>(p, n_groups, 128, team_smem<MAXT, SLOTS>(p));
 }
 template <int NT, int BW, bool DIRECT, int THREADS, int MINB>
 static void gemm_launch_few(GemmParams &p, int n_groups) {
@@ -841,7 +846,8 @@ static void gemm_launch(GemmParams &p, int n_groups, int tokens) {
     // The lines lie where the forms' times cross, see there; MAXT and the CTAs per SM by us of gate and up: 64 tokens (half a tile per
     // expert) <2, 4, 6> 124, <4, 8, 5> 136; 512 (four) <8, 16, 3> 257, <6, 12, 4> 267, <4, 8, 4> 285; down of 512 <6, 12, 4> 164, <8, 16, 3> 179.
     if (folded) {
-        if (tiles <= 4) gemm_launch_t<4, 8, 2, true>(p, n_groups);
+        // (an image of 24 blocks a row leaves no room for the rings of eight tiles)
+        if (tiles <= 4 || team_smem<8, 16>(p) > kMaxSmem) gemm_launch_t<4, 8, 2, true>(p, n_groups);
         else gemm_launch_t<8, 16, 2, true>(p, n_groups);
     } else if (direct) {
         if (tiles <= 1) gemm_launch_few<1, 3, true, 128, 5>(p, n_groups);

@@ -22,6 +22,46 @@ def _one_by_one(gm, toks):
     return want, logits
 
 
+def _check_batch(gm, toks, n):
+    got = gm.forward_batch(toks[:n], [0] * n)
+    rows = gm.logits(n).view(np.uint32)
+    for s in range(n):
+        assert got[s] == gm.forward(toks[s], 0) and np.array_equal(gm.logits()[0].view(np.uint32), rows[s]), f"sequence {s} of {n}"
+
+
+# 24: images that leave room for the rings of four token tiles only
+@pytest.mark.parametrize("blocks", [24, 23])
+def test_folded_rows(blocks):
+    """Tiles of up to 192 tokens and batches multiply with folded copies of the projections: up to four token tiles, and more."""
+    from llamd_rs_b200 import synth
+
+    gm, hp = _model(33, n_embd=256 * blocks, n_head=2 * blocks)
+    try:
+        toks = synth.token_ids(192, hp["n_vocab"], 11, "wide").tolist()
+        want, logits = _one_by_one(gm, toks)
+        for n in (32, 33, 64, 192):
+            assert gm.prefill(toks[:n], 0) == want[n - 1] and np.array_equal(gm.logits()[0].view(np.uint32), logits[n - 1]), f"prompt of {n}"
+        _check_batch(gm, toks, 33)
+    finally:
+        gm.free()
+
+
+@pytest.mark.parametrize("blocks", [24, 23])
+def test_prefolded_experts(blocks):
+    """prefill_prefold: 16 to 96 tokens per expert."""
+    from llamd_rs_b200 import synth
+
+    gm, hp = _model(1, n_embd=256 * blocks, n_head=2)
+    try:
+        gm.set_option("prefill_prefold", 1)
+        toks = synth.token_ids(192, hp["n_vocab"], 11, "wide").tolist()
+        want, logits = _one_by_one(gm, toks)
+        for n in (32, 64, 65, 130, 192):
+            assert gm.prefill(toks[:n], 0) == want[n - 1] and np.array_equal(gm.logits()[0].view(np.uint32), logits[n - 1]), f"prompt of {n}"
+    finally:
+        gm.free()
+
+
 def test_narrower_rows_after_a_refused_form():
     """Folded rows of 24 blocks and more than 32 tokens, whether or not a form takes them, leave those of 23 as they were."""
     from llamd_rs_b200 import backend, synth
