@@ -819,16 +819,18 @@ static int raw_tile_bytes(int units, bool aligned) {
 
 // n_groups > 0: that many token groups of about `tokens` each. 0: one group of p.n_tokens.
 static void gemm_launch(GemmParams &p, int n_groups, int tokens) {
-    // (24 blocks a row: what the rings and the blocks of 16 rows leave of an SM's shared memory)
-    if (p.nb < 1 || p.nb > 24) {
-        set_error_msg("q6k gemm: blocks per row must be 1..24");
+    // Blocks a row: 24 for one group of tokens and 26 for token groups from the stored blocks, 25 and 26 from folded images, of
+    // which 26 blocks are 214656 bytes of shared memory.
+    const bool folded = p.folded[0] != nullptr;
+    if (p.nb < 1 || p.nb > (n_groups ? kGroupedBlocks : folded ? kFoldedBlocks : kGemmBlocks)) {
+        set_error_msg(n_groups ? "q6k gemm: blocks per row must be 1..26" : folded ? "q6k gemm: blocks per folded row must be 1..25"
+                                                                                    : "q6k gemm: blocks per row must be 1..24");
         return;
     }
     if (n_groups > 65535) {
         set_error_msg("q6k gemm: too many groups");
         return;
     }
-    const bool folded = p.folded[0] != nullptr;
     p.one = kOne2;
     const int tiles = (tokens + 7) / 8;
     const bool direct = !folded && p.nb <= 3 && tokens <= 16, few = direct || (!folded && !p.gstart && tiles <= 1);
@@ -846,8 +848,9 @@ static void gemm_launch(GemmParams &p, int n_groups, int tokens) {
     // The lines lie where the forms' times cross, see there; MAXT and the CTAs per SM by us of gate and up: 64 tokens (half a tile per
     // expert) <2, 4, 6> 124, <4, 8, 5> 136; 512 (four) <8, 16, 3> 257, <6, 12, 4> 267, <4, 8, 4> 285; down of 512 <6, 12, 4> 164, <8, 16, 3> 179.
     if (folded) {
-        // (an image of 24 blocks a row leaves no room for the rings of eight tiles)
-        if (tiles <= 4 || team_smem<8, 16>(p) > kMaxSmem) gemm_launch_t<4, 8, 2, true>(p, n_groups);
+        // (an image of 24 blocks a row leaves no room for the rings of eight tiles, one of 26 none for those of four)
+        if (team_smem<4, 8>(p) > kMaxSmem) gemm_launch_t<2, 4, 2, true>(p, n_groups);
+        else if (tiles <= 4 || team_smem<8, 16>(p) > kMaxSmem) gemm_launch_t<4, 8, 2, true>(p, n_groups);
         else gemm_launch_t<8, 16, 2, true>(p, n_groups);
     } else if (direct) {
         if (tiles <= 1) gemm_launch_few<1, 3, true, 128, 5>(p, n_groups);
@@ -911,8 +914,8 @@ size_t llamd::expert_fold_bytes(int blocks, int rows, int n_expert) {
     return expert_fold_tile_bytes(blocks) * (size_t)((rows + kGemmRows - 1) / kGemmRows) * (size_t)n_expert;
 }
 void llamd::expert_prefold(const void *w, void *dst, int blocks, int rows, int n_expert) {
-    if (n_expert > 65535 || n_expert < 1 || rows < 1 || blocks < 1 || blocks > 24) {
-        set_error_msg("expert prefold: 1..65535 experts, rows positive, 1..24 blocks per row");
+    if (n_expert > 65535 || n_expert < 1 || rows < 1 || blocks < 1 || blocks > kGroupedBlocks) {
+        set_error_msg("expert prefold: 1..65535 experts, rows positive, 1..26 blocks per row");
         return;
     }
     const size_t smem = (size_t)raw_tile_bytes(kGemmRows * blocks, false);

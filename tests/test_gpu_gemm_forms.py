@@ -44,7 +44,7 @@ def test_dense_forms(be, blocks, rows):
         assert np.array_equal(dw.matvec_f32(x[:nseq].ravel(), nseq).view(np.uint32).reshape(nseq, rows), want[:nseq]), f"{nseq} sequences"
 
 
-@pytest.mark.parametrize("blocks", [2, 4, 5])
+@pytest.mark.parametrize("blocks", [2, 4, 5, 24, 25, 26])
 def test_grouped_token_counts(be, blocks):
     """Groups of no token, one, a tile and its neighbours, two tiles of teams and one more."""
     from llamd_rs_b200 import ops, synth

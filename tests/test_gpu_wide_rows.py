@@ -1,4 +1,4 @@
-"""Rows around the widest that the integer GEMM takes: models of one layer whose matrices have 23 to 32 blocks a row, tiles and
+"""Rows around the widest that the integer GEMM takes: models of one layer whose matrices have 23 to 25 blocks a row, tiles and
 batches against one token after the other. Everything is bit for bit."""
 import numpy as np
 import pytest
@@ -29,17 +29,17 @@ def _check_batch(gm, toks, n):
         assert got[s] == gm.forward(toks[s], 0) and np.array_equal(gm.logits()[0].view(np.uint32), rows[s]), f"sequence {s} of {n}"
 
 
-# 24: images that leave room for the rings of four token tiles only
-@pytest.mark.parametrize("blocks", [24, 23])
-def test_folded_rows(blocks):
+# 24 blocks: images that leave room for the rings of four token tiles only; 50 heads: an output projection of 25, the widest
+@pytest.mark.parametrize("blocks,n_head", [(24, 48), (23, 46), (2, 50)])
+def test_folded_rows(blocks, n_head):
     """Tiles of up to 192 tokens and batches multiply with folded copies of the projections: up to four token tiles, and more."""
     from llamd_rs_b200 import synth
 
-    gm, hp = _model(33, n_embd=256 * blocks, n_head=2 * blocks)
+    gm, hp = _model(33, n_embd=256 * blocks, n_head=n_head)
     try:
         toks = synth.token_ids(192, hp["n_vocab"], 11, "wide").tolist()
         want, logits = _one_by_one(gm, toks)
-        for n in (32, 33, 64, 192):
+        for n in (32, 33, 56, 64, 192):
             assert gm.prefill(toks[:n], 0) == want[n - 1] and np.array_equal(gm.logits()[0].view(np.uint32), logits[n - 1]), f"prompt of {n}"
         _check_batch(gm, toks, 33)
     finally:
