@@ -780,7 +780,9 @@ bool ensure_folded(Model &m, int n, int prompt = 0) {
         b.release();
         if (clean) llamd_fwd_last_error();
     };
-    if (m.dense_gemm && n >= m.dense_gemm && !m.dense_fold_ready && !m.dense_fold_failed && !(prompt && m.prompt_no_dense)) {
+    // (rows wider than the GEMM takes stay on the matvec)
+    if (m.dense_gemm && n >= m.dense_gemm && !m.dense_fold_ready && !m.dense_fold_failed && !(prompt && m.prompt_no_dense) &&
+        eb <= kFoldedBlocks && qd / 256 <= kFoldedBlocks) {
         auto padded = [](size_t b) { return (b + 255) & ~(size_t)255; };
         const size_t q = padded(expert_fold_bytes(eb, qd, 1)), kv = padded(expert_fold_bytes(eb, kvd, 1)),
                      o = padded(expert_fold_bytes(qd / 256, hp.n_embd, 1)), layer = q + 2 * kv + o;

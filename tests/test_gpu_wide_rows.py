@@ -1,4 +1,4 @@
-"""Rows around the widest that the integer GEMM takes: models of one layer whose matrices have 23 to 25 blocks a row, tiles and
+"""Rows around the widest that the integer GEMM takes: models of one layer whose matrices have 23 to 32 blocks a row, tiles and
 batches against one token after the other. Everything is bit for bit."""
 import numpy as np
 import pytest
@@ -60,6 +60,26 @@ def test_prefolded_experts(blocks):
             assert gm.prefill(toks[:n], 0) == want[n - 1] and np.array_equal(gm.logits()[0].view(np.uint32), logits[n - 1]), f"prompt of {n}"
     finally:
         gm.free()
+
+
+@pytest.mark.parametrize("n_head", [52, 64])
+def test_projections_wider_than_the_gemm_takes(n_head):
+    """An output projection of 26 and 32 blocks a row: batches, drafts and short prompts run on the matvecs, from the first pass on."""
+    from llamd_rs_b200 import synth
+
+    for first in ("batch", "prompt"):
+        gm, hp = _model(9, n_embd=512, n_head=n_head)
+        try:
+            toks = synth.token_ids(9, hp["n_vocab"], 11, "wide").tolist()
+            if first == "batch":
+                for n in (8, 4, 9):
+                    _check_batch(gm, toks, n)
+            want, logits = _one_by_one(gm, toks)  # (a batch writes position 0 of sequence 0)
+            for n in (9, 4):
+                assert gm.prefill(toks[:n], 0) == want[n - 1] and np.array_equal(gm.logits()[0].view(np.uint32), logits[n - 1]), f"prompt of {n}"
+                assert list(gm.verify(toks[:n], 0)) == want[:n], f"draft of {n}"
+        finally:
+            gm.free()
 
 
 def test_narrower_rows_after_a_refused_form():
