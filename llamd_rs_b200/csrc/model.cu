@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "lines.h"
 #include "mega.cuh"
 #include "../../include/llamd_cuda_model.h"
 
@@ -393,14 +394,10 @@ void queue_token_resident(Model &m) {
 constexpr int kNearPositions = 512;
 bool near_pass(const Model &m, int nseq, int n_kv) { return m.ep_world == 1 && nseq <= 2 && nseq * n_kv <= kNearPositions; }
 
-// From how many tokens (sequences of a pass, tokens of a tile) on the experts run as a grouped GEMM over the scatter plan instead
-// of a matvec per (token, expert): it folds an expert's weights once for all its tokens, the matvec repeats its integer work
-// for each. us a layer (plan or slot order, gate and up, down) of 128 experts of 768 x 2048, 8 per token, matvec / GEMM: 16 tokens
-// 95 / 129, 24: 137 / 162, 28: 158 / 167, 30: 168 / 170, 32: 179 / 173, 40: 220 / 182, 64: 345 / 194. The GEMM's rows are up to 24
-// blocks.
-constexpr int kExpertGemmMin = 31;
+// The experts of a pass over n tokens (sequences of a batch, tokens of a tile) as a grouped GEMM.
 bool expert_gemm_pass(const Model &m, int n) {
-    return n >= kExpertGemmMin && m.ep_world == 1 && m.hp.n_embd <= 24 * 256 && m.hp.n_ff_expert <= 24 * 256 && m.hp.n_expert <= 1024;
+    return m.ep_world == 1 && m.hp.n_embd <= 24 * 256 && m.hp.n_ff_expert <= 24 * 256 && m.hp.n_expert <= 1024 &&
+           experts_on_gemm((long long)n * m.hp.n_expert_used, m.hp.n_expert, (long long)m.hp.n_embd * m.hp.n_ff_expert);
 }
 
 // Queue one pass for `nseq` sequences. Does not synchronise. near: see near_pass.

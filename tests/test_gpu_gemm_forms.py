@@ -60,14 +60,15 @@ def test_grouped_token_counts(be, blocks):
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
 
 
-@pytest.mark.parametrize("embd,ffe", [(1280, 768), (512, 1536)])
-def test_expert_forms_by_tokens_per_expert(embd, ffe):
+@pytest.mark.parametrize("embd,ffe,n_expert,n_used", [(1280, 768, 64, 4), (512, 1536, 64, 4), (512, 768, 8, 2)])
+def test_expert_forms_by_tokens_per_expert(embd, ffe, n_expert, n_used):
     """64 experts, 4 per token: tiles of 30 to 400 tokens are 2 to 25 tokens per expert, where the experts go from matvecs over
-    the few-token forms to the teams; batches likewise. Tokens and logits are those of one token after the other."""
+    the few-token forms to the teams; batches likewise. They change over at 36, 39 and 32 tokens. Tokens and logits are those of
+    one token after the other."""
     from llamd_rs_b200 import synth
     from llamd_rs_b200.model import CudaModel
 
-    hp = dict(synth.TINY, n_layer=1, n_embd=embd, n_ff_expert=ffe, n_expert=64, n_expert_used=4, n_vocab=512)
+    hp = dict(synth.TINY, n_layer=1, n_embd=embd, n_ff_expert=ffe, n_expert=n_expert, n_expert_used=n_used, n_vocab=512)
     gm = CudaModel.load_batched(hp, synth.make_model(hp, seed=5), max_kv=400, max_seq=64)
     try:
         toks = synth.token_ids(400, hp["n_vocab"], 5, "forms").tolist()
@@ -75,10 +76,10 @@ def test_expert_forms_by_tokens_per_expert(embd, ffe):
         for pos, t in enumerate(toks):
             want.append(gm.forward(t, pos))
             logits.append(gm.logits()[0].view(np.uint32).copy())
-        for n in (26, 30, 31, 33, 100, 200, 400):
+        for n in (26, 30, 31, 32, 33, 35, 36, 38, 39, 56, 100, 200, 400):
             assert gm.prefill(toks[:n], 0) == want[n - 1] and np.array_equal(gm.logits()[0].view(np.uint32), logits[n - 1]), f"prompt of {n}"
             assert list(gm.verify(toks[:n], 0)) == want[:n], f"draft of {n}"
-        for n in (3, 4, 9, 30, 31, 56, 64):  # one position of n sequences
+        for n in (3, 4, 9, 30, 31, 32, 35, 36, 38, 39, 56, 64):  # one position of n sequences
             got = gm.forward_batch(toks[:n], [0] * n)
             rows = gm.logits(n).view(np.uint32)
             for s in range(n):

@@ -1,0 +1,36 @@
+"""The lines between kernels (csrc/lines.h) at the sizes whose two sides were measured; no GPU is needed."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "llamd_rs_b200", "csrc")
+SOURCE = """
+#include "lines.h"
+extern "C" {
+int experts(long long pairs, int n_expert, long long weights) { return llamd::experts_on_gemm(pairs, n_expert, weights); }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def lines(tmp_path_factory):
+    d = tmp_path_factory.mktemp("lines")
+    (d / "l.cpp").write_text(SOURCE)
+    subprocess.check_call(["g++", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, str(d / "l.cpp"), "-o", str(d / "l.so")])
+    L = C.CDLL(str(d / "l.so"))
+    L.experts.argtypes = [C.c_longlong, C.c_int, C.c_longlong]
+    return L
+
+
+# experts, used per token, width, n_embd; tokens that the matvec is faster for by 2 % and more, tokens that the GEMM is
+@pytest.mark.parametrize("n_expert,used,width,embd,matvec,gemm", [
+    (8, 2, 1536, 2048, (2, 4, 8), (12, 16, 24)), (8, 2, 3072, 4096, (4, 6), (10, 12, 32)), (16, 2, 1536, 4096, (8, 12, 14), (16, 20, 64)),
+    (16, 2, 256, 2048, (8, 16, 18), (36, 56, 64)), (32, 4, 768, 2048, (8, 14, 16), (20, 24, 32)), (64, 8, 768, 2048, (8, 14), (18, 20, 32)),
+    (64, 6, 1536, 2048, (10, 16, 18), (24, 28, 64)), (60, 4, 1536, 2048, (12, 20, 24), (32, 36, 64)), (64, 4, 256, 2048, (14, 32, 36), (48, 56, 64)),
+    (128, 8, 768, 2048, (8, 24), (32, 36, 64)), (128, 8, 256, 2048, (14, 28, 32), (44, 48, 64)), (128, 8, 512, 1024, (14, 28, 32), (44, 48, 64)),
+    (256, 8, 512, 2048, (32, 48, 56), (70,)), (512, 10, 512, 2048, (26, 51, 64), (120,))])
+def test_experts_change_over_by_pairs_per_expert(lines, n_expert, used, width, embd, matvec, gemm):
+    assert not any(lines.experts(n * used, n_expert, width * embd) for n in matvec)
+    assert all(lines.experts(n * used, n_expert, width * embd) for n in gemm)
