@@ -1,6 +1,7 @@
 // The lines between two kernels that compute the same bits, as plain functions of sizes. Each stands where the times of its
 // two sides cross; both are given beside it.
 #pragma once
+#include <stddef.h>
 
 namespace llamd {
 
@@ -20,5 +21,14 @@ namespace llamd {
 inline bool experts_on_gemm(long long pairs, int n_expert, long long weights) {
     return 20 * pairs >= 33LL * n_expert + (4LL * n_expert + 220) * (768 * 2048) / weights;
 }
+
+// Softmax and weighted values of one kv head's query heads (attn_out_gqa_kernel): four CTAs to an SM, with half the products ahead of
+// a chain, or three. Four wins only where four are there: where the launch has more than three and a half to an SM and their
+// shared memory lets them (smem bytes each and the 1 KB that the system takes, of 228 KB: rows of up to 768 positions).
+// us a layer, three / four, batches of 128: rows of 288 positions 311.4 / 307.5, 700: 425.8 / 419.5, 768: 442.0 / 435.5, 1000: 499.6 /
+// 499.7, 1500: 647.2 / 653.3, 2500: 913.7 / 926.7. Batches of 32 (512 CTAs): 133.2 / 132.0 to 171.9 / 171.5; 48: 161.5 / 162.1 to 216.7 / 216.6;
+// a 48-layer pass of 32 behind 72 to 264 positions 11985 / 12016.
+// Tiles of 37 tokens (592) behind 300 positions 164.9 / 161.0, 700: 0.980 times, 800: 208.6 / 209.0, 4000: 571.9 / 588.6.
+inline bool attn_out_four_ctas(long long ctas, size_t smem) { return 2 * ctas > 7 * 148 && 4 * (smem + 1024) <= 228 * 1024; }
 
 }  // namespace llamd

@@ -10,6 +10,7 @@
 
 #include <vector>
 
+#include "lines.h"
 #include "packed_f32.cuh"
 #include "q6k_layout.cuh"
 #include "quant.cuh"
@@ -1508,9 +1509,7 @@ __global__ void __launch_bounds__(256, 3) attn_rope_scores_gqa_kernel(const floa
 }
 
 // Softmax and weighted values for the query heads of one kv head: warp j is head j (ratio * hd / kSplit == 256 threads).
-// CTAS to an SM: three, with sixteen products ahead of a chain, or four with eight where the launch has more than three and a half to
-// an SM. us a pass, three / four: 128 sequences 19975 / 19868, a turn of 37 tokens (592 CTAs) 14546 / 14299; 32 sequences (512) 11985 /
-// 12016, 9 positions of a draft (144) 7440 / 7458.
+// CTAS to an SM: three, with sixteen products ahead of a chain, or four with eight (attn_out_four_ctas).
 template <class KVT, int CTAS>
 __global__ void __launch_bounds__(256, CTAS) attn_out_gqa_kernel(const float *__restrict__ scores, const KVT *__restrict__ vc, float *__restrict__ out,
                                                            int n_head, int n_head_kv, const int32_t *__restrict__ meta, int max_kv,
@@ -1610,8 +1609,8 @@ __global__ void __launch_bounds__(256, CTAS) attn_out_gqa_kernel(const float *__
     out[((size_t)seq * n_head + h0 + j) * hd + (size_t)c * cols + lane] = acc;
 }
 template <class KVT>
-static auto gqa_out_kernel(dim3 grid) {
-    return 2 * grid.x * grid.y * grid.z > 7 * 148 ? attn_out_gqa_kernel<KVT, 4> : attn_out_gqa_kernel<KVT, 3>;
+static auto gqa_out_kernel(dim3 grid, size_t smem) {
+    return attn_out_four_ctas((long long)grid.x * grid.y * grid.z, smem) ? attn_out_gqa_kernel<KVT, 4> : attn_out_gqa_kernel<KVT, 3>;
 }
 template <class KVT>
 static cudaError_t gqa_out_attribute() {  // (the batches' launch and the small tile's set the same)
@@ -2358,10 +2357,10 @@ static void attention_rope_launch(const float *q, const float *wq, const float *
             conf_gb[kv16] = 200 * 1024;
         }
         if (kv16)
-            launch_kc(PDL_ATTN, "attn_out_gqa", gqa_out_kernel<__half>(dim3(n_head_kv, kSplit, nseq)), dim3(n_head_kv, kSplit, nseq), dim3(256), smem_gb, (const float *)scores,
+            launch_kc(PDL_ATTN, "attn_out_gqa", gqa_out_kernel<__half>(dim3(n_head_kv, kSplit, nseq), smem_gb), dim3(n_head_kv, kSplit, nseq), dim3(256), smem_gb, (const float *)scores,
                       (const __half *)vc, out, n_head, n_head_kv, meta, max_kv, max_kv, flags);
         else
-            launch_kc(PDL_ATTN, "attn_out_gqa", gqa_out_kernel<float>(dim3(n_head_kv, kSplit, nseq)), dim3(n_head_kv, kSplit, nseq), dim3(256), smem_gb, (const float *)scores,
+            launch_kc(PDL_ATTN, "attn_out_gqa", gqa_out_kernel<float>(dim3(n_head_kv, kSplit, nseq), smem_gb), dim3(n_head_kv, kSplit, nseq), dim3(256), smem_gb, (const float *)scores,
                       (const float *)vc, out, n_head, n_head_kv, meta, max_kv, max_kv, flags);
         if (qs && qd) llamd_fwd_quantize(out, qs, qd, nseq * (n_head * hd / 256));
         return;
@@ -2426,13 +2425,13 @@ bool attention_small_tile(const float *q, const void *kc, const void *vc, float 
         launch_kc(PDL_ATTN, "attn_scores_small_tile", attn_rope_scores_gqa_kernel<__half, false>, grid_a, dim3(256), smem_a, q, (const float *)nullptr,
                   (const float *)nullptr, (const float *)nullptr, (const float *)nullptr, (__half *)kc, (__half *)vc, scores, n_head, n_head_kv, meta, row, 0,
                   (const float *)nullptr, 0.0f, 0);
-        launch_kc(PDL_ATTN, "attn_out_small_tile", gqa_out_kernel<__half>(grid_b), grid_b, dim3(256), smem_b, (const float *)scores, (const __half *)vc, out, n_head,
+        launch_kc(PDL_ATTN, "attn_out_small_tile", gqa_out_kernel<__half>(grid_b, smem_b), grid_b, dim3(256), smem_b, (const float *)scores, (const __half *)vc, out, n_head,
                   n_head_kv, meta, row, 0, 0);
     } else {
         launch_kc(PDL_ATTN, "attn_scores_small_tile", attn_rope_scores_gqa_kernel<float, false>, grid_a, dim3(256), smem_a, q, (const float *)nullptr,
                   (const float *)nullptr, (const float *)nullptr, (const float *)nullptr, (float *)kc, (float *)vc, scores, n_head, n_head_kv, meta, row, 0,
                   (const float *)nullptr, 0.0f, 0);
-        launch_kc(PDL_ATTN, "attn_out_small_tile", gqa_out_kernel<float>(grid_b), grid_b, dim3(256), smem_b, (const float *)scores, (const float *)vc, out, n_head,
+        launch_kc(PDL_ATTN, "attn_out_small_tile", gqa_out_kernel<float>(grid_b, smem_b), grid_b, dim3(256), smem_b, (const float *)scores, (const float *)vc, out, n_head,
                   n_head_kv, meta, row, 0, 0);
     }
     return true;

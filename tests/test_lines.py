@@ -10,6 +10,7 @@ SOURCE = """
 #include "lines.h"
 extern "C" {
 int experts(long long pairs, int n_expert, long long weights) { return llamd::experts_on_gemm(pairs, n_expert, weights); }
+int four_ctas(long long ctas, long long smem) { return llamd::attn_out_four_ctas(ctas, smem); }
 }
 """
 
@@ -21,6 +22,7 @@ def lines(tmp_path_factory):
     subprocess.check_call(["g++", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, str(d / "l.cpp"), "-o", str(d / "l.so")])
     L = C.CDLL(str(d / "l.so"))
     L.experts.argtypes = [C.c_longlong, C.c_int, C.c_longlong]
+    L.four_ctas.argtypes = [C.c_longlong, C.c_longlong]
     return L
 
 
@@ -34,3 +36,14 @@ def lines(tmp_path_factory):
 def test_experts_change_over_by_pairs_per_expert(lines, n_expert, used, width, embd, matvec, gemm):
     assert not any(lines.experts(n * used, n_expert, width * embd) for n in matvec)
     assert all(lines.experts(n * used, n_expert, width * embd) for n in gemm)
+
+
+def _values_smem(positions):
+    return 4 * (8 * ((positions + 3) & ~3) + 2 * 128 * 32)  # eight rows of scores, two tiles of values
+
+
+def test_four_attention_ctas_only_where_they_are_there(lines):
+    for n in (37, 96, 128, 256):  # sequences, or tokens of a small tile: 16 CTAs each
+        assert all(lines.four_ctas(16 * n, _values_smem(p)) for p in (40, 288, 700, 768)), n
+        assert not any(lines.four_ctas(16 * n, _values_smem(p)) for p in (769, 837, 1000, 1500, 2500, 4000)), n
+    assert not any(lines.four_ctas(16 * n, _values_smem(288)) for n in (4, 9, 32))
