@@ -31,4 +31,12 @@ inline bool experts_on_gemm(long long pairs, int n_expert, long long weights) {
 // Tiles of 37 tokens (592) behind 300 positions 164.9 / 161.0, 700: 0.980 times, 800: 208.6 / 209.0, 4000: 571.9 / 588.6.
 inline bool attn_out_four_ctas(long long ctas, size_t smem) { return 2 * ctas > 7 * 148 && 4 * (smem + 1024) <= 228 * 1024; }
 
+// Attention of a small tile of one sequence by kv head (attention_small_tile), or by the tiled kernels. positions: a row of its
+// scores; ctas: of its second launch, 16 a token for four kv heads. Rows of more than 4352 positions leave one CTA to an SM, and those
+// that wait for another's end lose more than the tiled kernels' emptier tiles. us a layer, tiled / by kv head, f32 cache:
+//   behind 4360 positions: 9 tokens (144 CTAs) 312 / 214, 10: 315 / 314, 14: 328 / 341, 19: 337 / 445, 24: 340 / 468, 56 behind 4500: 455 / 995
+//   behind 5300:           9: 360 / 239, 10: 362 / 358, 14: 375 / 391, 19: 385 / 511, 24: 388 / 543, 56: 508 / 1137
+// Beyond 5376 positions the rows do not fit.
+inline bool small_tile_by_kv_head(int positions, long long ctas) { return positions <= 4352 || (positions <= 5376 && ctas <= 148); }
+
 }  // namespace llamd

@@ -2401,7 +2401,7 @@ bool attention_small_tile(const float *q, const void *kc, const void *vc, float 
     const int row = (n_kv_max + 3) & ~3;  // a row of scores
     const size_t smem_a = (size_t)(kGqaMax * hd + kAttTile * (hd + 4) + (kGqaMax + 1) * hd + hd) * sizeof(float);
     const size_t smem_b = (size_t)((size_t)kGqaMax * row + 2 * kGqaPvTile * (hd / kSplit)) * sizeof(float);
-    if (smem_b > 200 * 1024) return false;
+    if (smem_b > 200 * 1024 || !small_tile_by_kv_head(row, (long long)n_head_kv * kSplit * ntok)) return false;
     static size_t conf_a[2] = {0, 0}, conf_b[2] = {0, 0};
     if (smem_a > conf_a[kv16] || smem_b > conf_b[kv16]) {
         const cudaError_t e =

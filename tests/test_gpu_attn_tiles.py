@@ -53,3 +53,30 @@ def test_per_kv_head_forms_by_ctas(kv_f16):
                 assert list(got) == [want[pos]] * n and all(np.array_equal(r, logits[pos]) for r in rows), f"{n} sequences at {pos}"
     finally:
         gm.free()
+
+
+@pytest.mark.parametrize("kv_f16", [False, True])
+def test_small_tiles_around_the_longest_rows(kv_f16):
+    """Drafts and turns whose rows end around 4352 positions (nine tokens of four kv heads are the most that stay with the launches
+    by kv head behind them), around 5376, and around the four-CTA form's last row of 768: as one token after the other."""
+    from llamd_rs_b200 import synth
+    from llamd_rs_b200.model import CudaModel
+
+    hp = dict(synth.TINY, n_layer=1, n_embd=512, n_head=32, n_head_kv=4, head_dim=128, n_vocab=512)
+    gm = CudaModel.load_batched(hp, synth.make_model(hp, seed=8), max_kv=5440, max_seq=1)
+    try:
+        if kv_f16:
+            gm.set_option("kv_f16", 1)
+        toks = synth.token_ids(5440, hp["n_vocab"], 8, "rows").tolist()
+        gm.prefill(toks, 0)
+        for base, counts in ((728, (40, 41)), (4320, (9, 32, 33, 37)), (4343, (9, 10)), (5360, (9, 16, 17))):
+            want, logits = [], []
+            for pos in range(base, base + max(counts)):
+                want.append(gm.forward(toks[pos], pos))
+                logits.append(gm.logits()[0].view(np.uint32).copy())
+            for n in counts:
+                assert list(gm.verify(toks[base : base + n], base)) == want[:n], f"draft of {n} at {base}"
+                assert gm.prefill(toks[base : base + n], base) == want[n - 1], f"turn of {n} at {base}"
+                assert np.array_equal(gm.logits()[0].view(np.uint32), logits[n - 1]), f"turn of {n} at {base}"
+    finally:
+        gm.free()

@@ -11,6 +11,7 @@ SOURCE = """
 extern "C" {
 int experts(long long pairs, int n_expert, long long weights) { return llamd::experts_on_gemm(pairs, n_expert, weights); }
 int four_ctas(long long ctas, long long smem) { return llamd::attn_out_four_ctas(ctas, smem); }
+int small_tile(int positions, long long ctas) { return llamd::small_tile_by_kv_head(positions, ctas); }
 }
 """
 
@@ -23,6 +24,7 @@ def lines(tmp_path_factory):
     L = C.CDLL(str(d / "l.so"))
     L.experts.argtypes = [C.c_longlong, C.c_int, C.c_longlong]
     L.four_ctas.argtypes = [C.c_longlong, C.c_longlong]
+    L.small_tile.argtypes = [C.c_int, C.c_longlong]
     return L
 
 
@@ -47,3 +49,11 @@ def test_four_attention_ctas_only_where_they_are_there(lines):
         assert all(lines.four_ctas(16 * n, _values_smem(p)) for p in (40, 288, 700, 768)), n
         assert not any(lines.four_ctas(16 * n, _values_smem(p)) for p in (769, 837, 1000, 1500, 2500, 4000)), n
     assert not any(lines.four_ctas(16 * n, _values_smem(288)) for n in (4, 9, 32))
+
+
+def test_small_tiles_by_kv_head_behind_long_contexts(lines):
+    assert all(lines.small_tile(p, 16 * n) for p in (40, 1000, 4352) for n in (2, 9, 37, 56))
+    for p in (4356, 4800, 5376):
+        assert all(lines.small_tile(p, 16 * n) for n in (2, 4, 9))
+        assert not any(lines.small_tile(p, 16 * n) for n in (14, 19, 24, 37, 56))
+    assert not any(lines.small_tile(5380, 16 * n) for n in (2, 9, 56))
