@@ -4,6 +4,7 @@
 #include <string.h>
 
 #include "common.cuh"
+#include "lines.h"
 
 using namespace llamd;
 
@@ -318,11 +319,6 @@ static int finish_out(const float *d_out, float *out, size_t bytes, bool staged)
     return 0;
 }
 
-// From this many sequences on a host-facing product of up to 24 blocks a row runs on the integer tensor path, which folds a weight
-// once for all of them (the same bits). us in the kernel, matvec / GEMM: 151936 x 2048, 2 sequences 78 / 82, 3: 143 / 83, 8: 296 / 86;
-// 5120 x 2048, 3: 7.1 / 6.5, 8: 13.7 / 7.2; 2048 x 4096, 3: 5.9 / 6.8, 4: 6.8 / 7.4, 8: 12.1 / 6.9.
-constexpr int kGemmSeqs = 3;
-
 int llamd_cuda_matvec_q6k_f32(const void *d_w, const float *x, float *out, int blocks, int rows, int nseq) {
     if (!d_w || !x || !out || blocks <= 0 || rows <= 0 || nseq < 1 || nseq > LLAMD_MAX_SEQ) return -1;
     const size_t k = (size_t)blocks * 256, out_bytes = (size_t)nseq * rows * sizeof(float);
@@ -331,7 +327,7 @@ int llamd_cuda_matvec_q6k_f32(const void *d_w, const float *x, float *out, int b
     float *d_d = (float *)scratch(1, (size_t)nseq * blocks * sizeof(float));
     bool staged;
     float *d_out = out_buffer(out_bytes, &staged);
-    const bool gemm = nseq >= kGemmSeqs && blocks <= 24;
+    const bool gemm = product_on_gemm(blocks, rows, nseq);
     int8_t *d_rm = gemm ? (int8_t *)scratch(5, nseq * k) : nullptr;
     if (!d_q || !d_d || !d_out || (gemm && !d_rm) || stage_x(x, nseq * k * sizeof(float), &d_x, true)) return -1;
     quantize_rm(d_x, d_q, d_d, nseq * blocks, d_rm);

@@ -39,4 +39,26 @@ inline bool attn_out_four_ctas(long long ctas, size_t smem) { return 2 * ctas > 
 // Beyond 5376 positions the rows do not fit.
 inline bool small_tile_by_kv_head(int positions, long long ctas) { return positions <= 4352 || (positions <= 5376 && ctas <= 148); }
 
+// A host-facing Q6_K product of several sequences on the integer GEMM, which folds a weight once for all of them, or by matvec. Up to
+// eight blocks a row from three sequences on: four CTAs of 16 rows share an SM there and a wave of them is as short as the matvec.
+// Wider rows leave room for two CTAs, beyond 16 blocks for one, so a matrix of few rows is one wave of long chains, and the line is
+// the matvec's work against the GEMM's waves. us of quantizing and product, matvec / GEMM (launches come in ticks of 2 us):
+//   rows x blocks   2 sequences      3              4              6              8
+//   2048 x 8         7.8 / 7.7     8.1 / 7.6      8.3 / 7.5      8.3 / 7.7      8.3 / 8.3
+//   151936 x 8      81.9 / 87.1  141.4 / 88.0   176.0 / 88.1   238.2 / 88.2   301.9 / 90.1
+//   3072 x 12        9.7 / 9.8     8.3 / 9.9     10.3 / 9.7     14.4 / 9.9     16.4 / 10.3
+//   512 x 16         8.2 / 8.3     7.5 / 8.3      8.2 / 8.3      8.2 / 8.3      8.2 / 8.3
+//   2048 x 16        8.2 / 8.3     8.3 / 8.3     10.2 / 9.1     12.3 / 10.1    14.4 / 10.2
+//   1024 x 20        8.3 / 10.3    8.2 / 10.3    10.3 / 10.3    10.3 / 10.3    14.4 / 10.3
+//   512 x 24         8.3 / 10.3    8.0 / 10.3     8.3 / 10.3    10.3 / 10.3    10.3 / 10.3
+//   3072 x 24       12.4 / 16.4   14.4 / 16.4    18.8 / 16.4    24.6 / 17.3    30.4 / 17.5
+//   5120 x 24       15.0 / 22.6   20.5 / 22.6    24.6 / 23.5    34.9 / 24.4    44.2 / 24.6
+//   10000 x 24      24.6 / 36.0   41.0 / 36.4    50.8 / 36.9    69.7 / 36.9   102.5 / 36.9
+inline bool product_on_gemm(int blocks, int rows, int nseq) {
+    if (nseq < 3 || blocks > 24) return false;
+    if (blocks <= 8) return true;
+    const long long per_sm = blocks <= 16 ? 2 : 1, tiles = (rows + 15LL) / 16, waves = (tiles + 148 * per_sm - 1) / (148 * per_sm);
+    return (nseq + 1LL) * rows * blocks * per_sm >= 160000 * waves;
+}
+
 }  // namespace llamd

@@ -44,6 +44,21 @@ def test_dense_forms(be, blocks, rows):
         assert np.array_equal(dw.matvec_f32(x[:nseq].ravel(), nseq).view(np.uint32).reshape(nseq, rows), want[:nseq]), f"{nseq} sequences"
 
 
+# around the number of sequences from which such a matrix runs on the GEMM, with part of a row tile at the end
+@pytest.mark.parametrize("rows,blocks,counts", [(2047, 12, (2, 3, 8)), (1030, 16, (3, 4)), (1030, 24, (5, 6))])
+def test_products_of_several_sequences(be, rows, blocks, counts):
+    import oracle as orc
+    from llamd_rs_b200 import synth
+
+    k, most = 256 * blocks, max(counts)
+    w = synth.q6k_blocks(rows * blocks, 94, "products", blocks)
+    dw = be.DeviceWeights.upload(w, rows, blocks)
+    x = synth.normal_f32(most * k, 94, "products.x", blocks).reshape(most, k)
+    want = np.stack([orc.matvec_q6k(w, x[t], k, rows) for t in range(most)]).view(np.uint32)
+    for n in counts:
+        assert np.array_equal(dw.matvec_f32(x[:n].ravel(), n).view(np.uint32).reshape(n, rows), want[:n]), f"{n} sequences"
+
+
 @pytest.mark.parametrize("blocks", [2, 4, 5, 24, 25, 26])
 def test_grouped_token_counts(be, blocks):
     """Groups of no token, one, a tile and its neighbours, two tiles of teams and one more."""

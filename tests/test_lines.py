@@ -12,6 +12,7 @@ extern "C" {
 int experts(long long pairs, int n_expert, long long weights) { return llamd::experts_on_gemm(pairs, n_expert, weights); }
 int four_ctas(long long ctas, long long smem) { return llamd::attn_out_four_ctas(ctas, smem); }
 int small_tile(int positions, long long ctas) { return llamd::small_tile_by_kv_head(positions, ctas); }
+int product(int blocks, int rows, int nseq) { return llamd::product_on_gemm(blocks, rows, nseq); }
 }
 """
 
@@ -57,3 +58,14 @@ def test_small_tiles_by_kv_head_behind_long_contexts(lines):
         assert all(lines.small_tile(p, 16 * n) for n in (2, 4, 9))
         assert not any(lines.small_tile(p, 16 * n) for n in (14, 19, 24, 37, 56))
     assert not any(lines.small_tile(5380, 16 * n) for n in (2, 9, 56))
+
+
+# rows x blocks, sequences that the matvec is faster for (or as fast), sequences that the GEMM is
+@pytest.mark.parametrize("rows,blocks,matvec,gemm", [
+    (2048, 8, (1, 2), (3, 4, 8)), (151936, 8, (1, 2), (3, 4, 8)), (5120, 1, (2,), (3, 8)), (512, 16, (2, 3, 5), ()), (1024, 16, (2, 3), (6, 8)),
+    (2048, 16, (2,), (4, 6, 8)), (1024, 12, (3, 4), (6, 8)), (20000, 16, (2,), (3, 8)), (512, 20, (3, 4, 6, 8), ()), (1024, 20, (3, 5), (8,)),
+    (3072, 20, (2, 3, 4), (5, 6, 8)), (512, 24, (2, 3, 4, 5), ()), (2048, 24, (2,), (3, 4, 8)), (3072, 24, (2, 3), (4, 6, 8)),
+    (10000, 24, (2,), (3, 4, 8)), (5120, 25, (2, 3, 8), ())])
+def test_products_of_several_sequences(lines, rows, blocks, matvec, gemm):
+    assert not any(lines.product(blocks, rows, n) for n in matvec)
+    assert all(lines.product(blocks, rows, n) for n in gemm)
