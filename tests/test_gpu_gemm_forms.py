@@ -59,20 +59,61 @@ def test_products_of_several_sequences(be, rows, blocks, counts):
         assert np.array_equal(dw.matvec_f32(x[:n].ravel(), n).view(np.uint32).reshape(n, rows), want[:n]), f"{n} sequences"
 
 
-@pytest.mark.parametrize("blocks", [2, 4, 5, 24, 25, 26])
-def test_grouped_token_counts(be, blocks):
-    """Groups of no token, one, a tile and its neighbours, two tiles of teams and one more."""
+COUNTS = (0, 1, 7, 8, 9, 63, 64, 65, 129)
+
+
+def _groups(be, blocks, rows, matrices):
+    """One expert per entry of COUNTS, its pairs scattered over the tokens, and what expert_major makes of them."""
     from llamd_rs_b200 import ops, synth
 
-    counts, rows, k = (0, 1, 7, 8, 9, 63, 64, 65, 129), 40, 256 * blocks
-    ids = np.repeat(np.arange(len(counts), dtype=np.int32), counts).reshape(-1, 1)
+    k = 256 * blocks
+    ids = np.repeat(np.arange(len(COUNTS), dtype=np.int32), COUNTS).reshape(-1, 1)
     ids = np.ascontiguousarray(ids[np.random.default_rng(blocks).permutation(len(ids))])
-    w = _largest(synth.q6k_blocks(len(counts) * rows * blocks, 92, "counts", blocks).copy(), rows * blocks)
-    dw = be.DeviceWeights.upload(w, len(counts) * rows, blocks)
+    ws = [be.DeviceWeights.upload(_largest(synth.q6k_blocks(len(COUNTS) * rows * blocks, 92 + i, "counts", blocks).copy(), rows * blocks),
+                                  len(COUNTS) * rows, blocks) for i in range(matrices)]
     x = synth.normal_f32(len(ids) * k, 92, "counts.x", blocks).reshape(len(ids), k)
-    (want,) = ops.expert_major([dw], x, ids, rows)
-    (got,) = ops.expert_major([dw], x, ids, rows, gemm=True)
-    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+    return ids, ws, x, ops.expert_major(ws, x, ids, rows)
+
+
+@pytest.mark.parametrize("blocks", [2, 4, 5, 24, 25, 26])
+def test_grouped_token_counts(be, blocks):
+    """Groups of no token, one, a tile and its neighbours, two tiles of teams and one more, in the form that the entry point takes
+    for 64 tokens per group."""
+    from llamd_rs_b200 import ops
+
+    ids, ws, x, want = _groups(be, blocks, 40, 1)
+    got = ops.expert_major(ws, x, ids, 40, gemm=True)
+    assert np.array_equal(got[0].view(np.uint32), want[0].view(np.uint32))
+
+
+# rows: experts that begin with a tile of 32 blocks, and (part of a row tile at the end) that do not
+@pytest.mark.parametrize("blocks", [1, 3, 4, 5, 8, 24])
+@pytest.mark.parametrize("rows", [64, 33])
+def test_grouped_forms_meet_any_count(be, blocks, rows):
+    """The form follows the mean of the groups; each is given groups of none to 129 tokens, two matrices at a time."""
+    import ctypes as C
+    from llamd_rs_b200._lib import lib
+    from llamd_rs_b200.backend import DevBuf
+
+    vp = C.c_void_p
+    scatter = lib()._ZN5llamd19expert_gemm_scatterEPKvS1_PKiS3_S3_S3_S1_PKfPfS6_iiiiPKS6_iS1_S1_  # (as the model's passes call it)
+    scatter.restype, scatter.argtypes = None, [vp] * 10 + [C.c_int] * 4 + [vp, C.c_int, vp, vp]
+    ids, ws, x, want = _groups(be, blocks, rows, 2)
+    n, ne = len(ids), len(COUNTS)
+    dx, dq, dd, di = DevBuf.from_array(x), DevBuf(x.size), DevBuf(n * blocks * 4), DevBuf.from_array(ids)
+    lib().llamd_fwd_quantize(dx.ptr, dq.ptr, dd.ptr, n * blocks)
+    drm = DevBuf(x.size)
+    lib().llamd_fwd_q8k_residue_major(dq.ptr, drm.ptr, n * blocks)
+    gs, gc, pt, ps = DevBuf(ne * 4), DevBuf(ne * 4), DevBuf(n * 4), DevBuf(n * 4)
+    work, n_work = DevBuf((n // 8 + ne + 1) * 12), DevBuf.zeroed(4)
+    lib().llamd_fwd_moe_group_work(di.ptr, ne, 1, n, gs.ptr, gc.ptr, pt.ptr, ps.ptr, work.ptr, n_work.ptr)
+    for per_group in (1, 9, 17, 25, 41, 129):
+        outs = [DevBuf.zeroed(n * rows * 4) for _ in ws]
+        scatter(ws[0].ptr, ws[1].ptr, gs.ptr, gc.ptr, pt.ptr, ps.ptr, drm.ptr, dd.ptr, outs[0].ptr, outs[1].ptr, blocks, rows, ne,
+                per_group * ne, None, 1, None, None)
+        be.sync()
+        for o, w in zip(outs, want):
+            assert np.array_equal(o.download_f32(n * rows).view(np.uint32), w.view(np.uint32).ravel()), f"{per_group} tokens per group"
 
 
 @pytest.mark.parametrize("embd,ffe,n_expert,n_used", [(1280, 768, 64, 4), (512, 1536, 64, 4), (512, 768, 8, 2)])
