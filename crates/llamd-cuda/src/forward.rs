@@ -642,7 +642,7 @@ pub mod op {
         launch!("moe_group", [(ids, np * 4), (gstart, n_expert * 4), (gcount, n_expert * 4), (ptoken, np * 4), (pslot, np * 4)],
                 ffi::llamd_fwd_moe_group(i(ids), n_expert as i32, n_used as i32, ntok as i32, i(gstart), i(gcount), i(ptoken), i(pslot)))
     }
-    /// Q8_K quants [nblocks][256] -> the residue-major words the integer GEMM reads.
+    /// Q8_K quants [nblocks][256] -> the words the integer GEMM reads, in the order of its operands.
     pub fn q8k_residue_major(aq: &DevBuf, aq_rm: &DevBuf, nblocks: usize) -> Result<()> {
         launch!("q8k_residue_major", [(aq, nblocks * QK), (aq_rm, nblocks * QK)], ffi::llamd_fwd_q8k_residue_major(q(aq), aq_rm.ptr(), nblocks))
     }

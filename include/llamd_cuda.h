@@ -295,8 +295,10 @@ void llamd_fwd_expert_major(const void *wa, const void *wb, const int32_t *work,
 /* The same two on the integer tensor path (mma.sync s8 x s8 -> s32 per
  * (block, residue) slice, f32 scaling per slice as crates/llamd-vulkan/shaders/
  * q6k_expert_cm.comp:18-31 does per 16-K group); results identical to the two
- * above. Activations are the residue-major words llamd_fwd_q8k_residue_major
- * makes from Q8_K quants; the expert form takes gstart/gcount of the plan. */
+ * above. Activations are the words that llamd_fwd_q8k_residue_major makes from
+ * Q8_K quants, 64 per block in the order of the MMA's operands (its inside is
+ * no interface: make them and pass them on); the expert form takes
+ * gstart/gcount of the plan. Rows of up to 24 blocks, of experts up to 26. */
 void llamd_fwd_q8k_residue_major(const int8_t *aq, void *aq_rm, size_t nblocks);
 void llamd_fwd_gemm_tokens(const void *w0, const void *w1, const void *w2, const void *aq_rm, const float *ad, float *o0,
                            float *o1, float *o2, int blocks, int rows0, int rows1, int rows2, int ntok);

@@ -8,7 +8,7 @@
 // output element is one thread-private accumulator that walks its reduction
 // index in order with an unfused multiply and add. What changes against the
 // per-token kernels is only WHO holds the chains: a thread owns an 8x4 (scores)
-// or 4x8 (output) patch of independent chains, so operands fetched from shared
+// or 4x4 (output) patch of independent chains, so operands fetched from shared
 // memory are reused 4-8 times and the FP32 pipe, not memory, sets the pace.
 //
 //   tile_scores_kernel   S[t][p] = scale * (q_t . k_p)        64 tokens x 128 positions x one head per CTA

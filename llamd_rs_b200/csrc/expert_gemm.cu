@@ -20,10 +20,12 @@
 // What it costs is instruction issue: the packed codes have to become operands (some 40 instructions per 512 weights and warp)
 // and every 128 sums need 2 MMAs (10 cycles each, which keep the FP32 pipe from issuing) and 8 packed FP32 instructions.
 // The operands are made in registers by the lane that multiplies with them -- the weight layout gives every lane its own words
-// (q6k_layout.cuh) -- and used for all the token tiles at hand. Three forms, by tokens per group:
-//   q6k_gemm_few_kernel     up to 16: a warp folds all residues of its blocks, one or two tiles;
-//   q6k_gemm_kernel         four warps, a residue pair each, share 16 rows and up to 8 tiles;
-//   q6k_gemm_shared_kernel  short rows and many tokens: rows folded into shared memory once for four warps.
+// (q6k_layout.cuh) -- and used for all the token tiles at hand. Three forms (gemm_launch):
+//   q6k_gemm_few_kernel     a warp folds all residues of its blocks: up to 16 tokens a group at up to three blocks a row, and up to 8
+//                           tokens of one group (a projection, the head) at any number;
+//   q6k_gemm_shared_kernel  groups of more than 40 tokens at up to four blocks a row: rows folded into shared memory once for four
+//                           warps;
+//   q6k_gemm_kernel         everything else: four warps, a residue pair each, share 16 rows and up to 8 tiles.
 // us for 128 experts, gate and up (2 x 768 x 2048) / down (2048 x 768), 8 experts per token, before (every row tile folded into
 // shared memory, a warp per token tile) and now: 32 tokens 200 / 101, 114 / 58; 128: 243 / 119, 141 / 82; 512: 360 / 180, 257 / 164; 2048:
 // 910 / 465, 795 / 465.
@@ -179,7 +181,7 @@ struct RowTile {
 
 // The operands of one block of a row tile, made by the lane that multiplies with them. u: block of the lane's row g4 + 8h,
 // counted from the tile at `raw`.
-__device__ __forceinline__ void fold_block(uint32_t raw, int u, int rp, int q4, const uint32_t (&word_off)[3], int h, uint32_t (&hi)[2][4],
+__device__ __forceinline__ void fold_block(uint32_t raw, int u, int q4, const uint32_t (&word_off)[3], int h, uint32_t (&hi)[2][4],
                                            uint32_t (&lo)[2][4], float &d) {
     const uint32_t tile = raw + (uint32_t)(u >> 5) * kTileBytes, sl = (uint32_t)(u & 31), at = tile + 16u * (uint32_t)t32_slot((int)sl);
     uint32_t s[3], sc;
@@ -269,7 +271,7 @@ __device__ __forceinline__ void team_tiles(const GemmParams &p, const RowTile &r
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 float df;
-                fold_block(rt.raw, u[h] + b, rp, q4, word_off, h, hi, lo, df);
+                fold_block(rt.raw, u[h] + b, q4, word_off, h, hi, lo, df);
                 d[h] = pack2(df, df);
             }
         }
@@ -363,7 +365,8 @@ __device__ __forceinline__ void store_pair(const GemmParams &p, int j, int row0,
 // Up to 8 NT tokens against one row tile, one warp per BW blocks of the rows: a warp folds all eight residues of its blocks, so
 // that a block's scales, addresses and token scales are prepared once for eight residues and not for two. The products of the
 // tail wait in registers; then the warps add theirs in block order, each to the sums that the warp before it left in shared
-// memory, and the last one adds the eight residues. DIRECT (short rows): one warp has all the blocks of its own row tile.
+// memory, and the last one adds the eight residues. DIRECT (short rows): one warp has all the blocks of its own row tile, and
+// takes one tile group after the other; otherwise there is one group of at most eight tokens.
 // us, a residue pair per warp / this: the head for 8 tokens 95 / 86; down of 128 experts, 32 tokens 72 / 58, 128: 94 / 82. (Groups of 8
 // blocks a row: no gain, 130 / 131 for gate and up of 64 tokens, the products' registers cost the occupancy.)
 template <int NT>
@@ -562,9 +565,12 @@ __global__ void __launch_bounds__(128, MINB) q6k_gemm_kernel(const GemmParams p)
 }
 
 // grid as q6k_gemm_kernel's; a warp per BW blocks of a row tile, or (DIRECT) a warp per row tile, four row tiles a CTA.
-// Shared memory: the blocks | the warps' activations, NT x BW x 2 KB each | the sums on their way from warp to warp.
+// Shared memory: the blocks | the warps' activations, NT x BW x 2 KB each | the sums on their way from warp to warp (not DIRECT).
+// (DIRECT at three blocks a row: 64896 bytes, three CTAs to an SM, where the launch bound of five costs 84 bytes of spills; two token
+// tiles 89472 bytes, two CTAs.)
 template <int NT, int BW, bool DIRECT, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) q6k_gemm_few_kernel(const GemmParams p) {
+    static_assert(DIRECT || NT == 1, "the sums that go from warp to warp are of one tile");
     extern __shared__ __align__(16) uint8_t smem[];
     const int nb = p.nb, tid = threadIdx.x, w = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
     const int j = job_of_tile(p, blockIdx.x);
@@ -572,7 +578,7 @@ __global__ void __launch_bounds__(THREADS, MINB) q6k_gemm_few_kernel(const GemmP
     int first = 0, tile_lo = 0, count = p.n_tokens, tile_hi;
     size_t unit0 = (size_t)row_a * nb;
     pdl_trigger();
-    if (p.gstart) {
+    if (DIRECT && p.gstart) {
         pdl_wait();
         prefetch_ahead(p, p.prefetch_ahead);
         first = p.gstart[blockIdx.y];
@@ -592,15 +598,18 @@ __global__ void __launch_bounds__(THREADS, MINB) q6k_gemm_few_kernel(const GemmP
         for (int i = tid; i < n16; i += blockDim.x) copy_async16(s_raw + 16u * (uint32_t)i, src + 16 * (size_t)i);
         copy_commit();
     }
-    if (!p.gstart) pdl_wait();
+    if (!DIRECT || !p.gstart) pdl_wait();
     const uint32_t s_act = s_raw + (uint32_t)p.raw_bytes + (uint32_t)(w * NT * BW * 2048);
     float *s_x = reinterpret_cast<float *>(smem + p.raw_bytes + nw * NT * BW * 2048);
     const int r0 = DIRECT ? min(w * kGemmRows, ((live - 1) / kGemmRows) * kGemmRows) : 0;  // (a warp without a row tile repeats the last one)
     const RowTile rt = {j, row_a + r0, min(kGemmRows, live - r0), s_raw, (int)(unit0 - (t_lo << 5)) + r0 * nb};
-    for (int t = tile_lo; t < tile_hi; t += NT) {
-        if (NT == 1 || tile_hi - t > 1) few_tiles<NT, BW, DIRECT>(p, rt, first, count, t, s_act, s_x, DIRECT ? 0 : w, nw, lane);
-        else few_tiles<1, BW, DIRECT>(p, rt, first, count, t, s_act, s_x, DIRECT ? 0 : w, nw, lane);
-        if (!DIRECT && t + NT < tile_hi) __syncthreads();  // (the sums' place is free again)
+    if constexpr (DIRECT) {
+        for (int t = tile_lo; t < tile_hi; t += NT) {
+            if (NT == 1 || tile_hi - t > 1) few_tiles<NT, BW, DIRECT>(p, rt, first, count, t, s_act, s_x, 0, nw, lane);
+            else few_tiles<1, BW, DIRECT>(p, rt, first, count, t, s_act, s_x, 0, nw, lane);
+        }
+    } else {
+        few_tiles<NT, BW, DIRECT>(p, rt, first, count, 0, s_act, s_x, w, nw, lane);
     }
 }
 
@@ -743,7 +752,7 @@ __global__ void __launch_bounds__(128) q6k_prefold_kernel(const uint8_t *__restr
         for (int h = 0; h < 2; h++) {
             float d;
             const int m = g4 + 8 * h;
-            fold_block(s_raw, (int)(unit0 - (t_lo << 5)) + min(m, live - 1) * nb + b, rp, q4, word_off, h, hi, lo, d);
+            fold_block(s_raw, (int)(unit0 - (t_lo << 5)) + min(m, live - 1) * nb + b, q4, word_off, h, hi, lo, d);
             if (rp == 0 && q4 == 0) reinterpret_cast<float *>(out + (size_t)nb * kImageBlockBytes)[m * nb + b] = m < live ? d : 0.0f;
         }
         uint4 *o = reinterpret_cast<uint4 *>(out + (size_t)b * kImageBlockBytes + rp * 2048) + lane;
@@ -804,7 +813,7 @@ static void gemm_launch_t(GemmParams &p, int n_groups) {
 template <int NT, int BW, bool DIRECT, int THREADS, int MINB>
 static void gemm_launch_few(GemmParams &p, int n_groups) {
     const int warps = DIRECT ? p.row_tiles : (p.nb + BW - 1) / BW;
-    gemm_launch_k<q6k_gemm_few_kernel<NT, BW, DIRECT, THREADS, MINB>>(p, n_groups, 32 * warps, (size_t)p.raw_bytes + (size_t)warps * NT * BW * 2048 + NT * 4096);
+    gemm_launch_k<q6k_gemm_few_kernel<NT, BW, DIRECT, THREADS, MINB>>(p, n_groups, 32 * warps, (size_t)p.raw_bytes + (size_t)warps * NT * BW * 2048 + (DIRECT ? 0 : 4096));
 }
 
 static void shared_launch(GemmParams &p, int n_groups) {

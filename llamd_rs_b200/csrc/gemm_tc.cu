@@ -26,7 +26,8 @@
 //   blocks alternate between two accumulator tiles in TMEM; one stage into the next block, the finished one is
 //   read back: tcgen05.ld (32 lanes x 32 columns per warp), acc += 64 d * D in registers
 //   at the end: scatter acc to out[token][row].
-// act_f16_rm_kernel writes the activations in the contraction order used here (residue-major inside a block).
+// act_f16_rm_kernel writes the activations in the contraction order used here: residue after residue inside a block, the two
+// elements of a scale group side by side.
 // Every wait on an mbarrier is bounded; a timeout raises a flag the host reads (llamd_fwd_gemm_tc_status).
 #include <cuda_fp16.h>
 

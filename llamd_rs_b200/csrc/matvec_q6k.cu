@@ -10,7 +10,7 @@
 //
 // Mapping. One thread owns one (row, block) unit of the tiled weight layout
 // (q6k_layout.cuh): it streams 13 x 16 B + 2 B from HBM with fully coalesced
-// loads, unpacks residue by residue and forms its eight integers with dp4a
+// loads, unpacks quad by quad and forms its eight integers with dp4a
 // against activations staged in shared memory. A CTA of 256 threads covers
 // floor(256/blocks) whole rows. The per-unit f32 products go through shared
 // memory to the threads that walk the ordered sums.

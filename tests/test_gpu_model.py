@@ -447,8 +447,8 @@ def test_verify_buffers_do_not_follow_the_prompt_tile():
     gm = CudaModel.load_batched(hp, synth.make_model(hp, seed=9), max_kv=2048, max_seq=1)
     try:
         toks = synth.token_ids(2048, hp["n_vocab"], 3, "verify memory").tolist()
-        gm.set_option("head_gemm", 0)  # (no folded copy of the head in the figures below)
-        gm.set_option("dense_gemm", 0)
+        gm.set_option("head_gemm", 0)
+        gm.set_option("dense_gemm", 0)  # (no folded copies of the projections in the figures below)
         gm.prefill(toks[:80], 0)
         want = list(gm.verify(toks[:80], 0))
         gm.prefill(toks, 0)  # one tile of 2048
