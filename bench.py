@@ -268,9 +268,9 @@ def run_prefill(args, m, hp, prompt, rank, world, backend, dist):
             "gpu_launches": int(L.llamd_fwd_launch_count() - launches0), "last_token": int(tok),
             "roofline": {"bound": "hbm", "achieved": wbytes / (ms.value / K * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": wbytes / (ms.value / K * 1e-3) / 1e9 / peak,
-                         # one ncu capture of the expert GEMMs read 1.01x their algorithmic bytes (pre-folded: 816.7 MB for the 811 MB of
-                         # gate+up images); the matmuls' weights are the pass's traffic to within that
-                         "traffic": 1.01 * hp["n_layer"] * (15482880 + 128 * 3 * 1290240 * (2.016 / 0.8203 if args.prefold else 1.0))
+                         # one ncu capture of the expert GEMMs read 1.01x their algorithmic bytes (of pre-folded images likewise); the matmuls'
+                         # weights are the pass's traffic to within that
+                         "traffic": 1.01 * hp["n_layer"] * (15482880 + 128 * (2 + (2.016 / 0.8203 if args.prefold else 1.0)) * 1290240)
                          if world == 1 else None,
                          "peak_source": peak_src,
                          "matmul_tops": tops, "matmul_frac_of_bf16_peak": tops / float(peaks.get("bf16_tflops_sustained", 1400.0)),
@@ -306,7 +306,7 @@ def main():
                     help="prefill workload: exact = integer tensor path (mma.sync), bit-identical to decode (default); dp4a = the same "
                          "bits, 8 tokens per weight pass; tc = tcgen05 on f16 pairs, tolerance level")
     ap.add_argument("--prefold", action="store_true", help="prefill workload: keep the expert matrices a second time, folded for the integer "
-                    "GEMM (model option prefill_prefold; +58 GB on the 48-layer model; same bits)")
+                    "GEMM (model option prefill_prefold; +19.5 GB for the down projections of the 48-layer model; same bits)")
     ap.add_argument("--tile", type=int, default=0, help="prefill workload: tokens per prefill tile (0: min(prompt, 2048))")
     ap.add_argument("--ep-nccl", action="store_true", help="with --parallelism ep: the two exchanges per layer as NCCL collectives "
                     "(all-gather + grouped send/recv) instead of peer stores with arrival counters")

@@ -146,7 +146,7 @@ size_t llamd_model_weight_bytes(llamd_model *m); /* device.rs:473 */
  * GPU cuts a prompt into equal tiles of up to 2048, several into tiles of 512), "prefill_gemm" (1: the exact integer tensor path,
  * default; 0: dp4a, 8 tokens per weight pass, exact; 2: tcgen05 on f16 pairs, tolerance level), "prefill_attn" (1: the
  * register-tiled attention kernels, default; 0: the per-token decode kernels), "prefill_prefold" (1: keep the expert
- * matrices a second time, folded for the integer GEMM, +2 bytes per weight; same bits).
+ * matrices of up to five blocks a row a second time, folded for the integer GEMM, +2 bytes per weight; same bits).
  * Experiments kept for A/B runs, results unchanged: "pdl" (mask of launch classes that use programmatic dependent
  * launch), "prefetch" (1: matvec launches ask L2 for the next matvec's weights), "batch_group" (sequences per CTA for
  * small matrices at batch > 1, default 2), "ep_rank_arrive" (expert parallelism: 1 = one arrival per rank and launch on

@@ -265,6 +265,7 @@ void moe_group_owned(const int32_t *ids, int n_expert, int n_used, int nseq, int
                      int32_t *pslot, int32_t *work, int32_t *n_work, int own_lo, int own_hi);
 // Blocks per row that the integer GEMM takes: one group of tokens from the stored blocks, from folded images, and token groups.
 constexpr int kGemmBlocks = 24, kFoldedBlocks = 25, kGroupedBlocks = 26;
+constexpr int kPrefoldBlocks = 5;  // wider rows of experts have no use for folded images (gemm_launch)
 // The grouped expert GEMM with its output rows scattered over several GPUs: row block o goes to out_tab[o / out_div],
 // local row block o % out_div (out_tab null: everything into oa / ob). pairs: how many the plan holds about (0: unknown).
 void expert_gemm_scatter(const void *wa, const void *wb, const int32_t *gstart, const int32_t *gcount, const int32_t *act_map,

@@ -57,7 +57,7 @@ struct GemmParams {
     // expert parallelism: output row block o lives on GPU o / out_div, at local row block o % out_div (null: out[j])
     float *const *out_tab;
     int out_div;
-    // copies of the matrices kept folded (null: fold from w): [expert][row tile] images of fold_tile_bytes, see fold_image
+    // copies of the matrices kept folded (null: fold from w): [expert][row tile] images of fold_tile_bytes (kImageBlockBytes)
     const uint8_t *folded[3];
     long long fold_tile_bytes;
     f32x2 one;  // kOne2
@@ -521,9 +521,9 @@ __global__ void __launch_bounds__(128, MINB) q6k_gemm_kernel(const GemmParams p)
     pdl_trigger();
     int first = 0, tile_lo = 0, count = p.n_tokens, tile_hi;
     size_t unit0 = (size_t)row_a * nb;
-    if (p.gstart) {
+    if (!FOLDED && p.gstart) {
         pdl_wait();
-        prefetch_ahead<FOLDED>(p, p.prefetch_ahead);
+        prefetch_ahead(p, p.prefetch_ahead);
         first = p.gstart[blockIdx.y];
         count = p.gcount[blockIdx.y];
         if (count <= 0) return;
@@ -539,14 +539,13 @@ __global__ void __launch_bounds__(128, MINB) q6k_gemm_kernel(const GemmParams p)
         const uint8_t *src = p.w[j] + t_lo * kTileBytes;
         int n16 = (int)(t_hi - t_lo + 1) * (kTileBytes / 16);
         if (FOLDED) {
-            const int tiles_j = (p.rows[j] + kGemmRows - 1) / kGemmRows;
-            src = p.folded[j] + ((p.gstart ? (size_t)blockIdx.y * tiles_j : 0) + (size_t)(row_a / kGemmRows)) * (size_t)p.fold_tile_bytes;
+            src = p.folded[j] + (size_t)(row_a / kGemmRows) * (size_t)p.fold_tile_bytes;
             n16 = (int)(p.fold_tile_bytes >> 4);
         }
         for (int i = tid; i < n16; i += 128) copy_async16(s_raw + 16u * (uint32_t)i, src + 16 * (size_t)i);
         copy_commit();
     }
-    if (!p.gstart) pdl_wait();
+    if (FOLDED || !p.gstart) pdl_wait();
     float *s_ring = reinterpret_cast<float *>(smem + p.raw_bytes), *s_ad = s_ring + SLOTS * 512;
     for (int r0 = 0; r0 < live; r0 += kGemmRows) {
         const RowTile rt = {j, row_a + r0, min(kGemmRows, live - r0), s_raw, (int)(unit0 - (t_lo << 5)) + r0 * nb};
@@ -616,22 +615,31 @@ __global__ void __launch_bounds__(THREADS, MINB) q6k_gemm_few_kernel(const GemmP
 // ---- short rows, many tokens per group ----
 // With four blocks a row and less, a token group's preparation in q6k_gemm_kernel is as long as its products (down of 2048 tokens
 // 519 us, here 465; 768: 236 / 226; 512: 164 / 180). Here a CTA folds its 16 rows
-// into shared memory once, in operand order, and each of its warps takes token tiles of its own, all residues of them.
+// into shared memory once, in operand order, and each of its warps takes token tiles of its own, all residues of them. FOLDED: it
+// copies the rows' image.
 constexpr int kTokStride = 80;  // words per staged token: 16-byte aligned, fragment reads in 32 banks
+template <bool FOLDED>
 __global__ void __launch_bounds__(128, 5) q6k_gemm_shared_kernel(const GemmParams p) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int nb = p.nb, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g4 = lane >> 2, q4 = lane & 3;
-    uint4 *s_frag = reinterpret_cast<uint4 *>(smem);  // [block][residue][hi, lo][lane]
+    uint4 *s_frag = reinterpret_cast<uint4 *>(smem);  // [block][residue][hi, lo][lane], or the image (kImageBlockBytes)
     float *s_d = reinterpret_cast<float *>(smem + (size_t)nb * 8 * 2 * 32 * 16);
     uint32_t *s_b = reinterpret_cast<uint32_t *>(s_d + kGemmRows * nb) + warp * 8 * kTokStride;
     const int j = job_of_tile(p, blockIdx.x), row0 = ((int)blockIdx.x - p.tile_begin[j]) * kGemmRows, rows = p.rows[j];
     pdl_trigger();
     pdl_wait();
-    prefetch_ahead(p, p.prefetch_ahead);
+    prefetch_ahead<FOLDED>(p, p.prefetch_ahead);
     const int first = p.gstart[blockIdx.y], count = p.gcount[blockIdx.y], live = min(kGemmRows, rows - row0);
     if (count <= 0) return;
     const size_t unit0 = (size_t)blockIdx.y * (size_t)p.expert_units + (size_t)row0 * nb;
-    for (int it = tid; it < 2 * kGemmRows * nb; it += 128) {  // a thread: half of a (row, block)
+    if (FOLDED) {
+        const uint8_t *src = p.folded[j] + ((size_t)blockIdx.y * ((rows + kGemmRows - 1) / kGemmRows) + row0 / kGemmRows) * (size_t)p.fold_tile_bytes;
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem);
+        for (int i = tid; i < (int)(p.fold_tile_bytes >> 4); i += 128) copy_async16(dst + 16u * (uint32_t)i, src + 16 * (size_t)i);
+        copy_commit();
+        copy_wait<0>();
+    }
+    for (int it = FOLDED ? 2 * kGemmRows * nb : tid; it < 2 * kGemmRows * nb; it += 128) {  // a thread: half of a (row, block)
         const int half = it >= kGemmRows * nb ? 1 : 0, rb = it - half * kGemmRows * nb, row = rb / nb, b = rb - row * nb;
         const size_t unit = unit0 + (size_t)min(row, live - 1) * nb + b;
         const uint8_t *tile = p.w[j] + (unit >> 5) * kTileBytes;
@@ -698,13 +706,14 @@ __global__ void __launch_bounds__(128, 5) q6k_gemm_shared_kernel(const GemmParam
                 for (int i = 0; i < 4; i++) st[i] = __ldg(src[i] + (size_t)(b + 1) * 16);
                 a = pack2(__ldg(ad0 + b + 1), __ldg(ad1 + b + 1));
             }
-            const uint4 *fr = s_frag + (size_t)b * 8 * 2 * 32 + (lane ^ (lane >> 3) ^ (b & 7));
+            const uint4 *fr = s_frag + (size_t)b * 8 * 2 * 32 + (FOLDED ? lane : lane ^ (lane >> 3) ^ (b & 7));
 #pragma unroll
             for (int rp = 0; rp < 4; rp++) {
                 const uint4 bw = *reinterpret_cast<const uint4 *>(s_b + g4 * kTokStride + rp * 16 + q4 * 4);
 #pragma unroll
                 for (int rr = 0; rr < 2; rr++) {
-                    const uint4 h4 = fr[((2 * rp + rr) * 2 + 0) * 32], l4 = fr[((2 * rp + rr) * 2 + 1) * 32];
+                    const int at = FOLDED ? 4 * rp + rr : 2 * (2 * rp + rr);
+                    const uint4 h4 = fr[at * 32], l4 = fr[(at + (FOLDED ? 2 : 1)) * 32];
                     const uint32_t ah[4] = {h4.x, h4.y, h4.z, h4.w}, al[4] = {l4.x, l4.y, l4.z, l4.w};
                     int ch[4], cl[4];
                     mma_8<false>(ch, ah, rr ? bw.z : bw.x, rr ? bw.w : bw.y, zero);
@@ -816,9 +825,10 @@ static void gemm_launch_few(GemmParams &p, int n_groups) {
     gemm_launch_k<q6k_gemm_few_kernel<NT, BW, DIRECT, THREADS, MINB>>(p, n_groups, 32 * warps, (size_t)p.raw_bytes + (size_t)warps * NT * BW * 2048 + (DIRECT ? 0 : 4096));
 }
 
+template <bool FOLDED>
 static void shared_launch(GemmParams &p, int n_groups) {
     p.row_tiles = 1;
-    gemm_launch_k<q6k_gemm_shared_kernel>(p, n_groups, 128, (size_t)p.nb * 8 * 2 * 32 * 16 + (size_t)kGemmRows * p.nb * 4 + 4 * 8 * kTokStride * 4);
+    gemm_launch_k<q6k_gemm_shared_kernel<FOLDED>>(p, n_groups, 128, (size_t)p.nb * 8 * 2 * 32 * 16 + (size_t)kGemmRows * p.nb * 4 + 4 * 8 * kTokStride * 4);
 }
 
 // Shared memory for `units` consecutive blocks: whole tiles, one more where they need not start with one.
@@ -828,9 +838,12 @@ static int raw_tile_bytes(int units, bool aligned) {
 
 // n_groups > 0: that many token groups of about `tokens` each. 0: one group of p.n_tokens.
 static void gemm_launch(GemmParams &p, int n_groups, int tokens) {
-    // Blocks a row: 24 for one group of tokens and 26 for token groups from the stored blocks, 25 and 26 from folded images, of
-    // which 26 blocks are 214656 bytes of shared memory.
-    const bool folded = p.folded[0] != nullptr;
+    // Groups take the images of short rows, for as many tokens as a warp per token tile pays for: folding on the way is faster
+    // everywhere else. us, stored blocks / images, by blocks a row and tokens per group: 1 (2048 rows) 12 tokens 38 / 68, 32: 105 / 89,
+    // 128: 227 / 211; 3 (2048) 12: 95 / 130, 32: 169 / 162, 128: 482 / 433; 4 (1024) 12: 71 / 87, 32: 111 / 107, 128: 330 / 290; 5 (1024)
+    // 32: 131 / 136, 44: 161 / 173, 64: 222 / 213, 128: 397 / 366; 6 (1024) 64: 243 / 277, 128: 439 / 471; 8 (2 x 768) 32: 257 / 318, 128: 806 / 878.
+    const bool images = p.gstart && p.folded[0] && p.nb <= kPrefoldBlocks && tokens > (p.nb < 5 ? 24 : 48);
+    const bool folded = !p.gstart && p.folded[0];
     if (p.nb < 1 || p.nb > (n_groups ? kGroupedBlocks : folded ? kFoldedBlocks : kGemmBlocks)) {
         set_error_msg(n_groups ? "q6k gemm: blocks per row must be 1..26" : folded ? "q6k gemm: blocks per folded row must be 1..25"
                                                                                     : "q6k gemm: blocks per row must be 1..24");
@@ -857,10 +870,11 @@ static void gemm_launch(GemmParams &p, int n_groups, int tokens) {
     // The lines lie where the forms' times cross, see there; MAXT and the CTAs per SM by us of gate and up: 64 tokens (half a tile per
     // expert) <2, 4, 6> 124, <4, 8, 5> 136; 512 (four) <8, 16, 3> 257, <6, 12, 4> 267, <4, 8, 4> 285; down of 512 <6, 12, 4> 164, <8, 16, 3> 179.
     if (folded) {
-        // (an image of 24 blocks a row leaves no room for the rings of eight tiles, one of 26 none for those of four)
-        if (team_smem<4, 8>(p) > kMaxSmem) gemm_launch_t<2, 4, 2, true>(p, n_groups);
-        else if (tiles <= 4 || team_smem<8, 16>(p) > kMaxSmem) gemm_launch_t<4, 8, 2, true>(p, n_groups);
+        // (an image of 24 blocks a row leaves no room for the rings of eight tiles)
+        if (tiles <= 4 || team_smem<8, 16>(p) > kMaxSmem) gemm_launch_t<4, 8, 2, true>(p, n_groups);
         else gemm_launch_t<8, 16, 2, true>(p, n_groups);
+    } else if (images) {
+        shared_launch<true>(p, n_groups);
     } else if (direct) {
         if (tiles <= 1) gemm_launch_few<1, 3, true, 128, 5>(p, n_groups);
         else gemm_launch_few<2, 3, true, 128, 3>(p, n_groups);
@@ -869,7 +883,7 @@ static void gemm_launch(GemmParams &p, int n_groups, int tokens) {
         else if (p.nb <= 16) gemm_launch_few<1, 2, false, 256, 2>(p, n_groups);
         else gemm_launch_few<1, 2, false, 384, 1>(p, n_groups);
     } else if (p.gstart && p.nb <= 4 && tokens > 40) {
-        shared_launch(p, n_groups);
+        shared_launch<false>(p, n_groups);
     } else if (tiles <= 1) {
         gemm_launch_t<2, 4, 6, false>(p, n_groups);
     } else if (tiles <= 3) {
@@ -923,8 +937,8 @@ size_t llamd::expert_fold_bytes(int blocks, int rows, int n_expert) {
     return expert_fold_tile_bytes(blocks) * (size_t)((rows + kGemmRows - 1) / kGemmRows) * (size_t)n_expert;
 }
 void llamd::expert_prefold(const void *w, void *dst, int blocks, int rows, int n_expert) {
-    if (n_expert > 65535 || n_expert < 1 || rows < 1 || blocks < 1 || blocks > kGroupedBlocks) {
-        set_error_msg("expert prefold: 1..65535 experts, rows positive, 1..26 blocks per row");
+    if (n_expert > 65535 || n_expert < 1 || rows < 1 || blocks < 1 || blocks > kFoldedBlocks) {
+        set_error_msg("expert prefold: 1..65535 experts, rows positive, 1..25 blocks per row");
         return;
     }
     const size_t smem = (size_t)raw_tile_bytes(kGemmRows * blocks, false);

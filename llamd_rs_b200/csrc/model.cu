@@ -1251,8 +1251,9 @@ int llamd_model_set_option(llamd_model *h, const char *name, int value) {
         return 0;
     }
     if (!strcmp(name, "prefill_prefold")) {
-        // 1: keep every expert matrix a second time, folded into the integer MMA's operand order (2 bytes per weight:
-        // +58 GB for the 48-layer model), so that a prefill tile's grouped GEMMs copy operands instead of folding them.
+        // 1: keep the expert matrices of up to kPrefoldBlocks blocks a row a second time, folded into the integer MMA's operand
+        // order (2 bytes per weight: +19.5 GB for the down projections of the 48-layer model), so that a prefill tile's grouped GEMMs
+        // copy operands instead of folding them, where that is the faster (gemm_launch).
         // Built at the next prefill; 0 releases the copies. Same bits either way.
         if (!value && m->prefold_ready) {
             cudaStreamSynchronize(stream());
@@ -1343,20 +1344,23 @@ static bool ensure_prefold(Model &m) {
     if (!m.prefold || m.prefold_ready) return true;
     const llamd_hparams &hp = m.hp;
     const int eb = hp.n_embd / 256, fb = hp.n_ff_expert / 256, n_local = m.own_hi - m.own_lo;
-    const size_t gu = expert_fold_bytes(eb, hp.n_ff_expert, n_local), dn = expert_fold_bytes(fb, hp.n_embd, n_local);
+    const size_t gu = eb <= kPrefoldBlocks ? expert_fold_bytes(eb, hp.n_ff_expert, n_local) : 0,
+                 dn = fb <= kPrefoldBlocks ? expert_fold_bytes(fb, hp.n_embd, n_local) : 0;
     const size_t need = (size_t)hp.n_layer * (2 * gu + dn);
     if (need + ((size_t)2 << 30) > llamd_cuda_free_mem()) {
         m.err = "prefill_prefold: the folded expert matrices need " + std::to_string(need >> 20) + " MiB of device memory";
         return false;
     }
     for (auto &l : m.layers) {
-        if (!l.gate_fold.alloc(gu) || !l.up_fold.alloc(gu) || !l.down_fold.alloc(dn)) {
+        if ((gu && (!l.gate_fold.alloc(gu) || !l.up_fold.alloc(gu))) || (dn && !l.down_fold.alloc(dn))) {
             m.err = std::string("prefill_prefold: ") + llamd_cuda_last_error_string();
             return false;
         }
-        expert_prefold(l.gate_exps.p, l.gate_fold.p, eb, hp.n_ff_expert, n_local);
-        expert_prefold(l.up_exps.p, l.up_fold.p, eb, hp.n_ff_expert, n_local);
-        expert_prefold(l.down_exps.p, l.down_fold.p, fb, hp.n_embd, n_local);
+        if (gu) {
+            expert_prefold(l.gate_exps.p, l.gate_fold.p, eb, hp.n_ff_expert, n_local);
+            expert_prefold(l.up_exps.p, l.up_fold.p, eb, hp.n_ff_expert, n_local);
+        }
+        if (dn) expert_prefold(l.down_exps.p, l.down_fold.p, fb, hp.n_embd, n_local);
     }
     if (llamd_fwd_sync() != 0) {
         m.err = std::string("prefill_prefold: ") + llamd_cuda_last_error_string();
@@ -1473,7 +1477,7 @@ static bool folded_tile(const Model &m, int T) { return m.ep_world == 1 && m.pre
 // (expert_gemm_pass), the dense matrices on the folded copies. The line is where a batch of sequences changes over
 // (matvec_batch_max).
 static bool small_tile(const Model &m, int T, bool multi_seq) {
-    return !multi_seq && m.ep_world == 1 && m.prefill_gemm == 1 && !m.prefold_ready && T <= m.matvec_batch_max;
+    return !multi_seq && m.ep_world == 1 && m.prefill_gemm == 1 && T <= m.matvec_batch_max;
 }
 
 // multi_seq: the T tokens belong to T different sequences, token i with its own cache (sequence i) and position:

@@ -1,5 +1,5 @@
-"""Rows around the widest that the integer GEMM takes: models of one layer whose matrices have 23 to 32 blocks a row, tiles and
-batches against one token after the other. Everything is bit for bit."""
+"""Rows around the widest that the integer GEMM takes, and around the widest that keep folded copies: models of one layer, tiles
+and batches against one token after the other. Everything is bit for bit."""
 import numpy as np
 import pytest
 
@@ -46,17 +46,18 @@ def test_folded_rows(blocks, n_head):
         gm.free()
 
 
-@pytest.mark.parametrize("blocks", [24, 23])
-def test_prefolded_experts(blocks):
-    """prefill_prefold: 16 to 96 tokens per expert."""
+# gate and up, and down, of 1 to 5 blocks a row (images are taken from 24 or 48 tokens per expert on), and wider (they are not)
+@pytest.mark.parametrize("blocks,down_blocks", [(1, 2), (3, 4), (5, 5), (6, 3), (24, 1)])
+def test_prefolded_experts(blocks, down_blocks):
+    """prefill_prefold: 2 to 96 tokens per expert."""
     from llamd_rs_b200 import synth
 
-    gm, hp = _model(1, n_embd=256 * blocks, n_head=2)
+    gm, hp = _model(1, n_embd=256 * blocks, n_head=2, n_ff_expert=256 * down_blocks)
     try:
         gm.set_option("prefill_prefold", 1)
         toks = synth.token_ids(192, hp["n_vocab"], 11, "wide").tolist()
         want, logits = _one_by_one(gm, toks)
-        for n in (32, 64, 65, 130, 192):
+        for n in (4, 32, 48, 50, 64, 65, 98, 130, 192):
             assert gm.prefill(toks[:n], 0) == want[n - 1] and np.array_equal(gm.logits()[0].view(np.uint32), logits[n - 1]), f"prompt of {n}"
     finally:
         gm.free()
