@@ -811,6 +811,15 @@ bool ensure_folded(Model &m, int n, int prompt = 0) {
     return true;
 }
 
+// The folded copies of the expert matrices (option "prefill_prefold") are given back; the next prompt makes them again.
+void drop_prefold(Model &m) {
+    if (!m.prefold_ready) return;
+    cudaStreamSynchronize(stream());
+    for (auto &l : m.layers)
+        for (Buf *b : {&l.gate_fold, &l.up_fold, &l.down_fold}) b->release();
+    m.prefold_ready = false;
+}
+
 // The graph of a pass over nseq sequences is the current one afterwards: recorded now unless it is there already. Two are
 // kept, for near contexts and for the rest; a graph recorded for another model, or another nseq, points at the wrong buffers.
 bool ensure_graph(Model &m, int nseq, bool near) {
@@ -1063,6 +1072,7 @@ int llamd_model_set_tensor(llamd_model *h, int layer, int which, size_t first_bl
             const size_t own0 = (size_t)m->own_lo * per, own1 = (size_t)m->own_hi * per;
             if (lo < own0) lo = own0;
             if (hi > own1) hi = own1;
+            drop_prefold(*m);  // (the folded copies are of the old bytes)
             if (!dst.p && !dst.alloc(llamd_cuda_q6k_tiled_bytes(total))) break;
             if (lo >= hi) {
                 ok = true;  // nothing of this slice lives here
@@ -1255,12 +1265,7 @@ int llamd_model_set_option(llamd_model *h, const char *name, int value) {
         // order (2 bytes per weight: +19.5 GB for the down projections of the 48-layer model), so that a prefill tile's grouped GEMMs
         // copy operands instead of folding them, where that is the faster (gemm_launch).
         // Built at the next prefill; 0 releases the copies. Same bits either way.
-        if (!value && m->prefold_ready) {
-            cudaStreamSynchronize(stream());
-            for (auto &l : m->layers)
-                for (Buf *b : {&l.gate_fold, &l.up_fold, &l.down_fold}) b->release();
-            m->prefold_ready = false;
-        }
+        if (!value) drop_prefold(*m);
         m->prefold = value != 0;
         return 0;
     }

@@ -63,6 +63,24 @@ def test_prefolded_experts(blocks, down_blocks):
         gm.free()
 
 
+@pytest.mark.parametrize("which", ["T_FFN_GATE_EXPS", "T_FFN_UP_EXPS", "T_FFN_DOWN_EXPS"])
+def test_prefolded_experts_follow_their_tensor(which):
+    """An expert tensor set after a prompt with prefill_prefold: the next prompt multiplies with the new bytes."""
+    from llamd_rs_b200 import model, synth
+
+    gm, hp = _model(1, n_embd=512, n_head=4, n_ff_expert=512)
+    try:
+        gm.set_option("prefill_prefold", 1)
+        toks = synth.token_ids(130, hp["n_vocab"], 11, "wide").tolist()
+        before = gm.prefill(toks, 0), gm.logits()[0].view(np.uint32).copy()
+        gm.set_tensor(0, getattr(model, which), synth.q6k_blocks(hp["n_expert"] * 512 * 512 // 256, 12, "other"))
+        want, logits = _one_by_one(gm, toks)
+        assert not np.array_equal(before[1], logits[-1])
+        assert gm.prefill(toks, 0) == want[-1] and np.array_equal(gm.logits()[0].view(np.uint32), logits[-1])
+    finally:
+        gm.free()
+
+
 @pytest.mark.parametrize("n_head", [52, 64])
 def test_projections_wider_than_the_gemm_takes(n_head):
     """An output projection of 26 and 32 blocks a row: batches, drafts and short prompts run on the matvecs, from the first pass on."""
