@@ -23,7 +23,7 @@
 // (q6k_layout.cuh) -- and used for all the token tiles at hand. Three forms (gemm_launch):
 //   q6k_gemm_few_kernel     a warp folds all residues of its blocks: up to 16 tokens a group at up to three blocks a row, and up to 8
 //                           tokens of one group (a projection, the head) at any number;
-//   q6k_gemm_shared_kernel  groups of more than 40 tokens at up to four blocks a row: rows folded into shared memory once for four
+//   q6k_gemm_shared_kernel  groups of more than 40 tokens at up to four blocks a row (24 at two): rows folded into shared memory once for four
 //                           warps;
 //   q6k_gemm_kernel         everything else: four warps, a residue pair each, share 16 rows and up to 8 tiles.
 // us for 128 experts, gate and up (2 x 768 x 2048) / down (2048 x 768), 8 experts per token, before (every row tile folded into
@@ -615,12 +615,14 @@ __global__ void __launch_bounds__(THREADS, MINB) q6k_gemm_few_kernel(const GemmP
 
 // ---- short rows, many tokens per group ----
 // With four blocks a row and less, a token group's preparation in q6k_gemm_kernel is as long as its products (down of 2048 tokens
-// 519 us, here 465; 768: 236 / 226; 512: 164 / 180). Here a CTA folds its 16 rows
+// 519 us, here 471; 768: 236 / 226; 512: 164 / 180; of one and two blocks, 512 tokens: 104 / 99 and 148 / 131). Here a CTA folds its 16 rows
 // into shared memory once, in operand order, and each of its warps takes token tiles of its own, all residues of them. FOLDED: it
 // copies the rows' image.
 constexpr int kTokStride = 80;  // words per staged token: 16-byte aligned, fragment reads in 32 banks
-template <bool FOLDED>
-__global__ void __launch_bounds__(128, 5) q6k_gemm_shared_kernel(const GemmParams p) {
+// CTAs to an SM: five, or where folding takes three blocks and more a row four with the registers it wants: down of 1024 / 2048 tokens 284
+// 481 / 281 471, four blocks (1024 rows) 195 331 / 189 318; one block (2048 rows) 142 228 / 156 244.
+template <bool FOLDED, int MINB>
+__global__ void __launch_bounds__(128, MINB) q6k_gemm_shared_kernel(const GemmParams p) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int nb = p.nb, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g4 = lane >> 2, q4 = lane & 3;
     uint4 *s_frag = reinterpret_cast<uint4 *>(smem);  // [block][residue][hi, lo][lane], or the image (kImageBlockBytes)
@@ -826,10 +828,10 @@ static void gemm_launch_few(GemmParams &p, int n_groups) {
     gemm_launch_k<q6k_gemm_few_kernel<NT, BW, DIRECT, THREADS, MINB>>(p, n_groups, 32 * warps, (size_t)p.raw_bytes + (size_t)warps * NT * BW * 2048 + (DIRECT ? 0 : 4096));
 }
 
-template <bool FOLDED>
+template <bool FOLDED, int MINB>
 static void shared_launch(GemmParams &p, int n_groups) {
     p.row_tiles = 1;
-    gemm_launch_k<q6k_gemm_shared_kernel<FOLDED>>(p, n_groups, 128, (size_t)p.nb * 8 * 2 * 32 * 16 + (size_t)kGemmRows * p.nb * 4 + 4 * 8 * kTokStride * 4);
+    gemm_launch_k<q6k_gemm_shared_kernel<FOLDED, MINB>>(p, n_groups, 128, (size_t)p.nb * 8 * 2 * 32 * 16 + (size_t)kGemmRows * p.nb * 4 + 4 * 8 * kTokStride * 4);
 }
 
 // Shared memory for `units` consecutive blocks: whole tiles, one more where they need not start with one.
@@ -840,8 +842,8 @@ static int raw_tile_bytes(int units, bool aligned) {
 // n_groups > 0: that many token groups of about `tokens` each. 0: one group of p.n_tokens.
 static void gemm_launch(GemmParams &p, int n_groups, int tokens) {
     // Groups take the images of short rows, for as many tokens as a warp per token tile pays for: folding on the way is faster
-    // everywhere else. us, stored blocks / images, by blocks a row and tokens per group: 1 (2048 rows) 12 tokens 38 / 68, 32: 105 / 89,
-    // 128: 227 / 211; 3 (2048) 12: 95 / 130, 32: 169 / 162, 128: 482 / 433; 4 (1024) 12: 71 / 87, 32: 111 / 107, 128: 330 / 290; 5 (1024)
+    // everywhere else. us, stored blocks / images, by blocks a row and tokens per group: 1 (2048 rows) 12 tokens 38 / 68, 32: 99 / 89,
+    // 128: 227 / 211; 3 (2048) 12: 95 / 130, 32: 169 / 162, 128: 472 / 433; 4 (1024) 12: 71 / 87, 32: 114 / 107, 128: 318 / 290; 5 (1024)
     // 32: 131 / 136, 44: 161 / 173, 64: 222 / 213, 128: 397 / 366; 6 (1024) 64: 243 / 277, 128: 439 / 471; 8 (2 x 768) 32: 257 / 318, 128: 806 / 878.
     const bool images = p.gstart && p.folded[0] && p.nb <= kPrefoldBlocks && tokens > (p.nb < 5 ? 24 : 48);
     const bool folded = !p.gstart && p.folded[0];
@@ -875,7 +877,7 @@ static void gemm_launch(GemmParams &p, int n_groups, int tokens) {
         if (tiles <= 4 || team_smem<8, 16>(p) > kMaxSmem) gemm_launch_t<4, 8, 2, true>(p, n_groups);
         else gemm_launch_t<8, 16, 2, true>(p, n_groups);
     } else if (images) {
-        shared_launch<true>(p, n_groups);
+        shared_launch<true, 5>(p, n_groups);
     } else if (direct) {
         if (tiles <= 1) gemm_launch_few<1, 3, true, 128, 5>(p, n_groups);
         else gemm_launch_few<2, 3, true, 128, 3>(p, n_groups);
@@ -883,8 +885,10 @@ static void gemm_launch(GemmParams &p, int n_groups, int tokens) {
         if (p.nb <= 8) gemm_launch_few<1, 2, false, 128, 4>(p, n_groups);
         else if (p.nb <= 16) gemm_launch_few<1, 2, false, 256, 2>(p, n_groups);
         else gemm_launch_few<1, 2, false, 384, 1>(p, n_groups);
+    } else if (p.gstart && p.nb <= 2 && tokens > 24) {
+        shared_launch<false, 5>(p, n_groups);
     } else if (p.gstart && p.nb <= 4 && tokens > 40) {
-        shared_launch<false>(p, n_groups);
+        shared_launch<false, 4>(p, n_groups);
     } else if (tiles <= 1) {
         gemm_launch_t<2, 4, 6, false>(p, n_groups);
     } else if (tiles <= 3) {
